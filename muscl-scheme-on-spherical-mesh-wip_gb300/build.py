@@ -33,8 +33,8 @@ CXXFLAGS = ["-std=c++17", "-O3", "-fPIC", "-fopenmp", "-ffp-contract=off", "-Wal
 # per-.cu extra flags: the FP64 path must not fuse multiply-adds (reference
 # operand order); the mixed path may.
 CU_FLAGS = {
-    "step_fp64.cu": ["-fmad=false"],
-    "adjoint.cu": ["-fmad=false"],
+    "step_fp64.cu": ["-fmad=false", "-DSPLASH_SWITCH_TABLE"],
+    "adjoint.cu": ["-fmad=false", "-DSPLASH_SWITCH_TABLE"],
     "diagnostics.cu": ["-fmad=false"],
     "cfl_noalloc.cu": ["-fmad=false"],
     "step_mixed.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
@@ -71,7 +71,10 @@ def build_library(verbose: bool = False, force: bool = False) -> Path:
     LIBDIR.mkdir(exist_ok=True)
     nvcc = _nvcc()
     cuda_inc = _cuda_home() / "include"
-    headers = list(CSRC.glob("*.hpp")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    table = OBJDIR / "limiter_switch_table.inc"
+    if force or _newer(CSRC / "limiter_table.py", table, []):
+        _run([sys.executable, str(CSRC / "limiter_table.py"), str(table)])
+    headers = [table, *CSRC.glob("*.hpp")] + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
     jobs = []
     objs = []
     for src in sorted(CSRC.glob("*.cpp")):
@@ -86,7 +89,7 @@ def build_library(verbose: bool = False, force: bool = False) -> Path:
         if force or _newer(src, obj, headers):
             jobs.append([nvcc, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
                          "-Xcompiler", "-fvisibility=hidden",
-                         *CU_FLAGS.get(src.name, []), f"-I{INCLUDE}", f"-I{CSRC}",
+                         *CU_FLAGS.get(src.name, []), f"-I{INCLUDE}", f"-I{CSRC}", f"-I{OBJDIR}",
                          "-c", str(src), "-o", str(obj)])
     with cf.ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 4))) as ex:
         for cmd, fut in [(c, ex.submit(_run, c)) for c in jobs]:

@@ -241,13 +241,12 @@ __global__ void __launch_bounds__(kRevBlock) adj_flux_kernel(DevGeom G, PhysPara
   if (mask[f] & bit) la[0] = 0.0;  // density floor: the output's Sigma is a constant
 #pragma unroll
   for (int k = 0; k < kDim; ++k) la_out[(size_t)k * fp + f] = la[k];
-  const double rd_dt = P.round_diff * dt_here;
-  const double area = G.area[f];
+  const Gas gas = gas_of(P);
   const int n = G.nslots[f];
   for (int j = 0; j < n; ++j) {
     const int s = j * fp + f;
     const int rv = G.rev[s];
-    const double coef = rd_dt * G.chord[s] / area;
+    const double coef = dt_here * G.coef[s];
     double uL[kDim], uR[kDim], Fb[kDim], uLb[kDim], uRb[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
@@ -257,12 +256,8 @@ __global__ void __launch_bounds__(kRevBlock) adj_flux_kernel(DevGeom G, PhysPara
       uLb[k] = 0.0;
       uRb[k] = 0.0;
     }
-    SlotGeom g;
-    g.ec = plane3(G.ec, (int)PS, s);
-    g.ecn = G.ecn[s];
-    g.en = plane3(G.en, (int)PS, s);
-    g.nxr = plane3(G.nxr, (int)PS, s);
-    rev::flux_star_rev(uL, uR, g, P.gam, P.solver, Fb, uLb, uRb);
+    const EdgeGeom g{plane3(G.ec, (int)PS, s), plane3(G.en, (int)PS, s), plane3(G.nxr, (int)PS, s)};
+    rev::riemann_flux_rev(uL, uR, g, gas, P.solver, Fb, uLb, uRb);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
       A[(size_t)k * PS + s] = uLb[k];

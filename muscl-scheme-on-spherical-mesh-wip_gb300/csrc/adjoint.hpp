@@ -18,7 +18,7 @@
 
 namespace splash {
 
-constexpr int kTapeJ = 16;  // limiter-Jacobian tape planes per slot and stage
+constexpr int kTapeJ = 15;  // limiter-Jacobian tape planes per slot and stage
 
 // Tangents of the TLM beside a value DevState.
 struct TlmTangents {
@@ -32,7 +32,7 @@ struct TlmTangents {
 
 // Primal data of one step, stored by the recomputation: the step's input
 // state and its stage-1 state, their (Sigma, l, Pi), both stages' edge
-// states, both stages' limiter Jacobians (16 planes per slot, see
+// states, both stages' limiter Jacobians (15 planes per slot, see
 // adjoint_rev.cuh) and the density-floor bits (1: stage 1, 2: stage 2).
 struct StepTape {
   double* U;

@@ -8,12 +8,12 @@
 // their inputs.  At a kink the derivative of the branch taken is used,
 // matching the forward-mode duals of dual.cuh.
 //
-//   flux_star_rev     hand-written reverse of the three Riemann solvers
+//   riemann_flux_rev  hand-written reverse of the three Riemann solvers
 //                     (HLLE_p.hpp:19-58, HLLC.hpp:138-242,
 //                     HLLCplus.hpp:17-177, char_vel adiabatic.hpp:594-683)
-//   recon_face_tape   find_U_edges (MUSCL_base.hpp:361-434) with the local
-//                     limiter Jacobian (adiabatic.hpp:685-828) taped per slot
-//   recon_face_rev    reverse of the reconstruction from that tape
+//   recon_side_tape   find_U_edges (MUSCL_base.hpp:361-434) of one side with
+//                     the local limiter Jacobian (adiabatic.hpp:685-828) taped
+//   recon_side_rev    reverse of the reconstruction from that tape
 //   source_rev        reverse of the source term (adiabatic.hpp:396-541)
 //                     from a Dual<10> Jacobian of its 5 state and 5
 //                     parameter inputs
@@ -29,414 +29,378 @@ namespace f64 {
 namespace rev {
 
 // ---------------------------------------------------------------------
-// One side (left or right edge state) of a Riemann flux.
-struct Side {
-  double u[kDim];
-  D3 c;        // cross(ec, l)
-  double s;    // 1 / ((-u0) |ec|)
-  D3 vel;      // edge velocity c * s
-  double n;    // |vel|
-  double e;    // unfloored pressure (u4 - u0 n^2 / 2)(gam - 1)
-  double p;    // max(1e-16, e)
-  double vn;   // en . vel
-  double a;    // sqrt(gam p / u0)
-  double F[kDim];
-};
-
+// Adjoints of the quantities of one side of a Riemann problem (EdgeSide).
 struct SideBar {
-  double u[kDim];
-  D3 vel;
-  double n, p, vn, a;
-  double F[kDim];
+  double u0, u4, vn, v2, p, e, gi, a2, a, q;
+  D3 l, vel;
 };
-
 SPLASH_HD void zero(SideBar& b) {
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) b.u[k] = b.F[k] = 0.0;
-  b.vel = d3(0, 0, 0);
-  b.n = b.p = b.vn = b.a = 0.0;
+  b.u0 = b.u4 = b.vn = b.v2 = b.p = b.e = b.gi = b.a2 = b.a = b.q = 0.0;
+  b.l = b.vel = d3(0, 0, 0);
+}
+SPLASH_HD void add_scaled(D3& a, const D3& b, double s) {
+  a.x = fma(b.x, s, a.x);
+  a.y = fma(b.y, s, a.y);
+  a.z = fma(b.z, s, a.z);
 }
 
-// edge_vel, pressure, phys_flux and the sound speed of char_vel, with the
-// operation order of physics_fp64.cuh.
-SPLASH_HD void side_forward(const double* u, const SlotGeom& g, double gam, Side& S) {
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) S.u[k] = u[k];
-  S.c = cross3(g.ec, d3(u[1], u[2], u[3]));
-  S.s = 1.0 / ((-u[0]) * g.ecn);
-  S.vel = scal(S.c, S.s);
-  S.n = norm3(S.vel);
-  S.e = (u[4] - u[0] * (S.n * S.n) / 2) * (gam - 1);
-  S.p = smax(1e-16, S.e);
-  S.vn = dot3(g.en, S.vel);
-  S.a = sqrt(gam * S.p / u[0]);
-  S.F[0] = u[0] * S.vn;
-  S.F[1] = (u[1] * S.vn - g.nxr.x * S.p);
-  S.F[2] = (u[2] * S.vn - g.nxr.y * S.p);
-  S.F[3] = (u[3] * S.vn - g.nxr.z * S.p);
-  S.F[4] = (u[4] + S.p) * S.vn;
+// Reverse of phys_flux
+SPLASH_HD void phys_flux_rev(const double* u, const EdgeSide<double>& S, const EdgeGeom& g, const double* Fb,
+                             SideBar& B) {
+  const D3 lb = d3(Fb[1], Fb[2], Fb[3]);
+  B.u0 = fma(Fb[0], S.vn, B.u0);
+  B.vn += fma(Fb[4], S.e + S.p, fma(Fb[0], u[0], fdot(lb, d3(u[1], u[2], u[3]))));
+  add_scaled(B.l, lb, S.vn);
+  B.p += fma(Fb[4], S.vn, -fdot(g.nxr, lb));
+  B.e = fma(Fb[4], S.vn, B.e);
 }
 
-SPLASH_HD void side_reverse(const Side& S, const SlotGeom& g, double gam, SideBar& B, double* ub) {
-  double u0b = B.u[0] + B.F[0] * S.vn;
-  double vnb = B.vn + B.F[0] * S.u[0];
-  double l1b = B.u[1] + B.F[1] * S.vn, l2b = B.u[2] + B.F[2] * S.vn, l3b = B.u[3] + B.F[3] * S.vn;
-  vnb += B.F[1] * S.u[1] + B.F[2] * S.u[2] + B.F[3] * S.u[3] + B.F[4] * (S.u[4] + S.p);
-  double pb = B.p - (g.nxr.x * B.F[1] + g.nxr.y * B.F[2] + g.nxr.z * B.F[3]) + B.F[4] * S.vn;
-  double u4b = B.u[4] + B.F[4] * S.vn;
-  // a = sqrt(gam p / u0)
-  if (S.a > 0.0) {
-    const double xb = B.a * 0.5 / S.a;
-    const double iu0 = 1.0 / S.u[0];
-    pb += xb * gam * iu0;
-    u0b -= xb * (gam * S.p * iu0) * iu0;
-  }
-  // vn = en . vel
-  D3 vb = d3(B.vel.x + vnb * g.en.x, B.vel.y + vnb * g.en.y, B.vel.z + vnb * g.en.z);
-  // p = max(1e-16, e)
-  double nb = B.n;
-  if (1e-16 < S.e) {
-    const double eb = pb * (gam - 1);
-    u4b += eb;
-    u0b -= eb * (S.n * S.n) / 2;
-    nb -= eb * S.u[0] * S.n;
-  }
-  // n = |vel|
-  if (S.n > 0.0) {
-    const double t = nb / S.n;
-    vb = d3(vb.x + t * S.vel.x, vb.y + t * S.vel.y, vb.z + t * S.vel.z);
-  }
-  // vel = c * s ; s = 1 / ((-u0) ecn)
-  const D3 cb = scal(vb, S.s);
-  const double sb = dot3(vb, S.c);
-  u0b += sb * S.s * S.s * g.ecn;
-  // c = ec x l  ->  lb += cb x ec
-  const D3 lb = cross3(cb, g.ec);
-  ub[0] += u0b;
-  ub[1] += l1b + lb.x;
-  ub[2] += l2b + lb.y;
-  ub[3] += l3b + lb.z;
-  ub[4] += u4b;
+// Reverse of edge_side: the adjoint of (Sigma, l, Pi)
+SPLASH_HD void edge_side_rev(const double* u, const EdgeSide<double>& S, const EdgeGeom& g, const Gas& gas,
+                             SideBar& B, double* ub) {
+  // a = sqrt(a2), a2 = gi p
+  if (S.a > 0.0) B.a2 = fma(B.a * 0.5, recip(S.a), B.a2);
+  B.gi = fma(B.a2, S.p, B.gi);
+  B.p = fma(B.a2, S.gi, B.p);
+  // e = Sigma v2 / 2 + Pi / (gam - 1), p = max(1e-16, Pi)
+  B.u0 = fma(0.5 * S.v2, B.e, B.u0);
+  B.v2 = fma(0.5 * u[0], B.e, B.v2);
+  B.u4 = fma(gas.inv_gm1, B.e, B.u4);
+  if (less(1e-16, u[4])) B.u4 += B.p;
+  add_scaled(B.vel, S.vel, 2 * B.v2);
+  add_scaled(B.vel, g.en, B.vn);
+  // vel = -(ec x l) / Sigma, gi = gam / Sigma
+  const double ir = recip(u[0]);
+  const D3 cb = scal(B.vel, -ir);
+  B.u0 -= ir * fma(B.gi, S.gi, fdot(B.vel, S.vel));
+  const D3 lb = fcross(cb, g.ec);
+  ub[0] += B.u0;
+  ub[1] += B.l.x + lb.x;
+  ub[2] += B.l.y + lb.y;
+  ub[3] += B.l.z + lb.z;
+  ub[4] += B.u4;
 }
 
-// ---------------------------------------------------------------------
-// Adjoint of F = flux_star(uL, uR): uLb += (dF/duL)^T Fb, uRb += (dF/duR)^T Fb.
-SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom& g, double gam, int solver,
-                             const double* Fb, double* uLb, double* uRb) {
-  Side L, R;
-  side_forward(uL, g, gam, L);
-  side_forward(uR, g, gam, R);
+// Reverse of wave_speed; returns the adjoint of p_star
+SPLASH_HD double wave_speed_rev(const EdgeSide<double>& S, double p_star, const Gas& gas, SideBar& B) {
+  if (less(S.p, p_star)) {
+    const double z = fma(gas.shock_k, p_star - S.p, S.p);
+    const double q = root(S.gi * z);
+    if (!odd_bits(q)) {
+      const double qq = B.q * 0.5 * recip(q);
+      B.gi = fma(qq, z, B.gi);
+      const double zb = qq * S.gi;
+      B.p = fma(zb, 1 - gas.shock_k, B.p);
+      return zb * gas.shock_k;
+    }
+  }
+  B.a += B.q;
+  return 0.0;
+}
+
+// Adjoint of F = riemann_flux(uL, uR): uLb += (dF/duL)^T Fb, uRb += (dF/duR)^T Fb.
+SPLASH_HD void riemann_flux_rev(const double* uL, const double* uR, const EdgeGeom& g, const Gas& gas, int solver,
+                                const double* Fb, double* uLb, double* uRb) {
+  EdgeSide<double> L = edge_side(uL, g, gas), R = edge_side(uR, g, gas);
+  const double pvrs = fma(-0.125 * ((R.vn - L.vn) * (uL[0] + uR[0])), L.a + R.a, 0.5 * (L.p + R.p));
+  const double p_star = smax(0., pvrs);
+  L.q = wave_speed(L, p_star, gas);
+  R.q = wave_speed(R, p_star, gas);
+  const double S_L = L.vn - L.q, S_R = R.vn + R.q;
   SideBar BL, BR;
   zero(BL);
   zero(BR);
-  // char_vel (adiabatic.hpp:594-683)
-  const double p_pvrs = 1 / 2. * (L.p + R.p) - 1 / 8. * (R.vn - L.vn) * (uL[0] + uR[0]) * (L.a + R.a);
-  const double p_star = smax(0., p_pvrs);
-  const double kk = (gam + 1) / (2 * gam);
-  double q_R = 1., q_L = 1.;
-  bool qRd = false, qLd = false;
-  if (!(p_star <= R.p)) {
-    q_R = sqrt(1 + kk * (p_star / R.p - 1));
-    if (is_nan(q_R) || is_inf(q_R))
-      q_R = 1.;
-    else
-      qRd = true;
-  }
-  if (!(p_star <= L.p)) {
-    q_L = sqrt(1 + kk * (p_star / L.p - 1));
-    if (is_nan(q_L) || is_inf(q_L))
-      q_L = 1.;
-    else
-      qLd = true;
-  }
-  const double S_L = L.vn - L.a * q_L;
-  const double S_R = R.vn + R.a * q_R;
   double SLb = 0.0, SRb = 0.0;
 
   if (solver == 1) {
-    if (S_L >= 0) {
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) BL.F[i] += Fb[i];
-    } else if (S_L < 0 && S_R > 0) {
-      const double inv = 1.0 / (S_R - S_L);
-      double invb = 0.0;
+    if (not_below_zero(S_L)) {
+      phys_flux_rev(uL, L, g, Fb, BL);
+    } else if (below_zero(S_L) && below_zero(-S_R)) {
+      double FL[kDim], FR[kDim], FLb[kDim], FRb[kDim];
+      phys_flux(uL, L, g, FL);
+      phys_flux(uR, R, g, FR);
+      const double inv = recip(S_R - S_L);
+      const double wl = S_R * inv;
+      const double t = wl * S_L;
+      double wb = 0.0, tb = 0.0, dub[kDim];
 #pragma unroll
       for (int i = 0; i < kDim; ++i) {
-        const double du = uR[i] - uL[i];
-        const double N = S_R * L.F[i] - S_L * R.F[i] + S_R * S_L * du;
-        const double Nb = Fb[i] * inv;
-        invb += Fb[i] * N;
-        SRb += Nb * (L.F[i] + S_L * du);
-        SLb += Nb * (-R.F[i] + S_R * du);
-        BL.F[i] += Nb * S_R;
-        BR.F[i] -= Nb * S_L;
-        BR.u[i] += Nb * S_R * S_L;
-        BL.u[i] -= Nb * S_R * S_L;
+        const double du = (i < 4) ? uR[i] - uL[i] : R.e - L.e;
+        wb = fma(Fb[i], FL[i] - FR[i], wb);
+        tb = fma(Fb[i], du, tb);
+        FLb[i] = wl * Fb[i];
+        FRb[i] = Fb[i] - FLb[i];
+        dub[i] = t * Fb[i];
       }
-      const double db = -invb * inv * inv;
+      // wl = S_R inv, t = wl S_L, inv = 1 / (S_R - S_L)
+      wb = fma(tb, S_L, wb);
+      SLb = fma(tb, wl, SLb);
+      SRb = fma(wb, inv, SRb);
+      const double db = -(wb * S_R) * inv * inv;
       SRb += db;
       SLb -= db;
+      BR.u0 += dub[0];
+      BL.u0 -= dub[0];
+      add_scaled(BR.l, d3(dub[1], dub[2], dub[3]), 1.0);
+      add_scaled(BL.l, d3(dub[1], dub[2], dub[3]), -1.0);
+      BR.e += dub[4];
+      BL.e -= dub[4];
+      phys_flux_rev(uL, L, g, FLb, BL);
+      phys_flux_rev(uR, R, g, FRb, BR);
     } else {
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) BR.F[i] += Fb[i];
+      phys_flux_rev(uR, R, g, Fb, BR);
     }
   } else {
-    const double rho_L = uL[0], rho_R = uR[0];
-    const double V_L = L.vn, V_R = R.vn;
-    const double p_L = L.p, p_R = R.p;
-    const double num = p_R - p_L + rho_L * V_L * (S_L - V_L) - rho_R * V_R * (S_R - V_R);
-    const double den = rho_L * (S_L - V_L) - rho_R * (S_R - V_R);
-    double S_star = num / den;
-    const bool ss_fb = is_nan(S_star) || is_inf(S_star);
-    if (ss_fb) S_star = (V_L + V_R) / 2;
-    const double P_LR =
-        (p_L + p_R + uL[0] * (S_L - V_L) * (S_star - V_L) + uR[0] * (S_R - V_R) * (S_star - V_R)) / 2;
+    const double mL = -(uL[0] * L.q), mR = uR[0] * R.q;
+    const double iden = recip(mL - mR);
+    const double num = fma(L.vn, mL, fma(-R.vn, mR, R.p - L.p));
+    double S_star = num * iden;
+    const bool mean = odd_bits(S_star);
+    if (mean) S_star = 0.5 * (L.vn + R.vn);
     int side;
-    if (S_L >= 0)
+    if (not_below_zero(S_L))
       side = 0;
-    else if (S_L < 0 && S_star >= 0)
+    else if (below_zero(S_L) && not_below_zero(S_star))
       side = 1;
-    else if (S_star < 0 && S_R >= 0)
+    else if (below_zero(S_star) && not_below_zero(S_R))
       side = 2;
     else
       side = 3;
     if (side == 0) {
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) BL.F[i] += Fb[i];
+      phys_flux_rev(uL, L, g, Fb, BL);
     } else if (side == 3) {
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) BR.F[i] += Fb[i];
+      phys_flux_rev(uR, R, g, Fb, BR);
     } else {
       const bool left = (side == 1);
+      const double P_LR = 0.5 * fma(mR, S_star - R.vn, fma(mL, S_star - L.vn, L.p + R.p));
       const double Sk = left ? S_L : S_R;
+      const double inv = recip(Sk - S_star);
       const double* uk = left ? uL : uR;
-      const Side& K = left ? L : R;
-      const double inv_k = 1.0 / (Sk - S_star);
-      const double D[kDim] = {0., -g.nxr.x, -g.nxr.y, -g.nxr.z, S_star};
-      double Skb = 0.0, Ssb = 0.0, PLRb = 0.0, invkb = 0.0, VLb = 0.0, VRb = 0.0;
-      double ukb[kDim] = {0, 0, 0, 0, 0}, Fkb[kDim] = {0, 0, 0, 0, 0};
+      const EdgeSide<double>& K = left ? L : R;
+      SideBar& BK = left ? BL : BR;
+      const double si = S_star * inv;
+      const double qk = left ? -L.q : R.q;
+      const double al = si * qk;
+      double Skb = 0.0, Ssb = 0.0, invb = 0.0, mLb = 0.0, mRb = 0.0, idenb = 0.0;
+      const D3 lb = d3(Fb[1], Fb[2], Fb[3]);
       if (solver == 3) {
-        // HLLC+ correction (HLLCplus.hpp:17-177)
-        const double phi_L = uL[0] * (S_L - V_L);
-        const double phi_R = uR[0] * (S_R - V_R);
-        const double a_L = L.a, a_R = R.a;
-        const double mL = L.n / a_L, mR = R.n / a_R;
-        const double inner = smax(mL, mR);
-        const double M = smin(1., inner);
-        int lambd_L = 0, lambd_R = 0;
-        if ((V_L - a_L) > 0 && (V_R - a_R) < 0) lambd_L = 1;
-        if ((V_L + a_L) > 0 && (V_R + a_R) < 0) lambd_L = 1;
-        if ((V_R - a_R) > 0 && (V_L - a_L) < 0) lambd_R = 1;
-        if ((V_R + a_R) > 0 && (V_L + a_L) < 0) lambd_R = 1;
-        const bool fs_on = (lambd_L == 0 && lambd_R == 0);
-        double f_star = 1., dfdM = 0.0;
-        if (fs_on) {
-          const Dual<1> Md = Dual<1>::seed(M, 0);
-          const Dual<1> fd = Md * sqrt(4 + (1 - Md * Md) * (1 - Md * Md)) / ((1 + Md * Md));
-          f_star = fd.v;
-          dfdM = fd.d[0];
+        const bool rfast = less(L.v2 * R.a2, R.v2 * L.a2);
+        double mm = divide(rfast ? R.v2 : L.v2, rfast ? R.a2 : L.a2);
+        const bool capped = !less(mm, 1.);
+        if (capped) mm = 1.;
+        Dual<1> Md;
+        const Dual<1> fd = hllcp_fstar(Dual<1>::seed(mm, 0), Md);
+        double f1 = fd.v - 1.0, df1 = fd.d[0];
+        if (!less_pos(mm, 0.999)) {
+          const double lm = L.vn - L.a, lp = L.vn + L.a, rm = R.vn - R.a, rp = R.vn + R.a;
+          if ((lm > 0 && rm < 0) || (lp > 0 && rp < 0) || (rm > 0 && lm < 0) || (rp > 0 && lp < 0)) f1 = df1 = 0.;
         }
-        const double hA = p_L / p_R, hB = p_R / p_L;
-        const double h = smin(hA, hB);
-        const double lg = log(h);
-        const double E = exp(M * lg);
-        const double gsw = 1 - E;
-        const double dV = V_R - V_L;
-        const D3 dv = sub(R.vel, L.vel);
-        const double cs = Sk * inv_k * gsw;
-        const double fm = f_star - 1;
-        const D3 vff = d3(fm * dV * g.en.x + cs * (dv.x - dV * g.en.x), fm * dV * g.en.y + cs * (dv.y - dV * g.en.y),
-                          fm * dV * g.en.z + cs * (dv.z - dV * g.en.z));
-        const D3 am = cross3(g.ec, vff);
-        const double w = phi_L * phi_R / (phi_R - phi_L);
-        const double X4 = fm * (V_R - V_L) * S_star;
-        // reverse
-        const double wb = Fb[1] * am.x + Fb[2] * am.y + Fb[3] * am.z + Fb[4] * X4;
-        const D3 amb = d3(Fb[1] * w, Fb[2] * w, Fb[3] * w);
-        const double X4b = Fb[4] * w;
-        double fmb = X4b * (V_R - V_L) * S_star;
-        const double dV2b = X4b * fm * S_star;
-        VRb += dV2b;
-        VLb -= dV2b;
-        Ssb += X4b * fm * (V_R - V_L);
-        const D3 vffb = cross3(amb, g.ec);
-        double dVb = 0.0, csb = 0.0;
-        fmb += vffb.x * dV * g.en.x + vffb.y * dV * g.en.y + vffb.z * dV * g.en.z;
-        dVb += vffb.x * (fm * g.en.x - cs * g.en.x) + vffb.y * (fm * g.en.y - cs * g.en.y) +
-               vffb.z * (fm * g.en.z - cs * g.en.z);
-        csb += vffb.x * (dv.x - dV * g.en.x) + vffb.y * (dv.y - dV * g.en.y) + vffb.z * (dv.z - dV * g.en.z);
-        const D3 dvb = scal(vffb, cs);
-        BR.vel = d3(BR.vel.x + dvb.x, BR.vel.y + dvb.y, BR.vel.z + dvb.z);
-        BL.vel = d3(BL.vel.x - dvb.x, BL.vel.y - dvb.y, BL.vel.z - dvb.z);
-        VRb += dVb;
-        VLb -= dVb;
-        Skb += csb * inv_k * gsw;
-        invkb += csb * Sk * gsw;
-        const double gswb = csb * Sk * inv_k;
-        const double yb = -gswb * E;
-        double Mb = yb * lg;
-        const double hb = yb * M / h;
-        if (hB < hA) {  // h = p_R / p_L
-          BR.p += hb / p_L;
-          BL.p -= hb * hB / p_L;
-        } else {  // h = p_L / p_R
-          BL.p += hb / p_R;
-          BR.p -= hb * hA / p_R;
+        const Dual<3> gd = pressure_switch(Dual<3>::seed(Md.v, 0), Dual<3>::seed(L.p, 1), Dual<3>::seed(R.p, 2));
+        const double dV = R.vn - L.vn;
+        const double cs = Sk * inv * gd.v;
+        const double k1 = (cs - f1) * dV;
+        const D3 ed = fcross(g.ec, sub(R.vel, L.vel));
+        const double w = -(mL * mR) * iden;
+        // F_l += w (k1 nxr + cs ed), F_E += w f1 dV S*
+        const double lbn = fdot(lb, g.nxr), lbe = fdot(lb, ed);
+        const double X = f1 * dV * S_star;
+        const double wb = fma(Fb[4], X, fma(k1, lbn, cs * lbe));
+        const double Xb = w * Fb[4];
+        const double k1b = w * lbn;
+        const double csb = fma(k1b, dV, w * lbe);
+        const D3 dvb = fcross(scal(lb, w * cs), g.ec);
+        add_scaled(BR.vel, dvb, 1.0);
+        add_scaled(BL.vel, dvb, -1.0);
+        const double f1b = fma(Xb * dV, S_star, -(k1b * dV));
+        const double dVb = fma(Xb * f1, S_star, k1b * (cs - f1));
+        Ssb = fma(Xb * f1, dV, Ssb);
+        BR.vn += dVb;
+        BL.vn -= dVb;
+        Skb = fma(csb * inv, gd.v, Skb);
+        invb = fma(csb * Sk, gd.v, invb);
+        const double gb = csb * Sk * inv;
+        BL.p = fma(gb, gd.d[1], BL.p);
+        BR.p = fma(gb, gd.d[2], BR.p);
+        if (!capped) {
+          const double mmb = fma(f1b, df1, gb * gd.d[0] * Md.d[0]);
+          const double ia = recip(rfast ? R.a2 : L.a2);
+          SideBar& BF = rfast ? BR : BL;
+          BF.v2 = fma(mmb, ia, BF.v2);
+          BF.a2 = fma(-mmb * mm, ia, BF.a2);
         }
-        if (fs_on) Mb += fmb * dfdM;
-        if (inner < 1.) {
-          if (mL < mR) {
-            BR.n += Mb / a_R;
-            BR.a -= Mb * mR / a_R;
-          } else {
-            BL.n += Mb / a_L;
-            BL.a -= Mb * mL / a_L;
-          }
-        }
-        // w = phi_L phi_R / (phi_R - phi_L)
-        const double Q = phi_R - phi_L;
-        const double Pb = wb / Q;
-        const double Qb = -wb * w / Q;
-        const double phiLb = Pb * phi_R - Qb;
-        const double phiRb = Pb * phi_L + Qb;
-        BL.u[0] += phiLb * (S_L - V_L);
-        SLb += phiLb * uL[0];
-        VLb -= phiLb * uL[0];
-        BR.u[0] += phiRb * (S_R - V_R);
-        SRb += phiRb * uR[0];
-        VRb -= phiRb * uR[0];
+        mLb = fma(-wb * mR, iden, mLb);
+        mRb = fma(-wb * mL, iden, mRb);
+        idenb = fma(-wb * mL, mR, idenb);
       }
-      // F_k* (HLLC.hpp:218-239)
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) {
-        const double Gi = S_star * (Sk * uk[i] - K.F[i]) + Sk * P_LR * D[i];
-        const double Gb = Fb[i] * inv_k;
-        invkb += Fb[i] * Gi;
-        Ssb += Gb * (Sk * uk[i] - K.F[i]);
-        const double t = Gb * S_star;
-        Skb += t * uk[i];
-        ukb[i] += t * Sk;
-        Fkb[i] -= t;
-        Skb += Gb * P_LR * D[i];
-        PLRb += Gb * Sk * D[i];
-      }
-      Ssb += (Fb[4] * inv_k) * Sk * P_LR;  // D[4] = S_star
-      // inv_k = 1 / (Sk - S_star)
-      const double db = -invkb * inv_k * inv_k;
+      // F_K* = (alpha Sigma, alpha l + beta nxr, alpha E + si (Sk P - p V))
+      const double alb = fma(Fb[4], K.e, fma(Fb[0], uk[0], fdot(lb, d3(uk[1], uk[2], uk[3]))));
+      BK.u0 = fma(Fb[0], al, BK.u0);
+      add_scaled(BK.l, lb, al);
+      BK.e = fma(Fb[4], al, BK.e);
+      const double t = fma(Sk, P_LR, -(K.p * K.vn));
+      const double beb = fdot(lb, g.nxr);
+      const double sib = fma(beb, K.p - P_LR, fma(alb, qk, Fb[4] * t));
+      const double tb = Fb[4] * si;
+      const double qkb = alb * si;
+      BK.p += fma(beb, si, -(tb * K.vn));
+      BK.vn = fma(-tb, K.p, BK.vn);
+      Skb = fma(tb, P_LR, Skb);
+      const double Pb = 0.5 * (fma(tb, Sk, -beb) - beb * si);
+      Ssb = fma(sib, inv, Ssb);
+      invb = fma(sib, S_star, invb);
+      // inv = 1 / (Sk - S*)
+      const double db = -invb * inv * inv;
       Skb += db;
       Ssb -= db;
-      SideBar& BK = left ? BL : BR;
-#pragma unroll
-      for (int i = 0; i < kDim; ++i) {
-        BK.u[i] += ukb[i];
-        BK.F[i] += Fkb[i];
-      }
-      if (left)
+      if (left) {
+        BL.q -= qkb;
         SLb += Skb;
-      else
-        SRb += Skb;
-      // P_LR
-      const double q = PLRb / 2;
-      BL.p += q;
-      BR.p += q;
-      {
-        const double X = uL[0] * (S_L - V_L), Y = S_star - V_L;
-        const double Xb = q * Y, Yb = q * X;
-        BL.u[0] += Xb * (S_L - V_L);
-        SLb += Xb * uL[0];
-        VLb -= Xb * uL[0];
-        Ssb += Yb;
-        VLb -= Yb;
-      }
-      {
-        const double X = uR[0] * (S_R - V_R), Y = S_star - V_R;
-        const double Xb = q * Y, Yb = q * X;
-        BR.u[0] += Xb * (S_R - V_R);
-        SRb += Xb * uR[0];
-        VRb -= Xb * uR[0];
-        Ssb += Yb;
-        VRb -= Yb;
-      }
-      // S_star
-      if (ss_fb) {
-        VLb += Ssb / 2;
-        VRb += Ssb / 2;
       } else {
-        const double numb = Ssb / den;
-        const double denb = -Ssb * S_star / den;
+        BR.q += qkb;
+        SRb += Skb;
+      }
+      // P_LR
+      BL.p += Pb;
+      BR.p += Pb;
+      mLb = fma(Pb, S_star - L.vn, mLb);
+      mRb = fma(Pb, S_star - R.vn, mRb);
+      Ssb = fma(Pb, mL + mR, Ssb);
+      BL.vn = fma(-Pb, mL, BL.vn);
+      BR.vn = fma(-Pb, mR, BR.vn);
+      // S* = num iden
+      if (mean) {
+        BL.vn = fma(0.5, Ssb, BL.vn);
+        BR.vn = fma(0.5, Ssb, BR.vn);
+      } else {
+        const double numb = Ssb * iden;
+        idenb = fma(Ssb, num, idenb);
         BR.p += numb;
         BL.p -= numb;
-        const double A = rho_L * V_L, Bq = S_L - V_L;
-        BL.u[0] += numb * Bq * V_L;
-        VLb += numb * Bq * rho_L;
-        SLb += numb * A;
-        VLb -= numb * A;
-        const double C = rho_R * V_R, Dd = S_R - V_R;
-        BR.u[0] -= numb * Dd * V_R;
-        VRb -= numb * Dd * rho_R;
-        SRb -= numb * C;
-        VRb += numb * C;
-        BL.u[0] += denb * (S_L - V_L);
-        SLb += denb * rho_L;
-        VLb -= denb * rho_L;
-        BR.u[0] -= denb * (S_R - V_R);
-        SRb -= denb * rho_R;
-        VRb += denb * rho_R;
+        BL.vn = fma(numb, mL, BL.vn);
+        mLb = fma(numb, L.vn, mLb);
+        BR.vn = fma(-numb, mR, BR.vn);
+        mRb = fma(-numb, R.vn, mRb);
       }
-      BL.vn += VLb;
-      BR.vn += VRb;
+      const double denb = -idenb * iden * iden;
+      mLb += denb;
+      mRb -= denb;
+      BL.u0 = fma(-mLb, L.q, BL.u0);
+      BL.q = fma(-mLb, uL[0], BL.q);
+      BR.u0 = fma(mRb, R.q, BR.u0);
+      BR.q = fma(mRb, uR[0], BR.q);
     }
   }
-  // char_vel reverse: S_L = vn_L - a_L q_L ; S_R = vn_R + a_R q_R
+  // S_L = vn_L - q_L ; S_R = vn_R + q_R
   BL.vn += SLb;
-  BL.a -= SLb * q_L;
-  const double qLb = -SLb * L.a;
+  BL.q -= SLb;
   BR.vn += SRb;
-  BR.a += SRb * q_R;
-  const double qRb = SRb * R.a;
-  double psb = 0.0;
-  if (qRd) {
-    const double zb = qRb * 0.5 / q_R;
-    psb += zb * kk / R.p;
-    BR.p -= zb * kk * p_star / (R.p * R.p);
-  }
-  if (qLd) {
-    const double zb = qLb * 0.5 / q_L;
-    psb += zb * kk / L.p;
-    BL.p -= zb * kk * p_star / (L.p * L.p);
-  }
-  const double ppb = (0. < p_pvrs) ? psb : 0.0;
-  BL.p += 0.5 * ppb;
-  BR.p += 0.5 * ppb;
+  BR.q += SRb;
+  const double psb = wave_speed_rev(L, p_star, gas, BL) + wave_speed_rev(R, p_star, gas, BR);
+  const double ppb = less(0., pvrs) ? psb : 0.0;
+  BL.p = fma(0.5, ppb, BL.p);
+  BR.p = fma(0.5, ppb, BR.p);
   {
     const double t = -ppb * 0.125;
     const double dvn = R.vn - L.vn, rs = uL[0] + uR[0], as = L.a + R.a;
     const double dvnb = t * rs * as, rsb = t * dvn * as, asb = t * dvn * rs;
     BR.vn += dvnb;
     BL.vn -= dvnb;
-    BL.u[0] += rsb;
-    BR.u[0] += rsb;
+    BL.u0 += rsb;
+    BR.u0 += rsb;
     BL.a += asb;
     BR.a += asb;
   }
-  side_reverse(L, g, gam, BL, uLb);
-  side_reverse(R, g, gam, BR, uRb);
+  edge_side_rev(uL, L, g, gas, BL, uLb);
+  edge_side_rev(uR, R, g, gas, BR, uRb);
+}
+
+// Adjoint of flux_star (states with the energy in field 4)
+SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom& sg, double gam, int solver,
+                             const double* Fb, double* uLb, double* uRb) {
+  const EdgeGeom g = edge_geom(sg);
+  Dual<5> pL, pR;
+  const double* us[2] = {uL, uR};
+  double st[2][kDim], bar[2][kDim] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};
+  Dual<5>* ps[2] = {&pL, &pR};
+  for (int i = 0; i < 2; ++i) {
+    Dual<5> ud[kDim];
+    for (int k = 0; k < kDim; ++k) ud[k] = Dual<5>::seed(us[i][k], k);
+    *ps[i] = edge_pressure(ud, g, gam);
+    for (int k = 0; k < 4; ++k) st[i][k] = us[i][k];
+    st[i][4] = ps[i]->v;
+  }
+  riemann_flux_rev(st[0], st[1], g, gas_of(gam), solver, Fb, bar[0], bar[1]);
+  double* out[2] = {uLb, uRb};
+  for (int i = 0; i < 2; ++i)
+    for (int k = 0; k < kDim; ++k) out[i][k] += (k < 4 ? bar[i][k] : 0.0) + bar[i][4] * ps[i]->d[k];
 }
 
 // ---------------------------------------------------------------------
 // Reconstruction with its reverse-sweep tape, and the reverse from the tape.
 //
-// Per slot and field the limited edge state is up = w + pp phi(r, nu) bmd
-// with pp = (Up - w)/H+, pm = (w - Um)/H-, r = pm/pp and nu the slot's
-// Courant factor (MUSCL_base.hpp:361-434, adiabatic.hpp:685-828).  The
-// recomputation evaluates phi once on Dual<2> over (r, nu) -- its value is
-// the primal's, bit for bit -- and stores the three partials
-//   d up / d pp = bmd (phi - r phi_r),  d up / d pm = bmd phi_r,
-//   d up / d nu = pp bmd phi_nu
+// Per side and field the limited edge state is up = w + hg dp phi(r, nu)
+// with dp = U+ - w, dm = w - U-, r = hr dm / dp (hr = H+/H-, hg = BM/H+)
+// and nu the side's Courant factor (MUSCL_base.hpp:361-434,
+// adiabatic.hpp:685-828).  The recomputation evaluates phi once on Dual<2>
+// over (r, nu) -- its value is the primal's, bit for bit -- and stores the
+// three partials
+//   d up / d dp = hg (phi - r phi_r),  d up / d dm = hg hr phi_r,
+//   d up / d nu = hg dp phi_nu
 // so that the reverse sweep needs no transcendental.  Where phi is flat in r
-// (r = +-inf or NaN) d up / d pp = bmd phi.
-constexpr int kTapePlanes = 16;  // 3 per field + the edge pressure before Pi -> E
+// (r = +-inf or NaN) d up / d dp = hg phi.
+constexpr int kTapePlanes = 15;  // 3 per field
 
+// nb as in recon_side; lj(3 k + i) receives the partials of field k
+template <class NbFn, class LjFn>
+SPLASH_HD void recon_side_tape(const SideGeom& g, double gam, double dt, const double* w, NbFn nb, double* up,
+                               LjFn lj) {
+  const Dual<2> nu = Dual<2>::seed(side_courant(g, gam, dt, w), 1);
+  const LimiterLine<Dual<2>> line = limiter_line(g, nu);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    double dp, dm;
+    side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
+    const double r = slope_ratio(g, dp, dm);
+    const Dual<2> lim = limiter_field(Dual<2>::seed(r, 0), line);
+    const double dg = dp * g.hg;
+    up[k] = fm(dg, lim.v, w[k]);
+    lj(3 * k, g.hg * ((lim.d[0] != 0.0) ? fma(-lim.d[0], r, lim.v) : lim.v));
+    lj(3 * k + 1, g.hg * g.hr * lim.d[0]);
+    lj(3 * k + 2, dg * lim.d[1]);
+  }
+}
+
+// upb: the adjoint of the edge state; LJ(i): the taped partials.  Gives the
+// adjoints of the interpolants U+ and U- (pu, mu) and adds the face's own
+// part to wb.
+template <class LjFn>
+SPLASH_HD void recon_side_rev(const SideGeom& g, double gam, double dt, const double* w, const double* upb, LjFn LJ,
+                              double* pu, double* mu, double* wb) {
+  double nub = 0.0;
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    const double dpb = upb[k] * LJ(3 * k), dmb = upb[k] * LJ(3 * k + 1);
+    nub = fma(upb[k], LJ(3 * k + 2), nub);
+    pu[k] = dpb;
+    mu[k] = -dmb;
+    wb[k] += upb[k] - dpb + dmb;
+  }
+  // nu = (c + vn) dt arc / area with c = sqrt(gam Pi / Sigma), vn = -(l . nxr) / Sigma
+  const double b = nub * (dt * g.arc_a);
+  const double ir = recip(w[0]);
+  double ic;
+  const double c = root_pair(gam * (w[4] * ir), ic);
+  const double vn = -(fdot(g.nxr, d3(w[1], w[2], w[3])) * ir);
+  const double cb = (c > 0.0) ? b * 0.5 * ic * gam * ir : 0.0;  // adjoint of Pi, and of Sigma times -Pi / Sigma
+  wb[0] -= ir * fma(cb, w[4], b * vn);
+  const double s = -b * ir;
+  wb[1] = fma(s, g.nxr.x, wb[1]);
+  wb[2] = fma(s, g.nxr.y, wb[2]);
+  wb[3] = fma(s, g.nxr.z, wb[3]);
+  wb[4] += cb;
+}
+
+// recon_side_tape for every slot of face f (planes: uplus 5, LJ kTapePlanes)
 SPLASH_HD void recon_face_tape(const DevGeom& G, const PhysParams& P, double dt, const double* W, double* uplus,
                                double* LJ, int f) {
   const int fp = G.fpad;
@@ -445,113 +409,45 @@ SPLASH_HD void recon_face_tape(const DevGeom& G, const PhysParams& P, double dt,
 #pragma unroll
   for (int k = 0; k < kDim; ++k) w[k] = W[(size_t)k * fp + f];
   const int n = G.nslots[f];
-  const double twoN = (double)(2 * n);
-  const double gam = P.gam;
-  const double c = sqrt(gam * (w[4] + 0.0) / (w[0] + 0.0));
   for (int j = 0; j < n; ++j) {
     const int s = j * fp + f;
-    const int ia = G.sten[s], ib = G.sten[PS + s], ic = G.sten[2 * PS + s], id = G.sten[3 * PS + s];
-    const double bp0 = G.beta[s], bp1 = G.beta[PS + s], bm0 = G.beta[2 * PS + s], bm1 = G.beta[3 * PS + s];
-    const double hp = G.hpm[s], hm = G.hpm[PS + s], bmd = G.bm[s];
-    const double ihp = 1.0 / hp, ihm = 1.0 / hm;
-    double pp[kDim], r[kDim];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      const double* Wk = W + (size_t)k * fp;
-      const double Up = bp0 * Wk[ia] + bp1 * Wk[ib];
-      pp[k] = (Up - w[k]) * ihp;
-      const double Um = bm0 * Wk[ic] + bm1 * Wk[id];
-      const double pm = (-Um + w[k]) * ihm;
-      r[k] = pm / pp[k];
-    }
-    const D3 ec = plane3(G.ec, PS, s);
-    const double ecn = G.ecn[s];
-    const D3 en = plane3(G.en, PS, s);
-    D3 vel = cross3(ec, d3(w[1], w[2], w[3]));
-    vel = scal(vel, 1.0 / ((-w[0] - 0.0) * ecn));
-    const double nu_plus = (c + dot3(vel, en)) * dt * G.arc_a[s];
-    const double eta_p = G.eta[s];
-    const Dual<2> nud = Dual<2>::seed(nu_plus, 1);
-    const Dual<2> sb_scale = G.eta[PS + s] / (twoN * nud);
-    const Dual<2> to_scale = (1 + nud) / 3;
+    const int st[4] = {G.sten[s], G.sten[PS + s], G.sten[2 * PS + s], G.sten[3 * PS + s]};
     double up[kDim];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      const Dual<2> lim = limiter_field(Dual<2>::seed(r[k], 0), eta_p, sb_scale, to_scale);
-      if (k == 0 || k == 4)
-        up[k] = w[k] + 0.0 + pp[k] * lim.v * bmd;
-      else
-        up[k] = w[k] + pp[k] * lim.v * bmd;
-      const double dpp = bmd * ((lim.d[0] != 0.0) ? lim.v - lim.d[0] * r[k] : lim.v);
-      LJ[(size_t)(3 * k) * PS + s] = dpp;
-      LJ[(size_t)(3 * k + 1) * PS + s] = bmd * lim.d[0];
-      LJ[(size_t)(3 * k + 2) * PS + s] = pp[k] * bmd * lim.d[1];
-    }
-    LJ[(size_t)15 * PS + s] = up[4];
-    up[4] = energy_at_edge(up, ec, gam);
+    recon_side_tape(
+        side_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W[(size_t)k * fp + st[q]]; }, up,
+        [&](int i, double x) { LJ[(size_t)i * PS + s] = x; });
 #pragma unroll
     for (int k = 0; k < kDim; ++k) uplus[(size_t)k * PS + s] = up[k];
   }
 }
 
-// Sound speed of a face as a Dual<5> over its (Sigma, l, Pi).
-SPLASH_HD Dual<5> face_sound_speed(const double* w, double gam) {
-  const Dual<5> w0 = Dual<5>::seed(w[0], 0), w4 = Dual<5>::seed(w[4], 4);
-  return sqrt(gam * (w4 + 0.0) / (w0 + 0.0));
-}
-
 // Reverse of recon_face_tape for face f.  W holds the primal (Sigma, l, Pi)
-// planes, uplus and LJ the slot's tape; upb_at(k, s) returns the adjoint of
+// planes and LJ the slots' tape; upb_at(k, s) returns the adjoint of
 // uplus[k * PS + s].  Writes the adjoints of the slot's stencil
-// interpolants to PU (planes 0..4: Up, 5..9: Um, each PS long) and adds the
+// interpolants to PU (planes 0..4: U+, 5..9: U-, each PS long) and adds the
 // face's own contribution to wb.  The interpolants' adjoints reach the
 // stencil faces through PU times the betas (scattered by the caller).
 template <class UpbFn>
 SPLASH_HD void recon_face_rev(const DevGeom& G, const PhysParams& P, double dt, const double* W,
-                              const double* uplus, const double* LJ, UpbFn upb_at, double* PU, double* wb, int f) {
+                              const double* /*uplus*/, const double* LJ, UpbFn upb_at, double* PU, double* wb, int f) {
   const int fp = G.fpad;
   const int PS = G.max_slots * fp;
   double w[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) w[k] = W[(size_t)k * fp + f];
   const int n = G.nslots[f];
-  const Dual<5> c = face_sound_speed(w, P.gam);
-  Dual<5> wd[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) wd[k] = Dual<5>::seed(w[k], k);
   for (int j = 0; j < n; ++j) {
     const int s = j * fp + f;
-    const D3 ec = plane3(G.ec, PS, s);
-    const D3 en = plane3(G.en, PS, s);
-    // energy at the edge centre from the limited (Sigma, l, Pi)
-    Dual<5> ud[kDim];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) ud[k] = Dual<5>::seed(uplus[(size_t)k * PS + s], k);
-    ud[4] = Dual<5>::seed(LJ[(size_t)15 * PS + s], 4);
-    const Dual<5> E = energy_at_edge(ud, ec, P.gam);
-    double upb[kDim], preb[kDim];
+    double upb[kDim], pu[kDim], mu[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) upb[k] = upb_at(k, s);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) preb[k] = upb[k] + upb[4] * E.d[k];
-    preb[4] = upb[4] * E.d[4];
-    // Courant factor as a function of w
-    V3<Dual<5>> vel = cross3(ec, v3(wd[1], wd[2], wd[3]));
-    vel = scal(vel, 1.0 / ((-wd[0] - 0.0) * G.ecn[s]));
-    const Dual<5> nu5 = (c + dot3(vel, en)) * dt * G.arc_a[s];
-    const double ihp = 1.0 / G.hpm[s], ihm = 1.0 / G.hpm[PS + s];
-    double nub = 0.0;
+    recon_side_rev(
+        side_geom(G, PS, s, n), P.gam, dt, w, upb, [&](int i) { return LJ[(size_t)i * PS + s]; }, pu, mu, wb);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
-      const double ppb = preb[k] * LJ[(size_t)(3 * k) * PS + s];
-      const double pmb = preb[k] * LJ[(size_t)(3 * k + 1) * PS + s];
-      nub += preb[k] * LJ[(size_t)(3 * k + 2) * PS + s];
-      PU[(size_t)k * PS + s] = ppb * ihp;
-      PU[(size_t)(kDim + k) * PS + s] = -pmb * ihm;
-      wb[k] += preb[k] - ppb * ihp + pmb * ihm;
+      PU[(size_t)k * PS + s] = pu[k];
+      PU[(size_t)(kDim + k) * PS + s] = mu[k];
     }
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) wb[k] += nub * nu5.d[k];
   }
 }
 

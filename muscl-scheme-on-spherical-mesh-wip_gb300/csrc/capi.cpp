@@ -202,6 +202,10 @@ void Solver::build_device_geometry(const RefGeometry& g) {
     G.hpm = upload(sp.hpm);
     G.bm = upload(sp.bm);
     G.eta = upload(sp.eta);
+    G.hr = upload(sp.hr);
+    G.hg = upload(sp.hg);
+    G.sbs = upload(sp.sbs);
+    G.coef = upload(sp.coef);
     G.arc_a = upload(sp.arc);
     G.ec = upload(sp.ec);
     G.ecn = upload(sp.ecn);

@@ -25,6 +25,7 @@ namespace splash {
 
 template <int N>
 struct Dual {
+  static constexpr int kN = N;
   double v;
   double d[N];
 

@@ -42,6 +42,8 @@ struct PhysParams {
   // (physics/adiabatic.hpp:563-566), and FP32 copies for the mixed path
   double fric_k;
   double gam_m1, fric_ak;  // gam - 1 and alpha * fric_k (mixed-path update)
+  double inv_gm1, gam_gm1; // 1 / (gam - 1), gam / (gam - 1)
+  double shock_k;          // (gam + 1) / (2 gam): the wave-speed factor of char_vel (physics/adiabatic.hpp:655-668)
   float gam_f, e_acc_f, alpha_f, omega_ns_f, fric_ak_f;
   float gam_m1_h, gam_m1_l;  // gam - 1 as a double-word (nearest float + residual)
   float cfl_num_f;           // h0 * 0.1 rounded to a float (numerator of the CFL bound)
@@ -54,6 +56,9 @@ inline void derive_params(PhysParams& P) {
   const double gam3d = 1 / (2 - P.gam);
   P.fric_k = gam3d / (2 * gam3d - 1);
   P.gam_m1 = P.gam - 1.0;
+  P.inv_gm1 = 1 / P.gam_m1;
+  P.gam_gm1 = P.gam / P.gam_m1;
+  P.shock_k = (P.gam + 1) / (2 * P.gam);
   P.fric_ak = P.alpha * P.fric_k;
   P.fric_ak_f = (float)P.fric_ak;
   P.gam_m1_h = (float)P.gam_m1;
@@ -87,12 +92,16 @@ struct DevGeom {
   const double* hpm;      // 2 planes: H_plus, H_minus
   const double* bm;       // BM_dist
   const double* eta;      // 2 planes: H_plus/BM, H_minus/BM
+  const double* hr;       // H_plus / H_minus
+  const double* hg;       // BM / H_plus
+  const double* sbs;      // (H_minus/BM) / (2 N): the superbee scale before the Courant factor
   const double* arc_a;    // great-circle edge length / face area (limiter Courant factor)
   const double* ec;       // 3 planes: unit edge centre
   const double* ecn;      // |ec| as evaluated in double
   const double* en;       // 3 planes: outward edge normal
   const double* nxr;      // 3 planes: cross(en, ec/|ec|)
   const double* chord;    // straight edge length
+  const double* coef;     // round_diff * chord / area
   const int* rev;         // slot-plane index of the same edge seen from the neighbour
 };
 

@@ -80,6 +80,10 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
   sp.en.assign(3 * PS, 0.0);
   sp.nxr.assign(3 * PS, 0.0);
   sp.chord.assign(PS, 0.0);
+  sp.hr.assign(PS, 1.0);
+  sp.hg.assign(PS, 1.0);
+  sp.sbs.assign(PS, 0.0);
+  sp.coef.assign(PS, 0.0);
 
   // every face writes only its own entries: the fill is order-independent
 #pragma omp parallel for schedule(static)
@@ -109,6 +113,9 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
       sp.bm[s] = g.bm_dist[sr];
       sp.eta[s] = g.h_plus[sr] / g.bm_dist[sr];
       sp.eta[PS + s] = g.h_minus[sr] / g.bm_dist[sr];
+      sp.hr[s] = sp.hpm[s] / sp.hpm[PS + s];
+      sp.hg[s] = sp.bm[s] / sp.hpm[s];
+      sp.sbs[s] = sp.eta[PS + s] / (2 * n);
       const int va = g.face_vtx[sr];
       const int vb = g.face_vtx[g.face_off[r] + ((j + 1 == n) ? 0 : j + 1)];
       const V3 A = at3(g.vertices, va), B = at3(g.vertices, vb);
@@ -131,6 +138,10 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
       sp.nxr[PS + s] = nxr.y;
       sp.nxr[2 * PS + s] = nxr.z;
       sp.chord[s] = vnorm(vsub(A, B));
+      {  // round_diff * chord / area with one rounding (the product's error and the quotient's remainder put back)
+        const double p = sp.round_diff * sp.chord[s], q = p / sp.area[i];
+        sp.coef[s] = q + (std::fma(-q, sp.area[i], p) + std::fma(sp.round_diff, sp.chord[s], -p)) / sp.area[i];
+      }
       sp.rev[s] = j0_of[sr] * fpad + iperm[g.nbr_edge[sr]];
     }
     // unused slots of low-valence faces point at themselves (never read)

@@ -24,6 +24,7 @@ struct SlotPlanes {
   std::vector<double> beta;  // 4 planes
   std::vector<double> hpm;   // 2 planes
   std::vector<double> bm, eta /*2 planes*/, arc, ec /*3*/, ecn, en /*3*/, nxr /*3*/, chord;
+  std::vector<double> hr, hg, sbs, coef;  // H+/H-, BM/H+, (H-/BM) / (2 N), round_diff * chord / area
   double round_diff = 0.0;
   size_t PS() const { return (size_t)max_slots * fpad; }
 };

@@ -2,7 +2,7 @@
 // (step_fp64.cu, scalar type double), the tangent-linear model (Dual<N>)
 // and the adjoint's forward recomputation (double, extra outputs).
 //
-// Every body evaluates one face with the reference's operation order
+// Every body evaluates one face or one side of an edge
 // (MUSCL_base.hpp:124-161, 238-276, 345-434, 517-562), so all users of a
 // body produce bit-identical primal values when compiled with -fmad=false.
 #pragma once
@@ -66,56 +66,114 @@ SPLASH_HD SrcParams<Q> face_src_params(const DevGeom& G, const PhysParams& P, in
                       Q(P.acc_rate), Q(P.total_mass)};
 }
 
-// find_U_edges (MUSCL_base.hpp:361-434) for every slot of face f: limited
-// edge states of W, written to uplus with the energy at the edge centre.
+// The constants of one side of an edge (one slot): interpolation weights,
+// H+/H-, BM/H+, the limiter's eta_plus and superbee scale eta_minus / (2 N),
+// arc / area and cross(normal, edge centre).
+struct SideGeom {
+  double b0, b1, b2, b3, hr, hg, eta_p, sbs, arc_a;
+  D3 nxr;
+};
+// ... from the planes of the slots (stride PS), at index s, of a face of n edges
+SPLASH_HD SideGeom side_geom(const DevGeom& G, int PS, int s, int n) {
+  SideGeom c;
+  c.b0 = G.beta[s];
+  c.b1 = G.beta[PS + s];
+  c.b2 = G.beta[2 * PS + s];
+  c.b3 = G.beta[3 * PS + s];
+  c.arc_a = G.arc_a[s];
+#if defined(__CUDA_ARCH__)
+  c.hr = G.hr[s];
+  c.hg = G.hg[s];
+  c.eta_p = G.eta[s];
+  c.sbs = G.sbs[s];
+  c.nxr = plane3(G.nxr, PS, s);
+#else
+  c.hr = G.hpm[s] / G.hpm[PS + s];
+  c.hg = G.bm[s] / G.hpm[s];
+  c.eta_p = G.eta[s];
+  c.sbs = G.eta[PS + s] / (2 * n);
+  const D3 ec = plane3(G.ec, PS, s), en = plane3(G.en, PS, s);
+  const double ecn = G.ecn[s];
+  c.nxr = cross3(en, d3(ec.x / ecn, ec.y / ecn, ec.z / ecn));
+#endif
+  return c;
+}
+
+// Courant factor of the limiter (adiabatic.hpp:741-758, 792-810) of the
+// face state w on one side of an edge, (c + v.n) dt arc / area with
+// v.n = -(l . (n x R)) / Sigma, and what the limiter makes of it.
 template <class T>
-SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt,
-                                           const Planes<T>& W, const Planes<T>& uplus, int f) {
+SPLASH_HD T side_courant(const SideGeom& g, double gam, double dt, const T* w) {
+  const T ir = recip(w[0]);
+  const T c = root(gam * (w[4] * ir));
+  const T vn = -(fdot(g.nxr, v3(w[1], w[2], w[3])) * ir);
+  return (c + vn) * (dt * g.arc_a);
+}
+template <class T>
+SPLASH_HD LimiterLine<T> limiter_line(const SideGeom& g, const T& nu) {
+  const T ts = fm(nu, 1.0 / 3, T(1.0 / 3));
+  return LimiterLine<T>{g.eta_p, divide(g.sbs, nu), ts, 1.0 - ts};
+}
+
+// The differences of one field across the side: dp = U+ - w, dm = w - U-
+// with the interpolants U+- at the distances H+- (MUSCL_base.hpp:361-434).
+template <class T>
+SPLASH_HD void side_differences(const SideGeom& g, const T& w, const T& a, const T& b, const T& c, const T& d, T& dp,
+                                T& dm) {
+  dp = fm(g.b1, b, fm(g.b0, a, -w));
+  dm = fm(-g.b3, d, fm(-g.b2, c, w));
+}
+// r = (dm / H-) / (dp / H+)
+template <class T>
+SPLASH_HD T slope_ratio(const SideGeom& g, const T& dp, const T& dm) {
+  const T num = dm * g.hr;
+  const double y = recip(val(dp));
+  double v = val(num) * y;
+  if (odd_bits(v)) v = val(num) / val(dp);
+  T r(v);
+  if constexpr (is_dual<T>::value) {
+#pragma unroll
+    for (int i = 0; i < T::kN; ++i) r.d[i] = fma(-v, dp.d[i], num.d[i]) * y;
+  }
+  return r;
+}
+
+// The limited state (Sigma, l, Pi) of one side: up = w + dp phi(r) BM / H+.
+// nb(k, q) returns field k of stencil face q (0, 1: plus pair, 2, 3: minus).
+template <class T, class NbFn>
+SPLASH_HD void recon_side(const SideGeom& g, double gam, double dt, const T* w, NbFn nb, T* up) {
+  const T nu = side_courant(g, gam, dt, w);
+  const LimiterLine<T> line = limiter_line(g, nu);
+  const bool pos = (int64_t)bits_of(val(line.sb)) > 0 && !odd_bits(val(line.sb));
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    T dp, dm;
+    side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
+    const T r = slope_ratio(g, dp, dm);
+    T lim;
+    if constexpr (std::is_same<T, double>::value)
+      lim = pos ? limiter_field_pos(r, line) : limiter_field(r, line);
+    else
+      lim = limiter_field(r, line);
+    up[k] = fm(dp * g.hg, lim, w[k]);
+  }
+}
+
+// find_U_edges for every slot of face f: the edge states (Sigma, l, Pi)
+template <class T>
+SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt, const Planes<T>& W,
+                          const Planes<T>& uplus, int f) {
   const int fp = G.fpad;
   const int PS = G.max_slots * fp;  // one slot-plane set
   T w[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) w[k] = W.ld((size_t)k * fp + f);
   const int n = G.nslots[f];
-  const double twoN = (double)(2 * n);
-  const double gam = P.gam;
-  const T c = sqrt(gam * (w[4] + 0.0) / (w[0] + 0.0));  // sound speed (per face)
   for (int j = 0; j < n; ++j) {
     const int s = j * fp + f;
-    const int ia = G.sten[s], ib = G.sten[PS + s], ic = G.sten[2 * PS + s], id = G.sten[3 * PS + s];
-    const double bp0 = G.beta[s], bp1 = G.beta[PS + s], bm0 = G.beta[2 * PS + s], bm1 = G.beta[3 * PS + s];
-    const double hp = G.hpm[s], hm = G.hpm[PS + s], bmd = G.bm[s];
-    const double ihp = 1.0 / hp, ihm = 1.0 / hm;
-    T pp[kDim], r[kDim];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      const size_t o = (size_t)k * fp;
-      const T Up = bp0 * W.ld(o + ia) + bp1 * W.ld(o + ib);
-      pp[k] = (Up - w[k]) * ihp;
-      const T Um = bm0 * W.ld(o + ic) + bm1 * W.ld(o + id);
-      const T pm = (-Um + w[k]) * ihm;
-      r[k] = pm / pp[k];
-    }
-    // Courant factor of the limiter (adiabatic.hpp:741-758, 792-810)
-    const D3 ec = plane3(G.ec, PS, s);
-    const double ecn = G.ecn[s];
-    const D3 en = plane3(G.en, PS, s);
-    V3<T> vel = cross3(ec, v3(w[1], w[2], w[3]));
-    vel = scal(vel, 1.0 / ((-w[0] - 0.0) * ecn));
-    const T nu_plus = (c + dot3(vel, en)) * dt * G.arc_a[s];
-    const double eta_p = G.eta[s];
-    const T sb_scale = G.eta[PS + s] / (twoN * nu_plus);
-    const T to_scale = (1 + nu_plus) / 3;
+    const int st[4] = {G.sten[s], G.sten[PS + s], G.sten[2 * PS + s], G.sten[3 * PS + s]};
     T up[kDim];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      const T lim = limiter_field(r[k], eta_p, sb_scale, to_scale);
-      if (k == 0 || k == 4)
-        up[k] = w[k] + 0.0 + pp[k] * lim * bmd;
-      else
-        up[k] = w[k] + pp[k] * lim * bmd;
-    }
-    up[4] = energy_at_edge(up, ec, gam);  // Pi -> E at the edge centre
+    recon_side(side_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W.ld((size_t)k * fp + st[q]); }, up);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) uplus.st((size_t)k * PS + s, up[k]);
   }
@@ -132,14 +190,11 @@ SPLASH_HD unsigned flux_face(const DevGeom& G, const PhysParams& P, const SrcPar
   const int fp = G.fpad;
   const int PS = G.max_slots * fp;
   const D3 fcn = plane3(G.fcn, fp, f);
-  const double area = G.area[f];
   T w[kDim], acc[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) w[k] = Win.ld((size_t)k * fp + f);
   source_term(w, fcn, sp, P, acc);
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) acc[k] = dt_here * acc[k];
-  const double rd_dt = P.round_diff * dt_here;
+  const Gas gas = gas_of(P);
   const int n = G.nslots[f];
   unsigned bits = 0;
   for (int j = 0; j < n; ++j) {
@@ -151,21 +206,17 @@ SPLASH_HD unsigned flux_face(const DevGeom& G, const PhysParams& P, const SrcPar
       uL[k] = uplus.ld((size_t)k * PS + s);
       uR[k] = uplus.ld((size_t)k * PS + rv);
     }
-    SlotGeom g;
-    g.ec = plane3(G.ec, PS, s);
-    g.ecn = G.ecn[s];
-    g.en = plane3(G.en, PS, s);
-    g.nxr = plane3(G.nxr, PS, s);
-    bits |= flux_star(uL, uR, g, P.gam, P.solver, F);
-    const double coef = rd_dt * G.chord[s] / area;
+    const EdgeGeom g{plane3(G.ec, PS, s), plane3(G.en, PS, s), plane3(G.nxr, PS, s)};
+    bits |= riemann_flux(uL, uR, g, gas, P.solver, F);
+    const double coef = -G.coef[s];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
-      if (is_nan(F[k])) bits |= 1u;
-      acc[k] -= coef * F[k];
+      if (nan_bits(val(F[k]))) bits |= 1u;
+      acc[k] = fm(coef, F[k], acc[k]);
     }
   }
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) u[k] = acc[k] + U0.ld((size_t)k * fp + f);
+  for (int k = 0; k < kDim; ++k) u[k] = fm(dt_here, acc[k], U0.ld((size_t)k * fp + f));
   floored = u[0] < 1e-8;
   if (floored) u[0] = T(1e-8);
   return bits;
