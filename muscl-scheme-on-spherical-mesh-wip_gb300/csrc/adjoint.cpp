@@ -50,7 +50,7 @@ struct Adjoint {
   Solver* base = nullptr;
   int K = 50;
   int n_faces = 0, fpad = 0, max_slots = 0;
-  size_t PS = 0, FS = 0;  // one slot-plane set / one face-plane set of 5 fields
+  size_t XS = 0, FS = 0;  // one side plane / one face-plane set of 5 fields
   DevGeom G{};
   PhysParams P{};
   splash_params par{};
@@ -121,10 +121,10 @@ struct Adjoint {
     t.W0 = tW0 + (size_t)m * FS;
     t.U1 = tU1 + (size_t)m * FS;
     t.W1 = tW1 + (size_t)m * FS;
-    t.P0 = tP0 + (size_t)m * kDim * PS;
-    t.P1 = tP1 + (size_t)m * kDim * PS;
-    t.J0 = tJ0 + (size_t)m * kTapeJ * PS;
-    t.J1 = tJ1 + (size_t)m * kTapeJ * PS;
+    t.P0 = tP0 + (size_t)m * kDim * XS;
+    t.P1 = tP1 + (size_t)m * kDim * XS;
+    t.J0 = tJ0 + (size_t)m * kTapeJ * XS;
+    t.J1 = tJ1 + (size_t)m * kTapeJ * XS;
     t.mask = tmask + (size_t)m * fpad;
     return t;
   }
@@ -224,7 +224,6 @@ int Adjoint::forward(const double* U0, const double* theta, int n, double dt0_, 
   ADJ_CUDA(cudaMemsetAsync(S.err, 0, 4 * sizeof(unsigned), st));
   ADJ_CUDA(cudaMemsetAsync(S.scal, 0, kScCount * sizeof(double), st));
   ADJ_CUDA(fp64_prepare(G, S, P, st));
-  ADJ_CUDA(fp64_set_dt0(S, dt0_, st));
   cudaEvent_t e0, e1;
   ADJ_CUDA(cudaEventCreate(&e0));
   ADJ_CUDA(cudaEventCreate(&e1));
@@ -232,7 +231,7 @@ int Adjoint::forward(const double* U0, const double* theta, int n, double dt0_, 
   for (int i = 0; i < n; ++i) {
     if (i % K == 0)
       ADJ_CUDA(cudaMemcpyAsync(d_ck + (size_t)(i / K) * FS, S.U, FS * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    ADJ_CUDA(fp64_step(G, S, P, st));
+    ADJ_CUDA(fp64_step(G, S, P, dt0_, st));
     ADJ_CUDA(cudaMemcpyAsync(d_dts + i, S.scal + kScDt, sizeof(double), cudaMemcpyDeviceToDevice, st));
   }
   ADJ_CUDA(cudaEventRecord(e1, st));
@@ -270,7 +269,7 @@ int Adjoint::backward(const double* lam_final, double* grad_U0, double* grad_the
     ADJ_CUDA(rc_prim(G, P, tU, tW0, st));
     for (int m = 0; m < len; ++m) {
       const bool last = (m + 1 == len);
-      ADJ_CUDA(rc_step(G, P, d_dts + c + m, tape(m), last ? d_scrU : tU + (size_t)(m + 1) * FS,
+      ADJ_CUDA(rc_step(G, P, d_dts + c + m, tape(m), S.fe, last ? d_scrU : tU + (size_t)(m + 1) * FS,
                        last ? d_scrW : tW0 + (size_t)(m + 1) * FS, st));
     }
     // reverse steps back to the interval start
@@ -337,12 +336,11 @@ int Adjoint::tlm(const double* U0, const double* theta, const double* dU0, const
   ADJ_CUDA(cudaMemsetAsync(S.err, 0, 4 * sizeof(unsigned), st));
   ADJ_CUDA(cudaMemsetAsync(S.scal, 0, kScCount * sizeof(double), st));
   ADJ_CUDA(tlm_prepare(G, S, T, P, st));
-  ADJ_CUDA(fp64_set_dt0(S, dt0_, st));
   cudaEvent_t e0, e1;
   ADJ_CUDA(cudaEventCreate(&e0));
   ADJ_CUDA(cudaEventCreate(&e1));
   ADJ_CUDA(cudaEventRecord(e0, st));
-  for (int i = 0; i < n; ++i) ADJ_CUDA(tlm_step(G, S, T, P, st));
+  for (int i = 0; i < n; ++i) ADJ_CUDA(tlm_step(G, S, T, P, dt0_, st));
   ADJ_CUDA(cudaEventRecord(e1, st));
   ADJ_CUDA(cudaEventSynchronize(e1));
   ADJ_CUDA(cudaEventElapsedTime(&ms_tlm, e0, e1));
@@ -459,34 +457,34 @@ int splash_adjoint_create(splash_solver* base_h, int checkpoint_every, splash_ad
     a->n_faces = base->n_faces;
     a->fpad = base->fpad;
     a->max_slots = base->max_slots;
-    a->PS = (size_t)base->max_slots * base->fpad;
+    a->XS = (size_t)base->G.xs;
     a->FS = (size_t)splash::kDim * base->fpad;
     a->G = base->G;
     a->P = base->P;
     a->par = base->par;
-    const size_t fp = a->fpad, PS = a->PS, FS = a->FS;
+    const size_t fp = a->fpad, XS = a->XS, FS = a->FS;
     // host copies of the geometry the adjoint needs
     a->fcn_h.assign(3 * fp, 0.0);
-    std::vector<int> sten(4 * PS);
-    std::vector<int8_t> nsl(fp);
+    std::vector<int> sten(4 * XS), face(XS);
     if (cudaMemcpy(a->fcn_h.data(), base->G.fcn, 3 * fp * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(sten.data(), base->G.sten, 4 * PS * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(nsl.data(), base->G.nslots, fp, cudaMemcpyDeviceToHost) != cudaSuccess)
+        cudaMemcpy(sten.data(), base->G.e_sten, 4 * XS * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(face.data(), base->G.e_face, XS * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
       return splash::set_error(SPLASH_E_CUDA, "geometry download failed");
-    // inverse stencil: for every face, the (slot, position) pairs whose
-    // interpolants read it, in slot-plane order
-    if (4 * PS > (size_t)INT32_MAX) return splash::set_error(SPLASH_E_UNSUPPORTED, "mesh too large for the adjoint");
+    // inverse stencil: for every face, the (side, position) pairs whose
+    // interpolants read it, and its own sides (position 4), in side order
+    auto each = [&](auto&& fn) {  // fn(face, code)
+      for (int k = 0; k < 2; ++k)
+        for (int e = 0; e < base->G.n_edges; ++e) {
+          const size_t x = (size_t)k * base->G.epad + e;
+          for (int p = 0; p < 4; ++p) fn(sten[p * XS + x], (int)(x * 8 + p));
+          fn(face[x], (int)(x * 8 + 4));
+        }
+    };
     std::vector<int> cnt(fp + 1, 0);
-    for (int f = 0; f < a->n_faces; ++f)
-      for (int j = 0; j < nsl[f]; ++j)
-        for (int p = 0; p < 4; ++p) cnt[sten[p * PS + (size_t)j * fp + f] + 1]++;
+    each([&](int f, int) { cnt[f + 1]++; });
     for (size_t i = 0; i < fp; ++i) cnt[i + 1] += cnt[i];
     std::vector<int> ent(cnt[fp]), fill(cnt.begin(), cnt.end() - 1);
-    for (size_t s = 0; s < PS; ++s) {
-      const int f = (int)(s % fp), j = (int)(s / fp);
-      if (f >= a->n_faces || j >= nsl[f]) continue;
-      for (int p = 0; p < 4; ++p) ent[fill[sten[p * PS + s]]++] = (int)(s * 4 + p);
-    }
+    each([&](int f, int code) { ent[fill[f]++] = code; });
     int* d_off = a->dalloc<int>(fp + 1);
     int* d_ent = a->dalloc<int>(ent.size());
     if (cudaMemcpy(d_off, cnt.data(), (fp + 1) * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -500,14 +498,15 @@ int splash_adjoint_create(splash_solver* base_h, int checkpoint_every, splash_ad
     S.U = a->dalloc<double>(FS);
     S.W0 = a->dalloc<double>(FS);
     S.W1 = a->dalloc<double>(FS);
-    S.uplus = a->dalloc<double>(splash::kDim * PS);
-    S.partial = a->dalloc<double>((size_t)splash::fp64_partial_blocks(a->n_faces) * splash::kPartialStride);
+    S.uplus = a->dalloc<double>(splash::kDim * XS);
+    S.fe = a->dalloc<double>(splash::kDim * (XS / 2));
+    S.fold = a->dalloc<unsigned long long>(splash::kFoldCount);
     S.scal = a->dalloc<double>(splash::kScCount);
     S.err = a->dalloc<unsigned int>(4);
     a->T.dU = a->dalloc<double>(FS);
     a->T.dW0 = a->dalloc<double>(FS);
     a->T.dW1 = a->dalloc<double>(FS);
-    a->T.duplus = a->dalloc<double>(splash::kDim * PS);
+    a->T.dfe = a->dalloc<double>(splash::kDim * (XS / 2));
     a->T.dacc = a->d_dacc;
     // tape of K steps
     const size_t K = a->K;
@@ -515,21 +514,17 @@ int splash_adjoint_create(splash_solver* base_h, int checkpoint_every, splash_ad
     a->tW0 = a->dalloc<double>(K * FS);
     a->tU1 = a->dalloc<double>(K * FS);
     a->tW1 = a->dalloc<double>(K * FS);
-    a->tP0 = a->dalloc<double>(K * splash::kDim * PS);
-    a->tP1 = a->dalloc<double>(K * splash::kDim * PS);
-    a->tJ0 = a->dalloc<double>(K * splash::kTapeJ * PS);
-    a->tJ1 = a->dalloc<double>(K * splash::kTapeJ * PS);
+    a->tP0 = a->dalloc<double>(K * splash::kDim * XS);
+    a->tP1 = a->dalloc<double>(K * splash::kDim * XS);
+    a->tJ0 = a->dalloc<double>(K * splash::kTapeJ * XS);
+    a->tJ1 = a->dalloc<double>(K * splash::kTapeJ * XS);
     a->tmask = a->dalloc<uint8_t>(K * fp);
     a->d_lam = a->dalloc<double>(FS);
     a->d_scrU = a->dalloc<double>(FS);
     a->d_scrW = a->dalloc<double>(FS);
     splash::AdjScratch& X = a->X;
-    X.A = a->dalloc<double>(splash::kDim * PS);
-    X.B = a->dalloc<double>(splash::kDim * PS);
-    X.PU = a->dalloc<double>(2 * splash::kDim * PS);
-    X.Lw = a->dalloc<double>(FS);
-    X.la2 = a->dalloc<double>(FS);
-    X.la1 = a->dalloc<double>(FS);
+    X.PU = a->dalloc<double>(2 * splash::kDim * XS);
+    X.own = a->dalloc<double>(splash::kDim * XS);
     X.lam1 = a->dalloc<double>(FS);
     X.th = a->dalloc<double>(FS);
     X.inv_off = d_off;

@@ -9,15 +9,17 @@
 // apply the hand-written reverses of adjoint_rev.cuh.
 //
 // Reverse of one step (adjoint.hpp gives the forward map), per stage:
-//   adj_flux    per face: la = mask(lam); per slot Fb = -coef la,
-//               A = (dF/duL)^T Fb, B = (dF/duR)^T Fb
-//   adj_recon   per face: the adjoint of slot s's edge state is
-//               A[s] + B[rev s] (the edge seen from both faces);
-//               reverse reconstruction from the recomputation's limiter
-//               tape -> interpolant adjoints PU, own Lw
-//   adj_face    per face: lamW = Lw + sum over the inverse stencil of
-//               beta * PU, + source reverse (dt_here la), -> prim reverse
+//   adj_edge    per edge: la = mask(lam) of its two faces, the adjoint of the
+//               edge's flux Fb = dt (coef_1 la_1 - coef_0 la_0), its reverse
+//               (dF/duL)^T Fb, (dF/duR)^T Fb; per side: reverse reconstruction
+//               from the recomputation's limiter tape -> the adjoints PU of the
+//               two interpolants and the side's own part
+//   adj_face    per face: lamW = sum over the inverse stencil of beta * PU and
+//               the own parts, + source reverse (dt_here la), -> prim reverse
 // Every sum has a fixed order (no atomics): the adjoint is deterministic.
+// Like the step itself (step_fp64.cu) all of it is bound by the FP64 pipe:
+// the flux reverse runs once per edge, the reconstruction on a thread per
+// side.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -27,8 +29,8 @@
 #include "dual.cuh"
 #include "kernels.hpp"
 #include "physics_fp64.cuh"
-#include "reduce.cuh"
 #include "step_body_fp64.cuh"
+#include "step_fold_fp64.cuh"
 #include "taped.cuh"
 
 namespace splash {
@@ -50,12 +52,11 @@ namespace {
 using namespace splash::f64;
 using D1 = Dual<1>;
 static_assert(kTapeJ == rev::kTapePlanes, "tape plane count");
-constexpr int kBlock = 64;     // TLM kernels: must match the FP64 step (partials per block)
-constexpr int kRevBlock = 64;  // recomputation and reverse kernels (FP64-bound, register-heavy:
-                               // small blocks spread the faces evenly over the SMs)
+constexpr int kBlock = 64;                // faces per block
+constexpr int kThreads = 2 * kEdgeBlock;  // edge launches: a thread per side, as in step_fp64.cu
 
 inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
-inline int rev_blocks_for(int n) { return (n + kRevBlock - 1) / kRevBlock; }
+inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
 
 __device__ __forceinline__ D1 dual1(double v, double d) {
   D1 r(v);
@@ -67,73 +68,112 @@ __device__ __forceinline__ D1 dual1(double v, double d) {
 // tangent-linear model
 __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0, rate2 = 0.0;
+  bool negative = false;
   if (f < G.n_faces) {
     const int fp = G.fpad;
     const Planes<D1> U{S.U, T.dU, 0}, W{S.W0, T.dW0, 0};
     D1 u[kDim], w[kDim];
-    double uv[kDim];
+    double wv[kDim];
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      u[k] = U.ld((size_t)k * fp + f);
-      uv[k] = u[k].v;
-    }
+    for (int k = 0; k < kDim; ++k) u[k] = U.ld((size_t)k * fp + f);
     const D3 r = plane3(G.fcn, fp, f);
     prim_of(u, r, P.gam, w);
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) W.st((size_t)k * fp + f, w[k]);
-    dt_candidates(uv, r, G.area[f], P, vmax, dmin, sums);
+    for (int k = 0; k < kDim; ++k) {
+      W.st((size_t)k * fp + f, w[k]);
+      wv[k] = w[k].v;
+    }
+    dt_fold(wv, r, P, vel2, rate2, negative);
   }
-  red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
-}
-
-__global__ void __launch_bounds__(kBlock) tlm_recon_kernel(DevGeom G, PhysParams P, const double* __restrict__ sc,
-                                                           Planes<D1> W, Planes<D1> uplus) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  recon_face<D1>(G, P, sc[kScDt], W, uplus, f);
+  fold_block<kBlock>(vel2, rate2, negative, S, P);
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) tlm_flux_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
+__global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
+                                                            double dt0) {
+  __shared__ double up[2][kDim][kThreads];
+  const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  if (live) {
+    const int x = (t < kEdgeBlock) ? e : G.epad + e;
+    const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
+    const Planes<D1> W = (STAGE == 1) ? Planes<D1>{S.W0, T.dW0, 0} : Planes<D1>{S.W1, T.dW1, 0};
+    const size_t fp = G.fpad;
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[G.xs + x], G.e_sten[2 * G.xs + x], G.e_sten[3 * G.xs + x]};
+    D1 w[kDim], u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) w[k] = W.ld(k * fp + f);
+    recon_side(side_geom(G, x), P.gam, dt, w, [&](int k, int q) { return W.ld(k * fp + st[q]); }, u);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      up[0][k][t] = u[k].v;
+      up[1][k][t] = u[k].d[0];
+    }
+    if (STAGE == 1 && x == 0) publish_dt(S, dt);
+  }
+  __syncthreads();
+  if (!live || t >= kEdgeBlock) return;
+  D1 L[kDim], R[kDim], F[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    L[k] = dual1(up[0][k][i], up[1][k][i]);
+    R[k] = dual1(up[0][k][kEdgeBlock + i], up[1][k][kEdgeBlock + i]);
+  }
+  unsigned bits = riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+  const Planes<D1> fe{S.fe, T.dfe, 0};
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    if (nan_bits(F[k].v)) bits |= 1u;
+    fe.st((size_t)k * G.epad + e, F[k]);
+  }
+  if (bits) atomicOr(S.err, bits);
+}
+
+template <int STAGE>
+__global__ void __launch_bounds__(kBlock) tlm_update_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0, rate2 = 0.0;
+  bool negative = false;
   if (f < G.n_faces) {
-    const int fp = G.fpad;
+    const size_t fp = G.fpad;
     const double dt = S.scal[kScDt];
-    const double dt_here = (STAGE == 1) ? dt / 2 : dt;
     const SrcParams<D1> sp{dual1(G.acc_src[f], T.dacc[f]),
                            v3(D1(P.omega_acc_x), dual1(P.omega_acc_y, T.d_omega_y), dual1(P.omega_acc_z, T.d_omega_z)),
                            dual1(P.acc_rate, T.d_rate), dual1(P.total_mass, T.d_total_mass)};
     const Planes<D1> Win = (STAGE == 1) ? Planes<D1>{S.W0, T.dW0, 0} : Planes<D1>{S.W1, T.dW1, 0};
-    const Planes<D1> U{S.U, T.dU, 0};
-    D1 u[kDim];
+    const Planes<D1> U{S.U, T.dU, 0}, fe{S.fe, T.dfe, 0};
+    D1 w[kDim], u0[kDim], u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      w[k] = Win.ld(k * fp + f);
+      u0[k] = U.ld(k * fp + f);
+    }
     bool floored;
-    const unsigned bits =
-        flux_face<D1, D1>(G, P, sp, dt_here, Win, U, Planes<D1>{S.uplus, T.duplus, 0}, f, u, floored);
-    if (bits) atomicOr(S.err, bits);
-    const D3 fcn = plane3(G.fcn, fp, f);
-    D1 w[kDim];
+    update_face<D1, D1>(G, P, sp, (STAGE == 1) ? 0.5 * dt : dt, w, u0,
+                        [&](int k, int e) { return fe.ld((size_t)k * G.epad + e); }, f, u, floored);
+    const D3 fcn = plane3(G.fcn, G.fpad, f);
     prim_of(u, fcn, P.gam, w);
     const Planes<D1> Wout = (STAGE == 1) ? Planes<D1>{S.W1, T.dW1, 0} : Planes<D1>{S.W0, T.dW0, 0};
+    double wv[kDim];
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) Wout.st((size_t)k * fp + f, w[k]);
-    if (STAGE == 2) {
-      double uv[kDim];
-#pragma unroll
-      for (int k = 0; k < kDim; ++k) {
-        U.st((size_t)k * fp + f, u[k]);
-        uv[k] = u[k].v;
-      }
-      dt_candidates(uv, fcn, G.area[f], P, vmax, dmin, sums);
+    for (int k = 0; k < kDim; ++k) {
+      Wout.st(k * fp + f, w[k]);
+      wv[k] = w[k].v;
+      if (STAGE == 2) U.st(k * fp + f, u[k]);
     }
+    if (STAGE == 2) dt_fold(wv, fcn, P, vel2, rate2, negative);
   }
-  if (STAGE == 2) red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
+  if (STAGE == 2) fold_block<kBlock>(vel2, rate2, negative, S, P);
 }
 
 // ---------------------------------------------------------------------
-// branch-frozen forward: the step bodies on Taped (taped.cuh)
-__global__ void __launch_bounds__(kRevBlock) tp_prim_kernel(DevGeom G, PhysParams P, const double* __restrict__ U,
+// branch-frozen forward: the step bodies on Taped (taped.cuh).  A thread per
+// face, since a face owns its slice of the tape; it evaluates the fluxes of
+// all its edges itself, each in its edge's orientation.
+__global__ void __launch_bounds__(kBlock) tp_prim_kernel(DevGeom G, PhysParams P, const double* __restrict__ U,
                                                          double* __restrict__ W) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= G.n_faces) return;
@@ -146,37 +186,72 @@ __global__ void __launch_bounds__(kRevBlock) tp_prim_kernel(DevGeom G, PhysParam
   for (int k = 0; k < kDim; ++k) W[(size_t)k * fp + f] = w[k].v;
 }
 
-__global__ void __launch_bounds__(kRevBlock) tp_recon_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                          double* W, double* uplus) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  recon_face<Taped>(G, P, *dtp, Planes<Taped>{W}, Planes<Taped>{uplus}, f);
+// the sides of one edge that a face's slot stands for
+__device__ __forceinline__ int side_index(const DevGeom& G, int se) {
+  return se < 0 ? G.epad + (se & 0x7fffffff) : se;
 }
 
-template <int STAGE>
-__global__ void __launch_bounds__(kRevBlock) tp_flux_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                         double* Win, double* U0, double* uplus, double* Uout,
-                                                         double* Wout) {
+__global__ void __launch_bounds__(kBlock) tp_recon_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
+                                                          const double* W, double* uplus) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= G.n_faces) return;
-  const int fp = G.fpad;
+  const size_t fp = G.fpad, xs = G.xs;
+  Taped w[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) w[k] = Taped(W[k * fp + f]);
+  const int n = G.nslots[f];
+  for (int j = 0; j < n; ++j) {
+    const int x = side_index(G, G.slot_edge[j * fp + f]);
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    Taped u[kDim];
+    recon_side(side_geom(G, x), P.gam, *dtp, w, [&](int k, int q) { return Taped(W[k * fp + st[q]]); }, u);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) uplus[k * xs + x] = u[k].v;
+  }
+}
+template <int STAGE>
+__global__ void __launch_bounds__(kBlock) tp_flux_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
+                                                         const double* Win, const double* U0, const double* uplus,
+                                                         double* Uout, double* Wout) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= G.n_faces) return;
+  const size_t fp = G.fpad, xs = G.xs;
   const double dt = *dtp;
-  const double dt_here = (STAGE == 1) ? dt / 2 : dt;
-  Taped u[kDim], w[kDim];
-  bool floored;
-  flux_face<Taped, double>(G, P, face_src_params<double>(G, P, f), dt_here, Planes<Taped>{Win}, Planes<Taped>{U0},
-                           Planes<Taped>{uplus}, f, u, floored);
-  prim_of(u, plane3(G.fcn, fp, f), P.gam, w);
+  Taped u[kDim], w[kDim], u0[kDim], F[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    Uout[(size_t)k * fp + f] = u[k].v;
-    Wout[(size_t)k * fp + f] = w[k].v;
+    w[k] = Taped(Win[k * fp + f]);
+    u0[k] = Taped(U0[k * fp + f]);
+  }
+  const Gas gas = gas_of(P);
+  int have = -1;  // the edge whose flux F holds: the sum asks for its fields in turn
+  bool floored;
+  update_face<Taped, double>(
+      G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
+      [&](int k, int e) {
+        if (have != e) {
+          Taped L[kDim], R[kDim];
+          for (int q = 0; q < kDim; ++q) {
+            L[q] = Taped(uplus[q * xs + e]);
+            R[q] = Taped(uplus[q * xs + (G.e_twin ? G.e_twin[e] : G.epad + e)]);
+          }
+          riemann_flux(L, R, edge_geom(G, e), gas, P.solver, F);
+          have = e;
+        }
+        return F[k];
+      },
+      f, u, floored);
+  prim_of(u, plane3(G.fcn, G.fpad, f), P.gam, w);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    Uout[k * fp + f] = u[k].v;
+    Wout[k * fp + f] = w[k].v;
   }
 }
 
 // ---------------------------------------------------------------------
 // recomputation (double, extra outputs)
-__global__ void __launch_bounds__(kRevBlock) rc_prim_kernel(DevGeom G, PhysParams P, const double* __restrict__ U,
+__global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P, const double* __restrict__ U,
                                                          double* __restrict__ W) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= G.n_faces) return;
@@ -189,35 +264,69 @@ __global__ void __launch_bounds__(kRevBlock) rc_prim_kernel(DevGeom G, PhysParam
   for (int k = 0; k < kDim; ++k) W[(size_t)k * fp + f] = w[k];
 }
 
-__global__ void __launch_bounds__(kRevBlock) rc_recon_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                             const double* __restrict__ W, double* __restrict__ uplus,
-                                                             double* __restrict__ LJ) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  rev::recon_face_tape(G, P, *dtp, W, uplus, LJ, f);
+// the edge launch of the step with the limiter's Jacobian (LJ) and the edge
+// states (uplus) kept
+__global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
+                                                           const double* __restrict__ W, double* __restrict__ uplus,
+                                                           double* __restrict__ LJ, double* __restrict__ fe) {
+  __shared__ double up[kDim][kThreads];
+  const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  if (live) {
+    const int x = (t < kEdgeBlock) ? e : G.epad + e;
+    const size_t fp = G.fpad, xs = G.xs;
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    double w[kDim], u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) w[k] = W[k * fp + f];
+    rev::recon_side_tape(
+        side_geom(G, x), P.gam, *dtp, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u,
+        [&](int k, double v) { LJ[k * xs + x] = v; });
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      up[k][t] = u[k];
+      uplus[k * xs + x] = u[k];
+    }
+  }
+  __syncthreads();
+  if (!live || t >= kEdgeBlock) return;
+  double L[kDim], R[kDim], F[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    L[k] = up[k][i];
+    R[k] = up[k][kEdgeBlock + i];
+  }
+  riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) fe[(size_t)k * G.epad + e] = F[k];
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kRevBlock) rc_flux_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                         const double* __restrict__ Win, const double* __restrict__ U0,
-                                                         const double* __restrict__ uplus, double* __restrict__ Uout,
-                                                         double* __restrict__ Wout, uint8_t* __restrict__ mask) {
+__global__ void __launch_bounds__(kBlock) rc_update_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
+                                                           const double* __restrict__ Win,
+                                                           const double* __restrict__ U0, const double* __restrict__ fe,
+                                                           double* __restrict__ Uout, double* __restrict__ Wout,
+                                                           uint8_t* __restrict__ mask) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= G.n_faces) return;
-  const int fp = G.fpad;
+  const size_t fp = G.fpad;
   const double dt = *dtp;
-  const double dt_here = (STAGE == 1) ? dt / 2 : dt;
-  double u[kDim], w[kDim];
-  bool floored;
-  flux_face<double, double>(G, P, face_src_params<double>(G, P, f), dt_here, Planes<double>{const_cast<double*>(Win)},
-                            Planes<double>{const_cast<double*>(U0)}, Planes<double>{const_cast<double*>(uplus)}, f, u,
-                            floored);
-  const D3 fcn = plane3(G.fcn, fp, f);
-  prim_of(u, fcn, P.gam, w);
+  double w[kDim], u0[kDim], u[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    Uout[(size_t)k * fp + f] = u[k];
-    Wout[(size_t)k * fp + f] = w[k];
+    w[k] = Win[k * fp + f];
+    u0[k] = U0[k * fp + f];
+  }
+  bool floored;
+  update_face<double, double>(G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
+                              [&](int k, int e) { return fe[(size_t)k * G.epad + e]; }, f, u, floored);
+  prim_of(u, plane3(G.fcn, G.fpad, f), P.gam, w);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    Uout[k * fp + f] = u[k];
+    Wout[k * fp + f] = w[k];
   }
   const uint8_t bit = floored ? (uint8_t)STAGE : (uint8_t)0;
   mask[f] = (STAGE == 1) ? bit : (uint8_t)(mask[f] | bit);
@@ -225,111 +334,113 @@ __global__ void __launch_bounds__(kRevBlock) rc_flux_kernel(DevGeom G, PhysParam
 
 // ---------------------------------------------------------------------
 // reverse sweep
-__global__ void __launch_bounds__(kRevBlock) adj_flux_kernel(DevGeom G, PhysParams P, double dt_here,
-                                                          const double* __restrict__ uplus,
-                                                          const double* __restrict__ lam,
-                                                          const uint8_t* __restrict__ mask, int bit,
-                                                          double* __restrict__ la_out, double* __restrict__ A,
-                                                          double* __restrict__ B) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  const int fp = G.fpad;
-  const size_t PS = (size_t)G.max_slots * fp;
-  double la[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) la[k] = lam[(size_t)k * fp + f];
-  if (mask[f] & bit) la[0] = 0.0;  // density floor: the output's Sigma is a constant
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) la_out[(size_t)k * fp + f] = la[k];
-  const Gas gas = gas_of(P);
-  const int n = G.nslots[f];
-  for (int j = 0; j < n; ++j) {
-    const int s = j * fp + f;
-    const int rv = G.rev[s];
-    const double coef = dt_here * G.coef[s];
-    double uL[kDim], uR[kDim], Fb[kDim], uLb[kDim], uRb[kDim];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      uL[k] = uplus[(size_t)k * PS + s];
-      uR[k] = uplus[(size_t)k * PS + rv];
-      Fb[k] = -coef * la[k];
-      uLb[k] = 0.0;
-      uRb[k] = 0.0;
-    }
-    const EdgeGeom g{plane3(G.ec, (int)PS, s), plane3(G.en, (int)PS, s), plane3(G.nxr, (int)PS, s)};
-    rev::riemann_flux_rev(uL, uR, g, gas, P.solver, Fb, uLb, uRb);
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      A[(size_t)k * PS + s] = uLb[k];
-      B[(size_t)k * PS + s] = uRb[k];
-    }
-  }
+
+// lam of face f with the density floor's mask: where the floor held, the
+// output's Sigma is a constant
+__device__ __forceinline__ double masked(const double* lam, const uint8_t* mask, int bit, size_t fp, int k, int f) {
+  return (k == 0 && (mask[f] & bit)) ? 0.0 : lam[k * fp + f];
 }
 
-__global__ void __launch_bounds__(kRevBlock) adj_recon_kernel(DevGeom G, PhysParams P, double dt,
-                                                              const double* __restrict__ W,
-                                                              const double* __restrict__ uplus,
-                                                              const double* __restrict__ LJ,
-                                                              const double* __restrict__ A,
-                                                              const double* __restrict__ B, double* __restrict__ PU,
-                                                              double* __restrict__ Lw) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  const int fp = G.fpad;
-  const size_t PS = (size_t)G.max_slots * fp;
-  double wb[kDim] = {0, 0, 0, 0, 0};
-  rev::recon_face_rev(
-      G, P, dt, W, uplus, LJ, [&](int k, int s) { return A[(size_t)k * PS + s] + B[(size_t)k * PS + G.rev[s]]; },
-      PU, wb, f);
+__global__ void __launch_bounds__(kThreads) adj_edge_kernel(DevGeom G, PhysParams P, double dt, double dt_here,
+                                                            const double* __restrict__ W,
+                                                            const double* __restrict__ uplus,
+                                                            const double* __restrict__ LJ,
+                                                            const double* __restrict__ lam,
+                                                            const uint8_t* __restrict__ mask, int bit,
+                                                            double* __restrict__ PU, double* __restrict__ own) {
+  __shared__ double ub[kDim][kThreads];
+  const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  const size_t fp = G.fpad, xs = G.xs;
+  if (live && t < kEdgeBlock) {
+    const double* coef = G.e_side + kSideCoef * xs + e;
+    const double c0 = dt_here * coef[0], c1 = dt_here * coef[G.epad];
+    const int f0 = G.e_face[e], f1 = G.e_face[G.epad + e];
+    double L[kDim], R[kDim], Fb[kDim], Lb[kDim], Rb[kDim];
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) Lw[(size_t)k * fp + f] = wb[k];
+    for (int k = 0; k < kDim; ++k) {
+      L[k] = uplus[k * xs + e];
+      R[k] = uplus[k * xs + G.epad + e];
+      Fb[k] = fma(c1, masked(lam, mask, bit, fp, k, f1), -(c0 * masked(lam, mask, bit, fp, k, f0)));
+      Lb[k] = 0.0;
+      Rb[k] = 0.0;
+    }
+    rev::riemann_flux_rev(L, R, edge_geom(G, e), gas_of(P), P.solver, Fb, Lb, Rb);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      ub[k][i] = Lb[k];
+      ub[k][kEdgeBlock + i] = Rb[k];
+    }
+  }
+  __syncthreads();
+  if (!live) return;
+  const int x = (t < kEdgeBlock) ? e : G.epad + e;
+  const int f = G.e_face[x];
+  double w[kDim], upb[kDim], pu[kDim], mu[kDim], wb[kDim] = {0, 0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    w[k] = W[k * fp + f];
+    upb[k] = ub[k][t];
+  }
+  rev::recon_side_rev(side_geom(G, x), P.gam, dt, w, upb, [&](int k) { return LJ[k * xs + x]; }, pu, mu, wb);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    PU[k * xs + x] = pu[k];
+    PU[(kDim + k) * xs + x] = mu[k];
+    own[k * xs + x] = wb[k];
+  }
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kRevBlock) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
+__global__ void __launch_bounds__(kBlock) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
                                                           const double* __restrict__ Win,
                                                           const double* __restrict__ Uin,
-                                                          const double* __restrict__ la,
-                                                          double* __restrict__ lam_out) {
+                                                          const uint8_t* __restrict__ mask, const double* lam,
+                                                          double* lam_out) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G.n_faces) return;
-  const int fp = G.fpad;
-  const size_t PS = (size_t)G.max_slots * fp;
-  double wb[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) wb[k] = X.Lw[(size_t)k * fp + g];
-  // the interpolants of the slots whose stencils hold face g
+  const size_t fp = G.fpad, xs = G.xs;
+  double wb[kDim] = {0, 0, 0, 0, 0};
+  // the interpolants whose stencils hold face g, and the sides that are its own
   for (int e = X.inv_off[g]; e < X.inv_off[g + 1]; ++e) {
     const int code = X.inv_ent[e];
-    const size_t s = (size_t)(code >> 2);
-    const int pos = code & 3;
-    const double bt = G.beta[(size_t)pos * PS + s];
-    const double* src = X.PU + (size_t)(pos >= 2 ? kDim : 0) * PS;
+    const size_t x = (size_t)(code >> 3);
+    const int pos = code & 7;
+    if (pos == 4) {
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) wb[k] += bt * src[(size_t)k * PS + s];
+      for (int k = 0; k < kDim; ++k) wb[k] += X.own[k * xs + x];
+      continue;
+    }
+    const double bt = G.e_side[(size_t)(kSideBeta + pos) * xs + x];
+    const double* src = X.PU + (pos >= 2 ? kDim : 0) * xs;
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) wb[k] = fma(bt, src[k * xs + x], wb[k]);
   }
-  const D3 fcn = plane3(G.fcn, fp, g);
-  double w[kDim], u[kDim], srcb[kDim], ub[kDim] = {0, 0, 0, 0, 0}, pb[5] = {0, 0, 0, 0, 0};
+  const D3 fcn = plane3(G.fcn, G.fpad, g);
+  // the adjoint of this stage's output state: stage 2's is lam, stage 1's lam1
+  const double* out = (STAGE == 2) ? lam : X.lam1;
+  double w[kDim], u[kDim], la[kDim], srcb[kDim], ub[kDim] = {0, 0, 0, 0, 0}, pb[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    w[k] = Win[(size_t)k * fp + g];
-    u[k] = Uin[(size_t)k * fp + g];
-    srcb[k] = dt_here * la[(size_t)k * fp + g];
+    w[k] = Win[k * fp + g];
+    u[k] = Uin[k * fp + g];
+    la[k] = masked(out, mask, STAGE, fp, k, g);
+    srcb[k] = dt_here * la[k];
   }
   if (P.accretion_on) {
     rev::source_rev(w, fcn, face_src_params<double>(G, P, g), P, srcb, wb, pb);
 #pragma unroll
-    for (int j = 0; j < 5; ++j) X.th[(size_t)j * fp + g] += pb[j];
+    for (int j = 0; j < 5; ++j) X.th[j * fp + g] += pb[j];
   }
   rev::prim_rev(u, fcn, P.gam, wb, ub);
   if (STAGE == 2) {
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) lam_out[(size_t)k * fp + g] = ub[k];
+    for (int k = 0; k < kDim; ++k) lam_out[k * fp + g] = ub[k];
   } else {
     // U1 = floor(U + acc1) and U2 = floor(U + acc2) both hold U directly
 #pragma unroll
-    for (int k = 0; k < kDim; ++k)
-      lam_out[(size_t)k * fp + g] = ub[k] + X.la1[(size_t)k * fp + g] + X.la2[(size_t)k * fp + g];
+    for (int k = 0; k < kDim; ++k) lam_out[k * fp + g] = ub[k] + la[k] + masked(lam, mask, 2, fp, k, g);
   }
 }
 
@@ -339,21 +450,19 @@ __global__ void __launch_bounds__(kRevBlock) adj_face_kernel(DevGeom G, PhysPara
 // ---- launchers ----------------------------------------------------------
 cudaError_t tlm_prepare(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P,
                         cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(S.fold, 0, kFoldCount * sizeof(*S.fold), st);
+  if (e != cudaSuccess) return e;
   adj::tlm_prepare_kernel<<<adj::blocks_for(G.n_faces), adj::kBlock, 0, st>>>(G, S, T, P);
   return cudaGetLastError();
 }
 
-cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P,
+cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P, double dt0,
                      cudaStream_t st) {
-  using adj::D1;
-  const int nb = adj::blocks_for(G.n_faces);
-  cudaError_t e = fp64_dt(S, P, G.n_faces, st);
-  if (e != cudaSuccess) return e;
-  const f64::Planes<D1> W0{S.W0, T.dW0, 0}, W1{S.W1, T.dW1, 0}, up{S.uplus, T.duplus, 0};
-  adj::tlm_recon_kernel<<<nb, adj::kBlock, 0, st>>>(G, P, S.scal, W0, up);
-  adj::tlm_flux_kernel<1><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
-  adj::tlm_recon_kernel<<<nb, adj::kBlock, 0, st>>>(G, P, S.scal, W1, up);
-  adj::tlm_flux_kernel<2><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
+  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  adj::tlm_edge_kernel<1><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
+  adj::tlm_update_kernel<1><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
+  adj::tlm_edge_kernel<2><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
+  adj::tlm_update_kernel<2><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
   return cudaGetLastError();
 }
 
@@ -377,15 +486,15 @@ cudaError_t taped_prim(const DevGeom& G, const PhysParams& P, double* U, double*
                        uint32_t* pos, unsigned* err, int mode, cudaStream_t st) {
   cudaError_t e = tape_region(G, region, pos, err, mode, st);
   if (e != cudaSuccess) return e;
-  adj::tp_prim_kernel<<<adj::rev_blocks_for(G.n_faces), adj::kRevBlock, 0, st>>>(G, P, U, W);
+  adj::tp_prim_kernel<<<adj::blocks_for(G.n_faces), adj::kBlock, 0, st>>>(G, P, U, W);
   return cudaGetLastError();
 }
 
 cudaError_t taped_step(const DevGeom& G, const PhysParams& P, const double* dtp, double* U, double* W0,
                        double* W1, double* uplus, double* U1, uint32_t* region, uint32_t* pos, unsigned* err,
                        int mode, cudaStream_t st) {
-  const int nb = adj::rev_blocks_for(G.n_faces);
-  constexpr int B = adj::kRevBlock;
+  const int nb = adj::blocks_for(G.n_faces);
+  constexpr int B = adj::kBlock;
   const size_t RW = (size_t)G.n_faces * tape::kTapeWords;
   cudaError_t e;
   if ((e = tape_region(G, region, pos, err, mode, st)) != cudaSuccess) return e;
@@ -400,34 +509,32 @@ cudaError_t taped_step(const DevGeom& G, const PhysParams& P, const double* dtp,
 }
 
 cudaError_t rc_prim(const DevGeom& G, const PhysParams& P, const double* U, double* W, cudaStream_t st) {
-  adj::rc_prim_kernel<<<adj::rev_blocks_for(G.n_faces), adj::kRevBlock, 0, st>>>(G, P, U, W);
+  adj::rc_prim_kernel<<<adj::blocks_for(G.n_faces), adj::kBlock, 0, st>>>(G, P, U, W);
   return cudaGetLastError();
 }
 
-cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t, double* U_next,
-                    double* W_next, cudaStream_t st) {
-  const int nb = adj::rev_blocks_for(G.n_faces);
-  constexpr int B = adj::kRevBlock;
-  adj::rc_recon_kernel<<<nb, B, 0, st>>>(G, P, dtp, t.W0, t.P0, t.J0);
-  adj::rc_flux_kernel<1><<<nb, B, 0, st>>>(G, P, dtp, t.W0, t.U, t.P0, t.U1, t.W1, t.mask);
-  adj::rc_recon_kernel<<<nb, B, 0, st>>>(G, P, dtp, t.W1, t.P1, t.J1);
-  adj::rc_flux_kernel<2><<<nb, B, 0, st>>>(G, P, dtp, t.W1, t.U, t.P1, U_next, W_next, t.mask);
+cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t, double* fe,
+                    double* U_next, double* W_next, cudaStream_t st) {
+  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  constexpr int B = adj::kBlock, E = adj::kThreads;
+  adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W0, t.P0, t.J0, fe);
+  adj::rc_update_kernel<1><<<nb, B, 0, st>>>(G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask);
+  adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W1, t.P1, t.J1, fe);
+  adj::rc_update_kernel<2><<<nb, B, 0, st>>>(G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask);
   return cudaGetLastError();
 }
 
 cudaError_t adj_step(const DevGeom& G, const PhysParams& P, double dt, const StepTape& t, const AdjScratch& X,
                      double* lam, cudaStream_t st) {
-  const int nb = adj::rev_blocks_for(G.n_faces);
-  constexpr int B = adj::kRevBlock;
+  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  constexpr int B = adj::kBlock, E = adj::kThreads;
   // stage 2: U2 = floor(U + dt Phi(W1, P1))
-  adj::adj_flux_kernel<<<nb, B, 0, st>>>(G, P, dt, t.P1, lam, t.mask, 2, X.la2, X.A, X.B);
-  adj::adj_recon_kernel<<<nb, B, 0, st>>>(G, P, dt, t.W1, t.P1, t.J1, X.A, X.B, X.PU, X.Lw);
-  adj::adj_face_kernel<2><<<nb, B, 0, st>>>(G, P, dt, X, t.W1, t.U1, X.la2, X.lam1);
+  adj::adj_edge_kernel<<<ne, E, 0, st>>>(G, P, dt, dt, t.W1, t.P1, t.J1, lam, t.mask, 2, X.PU, X.own);
+  adj::adj_face_kernel<2><<<nb, B, 0, st>>>(G, P, dt, X, t.W1, t.U1, t.mask, lam, X.lam1);
   // stage 1: U1 = floor(U + dt/2 Phi(W0, P0))
   const double dt_half = dt / 2;
-  adj::adj_flux_kernel<<<nb, B, 0, st>>>(G, P, dt_half, t.P0, X.lam1, t.mask, 1, X.la1, X.A, X.B);
-  adj::adj_recon_kernel<<<nb, B, 0, st>>>(G, P, dt, t.W0, t.P0, t.J0, X.A, X.B, X.PU, X.Lw);
-  adj::adj_face_kernel<1><<<nb, B, 0, st>>>(G, P, dt_half, X, t.W0, t.U, X.la1, lam);
+  adj::adj_edge_kernel<<<ne, E, 0, st>>>(G, P, dt, dt_half, t.W0, t.P0, t.J0, X.lam1, t.mask, 1, X.PU, X.own);
+  adj::adj_face_kernel<1><<<nb, B, 0, st>>>(G, P, dt_half, X, t.W0, t.U, t.mask, lam, lam);
   return cudaGetLastError();
 }
 

@@ -18,21 +18,21 @@
 
 namespace splash {
 
-constexpr int kTapeJ = 15;  // limiter-Jacobian tape planes per slot and stage
+constexpr int kTapeJ = 15;  // limiter-Jacobian tape planes per side and stage
 
 // Tangents of the TLM beside a value DevState.
 struct TlmTangents {
   double* dU;
   double* dW0;
   double* dW1;
-  double* duplus;
+  double* dfe;         // of the edge fluxes
   const double* dacc;  // tangent of the per-face accretion profile
   double d_omega_y, d_omega_z, d_rate, d_total_mass;
 };
 
 // Primal data of one step, stored by the recomputation: the step's input
 // state and its stage-1 state, their (Sigma, l, Pi), both stages' edge
-// states, both stages' limiter Jacobians (15 planes per slot, see
+// states, both stages' limiter Jacobians (15 planes per side, see
 // adjoint_rev.cuh) and the density-floor bits (1: stage 1, 2: stage 2).
 struct StepTape {
   double* U;
@@ -48,15 +48,11 @@ struct StepTape {
 
 // Scratch of the reverse sweep.
 struct AdjScratch {
-  double* A;    // [5][PS]  (dF/duL)^T Fb per slot
-  double* B;    // [5][PS]  (dF/duR)^T Fb per slot
-  double* PU;   // [10][PS] adjoints of the stencil interpolants
-  double* Lw;   // [5][fp]  own-face reconstruction adjoint
-  double* la2;  // [5][fp]  masked adjoint of the stage-2 increment
-  double* la1;  // [5][fp]  masked adjoint of the stage-1 increment
+  double* PU;   // [10][xs] adjoints of the stencil interpolants of every side
+  double* own;  // [5][xs]  the sides' own-face reconstruction adjoints
   double* lam1; // [5][fp]  adjoint of U1
   double* th;   // [5][fp]  per-face adjoints of (acc0, omega_y, omega_z, acc_rate, total_mass)
-  const int* inv_off;  // inverse stencil CSR: faces -> (slot * 4 + position)
+  const int* inv_off;  // inverse stencil CSR: faces -> side * 8 + position (4: the face's own side)
   const int* inv_ent;
 };
 
@@ -65,14 +61,15 @@ cudaError_t tlm_prepare(const DevGeom& G, const DevState& S, const TlmTangents& 
                         cudaStream_t st);
 // One step: dt clip of the value state, then the four stage launches on
 // Dual<1> (values bit-identical to fp64_step).
-cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P,
+cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P, double dt0,
                      cudaStream_t st);
 
 // ---- recomputation of one step from tape.U with dt = *dtp ----
 // tape.W0 must hold prim(tape.U) (rc_prim).  Writes the rest of the tape
-// and the step's output state to (U_next, W_next).
+// and the step's output state to (U_next, W_next); fe is scratch for the
+// edge fluxes.
 cudaError_t rc_prim(const DevGeom& G, const PhysParams& P, const double* U, double* W, cudaStream_t st);
-cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t,
+cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t, double* fe,
                     double* U_next, double* W_next, cudaStream_t st);
 
 // ---- reverse of one step: lam (adjoint of the step's output) is replaced

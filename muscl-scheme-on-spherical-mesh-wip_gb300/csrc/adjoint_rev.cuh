@@ -414,7 +414,7 @@ SPLASH_HD void recon_face_tape(const DevGeom& G, const PhysParams& P, double dt,
     const int st[4] = {G.sten[s], G.sten[PS + s], G.sten[2 * PS + s], G.sten[3 * PS + s]};
     double up[kDim];
     recon_side_tape(
-        side_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W[(size_t)k * fp + st[q]]; }, up,
+        slot_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W[(size_t)k * fp + st[q]]; }, up,
         [&](int i, double x) { LJ[(size_t)i * PS + s] = x; });
 #pragma unroll
     for (int k = 0; k < kDim; ++k) uplus[(size_t)k * PS + s] = up[k];
@@ -442,7 +442,7 @@ SPLASH_HD void recon_face_rev(const DevGeom& G, const PhysParams& P, double dt, 
 #pragma unroll
     for (int k = 0; k < kDim; ++k) upb[k] = upb_at(k, s);
     recon_side_rev(
-        side_geom(G, PS, s, n), P.gam, dt, w, upb, [&](int i) { return LJ[(size_t)i * PS + s]; }, pu, mu, wb);
+        slot_geom(G, PS, s, n), P.gam, dt, w, upb, [&](int i) { return LJ[(size_t)i * PS + s]; }, pu, mu, wb);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
       PU[(size_t)k * PS + s] = pu[k];

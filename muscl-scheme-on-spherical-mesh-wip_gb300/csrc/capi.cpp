@@ -100,8 +100,8 @@ T* Solver::dalloc(size_t n) {
   return static_cast<T*>(p);
 }
 
-template <typename T>
-T* Solver::upload(const std::vector<T>& h) {
+template <typename T, typename A>
+T* Solver::upload(const std::vector<T, A>& h) {
   T* d = dalloc<T>(h.size());
   if (!h.empty() && cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess)
     throw std::runtime_error("cudaMemcpy upload failed");
@@ -197,27 +197,20 @@ void Solver::build_device_geometry(const RefGeometry& g) {
     G.fcn = upload(sp.fcn);
     G.area = upload(sp.area);
     G.acc_src = upload(acc);
-    G.sten = upload(sp.sten);
-    G.beta = upload(sp.beta);
-    G.hpm = upload(sp.hpm);
-    G.bm = upload(sp.bm);
-    G.eta = upload(sp.eta);
-    G.hr = upload(sp.hr);
-    G.hg = upload(sp.hg);
-    G.sbs = upload(sp.sbs);
-    G.coef = upload(sp.coef);
-    G.arc_a = upload(sp.arc);
-    G.ec = upload(sp.ec);
-    G.ecn = upload(sp.ecn);
-    G.en = upload(sp.en);
-    G.nxr = upload(sp.nxr);
-    G.chord = upload(sp.chord);
-    G.rev = upload(sp.rev);
+    const EdgePlanes ep = make_edge_planes(sp, solver_kind == kSolverIsoHLLE);
+    G.n_edges = ep.n_edges;
+    G.epad = ep.epad;
+    G.xs = 2 * ep.epad;
+    G.slot_edge = upload(ep.slot_edge);
+    h_slot_edge = ep.slot_edge;
+    G.e_face = upload(ep.face);
+    G.e_sten = upload(ep.sten);
+    G.e_twin = ep.twin.empty() ? nullptr : upload(ep.twin);
+    G.e_side = upload(ep.side);
+    G.e_geo = upload(ep.geo);
     geometry_bytes = sp.nslots.size() + 8 * (sp.fcn.size() + sp.area.size() + acc.size()) +
-                     4 * (sp.sten.size() + sp.rev.size()) +
-                     8 * (sp.beta.size() + sp.hpm.size() + sp.bm.size() + sp.eta.size() +
-                          sp.arc.size() + sp.ec.size() + sp.ecn.size() + sp.en.size() +
-                          sp.nxr.size() + sp.chord.size());
+                     4 * (ep.slot_edge.size() + ep.face.size() + ep.sten.size() + ep.twin.size()) +
+                     8 * (ep.side.size() + ep.geo.size());
   }
   // keep what the writers need, in reference order
   wr_vertices = g.vertices;
@@ -269,15 +262,13 @@ int Solver::run_diagnostics(double* out9) {
   return SPLASH_OK;
 }
 
-// FP64 path: W and the dt partial records of the current U (the mixed path
+// FP64 path: W and the dt bounds of the current U (the mixed path
 // computes its face states and dt keys in the set_state pass)
 cudaError_t Solver::launch_prepare() { return fp64_prepare(G, S, P, stream); }
 
 cudaError_t Solver::launch_step(cudaEvent_t* ev, double dt0, bool per_launch) {
   if (precision == SPLASH_PREC_MIXED) return mixed_step(GM, S, P, dt0, stream, ev, per_launch);
-  cudaError_t e = fp64_set_dt0(S, dt0, stream);
-  if (e != cudaSuccess) return e;
-  return fp64_step(G, S, P, stream, ev);
+  return fp64_step(G, S, P, dt0, stream, ev);
 }
 
 int Solver::upload_state(const double* U_ref) {
@@ -317,66 +308,42 @@ int Solver::read_scalars(double* out) {
   return SPLASH_OK;
 }
 
-int Solver::capture_graph() {
+// Captures n_steps steps into a graph and collects its stage-1 edge nodes,
+// whose argument dt0 is.
+int Solver::capture_steps(int n_steps, cudaGraph_t* g, cudaGraphExec_t* exec, std::vector<cudaGraphNode_t>* dt0_nodes) {
   SPLASH_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-  // FP64: the graph holds the five step launches, dt0 is set by a launch
-  // before each replay; mixed: the graph holds the whole step, dt0 being an
-  // argument of its first node
-  cudaError_t le = (precision == SPLASH_PREC_MIXED) ? mixed_step(GM, S, P, graph_dt0, stream, nullptr)
-                                                     : fp64_step(G, S, P, stream, nullptr);
-  cudaGraph_t g = nullptr;
-  cudaError_t ce = cudaStreamEndCapture(stream, &g);
+  cudaError_t le = cudaSuccess;
+  for (int k = 0; k < n_steps && le == cudaSuccess; ++k) le = launch_step(nullptr, graph_dt0);
+  cudaGraph_t got = nullptr;
+  cudaError_t ce = cudaStreamEndCapture(stream, &got);
   if (le != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
+    if (got) cudaGraphDestroy(got);
     return fail(SPLASH_E_CUDA, "step launch during capture: %s", cudaGetErrorString(le));
   }
   SPLASH_CUDA(ce);
-  graph = g;
-  SPLASH_CUDA(cudaGraphInstantiate(&graph_exec, graph, 0));
-  if (precision == SPLASH_PREC_MIXED) {
-    size_t n = 0;
-    SPLASH_CUDA(cudaGraphGetNodes(graph, nullptr, &n));
-    std::vector<cudaGraphNode_t> nodes(n);
-    SPLASH_CUDA(cudaGraphGetNodes(graph, nodes.data(), &n));
-    for (cudaGraphNode_t nd : nodes) {
-      cudaGraphNodeType t;
-      SPLASH_CUDA(cudaGraphNodeGetType(nd, &t));
-      if (t != cudaGraphNodeTypeKernel) continue;
-      cudaKernelNodeParams kp{};
-      SPLASH_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
-      if (kp.func == mixed_dt0_kernel_ptr()) dt0_node = nd;
-    }
-    if (!dt0_node) return fail(SPLASH_E_CUDA, "dt node not found in the captured step");
-    // the same step kGraphSteps times in one graph
-    SPLASH_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t lk = cudaSuccess;
-    for (int k = 0; k < kGraphSteps && lk == cudaSuccess; ++k)
-      lk = mixed_step(GM, S, P, graph_dt0, stream, nullptr);
-    cudaGraph_t gk = nullptr;
-    cudaError_t ck = cudaStreamEndCapture(stream, &gk);
-    if (lk != cudaSuccess) {
-      if (gk) cudaGraphDestroy(gk);
-      return fail(SPLASH_E_CUDA, "step launch during capture: %s", cudaGetErrorString(lk));
-    }
-    SPLASH_CUDA(ck);
-    graph_k = gk;
-    SPLASH_CUDA(cudaGraphInstantiate(&graph_k_exec, graph_k, 0));
-    SPLASH_CUDA(cudaGraphGetNodes(graph_k, nullptr, &n));
-    nodes.resize(n);
-    SPLASH_CUDA(cudaGraphGetNodes(graph_k, nodes.data(), &n));
-    dt0_nodes_k.clear();
-    for (cudaGraphNode_t nd : nodes) {
-      cudaGraphNodeType t;
-      SPLASH_CUDA(cudaGraphNodeGetType(nd, &t));
-      if (t != cudaGraphNodeTypeKernel) continue;
-      cudaKernelNodeParams kp{};
-      SPLASH_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
-      if (kp.func == mixed_dt0_kernel_ptr()) dt0_nodes_k.push_back(nd);
-    }
-    if ((int)dt0_nodes_k.size() != kGraphSteps)
-      return fail(SPLASH_E_CUDA, "dt nodes not found in the captured steps");
+  *g = got;
+  SPLASH_CUDA(cudaGraphInstantiate(exec, got, 0));
+  const void* first = precision == SPLASH_PREC_MIXED ? mixed_dt0_kernel_ptr() : fp64_dt0_kernel_ptr(solver_kind);
+  size_t n = 0;
+  SPLASH_CUDA(cudaGraphGetNodes(got, nullptr, &n));
+  std::vector<cudaGraphNode_t> nodes(n);
+  SPLASH_CUDA(cudaGraphGetNodes(got, nodes.data(), &n));
+  dt0_nodes->clear();
+  for (cudaGraphNode_t nd : nodes) {
+    cudaGraphNodeType t;
+    SPLASH_CUDA(cudaGraphNodeGetType(nd, &t));
+    if (t != cudaGraphNodeTypeKernel) continue;
+    cudaKernelNodeParams kp{};
+    SPLASH_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
+    if (kp.func == first) dt0_nodes->push_back(nd);
   }
+  if ((int)dt0_nodes->size() != n_steps) return fail(SPLASH_E_CUDA, "dt nodes not found in the captured steps");
   return SPLASH_OK;
+}
+
+int Solver::capture_graph() {
+  const int rc = capture_steps(1, &graph, &graph_exec, &dt0_nodes);
+  return rc ? rc : capture_steps(kGraphSteps, &graph_k, &graph_k_exec, &dt0_nodes_k);
 }
 
 int Solver::set_graph_dt0(double dt0) {
@@ -384,37 +351,27 @@ int Solver::set_graph_dt0(double dt0) {
   // new dt0: rewrite the stage-1 edge nodes' arguments in the instantiated
   // graphs (takes effect from the next launch; launches in flight keep theirs)
   cudaKernelNodeParams kp{};
-  SPLASH_CUDA(cudaGraphKernelNodeGetParams(dt0_node, &kp));
+  SPLASH_CUDA(cudaGraphKernelNodeGetParams(dt0_nodes[0], &kp));
   float dt0f = splash::fpc::d2f(dt0);
-  void* args[] = {&GM, &S, &P, &dt0, &dt0f};
-  kp.kernelParams = args;
+  void* mixed_args[] = {&GM, &S, &P, &dt0, &dt0f};
+  void* fp64_args[] = {&G, &S, &P, &dt0};
+  kp.kernelParams = precision == SPLASH_PREC_MIXED ? mixed_args : fp64_args;
   kp.extra = nullptr;
-  SPLASH_CUDA(cudaGraphExecKernelNodeSetParams(graph_exec, dt0_node, &kp));
+  for (cudaGraphNode_t nd : dt0_nodes) SPLASH_CUDA(cudaGraphExecKernelNodeSetParams(graph_exec, nd, &kp));
   for (cudaGraphNode_t nd : dt0_nodes_k) SPLASH_CUDA(cudaGraphExecKernelNodeSetParams(graph_k_exec, nd, &kp));
   graph_dt0 = dt0;
   return SPLASH_OK;
 }
 
 int Solver::step(double dt0) {
-  if (precision == SPLASH_PREC_MIXED) {
-    const int rc = set_graph_dt0(dt0);
-    if (rc) return rc;
-  } else {
-    SPLASH_CUDA(fp64_set_dt0(S, dt0, stream));
-  }
+  const int rc = set_graph_dt0(dt0);
+  if (rc) return rc;
   SPLASH_CUDA(cudaGraphLaunch(graph_exec, stream));
   ++steps;
   return SPLASH_OK;
 }
 
 int Solver::steps_n(int n, double dt0) {
-  if (precision != SPLASH_PREC_MIXED || !graph_k_exec) {
-    for (int i = 0; i < n; ++i) {
-      const int rc = step(dt0);
-      if (rc) return rc;
-    }
-    return SPLASH_OK;
-  }
   const int rc = set_graph_dt0(dt0);
   if (rc) return rc;
   int left = n;
@@ -509,7 +466,6 @@ int splash_create(const splash_mesh_desc* mesh, const double* U_in, int dim, dou
     splash::derive_params(P);
 
     const size_t fp = (size_t)s->fpad;
-    const size_t PS = (size_t)s->max_slots * fp;
     splash::DevState& S = s->S;
     S.U = s->dalloc<double>(splash::kDim * fp);
     if (precision == SPLASH_PREC_MIXED) {
@@ -521,16 +477,17 @@ int splash_create(const splash_mesh_desc* mesh, const double* U_in, int dim, dou
       SPLASH_CUDA(cudaMemset(S.W32, 0, splash::kDim * fp * sizeof(float)));
       SPLASH_CUDA(cudaMemset(S.W32b, 0, splash::kDim * fp * sizeof(float)));
       SPLASH_CUDA(cudaMemset(S.uplus32, 0, splash::kDim * 2 * (size_t)s->GM.epad * sizeof(float)));
-      s->n_partials = 0;  // the mixed path reduces the dt candidates as keys
     } else {
       S.W0 = s->dalloc<double>(splash::kDim * fp);
       S.W1 = s->dalloc<double>(splash::kDim * fp);
       SPLASH_CUDA(cudaMemset(S.W0, 0, splash::kDim * fp * sizeof(double)));
       SPLASH_CUDA(cudaMemset(S.W1, 0, splash::kDim * fp * sizeof(double)));
-      S.uplus = s->dalloc<double>(splash::kDim * PS);
-      SPLASH_CUDA(cudaMemset(S.uplus, 0, splash::kDim * PS * sizeof(double)));
-      s->n_partials = splash::fp64_partial_blocks(s->n_faces);
-      S.partial = s->dalloc<double>((size_t)s->n_partials * splash::kPartialStride);
+      const size_t xs = (size_t)s->G.xs;
+      S.uplus = s->dalloc<double>(splash::kDim * xs);
+      SPLASH_CUDA(cudaMemset(S.uplus, 0, splash::kDim * xs * sizeof(double)));
+      S.fe = s->dalloc<double>(splash::kDim * (xs / 2));
+      S.fold = s->dalloc<unsigned long long>(splash::kFoldCount);
+      SPLASH_CUDA(cudaMemset(S.fold, 0, splash::kFoldCount * sizeof(unsigned long long)));
     }
     S.scal = s->dalloc<double>(splash::kScCount);
     S.err = s->dalloc<unsigned int>(4);
@@ -669,13 +626,12 @@ int splash_launch_times(splash_solver* h, int reps, double dt0, double* ms, int 
 int splash_memory(splash_solver* h, int64_t out[2]) {
   Solver* s = reinterpret_cast<Solver*>(h);
   if (!s || !out) return fail(SPLASH_E_INVALID, "NULL argument");
-  const size_t fp = (size_t)s->fpad, PS = (size_t)s->max_slots * fp;
+  const size_t fp = (size_t)s->fpad;
   out[0] = (int64_t)s->geometry_bytes;
   if (s->precision == SPLASH_PREC_MIXED)  // U; W32 and W32b; edge states (2 per edge); edge fluxes
     out[1] = (int64_t)(8 * splash::kDim * fp + 4 * splash::kDim * (2 * fp + 3 * (size_t)s->GM.epad));
   else
-    out[1] = (int64_t)(8 * (3 * splash::kDim * fp + splash::kDim * PS) +
-                       8 * (size_t)s->n_partials * splash::kPartialStride);
+    out[1] = (int64_t)(8 * splash::kDim * (3 * fp + 3 * (size_t)s->G.epad));  // U, W0, W1; edge states; fluxes
   return SPLASH_OK;
 }
 
@@ -849,31 +805,35 @@ int splash_write_t_curl(splash_solver* h, const char* path) {
   if (rc) return rc;
   std::vector<double> U((size_t)s->n_faces * s->dim);
   if ((rc = s->download_state(U.data()))) return rc;
-  // U_plus of the last stage, slot planes -> host
+  // U_plus of the last stage -> host, slot planes
   const size_t PS = (size_t)s->max_slots * s->fpad;
   std::vector<double> up(splash::kDim * PS);
-  if (s->S.uplus) {
-    SPLASH_CUDA(cudaMemcpy(up.data(), s->S.uplus, up.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  } else {
-    // packed FP32 edge states of the last stage, edge-major (owner side of
-    // edge e at e, reverse side at epad + e): [2 epad][4] (Sigma, l), then Pi,
-    // recomputed from the last stage-2 input (zeros before the first step,
-    // like the reference's freshly allocated U_plus)
-    const size_t ne = 2 * (size_t)s->GM.epad;
-    std::vector<float> up32(splash::kDim * ne);
-    if (s->steps > 0) SPLASH_CUDA(splash::mixed_edge_states(s->GM, s->S, s->P, s->stream));
-    SPLASH_CUDA(cudaStreamSynchronize(s->stream));
-    SPLASH_CUDA(cudaMemcpy(up32.data(), s->S.uplus32, up32.size() * sizeof(float), cudaMemcpyDeviceToHost));
+  auto from_sides = [&](size_t epad, auto&& at) {  // at(k, x): field k of side x (edge e at e, its other side at epad + e)
     for (int i = 0; i < s->n_faces; ++i) {
       const int n = s->wr_face_off[s->perm[i] + 1] - s->wr_face_off[s->perm[i]];
       for (int j = 0; j < n; ++j) {
         const size_t q = (size_t)j * s->fpad + i;
         const unsigned se = (unsigned)s->h_slot_edge[q];
-        const size_t x = (se & 0x7fffffffu) + ((se >> 31) ? (size_t)s->GM.epad : 0);
-        for (int k = 0; k < 4; ++k) up[k * PS + q] = up32[4 * x + k];
-        up[4 * PS + q] = up32[4 * ne + x];
+        const size_t x = (se & 0x7fffffffu) + ((se >> 31) ? epad : 0);
+        for (int k = 0; k < 4; ++k) up[k * PS + q] = at(k, x);
       }
     }
+  };
+  if (s->S.uplus) {
+    const size_t xs = (size_t)s->G.xs;
+    std::vector<double> u(4 * xs);
+    SPLASH_CUDA(cudaMemcpy(u.data(), s->S.uplus, u.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    from_sides(xs / 2, [&](int k, size_t x) { return u[k * xs + x]; });
+  } else {
+    // packed FP32 edge states of the last stage: [2 epad][4] (Sigma, l), then
+    // Pi, recomputed from the last stage-2 input (zeros before the first step,
+    // like the reference's freshly allocated U_plus)
+    const size_t ne = 2 * (size_t)s->GM.epad;
+    std::vector<float> up32(4 * ne);
+    if (s->steps > 0) SPLASH_CUDA(splash::mixed_edge_states(s->GM, s->S, s->P, s->stream));
+    SPLASH_CUDA(cudaStreamSynchronize(s->stream));
+    SPLASH_CUDA(cudaMemcpy(up32.data(), s->S.uplus32, up32.size() * sizeof(float), cudaMemcpyDeviceToHost));
+    from_sides(ne / 2, [&](int k, size_t x) { return (double)up32[4 * x + k]; });
   }
   double t;
   if ((rc = splash_time(h, &t))) return rc;

@@ -9,17 +9,17 @@
 namespace splash {
 
 // ---- FP64 path (step_fp64.cu) ----
-int fp64_partial_blocks(int n_faces);
-// W0 and the dt partials of the current U (after the state is set).
+// W0 and the bounds of the next dt of the current U (after the state is set).
 cudaError_t fp64_prepare(const DevGeom& G, const DevState& S, const PhysParams& P, cudaStream_t st);
-cudaError_t fp64_set_dt0(const DevState& S, double dt0, cudaStream_t st);
-// The dt clip of one step alone (first launch of fp64_step): reduces the
-// per-block partials of the current state into S.scal.
-cudaError_t fp64_dt(const DevState& S, const PhysParams& P, int n_faces, cudaStream_t st);
-// One do_step (five launches; capturable).  With `ev` non-null (6 events)
-// an event is recorded before the first and after every launch.
-cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, cudaStream_t st,
+// One do_step: four launches (edge, update per stage), the stage-1 edge
+// launch (argument dt0) clipping dt to the bounds that the previous stage-2
+// update (or fp64_prepare) made.  Capturable; the stage-1 edge node's dt0 can
+// be updated in an instantiated graph (fp64_dt0_kernel_ptr identifies the
+// node).  ev (optional): six events recorded on st (before the step, an empty
+// dt slot, after every launch).
+cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, double dt0, cudaStream_t st,
                       cudaEvent_t* ev = nullptr);
+const void* fp64_dt0_kernel_ptr(int solver);
 // reference-order [n_faces][dim] <-> internal planes (dim 5, or 4 for the
 // isothermal solver, whose fifth plane is zero); iperm[reference face] =
 // internal face.  aos may be host memory the device can access.

@@ -21,7 +21,7 @@ namespace splash {
 
 constexpr int kDim = 5;          // conserved fields: Sigma, l_x, l_y, l_z, E
 constexpr int kMaxSlots = 6;     // hexagons (pentagons and quads use fewer)
-constexpr int kPartialStride = 8;  // doubles per block partial record
+constexpr int kEdgeBlock = 64;   // edges per block of the FP64 edge launches
 
 // Physics constants of the adiabatic model (physics/adiabatic.hpp).
 struct PhysParams {
@@ -76,7 +76,38 @@ inline void derive_params(PhysParams& P) {
 
 constexpr int kSolverIsoHLLE = 4;  // the isothermal solver (4 state fields)
 
-// FP64 geometry, slot planes of length max_slots * fpad unless noted.
+// Planes of DevGeom::e_side, one value per side of an edge.  Adiabatic: the
+// interpolation weights, H+/H-, BM/H+, H+/BM, (H-/BM) / (2 N), arc / area,
+// cross(normal, centre) and round_diff * chord / area (0 on the side whose
+// face does not take this edge's flux).  Isothermal: weights, H+, H-, their
+// reciprocals, BM, H-/BM, arc / area, the normal and the straight edge length.
+enum SidePlane : int {
+  kSideBeta = 0,  // 0..3
+  kSideHr = 4,
+  kSideHg = 5,
+  kSideEtaP = 6,
+  kSideSbs = 7,
+  kSideArc = 8,
+  kSideNxr = 9,   // 9..11
+  kSideCoef = 12,
+  kSidePlanes = 13,
+  kIsoHp = 4,
+  kIsoHm = 5,
+  kIsoRhp = 6,
+  kIsoRhm = 7,
+  kIsoArc = 8,
+  kIsoEn = 9,     // 9..11
+  kIsoChord = 12,
+  kIsoBm = 13,
+  kIsoEta = 14,
+  kIsoPlanes = 15
+};
+
+// FP64 geometry.  The step works on interior edges: one thread per side (the
+// slot of one of the edge's two faces) reconstructs that side's edge state,
+// one thread per edge evaluates the flux, in the orientation of side 0.
+// Side arrays have length xs = 2 epad: side 0 of edge e at e, side 1 at
+// epad + e.  Edges are numbered face-major (owner face, then slot).
 struct DevGeom {
   int n_faces;
   int fpad;
@@ -86,23 +117,27 @@ struct DevGeom {
   const double* fcn;      // unit face centre, 3 planes of fpad (x | y | z)
   const double* area;     // spherical excess
   const double* acc_src;  // accretion mass source res[0] (0 when accretion is off)
-  // per slot
-  const int* sten;        // 4 planes: flux_faces_plus[0..1], flux_faces_minus[0..1] (internal ids)
+  // edges
+  int n_edges;
+  int epad;               // n_edges rounded up to the edges of a block
+  int xs;                 // 2 epad
+  const int* slot_edge;   // per slot (slot planes): its edge, bit 31 set where the slot is side 1
+  const int* e_face;      // [xs] the side's face
+  const int* e_sten;      // 4 planes of xs: flux_faces_plus[0..1], flux_faces_minus[0..1] (internal ids)
+  const double* e_side;   // SidePlane planes of xs
+  const int* e_twin;      // null, or on a mesh with one edge per slot (make_edge_planes): the edge whose side 0 is
+                          // the same slot as side 1 of edge e
+  const double* e_geo;    // planes of epad: unit edge centre (3), side 0's outward normal (3), |centre| as evaluated
+  // per slot, slot planes: for the evaluation of single faces on the host
+  const int* sten;        // 4 planes
   const double* beta;     // 4 planes: betas_plus[0..1], betas_minus[0..1]
   const double* hpm;      // 2 planes: H_plus, H_minus
   const double* bm;       // BM_dist
   const double* eta;      // 2 planes: H_plus/BM, H_minus/BM
-  const double* hr;       // H_plus / H_minus
-  const double* hg;       // BM / H_plus
-  const double* sbs;      // (H_minus/BM) / (2 N): the superbee scale before the Courant factor
   const double* arc_a;    // great-circle edge length / face area (limiter Courant factor)
   const double* ec;       // 3 planes: unit edge centre
   const double* ecn;      // |ec| as evaluated in double
   const double* en;       // 3 planes: outward edge normal
-  const double* nxr;      // 3 planes: cross(en, ec/|ec|)
-  const double* chord;    // straight edge length
-  const double* coef;     // round_diff * chord / area
-  const int* rev;         // slot-plane index of the same edge seen from the neighbour
 };
 
 // Geometry of the FP32/FP64 mixed path: FP32 slot planes, FP64 where the
@@ -137,14 +172,15 @@ struct DevState {
   double* U;      // conserved state, kDim planes of fpad
   double* W0;     // (Sigma, l, Pi) of U, kDim planes
   double* W1;     // (Sigma, l, Pi) after stage 1, kDim planes
-  double* uplus;  // reconstructed edge states, kDim * max_slots planes of fpad
+  double* uplus;  // the last stage-2 edge states (Sigma, l, Pi), kDim planes of xs
+  double* fe;     // Riemann flux of every edge, kDim planes of epad
+  unsigned long long* fold;  // FP64 path: the candidates of the next dt, see FoldSlot
   float* W32;     // mixed path: stage-1 input (Sigma, l, Pi) in FP32: [fpad] float4 (Sigma, l), then a Pi plane
   float* W32b;    // mixed path: stage-2 input, the same layout (written by the stage-1 update)
   float* uplus32; // mixed path: the last stage-2 edge states, packed like W32 over 2 * epad entries
                   // (owner side of edge e at e, reverse side at epad + e), recomputed for the
                   // writers (mixed_edge_states); may be null
   float* fe32;    // mixed path: FP32 Riemann flux of every edge, packed like W32 over epad edges
-  double* partial;  // per-block partial records (kPartialStride doubles)
   double* scal;   // device scalars, see ScalarSlot
   unsigned int* err;  // stop bits
   unsigned* keys;  // mixed path: [0] max |v|^2 key, [1] min signed-square extra-dt key (FP32 order keys)
@@ -159,13 +195,24 @@ struct EnsInstance {
   PhysParams P;
 };
 
+// The FP64 path's dt candidates, folded as integers (the bit patterns of
+// non-negative doubles order like the doubles).
+enum FoldSlot : int {
+  kFoldVel2 = 0,   // max of |v|^2 and the squared sound speed
+  kFoldRate2 = 1,  // max squared reciprocal of the extra dt, but for a constant factor
+  kFoldNeg = 2,    // 1 where some face's extra dt is negative
+  kFoldDone = 3,   // blocks that have folded
+  kFoldCount = 4
+};
+
 enum ScalarSlot : int {
   kScDt = 0,       // dt of the current step (clipped)
   kScTime = 1,     // simulation time after the current step
   kScMaxVel = 2,   // max_vel of the step's input state
   kScExtraDt = 3,  // extra_dt_constr of the step's input state
-  kScMass = 4,     // 4..8: sum Sigma A, l_x A, l_y A, l_z A, E A of the step's input state
-  kScDt0 = 9,      // dt0 requested by the caller
+  kScBound = 4,    // FP64 path: min(CFL bound, extra dt) of the current state
+  kScNegExtra = 5, // FP64 path: 1 if the current state's extra dt is negative
+  kScDt0 = 9,      // mixed path: dt0 requested by the caller
   kScDtF = 10,     // mixed path: (float dt, float dt/2) packed in one slot
   kScDtHalf = 11,  // mixed path: dt / 2 (FP64)
   kScCount = 16

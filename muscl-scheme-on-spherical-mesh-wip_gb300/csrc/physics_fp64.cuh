@@ -43,13 +43,6 @@ template <class T, class S>
 SPLASH_HD auto scal(const V3<T>& a, const S& s) -> V3<wider_t<T, S>> {
   return V3<wider_t<T, S>>{a.x * s, a.y * s, a.z * s};
 }
-// vec3d.hpp:56-64 : sqrt(((0 + x^2) + y^2) + z^2)
-SPLASH_HD double norm3(const D3& a) {
-  double s = a.x * a.x;
-  s = s + a.y * a.y;
-  s = s + a.z * a.z;
-  return sqrt(s);
-}
 template <class A, class B>
 SPLASH_HD auto cross3(const V3<A>& a, const V3<B>& b) -> V3<wider_t<A, B>> {
   return V3<wider_t<A, B>>{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
@@ -348,6 +341,31 @@ SPLASH_HD void dt_candidates(const double* u, D3 r, double area, const PhysParam
   dmin = 0.01 * p / (P.alpha * P.fric_k * g_eff * u[0] * root(fdot(rel, rel)));
 #pragma unroll
   for (int k = 0; k < 5; ++k) sums[k] = u[k] * area;
+}
+
+// The candidates of one face for the next dt in the form in which they are
+// folded (FoldSlot): the larger of |v|^2 and the squared sound speed, and
+// rate2 = (g_eff Sigma |v - v0| / Pi)^2, the squared reciprocal of the extra
+// dt 0.01 Pi / (alpha fric_k g_eff Sigma |v - v0|) but for the constant factor
+// (no root and no quotient but 1 / Sigma and 1 / Pi per face).  `negative`
+// reports a negative extra dt; NaN candidates are 0, like the reference's
+// comparisons skip them.  w holds (Sigma, l, Pi).
+SPLASH_HD void dt_fold(const double* w, const D3& r, const PhysParams& P, double& vel2, double& rate2,
+                       bool& negative) {
+  const double ir = recip(w[0]);
+  const D3 vel = scal(fcross(r, d3(w[1], w[2], w[3])), -ir);
+  const double v2 = fdot(vel, vel);
+  const double a2 = P.gam * (w[4] * ir);
+  const D3 rel = d3(fma(P.omega_ns, r.y, vel.x), fma(-P.omega_ns, r.x, vel.y), vel.z);
+  const double n2 = fdot(rel, rel);
+  const double GM = 0.217909;
+  const double t = (GM - v2) * w[0] * recip(w[4]);
+  vel2 = 0.0;
+  if (!nan_bits(v2)) vel2 = v2;
+  if (not_below_zero(a2) && less_pos(vel2, a2)) vel2 = a2;
+  rate2 = t * t * n2;
+  negative = below_zero(t) && !nan_bits(n2);
+  if (nan_bits(rate2)) rate2 = 0.0;
 }
 
 // The parameters of the source term that the derivative kernels

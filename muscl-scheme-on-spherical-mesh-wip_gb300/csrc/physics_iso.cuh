@@ -2,9 +2,10 @@
 // Sigma, l_x, l_y, l_z; pressure a^2 Sigma with a = 1).
 //
 // Each function restates one reference function with the reference's
-// operation order, divisions included (this path has no transcendental, so
-// exact IEEE division costs little), so that the FP64 kernels reproduce the
-// CPU restatement bit for bit.  The reference's isothermal limiter reads an
+// operation order, and quotients are rounded as the operator rounds them
+// (fp64_math.cuh: a reciprocal per divisor, Markstein's correction per
+// quotient), so that the FP64 kernels reproduce the CPU restatement bit for
+// bit.  The reference's isothermal limiter reads an
 // uninitialised etha_minus (physics/isothermal.hpp:272, 307); it is taken as
 // H_minus / BM_dist (its value in the adiabatic superbee), and etha_plus keeps
 // its value as written (H_minus / BM_dist, isothermal.hpp:301-302).
@@ -20,14 +21,16 @@ using f64::D3;
 using f64::cross3;
 using f64::d3;
 using f64::dot3;
-using f64::norm3;
 using f64::smax;
 using f64::smin;
 
 constexpr int kIsoDim = 4;
 constexpr double kA = 1;  // isothermal sound speed (isothermal.hpp:138)
 
-SPLASH_HD D3 div3(const D3& a, double s) { return D3{a.x / s, a.y / s, a.z / s}; }
+SPLASH_HD D3 div3(const D3& a, double s) {
+  const double y = f64::recip(s);
+  return D3{f64::quotient(a.x, s, y), f64::quotient(a.y, s, y), f64::quotient(a.z, s, y)};
+}
 
 // physics/isothermal.hpp:141-195 ; ec is the unit edge centre
 SPLASH_HD void flux(const double* u, const D3& ec, const D3& en, double* res) {
@@ -60,27 +63,34 @@ SPLASH_HD unsigned flux_star(const double* uL, const double* uR, const D3& ec, d
   char_vel(uL, uR, ec, ecn, en, S_L, S_R);
   flux(uL, ec, en, FL);
   flux(uR, ec, en, FR);
-  unsigned bits = (is_nan(S_L) || is_nan(S_R)) ? 2u : 0u;
-  if (S_L >= 0) {
+  unsigned bits = (f64::nan_bits(S_L) || f64::nan_bits(S_R)) ? 2u : 0u;
+  if (f64::not_below_zero(S_L)) {
 #pragma unroll
     for (int i = 0; i < kIsoDim; ++i) F[i] = FL[i];
-  } else if (S_L < 0 && S_R > 0) {
+  } else if (f64::below_zero(S_L) && f64::below_zero(-S_R)) {
+    const double d = S_R - S_L, y = f64::recip(d);
 #pragma unroll
-    for (int i = 0; i < kIsoDim; ++i) F[i] = (S_R * FL[i] - S_L * FR[i] + S_R * S_L * (uR[i] - uL[i])) / (S_R - S_L);
+    for (int i = 0; i < kIsoDim; ++i)
+      F[i] = f64::quotient(S_R * FL[i] - S_L * FR[i] + S_R * S_L * (uR[i] - uL[i]), d, y);
   } else {
-    if (!(S_R <= 0)) bits |= 4u;
+    if (!f64::not_below_zero(-S_R)) bits |= 4u;
 #pragma unroll
     for (int i = 0; i < kIsoDim; ++i) F[i] = FR[i];
   }
   return bits;
 }
 
-// physics/isothermal.hpp:269-320 for one field, given the slot's Courant
+// physics/isothermal.hpp:269-320 for one field, given the side's Courant
 // factor nu_plus, eta = H_minus / BM_dist and 2 N (N the face's edge count)
-SPLASH_HD double limiter_field(double r, double eta, double twoN, double nu_plus) {
-  if (is_nan(r)) return 0.;
-  return smax(0., smax(smin(1., eta * r * 2 / (twoN * nu_plus)), smin(r, eta)));
-}
+struct Limiter {
+  double eta, den, y;  // the quotients' divisor 2 N nu_plus and its reciprocal
+  SPLASH_HD Limiter(double eta_, double twoN, double nu_plus)
+      : eta(eta_), den(twoN * nu_plus), y(f64::recip(den)) {}
+  SPLASH_HD double operator()(double r) const {
+    if (f64::nan_bits(r)) return 0.;
+    return smax(0., smax(smin(1., f64::quotient(eta * r * 2, den, y)), smin(r, eta)));
+  }
+};
 
 // Courant factor of the isothermal limiter: (a + v.n) dt arc / area with
 // v = cross(ec, l) / (-Sigma) of the face state w
@@ -89,17 +99,15 @@ SPLASH_HD double courant(const double* w, const D3& ec, const D3& en, double dt,
   return (kA + dot3(vel, en)) * dt * arc_a;
 }
 
-// find_v_max (MUSCL_base.hpp:311-343) of a 4-field state: the CFL speed is
-// max(|v|, a) (the reference reads a fifth field for the sound speed); the
-// extra constraint is 1e20 (isothermal.hpp:262-267).
-SPLASH_HD void dt_candidates(const double* u, const D3& r, double area, double& vmax, double& dmin,
-                             double sums[5]) {
-  const D3 vel = div3(cross3(r, d3(u[1], u[2], u[3])), u[0]);
-  vmax = fmax(norm3(vel), kA);
-  dmin = 1e20;
-#pragma unroll
-  for (int k = 0; k < kIsoDim; ++k) sums[k] = u[k] * area;
-  sums[4] = 0.0;
+// The squared CFL speed max(|v|, a)^2 of a 4-field state (find_v_max,
+// MUSCL_base.hpp:311-343; the reference reads a fifth field for the sound
+// speed).  The extra constraint is 1e20 (isothermal.hpp:262-267).
+SPLASH_HD double dt_fold(const double* u, const D3& r) {
+  const D3 v = div3(cross3(r, d3(u[1], u[2], u[3])), u[0]);
+  double s = v.x * v.x;
+  s = s + v.y * v.y;
+  s = s + v.z * v.z;
+  return f64::less(kA * kA, s) ? s : kA * kA;
 }
 
 }  // namespace iso

@@ -1,10 +1,13 @@
-// Deterministic block reduction of the per-block partial records used by
-// the dt clip and the diagnostics sums (shared by both precision paths).
+// Deterministic block reduction of the per-block partial records of the
+// allocation-free dt clip (cfl_noalloc.cu).
 #pragma once
 
 #include "layout.hpp"
 
 namespace splash {
+
+constexpr int kPartialStride = 8;  // doubles per block partial record
+
 namespace red {
 
 // Warp + block reduction of one partial record; thread 0 of the block

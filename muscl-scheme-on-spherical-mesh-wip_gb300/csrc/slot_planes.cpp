@@ -7,6 +7,7 @@
 #include <stdexcept>
 
 #include "hilbert.hpp"
+#include "layout.hpp"
 
 namespace splash {
 
@@ -68,22 +69,18 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
   sp.nslots.assign(fpad, 0);
   sp.fcn.assign(3 * (size_t)fpad, 0.0);
   sp.area.assign(fpad, 1.0);
-  sp.sten.assign(4 * PS, 0);
-  sp.rev.assign(PS, 0);
-  sp.beta.assign(4 * PS, 0.0);
-  sp.hpm.assign(2 * PS, 1.0);
-  sp.bm.assign(PS, 1.0);
-  sp.eta.assign(2 * PS, 1.0);
-  sp.arc.assign(PS, 0.0);
-  sp.ec.assign(3 * PS, 0.0);
-  sp.ecn.assign(PS, 1.0);
-  sp.en.assign(3 * PS, 0.0);
-  sp.nxr.assign(3 * PS, 0.0);
-  sp.chord.assign(PS, 0.0);
-  sp.hr.assign(PS, 1.0);
-  sp.hg.assign(PS, 1.0);
-  sp.sbs.assign(PS, 0.0);
-  sp.coef.assign(PS, 0.0);
+  sp.sten.resize(4 * PS);
+  sp.rev.resize(PS);
+  sp.beta.resize(4 * PS);
+  sp.hpm.resize(2 * PS);
+  sp.bm.resize(PS);
+  sp.eta.resize(2 * PS);
+  sp.arc.resize(PS);
+  sp.ec.resize(3 * PS);
+  sp.ecn.resize(PS);
+  sp.en.resize(3 * PS);
+  sp.nxr.resize(3 * PS);
+  sp.chord.resize(PS);
 
   // every face writes only its own entries: the fill is order-independent
 #pragma omp parallel for schedule(static)
@@ -113,9 +110,6 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
       sp.bm[s] = g.bm_dist[sr];
       sp.eta[s] = g.h_plus[sr] / g.bm_dist[sr];
       sp.eta[PS + s] = g.h_minus[sr] / g.bm_dist[sr];
-      sp.hr[s] = sp.hpm[s] / sp.hpm[PS + s];
-      sp.hg[s] = sp.bm[s] / sp.hpm[s];
-      sp.sbs[s] = sp.eta[PS + s] / (2 * n);
       const int va = g.face_vtx[sr];
       const int vb = g.face_vtx[g.face_off[r] + ((j + 1 == n) ? 0 : j + 1)];
       const V3 A = at3(g.vertices, va), B = at3(g.vertices, vb);
@@ -138,10 +132,6 @@ SlotPlanes make_slot_planes(const RefGeometry& g) {
       sp.nxr[PS + s] = nxr.y;
       sp.nxr[2 * PS + s] = nxr.z;
       sp.chord[s] = vnorm(vsub(A, B));
-      {  // round_diff * chord / area with one rounding (the product's error and the quotient's remainder put back)
-        const double p = sp.round_diff * sp.chord[s], q = p / sp.area[i];
-        sp.coef[s] = q + (std::fma(-q, sp.area[i], p) + std::fma(sp.round_diff, sp.chord[s], -p)) / sp.area[i];
-      }
       sp.rev[s] = j0_of[sr] * fpad + iperm[g.nbr_edge[sr]];
     }
     // unused slots of low-valence faces point at themselves (never read)
@@ -202,20 +192,9 @@ std::vector<double> accretion_source_fcn(const std::vector<double>& fcn, int n_f
   return acc;
 }
 
-MixedPlanes make_mixed_planes(const SlotPlanes& sp) {
-  MixedPlanes mp;
+EdgeList make_edge_list(const SlotPlanes& sp) {
+  EdgeList el;
   const size_t PS = sp.PS();
-  mp.fcn32.assign(sp.fcn.begin(), sp.fcn.end());
-  mp.fcn_lo.resize(sp.fcn.size());
-  for (size_t i = 0; i < sp.fcn.size(); ++i) mp.fcn_lo[i] = (float)(sp.fcn[i] - (double)mp.fcn32[i]);
-  mp.coef.assign(PS, 0.0f);
-#pragma omp parallel for schedule(static)
-  for (int i = 0; i < sp.n_faces; ++i)
-    for (int j = 0; j < (int)sp.nslots[i]; ++j) {
-      const size_t q = (size_t)j * sp.fpad + i;
-      mp.coef[q] = (float)(sp.round_diff * sp.chord[q] / sp.area[i]);
-    }
-  if (sp.n_faces >= (1 << 28)) throw std::runtime_error("too many faces for the edge records");
   // Owner slots: of the two slots of an edge, the one with the smaller
   // slot-plane index.  Edge e is the e-th owner slot in the visiting order
   // below, its index an exclusive prefix sum of the owner flags.
@@ -250,9 +229,10 @@ MixedPlanes make_mixed_planes(const SlotPlanes& sp) {
     base[c + 1] = cnt;
   }
   for (long long c = 0; c < nchunk; ++c) base[c + 1] += base[c];
-  mp.n_edges = (int)base[nchunk];
-  std::vector<int> own(mp.n_edges), nbr(mp.n_edges);
-  mp.slot_edge.assign(PS, 0);
+  el.n_edges = (int)base[nchunk];
+  el.own.resize(el.n_edges);
+  el.nbr.resize(el.n_edges);
+  el.slot_edge.assign(PS, 0);
 #pragma omp parallel for schedule(static)
   for (long long c = 0; c < nchunk; ++c) {
     long long e = base[c];
@@ -260,13 +240,117 @@ MixedPlanes make_mixed_planes(const SlotPlanes& sp) {
       visit(v, [&](long long q) {
         if (!is_own[q]) return;
         const int r = sp.rev[q];
-        own[e] = (int)q;
-        nbr[e] = r;
-        mp.slot_edge[q] = (int)e;
-        mp.slot_edge[r] = (int)((unsigned)e | 0x80000000u);
+        el.own[e] = (int)q;
+        el.nbr[e] = r;
+        el.slot_edge[q] = (int)e;
+        el.slot_edge[r] = (int)((unsigned)e | 0x80000000u);
         ++e;
       });
   }
+  return el;
+}
+
+EdgePlanes make_edge_planes(const SlotPlanes& sp, bool isothermal) {
+  EdgePlanes ep;
+  const size_t PS = sp.PS();
+  bool paired = true;
+#pragma omp parallel for schedule(static) reduction(&& : paired)
+  for (int i = 0; i < sp.n_faces; ++i)
+    for (int j = 0; j < (int)sp.nslots[i]; ++j) {
+      const size_t q = (size_t)j * sp.fpad + i, r = (size_t)sp.rev[q];
+      bool ok = r != q && (size_t)sp.rev[r] == q;
+      for (size_t c = 0; c < 3; ++c)
+        ok = ok && sp.en[c * PS + q] == -sp.en[c * PS + r] && sp.ec[c * PS + q] == sp.ec[c * PS + r];
+      paired = paired && ok;
+    }
+  EdgeList el;
+  if (paired) {
+    el = make_edge_list(sp);
+  } else {
+    el.slot_edge.assign(PS, 0);
+    for (int i = 0; i < sp.n_faces; ++i)
+      for (int j = 0; j < (int)sp.nslots[i]; ++j) {
+        const size_t q = (size_t)j * sp.fpad + i;
+        el.slot_edge[q] = (int)el.own.size();
+        el.own.push_back((int)q);
+        el.nbr.push_back(sp.rev[q]);
+      }
+    el.n_edges = (int)el.own.size();
+    for (int q : el.nbr) ep.twin.push_back(el.slot_edge[q]);
+  }
+  const int ne = ep.n_edges = el.n_edges;
+  const size_t pad = ep.epad = (ne + kEdgeBlock - 1) / kEdgeBlock * kEdgeBlock, xs = 2 * pad;
+  if (xs >= (size_t)1 << 28) throw std::runtime_error("too many edges");
+  ep.slot_edge = std::move(el.slot_edge);
+  ep.face.resize(xs);
+  ep.sten.resize(4 * xs);
+  ep.side.resize((size_t)(isothermal ? kIsoPlanes : kSidePlanes) * xs);
+  ep.geo.resize(7 * pad);
+#pragma omp parallel for schedule(static)
+  for (int e = 0; e < ne; ++e) {
+    const size_t so = (size_t)el.own[e];
+    for (size_t c = 0; c < 3; ++c) {
+      ep.geo[c * pad + e] = sp.ec[c * PS + so];
+      ep.geo[(3 + c) * pad + e] = sp.en[c * PS + so];
+    }
+    ep.geo[6 * pad + e] = sp.ecn[so];
+    for (int k = 0; k < 2; ++k) {
+      const size_t q = k ? (size_t)el.nbr[e] : so, x = k * pad + e;
+      const int f = (int)(q % sp.fpad);
+      double* s = &ep.side[x];
+      auto put = [&](int plane, double v) { s[(size_t)plane * xs] = v; };
+      ep.face[x] = f;
+      for (size_t c = 0; c < 4; ++c) {
+        ep.sten[c * xs + x] = sp.sten[c * PS + q];
+        put(kSideBeta + (int)c, sp.beta[c * PS + q]);
+      }
+      const double hp = sp.hpm[q], hm = sp.hpm[PS + q];
+      if (isothermal) {
+        put(kIsoHp, hp);
+        put(kIsoHm, hm);
+        put(kIsoRhp, 1.0 / hp);
+        put(kIsoRhm, 1.0 / hm);
+        put(kIsoArc, sp.arc[q]);
+        for (int c = 0; c < 3; ++c) put(kIsoEn + c, sp.en[c * PS + q]);
+        put(kIsoChord, sp.chord[q]);
+        put(kIsoBm, sp.bm[q]);
+        put(kIsoEta, sp.eta[PS + q]);
+        continue;
+      }
+      put(kSideHr, hp / hm);
+      put(kSideHg, sp.bm[q] / hp);
+      put(kSideEtaP, sp.eta[q]);
+      put(kSideSbs, sp.eta[PS + q] / (2 * sp.nslots[f]));
+      put(kSideArc, sp.arc[q]);
+      for (int c = 0; c < 3; ++c) put(kSideNxr + c, sp.nxr[c * PS + q]);
+      // round_diff * chord / area with one rounding (the product's error and
+      // the quotient's remainder put back)
+      const double a = sp.area[f], p = sp.round_diff * sp.chord[q], c0 = p / a;
+      const double coef = c0 + (std::fma(-c0, a, p) + std::fma(sp.round_diff, sp.chord[q], -p)) / a;
+      put(kSideCoef, (k == 0 || paired) ? coef : 0.0);
+    }
+  }
+  return ep;
+}
+
+MixedPlanes make_mixed_planes(const SlotPlanes& sp) {
+  MixedPlanes mp;
+  const size_t PS = sp.PS();
+  mp.fcn32.assign(sp.fcn.begin(), sp.fcn.end());
+  mp.fcn_lo.resize(sp.fcn.size());
+  for (size_t i = 0; i < sp.fcn.size(); ++i) mp.fcn_lo[i] = (float)(sp.fcn[i] - (double)mp.fcn32[i]);
+  mp.coef.assign(PS, 0.0f);
+#pragma omp parallel for schedule(static)
+  for (int i = 0; i < sp.n_faces; ++i)
+    for (int j = 0; j < (int)sp.nslots[i]; ++j) {
+      const size_t q = (size_t)j * sp.fpad + i;
+      mp.coef[q] = (float)(sp.round_diff * sp.chord[q] / sp.area[i]);
+    }
+  if (sp.n_faces >= (1 << 28)) throw std::runtime_error("too many faces for the edge records");
+  const EdgeList el = make_edge_list(sp);
+  const std::vector<int>&own = el.own, &nbr = el.nbr;
+  mp.n_edges = el.n_edges;
+  mp.slot_edge = el.slot_edge;
   const int ep = mp.epad = (mp.n_edges + 31) / 32 * 32;
   mp.e_ids.assign(4 * (size_t)ep, 0);
   mp.e_ec.assign(4 * (size_t)ep, 0.f);

@@ -4,12 +4,35 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
+#include <new>
+#include <utility>
 #include <vector>
 
 #include "geometry.hpp"
 #include "splash_gb300.h"
 
 namespace splash {
+
+// A vector whose resize leaves new elements uninitialised, so that the
+// parallel loop that fills a plane is the first to touch it.
+template <class T>
+struct RawAllocator : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = RawAllocator<U>;
+  };
+  template <class U>
+  void construct(U* p) {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <class U, class... A>
+  void construct(U* p, A&&... a) {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+  }
+};
+template <class T>
+using RawVector = std::vector<T, RawAllocator<T>>;
 
 struct SlotPlanes {
   int n_faces = 0, fpad = 0, max_slots = 0;
@@ -18,13 +41,13 @@ struct SlotPlanes {
   std::vector<int8_t> nslots;
   std::vector<double> fcn;   // 3 planes
   std::vector<double> area;
-  // per slot [max_slots * fpad] (x planes)
-  std::vector<int> sten;     // 4 planes, internal ids
-  std::vector<int> rev;      // slot-plane index of the reverse slot
-  std::vector<double> beta;  // 4 planes
-  std::vector<double> hpm;   // 2 planes
-  std::vector<double> bm, eta /*2 planes*/, arc, ec /*3*/, ecn, en /*3*/, nxr /*3*/, chord;
-  std::vector<double> hr, hg, sbs, coef;  // H+/H-, BM/H+, (H-/BM) / (2 N), round_diff * chord / area
+  // per slot [max_slots * fpad] (x planes); the entries of a face's unused
+  // slots and of the padding hold nothing, but for sten and rev
+  RawVector<int> sten;     // 4 planes, internal ids
+  RawVector<int> rev;      // slot-plane index of the reverse slot
+  RawVector<double> beta;  // 4 planes
+  RawVector<double> hpm;   // 2 planes
+  RawVector<double> bm, eta /*2 planes*/, arc, ec /*3*/, ecn, en /*3*/, nxr /*3*/, chord;
   double round_diff = 0.0;
   size_t PS() const { return (size_t)max_slots * fpad; }
 };
@@ -47,6 +70,30 @@ std::vector<double> accretion_source_fcn(const std::vector<double>& fcn, int n_f
                                          const splash_params& par, double area_coeff, bool accretion_on,
                                          std::vector<double>* d_rate = nullptr,
                                          std::vector<double>* d_tilt = nullptr);
+
+// The interior edges: each once, its owner slot (the one with the smaller
+// slot-plane index) and the slot of its other side.  Edges are numbered
+// face-major; slot_edge maps every slot to its edge, with bit 31 set where
+// the slot is the other side.
+struct EdgeList {
+  int n_edges = 0;
+  std::vector<int> own, nbr;   // [n_edges] slot-plane indices
+  std::vector<int> slot_edge;  // [max_slots * fpad]
+};
+EdgeList make_edge_list(const SlotPlanes& sp);
+
+// Edge and side planes of the FP64 path (DevGeom).  A mesh whose reverse
+// slots do not pair up, or whose two normals of an edge are not exactly
+// opposite, gets one edge per slot, whose flux only that slot's face takes:
+// every face then sees the flux of its own side, as in the reference.
+struct EdgePlanes {
+  int n_edges = 0, epad = 0;
+  std::vector<int> slot_edge;
+  std::vector<int> twin;  // one edge per slot: the edge of every edge's reverse slot
+  RawVector<int> face, sten;
+  RawVector<double> side, geo;
+};
+EdgePlanes make_edge_planes(const SlotPlanes& sp, bool isothermal);
 
 // FP32 planes of the mixed path.  The mixed step works per interior edge:
 // one thread reconstructs the edge states of the edge's two slots (owner:

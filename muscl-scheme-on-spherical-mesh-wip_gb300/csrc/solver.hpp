@@ -35,12 +35,11 @@ struct Solver {
   int n_faces = 0;
   int fpad = 0;
   int max_slots = 0;
-  int n_partials = 0;
   size_t geometry_bytes = 0;
 
   // numbering: perm[internal] = reference face id, iperm = inverse
   std::vector<int> perm, iperm;
-  std::vector<int> h_slot_edge;  // mixed path: slot -> edge map (the writers' edge-state lookup)
+  std::vector<int> h_slot_edge;  // slot -> edge map (the writers' edge-state lookup)
 
   // reference-order host copies used by the writers
   std::vector<double> wr_vertices, wr_face_centers, wr_area;
@@ -66,11 +65,11 @@ struct Solver {
   std::vector<void*> dev_allocs;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
-  cudaGraphNode_t dt0_node = nullptr;  // mixed path: the stage-1 edge node taking dt0
-  double graph_dt0 = 0.0;              // dt0 the instantiated graphs currently use
-  // mixed path: kGraphSteps consecutive steps in one graph, so that each
-  // step's first launch overlaps the previous step's last one (programmatic
-  // dependent launch works within a graph, not across graph launches)
+  std::vector<cudaGraphNode_t> dt0_nodes;  // the stage-1 edge node, which takes dt0
+  double graph_dt0 = 0.0;                  // dt0 the instantiated graphs currently use
+  // kGraphSteps consecutive steps in one graph, so that each step's first
+  // launch overlaps the previous step's last one (programmatic dependent
+  // launch works within a graph, not across graph launches)
   static constexpr int kGraphSteps = 4;
   cudaGraph_t graph_k = nullptr;
   cudaGraphExec_t graph_k_exec = nullptr;
@@ -81,21 +80,22 @@ struct Solver {
 
   template <typename T>
   T* dalloc(size_t n);
-  template <typename T>
-  T* upload(const std::vector<T>& h);
+  template <typename T, typename A>
+  T* upload(const std::vector<T, A>& h);
 
   void build_device_geometry(const RefGeometry& g);
   int upload_state(const double* U_ref);
   int download_state(double* U_ref);
   int read_scalars(double* out);
   int capture_graph();
-  int set_graph_dt0(double dt0);  // mixed path: rewrite dt0 in the instantiated graphs
+  int capture_steps(int n_steps, cudaGraph_t* g, cudaGraphExec_t* exec, std::vector<cudaGraphNode_t>* dt0_nodes);
+  int set_graph_dt0(double dt0);  // rewrites dt0 in the instantiated graphs
   int steps_n(int n, double dt0);  // n steps (K-step graphs where they fit)
   int step(double dt0);
   // one un-captured step; ev as for mixed_step (six events, five slots on
   // both paths)
   cudaError_t launch_step(cudaEvent_t* ev, double dt0, bool per_launch = false);
-  int launches_per_step() const { return 5; }  // timing slots (the mixed step launches 4 kernels)
+  int launches_per_step() const { return 5; }  // timing slots (a step launches 4 kernels; the dt slot is empty)
   cudaError_t launch_prepare();
   static int check_cuda(cudaError_t e, const char* what);
 };

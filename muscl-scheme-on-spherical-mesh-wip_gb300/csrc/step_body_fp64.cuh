@@ -73,21 +73,31 @@ struct SideGeom {
   double b0, b1, b2, b3, hr, hg, eta_p, sbs, arc_a;
   D3 nxr;
 };
-// ... from the planes of the slots (stride PS), at index s, of a face of n edges
-SPLASH_HD SideGeom side_geom(const DevGeom& G, int PS, int s, int n) {
+// ... of side x (DevGeom::e_side)
+SPLASH_HD SideGeom side_geom(const DevGeom& G, int x) {
+  const size_t xs = (size_t)G.xs;
+  const double* p = G.e_side + x;
+  SideGeom c;
+  c.b0 = p[kSideBeta * xs];
+  c.b1 = p[(kSideBeta + 1) * xs];
+  c.b2 = p[(kSideBeta + 2) * xs];
+  c.b3 = p[(kSideBeta + 3) * xs];
+  c.hr = p[kSideHr * xs];
+  c.hg = p[kSideHg * xs];
+  c.eta_p = p[kSideEtaP * xs];
+  c.sbs = p[kSideSbs * xs];
+  c.arc_a = p[kSideArc * xs];
+  c.nxr = D3{p[kSideNxr * xs], p[(kSideNxr + 1) * xs], p[(kSideNxr + 2) * xs]};
+  return c;
+}
+// ... from the slot planes (stride PS), at index s, of a face of n edges
+SPLASH_HD SideGeom slot_geom(const DevGeom& G, int PS, int s, int n) {
   SideGeom c;
   c.b0 = G.beta[s];
   c.b1 = G.beta[PS + s];
   c.b2 = G.beta[2 * PS + s];
   c.b3 = G.beta[3 * PS + s];
   c.arc_a = G.arc_a[s];
-#if defined(__CUDA_ARCH__)
-  c.hr = G.hr[s];
-  c.hg = G.hg[s];
-  c.eta_p = G.eta[s];
-  c.sbs = G.sbs[s];
-  c.nxr = plane3(G.nxr, PS, s);
-#else
   c.hr = G.hpm[s] / G.hpm[PS + s];
   c.hg = G.bm[s] / G.hpm[s];
   c.eta_p = G.eta[s];
@@ -95,8 +105,13 @@ SPLASH_HD SideGeom side_geom(const DevGeom& G, int PS, int s, int n) {
   const D3 ec = plane3(G.ec, PS, s), en = plane3(G.en, PS, s);
   const double ecn = G.ecn[s];
   c.nxr = cross3(en, d3(ec.x / ecn, ec.y / ecn, ec.z / ecn));
-#endif
   return c;
+}
+// The edge as the flux sees it, in the orientation of side 0
+SPLASH_HD EdgeGeom edge_geom(const DevGeom& G, int e) {
+  const size_t ep = (size_t)G.epad, xs = (size_t)G.xs;
+  const double *p = G.e_geo + e, *q = G.e_side + kSideNxr * xs + e;
+  return EdgeGeom{D3{p[0], p[ep], p[2 * ep]}, D3{p[3 * ep], p[4 * ep], p[5 * ep]}, D3{q[0], q[xs], q[2 * xs]}};
 }
 
 // Courant factor of the limiter (adiabatic.hpp:741-758, 792-810) of the
@@ -129,7 +144,7 @@ SPLASH_HD T slope_ratio(const SideGeom& g, const T& dp, const T& dm) {
   const T num = dm * g.hr;
   const double y = recip(val(dp));
   double v = val(num) * y;
-  if (odd_bits(v)) v = val(num) / val(dp);
+  if (odd_bits(v)) v = exact_quotient(val(num), val(dp));
   T r(v);
   if constexpr (is_dual<T>::value) {
 #pragma unroll
@@ -159,7 +174,8 @@ SPLASH_HD void recon_side(const SideGeom& g, double gam, double dt, const T* w, 
   }
 }
 
-// find_U_edges for every slot of face f: the edge states (Sigma, l, Pi)
+// find_U_edges for every slot of face f from the slot planes: the edge
+// states (Sigma, l, Pi)
 template <class T>
 SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt, const Planes<T>& W,
                           const Planes<T>& uplus, int f) {
@@ -173,53 +189,35 @@ SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt, cons
     const int s = j * fp + f;
     const int st[4] = {G.sten[s], G.sten[PS + s], G.sten[2 * PS + s], G.sten[3 * PS + s]};
     T up[kDim];
-    recon_side(side_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W.ld((size_t)k * fp + st[q]); }, up);
+    recon_side(slot_geom(G, PS, s, n), P.gam, dt, w, [&](int k, int q) { return W.ld((size_t)k * fp + st[q]); }, up);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) uplus.st((size_t)k * PS + s, up[k]);
   }
 }
 
-// find_flux_var + res2d + the RK combine with the density floor
-// (MUSCL_base.hpp:345-359, 238-276, 124-161) for face f: the updated
-// conserved state U0 + dt_here (source - flux divergence), floored.
-// Returns the stop bits; `floored` reports the density floor.
-template <class T, class Q>
-SPLASH_HD unsigned flux_face(const DevGeom& G, const PhysParams& P, const SrcParams<Q>& sp,
-                                              double dt_here, const Planes<T>& Win, const Planes<T>& U0,
-                                              const Planes<T>& uplus, int f, T* u, bool& floored) {
+// res2d + the RK combine with the density floor (MUSCL_base.hpp:238-276,
+// 124-161) for face f: the updated conserved state
+// U0 + dt_here (source - flux divergence), floored, from the edges' fluxes
+// (flux(k, e) gives field k of edge e).
+template <class T, class Q, class FluxFn>
+SPLASH_HD void update_face(const DevGeom& G, const PhysParams& P, const SrcParams<Q>& sp, double dt_here,
+                           const T* w, const T* u0, FluxFn flux, int f, T* u, bool& floored) {
   const int fp = G.fpad;
-  const int PS = G.max_slots * fp;
-  const D3 fcn = plane3(G.fcn, fp, f);
-  T w[kDim], acc[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) w[k] = Win.ld((size_t)k * fp + f);
-  source_term(w, fcn, sp, P, acc);
-  const Gas gas = gas_of(P);
+  T acc[kDim];
+  source_term(w, plane3(G.fcn, fp, f), sp, P, acc);
   const int n = G.nslots[f];
-  unsigned bits = 0;
   for (int j = 0; j < n; ++j) {
-    const int s = j * fp + f;
-    const int rv = G.rev[s];
-    T uL[kDim], uR[kDim], F[kDim];
+    const int se = G.slot_edge[j * fp + f];
+    const int e = se & 0x7fffffff;
+    const double c = G.e_side[(size_t)kSideCoef * G.xs + (se < 0 ? G.epad + e : e)];
+    const double coef = (se < 0) ? c : -c;
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      uL[k] = uplus.ld((size_t)k * PS + s);
-      uR[k] = uplus.ld((size_t)k * PS + rv);
-    }
-    const EdgeGeom g{plane3(G.ec, PS, s), plane3(G.en, PS, s), plane3(G.nxr, PS, s)};
-    bits |= riemann_flux(uL, uR, g, gas, P.solver, F);
-    const double coef = -G.coef[s];
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      if (nan_bits(val(F[k]))) bits |= 1u;
-      acc[k] = fm(coef, F[k], acc[k]);
-    }
+    for (int k = 0; k < kDim; ++k) acc[k] = fm(coef, flux(k, e), acc[k]);
   }
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) u[k] = fm(dt_here, acc[k], U0.ld((size_t)k * fp + f));
-  floored = u[0] < 1e-8;
+  for (int k = 0; k < kDim; ++k) u[k] = fm(dt_here, acc[k], u0[k]);
+  floored = less(u[0], T(1e-8));
   if (floored) u[0] = T(1e-8);
-  return bits;
 }
 
 }  // namespace f64

@@ -1,0 +1,78 @@
+// The dt clip of the FP64 step (MUSCL_base.hpp:100-115): folding the faces'
+// candidates into the bounds of the next step, and the clip itself.
+#pragma once
+
+#include <cstdint>
+
+#include "fp64_math.cuh"
+#include "layout.hpp"
+
+namespace splash {
+namespace f64 {
+
+// max over the block of non-negative doubles' bit patterns, in thread 0
+template <int BLOCK>
+__device__ __forceinline__ unsigned long long block_max(unsigned long long v, unsigned long long* sm) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long a = __shfl_down_sync(0xffffffffu, v, o);
+    v = a > v ? a : v;
+  }
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < BLOCK / 32; ++w) v = sm[w] > v ? sm[w] : v;
+  }
+  return v;
+}
+
+// Folds the block's candidates (integer maxima: exact in any order) and, in
+// the last block to do so, makes the bounds of the next step's dt of them:
+//   CFL bound h0 0.1 / max_vel, max_vel = max(1e-8, sqrt(vel2)),
+//   extra dt 0.01 / (alpha fric_k sqrt(rate2)), at most 1e20; 1e20 and a flag
+//   when some face's is negative (physics/adiabatic.hpp:543-580),
+// and gives the folds a fresh start.  Every thread of the block calls it.
+template <int BLOCK>
+__device__ __forceinline__ void fold_block(double vel2, double rate2, bool negative, const DevState& S,
+                                           const PhysParams& P) {
+  __shared__ unsigned long long sm[2][BLOCK / 32];
+  const int neg = __syncthreads_or(negative);
+  const unsigned long long v = block_max<BLOCK>(bits_of(vel2), sm[0]);
+  const unsigned long long r = block_max<BLOCK>(bits_of(rate2), sm[1]);
+  if (threadIdx.x != 0) return;
+  unsigned long long* F = S.fold;
+  if (v) atomicMax(F + kFoldVel2, v);
+  if (r) atomicMax(F + kFoldRate2, r);
+  if (neg) atomicMax(F + kFoldNeg, 1ull);
+  __threadfence();
+  if (atomicAdd(F + kFoldDone, 1ull) != gridDim.x - 1) return;
+  __threadfence();
+  const double vmax = fmax(1e-8, sqrt(from_bits(atomicExch(F + kFoldVel2, 0ull))));
+  const double rate = sqrt(from_bits(atomicExch(F + kFoldRate2, 0ull)));
+  const bool below = atomicExch(F + kFoldNeg, 0ull) != 0;
+  atomicExch(F + kFoldDone, 0ull);
+  double extra = 1e20;
+  if (!below && rate > 0) extra = fmin(1e20, 0.01 / (P.alpha * P.fric_k * rate));
+  const double cfl = P.h0 * 0.1 / vmax;
+  S.scal[kScMaxVel] = vmax;
+  S.scal[kScExtraDt] = extra;
+  S.scal[kScBound] = (cfl > extra) ? extra : cfl;
+  S.scal[kScNegExtra] = below ? 1.0 : 0.0;
+}
+
+// dt = min(dt0, 0.1 h0 / max_vel, extra_dt)
+__device__ __forceinline__ double step_dt(const double* scal, double dt0) {
+  const double bound = scal[kScBound];
+  return less(bound, dt0) ? bound : dt0;
+}
+// One thread of the step: its dt and time, and the stop bit of a negative
+// extra dt, which the reference latches when the step begins.
+__device__ __forceinline__ void publish_dt(const DevState& S, double dt) {
+  S.scal[kScDt] = dt;
+  S.scal[kScTime] = S.scal[kScTime] + dt;
+  if (S.scal[kScNegExtra] != 0.0) atomicOr(S.err, 8u);  // SPLASH_STOP_NEG_EXTRA_DT
+}
+
+}  // namespace f64
+}  // namespace splash

@@ -1,129 +1,135 @@
 // FP64 kernels of the MUSCL time step (the reference method in FP64).
 //
-// One do_step(dt0) (MUSCL_base/MUSCL_base.hpp:97-225) is five launches on
-// one stream, captured once into a CUDA graph by the host:
+// One do_step(dt0) (MUSCL_base/MUSCL_base.hpp:97-225) is four launches on
+// one stream, captured into a CUDA graph by the host:
 //
-//   dt_kernel          1 block  : reduce the previous launch's per-block
-//                                 partials -> max_vel, extra_dt, clipped dt,
-//                                 time; diagnostics sums
-//   reconstruct(W0)    per face : limited edge states of every slot
-//   flux_update(1)     per face : Riemann fluxes, source, res2d(dt/2) + U0
-//                                 -> W1 (Sigma, l, Pi)
-//   reconstruct(W1)    per face
-//   flux_update(2)     per face : res2d(dt) + U0 -> U, W0 for the next step,
-//                                 per-block partials of the new state
+//   edge(W0)    per edge : dt clip; limited states of both sides, Riemann flux
+//   update(1)   per face : source, res2d(dt/2) + U0 -> W1 (Sigma, l, Pi)
+//   edge(W1)    per edge
+//   update(2)   per face : res2d(dt) + U0 -> U, W0 for the next step, and the
+//                          candidates of its dt, folded; the last block makes
+//                          the bounds of them
 //
-// Per-face threads loop over the face's slots in the reference slot order,
-// so the flux divergence accumulates in exactly the reference order.
+// What bounds them is the FP64 pipe (fp64_math.cuh: one warp instruction per
+// SM every 9.8 ns), so the layout serves the instruction count: every edge's
+// flux is evaluated once (every Riemann solver here satisfies
+// F(uR, uL, -n) = -F(uL, uR, n) term by term; the reference evaluates it from
+// both faces), and the work is spread over sides and edges instead of faces,
+// so that small meshes reach every SM.  Faces sum their edges' fluxes in the
+// reference's slot order.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "physics_fp64.cuh"
 #include "physics_iso.cuh"
 #include "step_body_fp64.cuh"
-#include "reduce.cuh"
+#include "step_fold_fp64.cuh"
 
 namespace splash {
 namespace f64 {
 namespace {
 
-constexpr int kBlock = 64;  // FP64-pipe bound, register-heavy: small blocks balance the SMs
+// Edge launches: blocks of kEdgeBlock edges and twice as many threads.
+// Thread t reconstructs one side of edge t mod kEdgeBlock, the two states
+// meet in shared memory, and the first half of the threads evaluates the
+// fluxes.  The other half has nothing left to do then, but the pipe is fed by
+// the SM's other blocks: a block of 64 edges measured as fast as larger ones
+// on hex(7) and spreads the smallest meshes over the most SMs.
+constexpr int kThreads = 2 * kEdgeBlock;
+constexpr int kFaceBlock = 64;
 
-// ---------------------------------------------------------------------
-// W = (Sigma, l, Pi) of the conserved state and the partials of it
-// (used once after the state is set; afterwards flux_update stage 2
-// produces both).
-__global__ void __launch_bounds__(kBlock) prepare_kernel(DevGeom G, DevState S, PhysParams P) {
+// W = (Sigma, l, Pi) of the conserved state and the candidates of its dt
+// (once after the state is set; afterwards the stage-2 update does both).
+__global__ void __launch_bounds__(kFaceBlock) prepare_kernel(DevGeom G, DevState S, PhysParams P) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0, rate2 = 0.0;
+  bool negative = false;
   if (f < G.n_faces) {
-    double u[kDim];
+    double u[kDim], w[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) u[k] = S.U[k * G.fpad + f];
     const D3 r = plane3(G.fcn, G.fpad, f);
-    double w[kDim];
     prim_of(u, r, P.gam, w);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) S.W0[k * G.fpad + f] = w[k];
-    dt_candidates(u, r, G.area[f], P, vmax, dmin, sums);
+    dt_fold(w, r, P, vel2, rate2, negative);
   }
-  red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
+  fold_block<kFaceBlock>(vel2, rate2, negative, S, P);
 }
 
-// dt = min(dt0, 0.1 h0 / max_vel, extra_dt)  (MUSCL_base.hpp:100-115)
-__global__ void __launch_bounds__(256) dt_kernel(DevState S, PhysParams P, int nblocks) {
-  __shared__ double sm[256][7];
-  double v[7] = {1e-8, 1e20, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    const double* p = S.partial + (size_t)b * kPartialStride;
-    v[0] = fmax(v[0], p[0]);
-    v[1] = fmin(v[1], p[1]);
-#pragma unroll
-    for (int k = 2; k < 7; ++k) v[k] = v[k] + p[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 7; ++k) sm[threadIdx.x][k] = v[k];
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sm[threadIdx.x][0] = fmax(sm[threadIdx.x][0], sm[threadIdx.x + s][0]);
-      sm[threadIdx.x][1] = fmin(sm[threadIdx.x][1], sm[threadIdx.x + s][1]);
-#pragma unroll
-      for (int k = 2; k < 7; ++k) sm[threadIdx.x][k] = sm[threadIdx.x][k] + sm[threadIdx.x + s][k];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const double max_vel = sm[0][0];
-    double extra = sm[0][1];
-    if (extra < 0) {
-      atomicOr(S.err, 8u);  // SPLASH_STOP_NEG_EXTRA_DT
-      extra = 1e20;
-    }
-    double dt = S.scal[kScDt0];
-    if (dt > P.h0 * 0.1 / max_vel) dt = P.h0 * 0.1 / max_vel;
-    if (dt > extra) dt = extra;
-    S.scal[kScDt] = dt;
-    S.scal[kScMaxVel] = max_vel;
-    S.scal[kScExtraDt] = extra;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) S.scal[kScMass + k] = sm[0][2 + k];
-    S.scal[kScTime] = S.scal[kScTime] + dt;
-  }
-}
-
-// find_U_edges (MUSCL_base.hpp:361-434) for every slot of one face.
-__global__ void __launch_bounds__(kBlock) reconstruct_kernel(DevGeom G, const double* __restrict__ W,
-                                                             double* __restrict__ uplus,
-                                                             const double* __restrict__ sc,
-                                                             PhysParams P) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  recon_face<double>(G, P, sc[kScDt], Planes<double>{const_cast<double*>(W)}, Planes<double>{uplus}, f);
-}
-
-// find_flux_var + res2d + the RK combine with the density floor
-// (MUSCL_base.hpp:345-359, 238-276, 124-161).  stage 1: dt_here = dt/2,
-// writes W1; stage 2: dt_here = dt, writes U, W0 and the partials.
+// find_U_edges (MUSCL_base.hpp:361-434) of both sides of every edge and the
+// Riemann flux (find_flux_var, MUSCL_base.hpp:345-359).
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) flux_update_kernel(DevGeom G, DevState S, PhysParams P) {
+__global__ void __launch_bounds__(kThreads, 3) edge_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
+  griddep_launch_dependents();
+  __shared__ double up[kDim][kThreads];
+  const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  if (live) {
+    const int x = (t < kEdgeBlock) ? e : G.epad + e;
+    const SideGeom g = side_geom(G, x);
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[G.xs + x], G.e_sten[2 * G.xs + x], G.e_sten[3 * G.xs + x]};
+    griddep_wait();
+    const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
+    const double* W = (STAGE == 1) ? S.W0 : S.W1;
+    const int fp = G.fpad;
+    double w[kDim], u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) w[k] = W[k * fp + f];
+    recon_side(g, P.gam, dt, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) up[k][t] = u[k];
+    if (STAGE == 2) {
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) S.uplus[(size_t)k * G.xs + x] = u[k];
+    }
+    if (STAGE == 1 && x == 0) publish_dt(S, dt);
+  }
+  __syncthreads();
+  if (!live || t >= kEdgeBlock) return;
+  double L[kDim], R[kDim], F[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    L[k] = up[k][i];
+    R[k] = up[k][kEdgeBlock + i];
+  }
+  unsigned bits = riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    if (nan_bits(F[k])) bits |= 1u;
+    S.fe[(size_t)k * G.epad + e] = F[k];
+  }
+  if (bits) atomicOr(S.err, bits);
+}
+
+// res2d + the RK combine; stage 1: dt/2, writes W1; stage 2: dt, writes U, W0
+// and folds the candidates of the next dt.
+template <int STAGE>
+__global__ void __launch_bounds__(kFaceBlock) update_kernel(DevGeom G, DevState S, PhysParams P) {
+  griddep_launch_dependents();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0, rate2 = 0.0;
+  bool negative = false;
+  griddep_wait();
   if (f < G.n_faces) {
     const int fp = G.fpad;
     const double dt = S.scal[kScDt];
-    const double dt_here = (STAGE == 1) ? dt / 2 : dt;
-    double u[kDim];
+    const double* Win = (STAGE == 1) ? S.W0 : S.W1;
+    double w[kDim], u0[kDim], u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      w[k] = Win[k * fp + f];
+      u0[k] = S.U[k * fp + f];
+    }
     bool floored;
-    const unsigned bits =
-        flux_face<double, double>(G, P, face_src_params<double>(G, P, f), dt_here,
-                                  Planes<double>{(STAGE == 1) ? S.W0 : S.W1}, Planes<double>{S.U},
-                                  Planes<double>{S.uplus}, f, u, floored);
-    if (bits) atomicOr(S.err, bits);
+    update_face<double, double>(G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
+                                [&](int k, int e) { return S.fe[(size_t)k * G.epad + e]; }, f, u, floored);
     const D3 fcn = plane3(G.fcn, fp, f);
-    double w[kDim];
     prim_of(u, fcn, P.gam, w);
     double* Wout = (STAGE == 1) ? S.W1 : S.W0;
 #pragma unroll
@@ -131,123 +137,126 @@ __global__ void __launch_bounds__(kBlock) flux_update_kernel(DevGeom G, DevState
     if (STAGE == 2) {
 #pragma unroll
       for (int k = 0; k < kDim; ++k) S.U[k * fp + f] = u[k];
-      dt_candidates(u, fcn, G.area[f], P, vmax, dmin, sums);
+      dt_fold(w, fcn, P, vel2, rate2, negative);
     }
   }
-  if (STAGE == 2) red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
+  if (STAGE == 2) fold_block<kFaceBlock>(vel2, rate2, negative, S, P);
 }
 
 // ---- isothermal solver (MUSCL_HLLE, 4 fields; planes 0..3 of U/W/U+) ----
 // W of a 4-field state is the state itself (find_U_edges subtracts the
 // zero profile rho_an from field 0, MUSCL_base.hpp:366-371).
-__global__ void __launch_bounds__(kBlock) iso_prepare_kernel(DevGeom G, DevState S) {
+__global__ void __launch_bounds__(kFaceBlock) iso_prepare_kernel(DevGeom G, DevState S, PhysParams P) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0;
   if (f < G.n_faces) {
-    double u[kDim];
+    double u[iso::kIsoDim];
 #pragma unroll
-    for (int k = 0; k < iso::kIsoDim; ++k) u[k] = S.U[k * G.fpad + f];
-    u[4] = 0.0;
-    S.W0[f] = u[0] - 0.0;
-#pragma unroll
-    for (int k = 1; k < iso::kIsoDim; ++k) S.W0[k * G.fpad + f] = u[k];
-    iso::dt_candidates(u, plane3(G.fcn, G.fpad, f), G.area[f], vmax, dmin, sums);
+    for (int k = 0; k < iso::kIsoDim; ++k) {
+      u[k] = S.U[k * G.fpad + f];
+      S.W0[k * G.fpad + f] = u[k];
+    }
+    vel2 = iso::dt_fold(u, plane3(G.fcn, G.fpad, f));
   }
-  red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
+  fold_block<kFaceBlock>(vel2, 0.0, false, S, P);
 }
 
-// find_U_edges with the isothermal limiter (MUSCL_base.hpp:361-434,
-// physics/isothermal.hpp:269-320) for every slot of one face
-__global__ void __launch_bounds__(kBlock) iso_reconstruct_kernel(DevGeom G, const double* __restrict__ W,
-                                                                 double* __restrict__ uplus,
-                                                                 const double* __restrict__ sc) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
-  const int fp = G.fpad;
-  const int PS = G.max_slots * fp;
-  const double dt = sc[kScDt];
-  double w[iso::kIsoDim];
+// the two sides' states with the isothermal limiter (MUSCL_base.hpp:361-434,
+// physics/isothermal.hpp:269-320) and the HLLE flux of every edge
+template <int STAGE>
+__global__ void __launch_bounds__(kThreads) iso_edge_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
+  griddep_launch_dependents();
+  __shared__ double up[iso::kIsoDim][kThreads];
+  const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  const size_t ep = (size_t)G.epad, xs = (size_t)G.xs;
+  const D3 ec = live ? D3{G.e_geo[e], G.e_geo[ep + e], G.e_geo[2 * ep + e]} : D3{0, 0, 0};
+  if (live) {
+    const int x = (t < kEdgeBlock) ? e : G.epad + e;
+    const double* c = G.e_side + x;
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    const double twoN = (double)(2 * G.nslots[f]);
+    griddep_wait();
+    const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
+    const double* W = (STAGE == 1) ? S.W0 : S.W1;
+    const int fp = G.fpad;
+    double w[iso::kIsoDim];
 #pragma unroll
-  for (int k = 0; k < iso::kIsoDim; ++k) w[k] = W[k * fp + f];
-  const int n = G.nslots[f];
-  const double twoN = (double)(2 * n);
-  for (int j = 0; j < n; ++j) {
-    const int s = j * fp + f;
-    const int ia = G.sten[s], ib = G.sten[PS + s], ic = G.sten[2 * PS + s], id = G.sten[3 * PS + s];
-    const double bp0 = G.beta[s], bp1 = G.beta[PS + s], bm0 = G.beta[2 * PS + s], bm1 = G.beta[3 * PS + s];
-    const double hp = G.hpm[s], hm = G.hpm[PS + s], bmd = G.bm[s];
-    const D3 ec = plane3(G.ec, PS, s);
-    const D3 en = plane3(G.en, PS, s);
-    const double nu_plus = iso::courant(w, ec, en, dt, G.arc_a[s]);
-    const double eta = G.eta[PS + s];
+    for (int k = 0; k < iso::kIsoDim; ++k) w[k] = W[k * fp + f];
+    const D3 en = D3{c[kIsoEn * xs], c[(kIsoEn + 1) * xs], c[(kIsoEn + 2) * xs]};
+    const iso::Limiter lim(c[kIsoEta * xs], twoN, iso::courant(w, ec, en, dt, c[kIsoArc * xs]));
 #pragma unroll
     for (int k = 0; k < iso::kIsoDim; ++k) {
       const double* Wk = W + k * fp;
-      const double Up = bp0 * Wk[ia] + bp1 * Wk[ib];
-      const double pp = (Up - w[k]) / hp;
-      const double Um = bm0 * Wk[ic] + bm1 * Wk[id];
-      const double pm = (-Um + w[k]) / hm;
-      const double lim = iso::limiter_field(pm / pp, eta, twoN, nu_plus);
-      uplus[k * PS + s] = (k == 0) ? w[k] + 0.0 + pp * lim * bmd : w[k] + pp * lim * bmd;
+      const double Up = c[kSideBeta * xs] * Wk[st[0]] + c[(kSideBeta + 1) * xs] * Wk[st[1]];
+      const double pp = quotient(Up - w[k], c[kIsoHp * xs], c[kIsoRhp * xs]);
+      const double Um = c[(kSideBeta + 2) * xs] * Wk[st[2]] + c[(kSideBeta + 3) * xs] * Wk[st[3]];
+      const double pm = quotient(-Um + w[k], c[kIsoHm * xs], c[kIsoRhm * xs]);
+      const double u = w[k] + pp * lim(divide(pm, pp)) * c[kIsoBm * xs];
+      up[k][t] = u;
+      if (STAGE == 2) S.uplus[k * xs + x] = u;
     }
+    if (STAGE == 1 && x == 0) publish_dt(S, dt);
   }
+  __syncthreads();
+  if (!live || t >= kEdgeBlock) return;
+  double L[iso::kIsoDim], R[iso::kIsoDim], F[iso::kIsoDim];
+#pragma unroll
+  for (int k = 0; k < iso::kIsoDim; ++k) {
+    L[k] = up[k][i];
+    R[k] = up[k][kEdgeBlock + i];
+  }
+  unsigned bits = iso::flux_star(L, R, ec, G.e_geo[6 * ep + e],
+                                 D3{G.e_geo[3 * ep + e], G.e_geo[4 * ep + e], G.e_geo[5 * ep + e]}, F);
+#pragma unroll
+  for (int k = 0; k < iso::kIsoDim; ++k) {
+    if (nan_bits(F[k])) bits |= 1u;
+    S.fe[k * ep + e] = F[k];
+  }
+  if (bits) atomicOr(S.err, bits);
 }
 
-// find_flux_var + res2d + the RK combine (zero source) for one face;
-// stage 1: dt/2, writes W1; stage 2: dt, writes U, W0 and the partials
+// res2d + the RK combine (zero source) for one face
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) iso_flux_update_kernel(DevGeom G, DevState S, PhysParams P) {
+__global__ void __launch_bounds__(kFaceBlock) iso_update_kernel(DevGeom G, DevState S, PhysParams P) {
+  griddep_launch_dependents();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double vel2 = 0.0;
+  griddep_wait();
   if (f < G.n_faces) {
     const int fp = G.fpad;
-    const int PS = G.max_slots * fp;
     const double dt = S.scal[kScDt];
     const double dt_here = (STAGE == 1) ? dt / 2 : dt;
-    const double area = G.area[f];
-    double acc[iso::kIsoDim];
+    const double area = G.area[f], iarea = recip(area);
+    double u[iso::kIsoDim];
 #pragma unroll
-    for (int k = 0; k < iso::kIsoDim; ++k) acc[k] = dt_here * 0.0;
+    for (int k = 0; k < iso::kIsoDim; ++k) u[k] = 0.0;
     const double rd_dt = P.round_diff * dt_here;
     const int n = G.nslots[f];
-    unsigned bits = 0;
     for (int j = 0; j < n; ++j) {
-      const int s = j * fp + f;
-      const int rv = G.rev[s];
-      double uL[iso::kIsoDim], uR[iso::kIsoDim], F[iso::kIsoDim];
+      const int se = G.slot_edge[j * fp + f];
+      const int e = se & 0x7fffffff;
+      const double chord = G.e_side[(size_t)kIsoChord * G.xs + (se < 0 ? G.epad + e : e)];
+      const double q = quotient(rd_dt * chord, area, iarea);
+      const double coef = (se < 0) ? -q : q;
 #pragma unroll
-      for (int k = 0; k < iso::kIsoDim; ++k) {
-        uL[k] = S.uplus[k * PS + s];
-        uR[k] = S.uplus[k * PS + rv];
-      }
-      bits |= iso::flux_star(uL, uR, plane3(G.ec, PS, s), G.ecn[s], plane3(G.en, PS, s), F);
-      const double coef = rd_dt * G.chord[s] / area;
-#pragma unroll
-      for (int k = 0; k < iso::kIsoDim; ++k) {
-        if (isnan(F[k])) bits |= 1u;
-        acc[k] -= coef * F[k];
-      }
+      for (int k = 0; k < iso::kIsoDim; ++k) u[k] -= coef * S.fe[(size_t)k * G.epad + e];
     }
-    if (bits) atomicOr(S.err, bits);
-    double u[kDim];
 #pragma unroll
-    for (int k = 0; k < iso::kIsoDim; ++k) u[k] = acc[k] + S.U[k * fp + f];
-    u[4] = 0.0;
+    for (int k = 0; k < iso::kIsoDim; ++k) u[k] = u[k] + S.U[k * fp + f];
     if (u[0] < 1e-8) u[0] = 1e-8;
     double* Wout = (STAGE == 1) ? S.W1 : S.W0;
-    Wout[f] = u[0] - 0.0;
 #pragma unroll
-    for (int k = 1; k < iso::kIsoDim; ++k) Wout[k * fp + f] = u[k];
-    if (STAGE == 2) {
-#pragma unroll
-      for (int k = 0; k < iso::kIsoDim; ++k) S.U[k * fp + f] = u[k];
-      iso::dt_candidates(u, plane3(G.fcn, fp, f), area, vmax, dmin, sums);
+    for (int k = 0; k < iso::kIsoDim; ++k) {
+      Wout[k * fp + f] = u[k];
+      if (STAGE == 2) S.U[k * fp + f] = u[k];
     }
+    if (STAGE == 2) vel2 = iso::dt_fold(u, plane3(G.fcn, fp, f));
   }
-  if (STAGE == 2) red::block_partials<kBlock>(vmax, dmin, sums, S.partial + (size_t)blockIdx.x * kPartialStride);
+  if (STAGE == 2) fold_block<kFaceBlock>(vel2, 0.0, false, S, P);
 }
-
-__global__ void set_scalar_kernel(double* dst, double v) { *dst = v; }
 
 // reference order [F][dim] <-> internal planes
 // One thread per element of the [n_faces][dim] array, in its memory order,
@@ -295,59 +304,48 @@ __global__ void gather_state2_kernel(const double* __restrict__ U, const int* __
 }
 constexpr int kMoveBlock = 256;
 
-inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
+inline int face_blocks(int n) { return (n + kFaceBlock - 1) / kFaceBlock; }
+inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
 
 }  // namespace
 }  // namespace f64
 
 // ---- launchers (declared in kernels.hpp) --------------------------------
-int fp64_partial_blocks(int n_faces) { return f64::blocks_for(n_faces); }
-
-cudaError_t fp64_prepare(const DevGeom& G, const DevState& S, const PhysParams& P,
-                         cudaStream_t st) {
+cudaError_t fp64_prepare(const DevGeom& G, const DevState& S, const PhysParams& P, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(S.fold, 0, kFoldCount * sizeof(*S.fold), st);
+  if (e != cudaSuccess) return e;
   if (P.solver == kSolverIsoHLLE)
-    f64::iso_prepare_kernel<<<f64::blocks_for(G.n_faces), f64::kBlock, 0, st>>>(G, S);
+    f64::iso_prepare_kernel<<<f64::face_blocks(G.n_faces), f64::kFaceBlock, 0, st>>>(G, S, P);
   else
-    f64::prepare_kernel<<<f64::blocks_for(G.n_faces), f64::kBlock, 0, st>>>(G, S, P);
+    f64::prepare_kernel<<<f64::face_blocks(G.n_faces), f64::kFaceBlock, 0, st>>>(G, S, P);
   return cudaGetLastError();
 }
 
-cudaError_t fp64_dt(const DevState& S, const PhysParams& P, int n_faces, cudaStream_t st) {
-  f64::dt_kernel<<<1, 256, 0, st>>>(S, P, f64::blocks_for(n_faces));
-  return cudaGetLastError();
+const void* fp64_dt0_kernel_ptr(int solver) {
+  return solver == kSolverIsoHLLE ? (const void*)f64::iso_edge_kernel<1> : (const void*)f64::edge_kernel<1>;
 }
 
-cudaError_t fp64_set_dt0(const DevState& S, double dt0, cudaStream_t st) {
-  f64::set_scalar_kernel<<<1, 1, 0, st>>>(S.scal + kScDt0, dt0);
-  return cudaGetLastError();
-}
-
-cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, cudaStream_t st,
+cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, double dt0, cudaStream_t st,
                       cudaEvent_t* ev) {
-  const int nb = f64::blocks_for(G.n_faces);
+  const bool iso = P.solver == kSolverIsoHLLE;
+  const dim3 eg(f64::edge_blocks(G.n_edges)), fg(f64::face_blocks(G.n_faces)), eb(f64::kThreads), fb(f64::kFaceBlock);
+  cudaError_t e = cudaSuccess;
+  auto chk = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+  };
+  // ev[0]..ev[1] is the (empty) slot of the dt clip, which the stage-1 edge
+  // launch evaluates itself
   if (ev) cudaEventRecord(ev[0], st);
-  f64::dt_kernel<<<1, 256, 0, st>>>(S, P, nb);
   if (ev) cudaEventRecord(ev[1], st);
-  if (P.solver == kSolverIsoHLLE) {
-    f64::iso_reconstruct_kernel<<<nb, f64::kBlock, 0, st>>>(G, S.W0, S.uplus, S.scal);
-    if (ev) cudaEventRecord(ev[2], st);
-    f64::iso_flux_update_kernel<1><<<nb, f64::kBlock, 0, st>>>(G, S, P);
-    if (ev) cudaEventRecord(ev[3], st);
-    f64::iso_reconstruct_kernel<<<nb, f64::kBlock, 0, st>>>(G, S.W1, S.uplus, S.scal);
-    if (ev) cudaEventRecord(ev[4], st);
-    f64::iso_flux_update_kernel<2><<<nb, f64::kBlock, 0, st>>>(G, S, P);
-    if (ev) cudaEventRecord(ev[5], st);
-    return cudaGetLastError();
-  }
-  f64::reconstruct_kernel<<<nb, f64::kBlock, 0, st>>>(G, S.W0, S.uplus, S.scal, P);
+  chk(launch_pdl(iso ? f64::iso_edge_kernel<1> : f64::edge_kernel<1>, eg, eb, st, G, S, P, dt0));
   if (ev) cudaEventRecord(ev[2], st);
-  f64::flux_update_kernel<1><<<nb, f64::kBlock, 0, st>>>(G, S, P);
+  chk(launch_pdl(iso ? f64::iso_update_kernel<1> : f64::update_kernel<1>, fg, fb, st, G, S, P));
   if (ev) cudaEventRecord(ev[3], st);
-  f64::reconstruct_kernel<<<nb, f64::kBlock, 0, st>>>(G, S.W1, S.uplus, S.scal, P);
+  chk(launch_pdl(iso ? f64::iso_edge_kernel<2> : f64::edge_kernel<2>, eg, eb, st, G, S, P, dt0));
   if (ev) cudaEventRecord(ev[4], st);
-  f64::flux_update_kernel<2><<<nb, f64::kBlock, 0, st>>>(G, S, P);
+  chk(launch_pdl(iso ? f64::iso_update_kernel<2> : f64::update_kernel<2>, fg, fb, st, G, S, P));
   if (ev) cudaEventRecord(ev[5], st);
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t fp64_scatter_state(const double* aos, const int* iperm, double* U, int n_faces,

@@ -23,6 +23,7 @@
 #include "dword.cuh"
 #include "fp_convert.cuh"
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "physics_fp64.cuh"
 #include "physics_mixed.cuh"
 #include "reduce.cuh"
@@ -43,18 +44,6 @@ constexpr int kMaxFaceSlots = 8;
 __device__ __forceinline__ F3 plane3f(const float* p, int stride, int i) {
   return F3{p[i], p[stride + i], p[2 * stride + i]};
 }
-// Programmatic dependent launch.  The step's kernels are launched with
-// programmatic stream serialization: a kernel may start while its
-// predecessor drains, loads what does not depend on it (stencil indices,
-// geometry), then waits in griddep_wait() for the predecessor grid to
-// complete and its writes to be visible.  Every read of state and every
-// write comes after the wait, so no kernel overwrites what its predecessor
-// is still reading.  Without a programmatic predecessor the wait returns at
-// once.  launch_dependents lets the next kernel start as soon as every
-// block of this one has begun.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
-
 // Two FP32 lanes per instruction (PTX .f32x2: round to nearest,
 // flush-to-zero like the rest of this file); each lane rounds exactly as the
 // scalar add / sub / mul.
@@ -1046,24 +1035,6 @@ cudaError_t mixed_scatter_prepare(const double* aos, const int* iperm, const Dev
     mx::scatter_prepare_kernel<false><<<mx::blocks_for(G.n_faces), mx::kBlock, 0, st>>>(aos, iperm, G, S, P, dim);
   return cudaGetLastError();
 }
-
-namespace {
-// A launch with programmatic stream serialization (see griddep_wait).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-}  // namespace
 
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
                        cudaStream_t st, cudaEvent_t* ev, bool /*per_launch: four launches, same layout*/) {
