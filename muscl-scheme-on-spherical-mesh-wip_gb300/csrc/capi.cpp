@@ -255,8 +255,7 @@ int Solver::run_diagnostics(double* out9) {
   in.cos_obs = d_cos_obs;
   in.gam = P.gam;
   in.light_curves = dim == kDim ? 1 : 0;
-  SPLASH_CUDA(diag_launch(in, d_diag_partial, d_diag_out, stream));
-  SPLASH_CUDA(cudaMemcpyAsync(h_diag, d_diag_out, 9 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+  SPLASH_CUDA(diag_launch(in, d_diag_partial, d_diag_done, h_diag, stream));
   SPLASH_CUDA(cudaStreamSynchronize(stream));
   std::memcpy(out9, h_diag, 9 * sizeof(double));
   return SPLASH_OK;
@@ -487,7 +486,6 @@ int splash_create(const splash_mesh_desc* mesh, const double* U_in, int dim, dou
       SPLASH_CUDA(cudaMemset(S.uplus, 0, splash::kDim * xs * sizeof(double)));
       S.fe = s->dalloc<double>(splash::kDim * (xs / 2));
       S.fold = s->dalloc<unsigned long long>(splash::kFoldCount);
-      SPLASH_CUDA(cudaMemset(S.fold, 0, splash::kFoldCount * sizeof(unsigned long long)));
     }
     S.scal = s->dalloc<double>(splash::kScCount);
     S.err = s->dalloc<unsigned int>(4);
@@ -497,7 +495,8 @@ int splash_create(const splash_mesh_desc* mesh, const double* U_in, int dim, dou
     s->d_iperm = s->upload(s->iperm);
     s->d_cos_obs = s->upload(observer_planes(*s));
     s->d_diag_partial = s->dalloc<double>((size_t)splash::diag_partial_blocks(s->n_faces) * 9);
-    s->d_diag_out = s->dalloc<double>(9);
+    s->d_diag_done = s->dalloc<unsigned>(1);
+    SPLASH_CUDA(cudaMemset(s->d_diag_done, 0, sizeof(unsigned)));
     SPLASH_CUDA(cudaMallocHost(&s->h_diag, 9 * sizeof(double)));
     {
       // Grace-class hosts: the device can dereference pageable host memory,

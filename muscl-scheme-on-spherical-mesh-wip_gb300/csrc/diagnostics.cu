@@ -9,11 +9,17 @@
 // cos(alpha) depend on the geometry only and are precomputed on the host with
 // the reference's expressions (one plane per observer, 0 where not visible);
 // the device evaluates Pi per face and the products in the reference order
-// (Pi * cos) * area.  The sums are reduced in a fixed tree order (per-block
-// partials, then one block), so the result is deterministic; it differs from
-// the reference's serial sum only by summation order.
+// (Pi * cos) * area.  The sums are reduced in a fixed order (per thread, warp
+// and block, then the blocks' partials by the last block to finish), so the
+// result is deterministic; it differs from the reference's serial sum only by
+// summation order.
 //
-// Compiled with -fmad=false like the FP64 step.
+// A caller of the light curves waits for them every step, so the pass is one
+// launch that leaves its 9 numbers in page-locked host memory (two launches
+// and a copy before).  What it takes beyond that is the FP64 pipe's latency,
+// 36 ns per dependent instruction (fp64_math.cuh): the 9 sums of a warp are
+// reduced together in 16 instructions, each exchange halving the sums a lane
+// still carries, instead of 45.  Compiled with -fmad=false like the FP64 step.
 #include <cuda_runtime.h>
 
 #include "diagnostics.hpp"
@@ -23,84 +29,98 @@ namespace splash {
 namespace diag {
 namespace {
 
-constexpr int kBlock = 256;
+constexpr int kBlock = 128;
 constexpr int kVals = 9;
+constexpr int kMaxBlocks = 304;  // 2 per SM: each thread of a large mesh sums several faces
 
-__device__ __forceinline__ double pressure_of(const double* u, double rx, double ry, double rz, double gam) {
-  // vel = cross(r, l) / (-Sigma) ; Pi = max(1e-16, (E - Sigma |v|^2 / 2)(gam - 1))
-  const double cx = ry * u[3] - rz * u[2], cy = rz * u[1] - rx * u[3], cz = rx * u[2] - ry * u[1];
-  const double vx = cx / (-u[0]), vy = cy / (-u[0]), vz = cz / (-u[0]);
-  double s = vx * vx;
-  s = s + vy * vy;
-  s = s + vz * vz;
-  const double n = sqrt(s);
-  return f64::smax(1e-16, (u[4] - u[0] * (n * n) / 2) * (gam - 1));
+// Sums v[0 .. 16) over the warp: every exchange passes on the half of the
+// values that the partner keeps, so lane l ends with the sum of v[l >> 1].
+__device__ __forceinline__ double warp_sums(double (&v)[16], int lane) {
+#pragma unroll
+  for (int o = 16, n = 8; o > 1; o >>= 1, n >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const double got = __shfl_xor_sync(0xffffffffu, up ? v[k] : v[n + k], o);
+      v[k] = (up ? v[n + k] : v[k]) + got;
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__global__ void __launch_bounds__(kBlock) partials_kernel(DiagInput in, double* __restrict__ partial) {
-  __shared__ double sm[kVals][kBlock];
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double v[kVals] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (f < in.n_faces) {
-    const int fp = in.fpad;
+// Sums v over the block; thread k < kVals returns the sum of v[k].
+__device__ __forceinline__ double block_sums(double (&v)[16]) {
+  __shared__ double sm[kBlock / 32][16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double s = warp_sums(v, lane);
+  __syncthreads();  // the last use of sm
+  if ((lane & 1) == 0) sm[warp][lane >> 1] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < kVals) {
+    t = sm[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < kBlock / 32; ++w) t = t + sm[w][threadIdx.x];
+  }
+  return t;
+}
+
+__global__ void __launch_bounds__(kBlock) sums_kernel(DiagInput in, double* __restrict__ partial,
+                                                      unsigned* __restrict__ done, double* __restrict__ out) {
+  double v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = 0.0;
+  const size_t fp = in.fpad;
+  for (int f = blockIdx.x * kBlock + threadIdx.x; f < in.n_faces; f += gridDim.x * kBlock) {
     double u[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) u[k] = (k < in.dim) ? in.U[(size_t)k * fp + f] : 0.0;
+    for (int k = 0; k < 5; ++k) u[k] = (k < in.dim) ? in.U[k * fp + f] : 0.0;
     const double a = in.area[f];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] = u[k] * a;
+    for (int k = 0; k < 5; ++k) v[k] = fma(u[k], a, v[k]);
     if (in.light_curves) {
-      const double PI = pressure_of(u, in.fcn[f], in.fcn[fp + f], in.fcn[2 * (size_t)fp + f], in.gam);
+      const f64::D3 r{in.fcn[f], in.fcn[fp + f], in.fcn[2 * fp + f]};
+      const double pa = f64::pressure_fc(u, r, in.gam) * a;
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
-        const double c = in.cos_obs[(size_t)o * fp + f];
-        if (c != 0.0) v[5 + o] = PI * c * a;
+        const double c = in.cos_obs[o * fp + f];
+        if (f64::bits_of(c) << 1) v[5 + o] = fma(pa, c, v[5 + o]);  // 0 where the observer does not see the face
       }
     }
   }
-#pragma unroll
-  for (int k = 0; k < kVals; ++k) sm[k][threadIdx.x] = v[k];
+  const double s = block_sums(v);
+  if (threadIdx.x < kVals) {
+    partial[(size_t)blockIdx.x * kVals + threadIdx.x] = s;
+    __threadfence();
+  }
+  __shared__ unsigned last;
   __syncthreads();
-  for (int h = kBlock / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) {
-#pragma unroll
-      for (int k = 0; k < kVals; ++k) sm[k][threadIdx.x] = sm[k][threadIdx.x] + sm[k][threadIdx.x + h];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < kVals) partial[(size_t)blockIdx.x * kVals + threadIdx.x] = sm[threadIdx.x][0];
-}
-
-__global__ void __launch_bounds__(kBlock) final_kernel(const double* __restrict__ partial, int nblocks,
-                                                       double* __restrict__ out) {
-  __shared__ double sm[kVals][kBlock];
-  double v[kVals] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += kBlock) {
-#pragma unroll
-    for (int k = 0; k < kVals; ++k) v[k] = v[k] + partial[(size_t)b * kVals + k];
-  }
-#pragma unroll
-  for (int k = 0; k < kVals; ++k) sm[k][threadIdx.x] = v[k];
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
   __syncthreads();
-  for (int h = kBlock / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) {
+  if (!last) return;
+  __threadfence();
 #pragma unroll
-      for (int k = 0; k < kVals; ++k) sm[k][threadIdx.x] = sm[k][threadIdx.x] + sm[k][threadIdx.x + h];
-    }
-    __syncthreads();
+  for (int k = 0; k < 16; ++k) v[k] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kBlock) {
+    const volatile double* p = partial + (size_t)b * kVals;
+#pragma unroll
+    for (int k = 0; k < kVals; ++k) v[k] = v[k] + p[k];
   }
-  if (threadIdx.x < kVals) out[threadIdx.x] = sm[threadIdx.x][0];
+  const double t = block_sums(v);
+  if (threadIdx.x < kVals) out[threadIdx.x] = t;
+  if (threadIdx.x == 0) *done = 0u;
 }
 
 }  // namespace
 }  // namespace diag
 
-int diag_partial_blocks(int n_faces) { return (n_faces + diag::kBlock - 1) / diag::kBlock; }
+int diag_partial_blocks(int n_faces) {
+  const int nb = (n_faces + diag::kBlock - 1) / diag::kBlock;
+  return nb < diag::kMaxBlocks ? nb : diag::kMaxBlocks;
+}
 
-cudaError_t diag_launch(const DiagInput& in, double* partial, double* out, cudaStream_t st) {
-  const int nb = diag_partial_blocks(in.n_faces);
-  diag::partials_kernel<<<nb, diag::kBlock, 0, st>>>(in, partial);
-  diag::final_kernel<<<1, diag::kBlock, 0, st>>>(partial, nb, out);
+cudaError_t diag_launch(const DiagInput& in, double* partial, unsigned* done, double* out, cudaStream_t st) {
+  diag::sums_kernel<<<diag_partial_blocks(in.n_faces), diag::kBlock, 0, st>>>(in, partial, done, out);
   return cudaGetLastError();
 }
 

@@ -19,8 +19,10 @@ struct DiagInput {
 
 // Per-block partial records needed by diag_launch.
 int diag_partial_blocks(int n_faces);
-// out (device, 9 doubles): sum Sigma A, sum l_x A, sum l_y A, sum l_z A,
-// sum E A, then the light curves (observer 0, 45, 90, 180 degrees).
-cudaError_t diag_launch(const DiagInput& in, double* partial, double* out, cudaStream_t st);
+// out (9 doubles in memory that the device can write, page-locked host memory
+// too): sum Sigma A, sum l_x A, sum l_y A, sum l_z A, sum E A, then the light
+// curves (observer 0, 45, 90, 180 degrees).  done: a device counter, zero
+// before the first call and left so.
+cudaError_t diag_launch(const DiagInput& in, double* partial, unsigned* done, double* out, cudaStream_t st);
 
 }  // namespace splash
