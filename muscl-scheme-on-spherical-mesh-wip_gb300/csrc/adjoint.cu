@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState
 template <int STAGE>
 __global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
                                                             double dt0) {
-  __shared__ double up[2][kDim][kThreads];
+  __shared__ SideExchange<D1, kThreads> sides;
+  const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
   const int e = blockIdx.x * kEdgeBlock + i;
   const bool live = e < G.n_edges;
@@ -107,22 +108,16 @@ __global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState 
 #pragma unroll
     for (int k = 0; k < kDim; ++k) w[k] = W.ld(k * fp + f);
     recon_side(side_geom(G, x), P.gam, dt, w, [&](int k, int q) { return W.ld(k * fp + st[q]); }, u);
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      up[0][k][t] = u[k].v;
-      up[1][k][t] = u[k].d[0];
-    }
     if (STAGE == 1 && x == 0) publish_dt(S, dt);
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
   D1 L[kDim], R[kDim], F[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    L[k] = dual1(up[0][k][i], up[1][k][i]);
-    R[k] = dual1(up[0][k][kEdgeBlock + i], up[1][k][kEdgeBlock + i]);
-  }
-  unsigned bits = riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+  EdgeSide<D1> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
   const Planes<D1> fe{S.fe, T.dfe, 0};
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
@@ -269,7 +264,8 @@ __global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P
 __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
                                                            const double* __restrict__ W, double* __restrict__ uplus,
                                                            double* __restrict__ LJ, double* __restrict__ fe) {
-  __shared__ double up[kDim][kThreads];
+  __shared__ SideExchange<double, kThreads> sides;
+  const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
   const int e = blockIdx.x * kEdgeBlock + i;
   const bool live = e < G.n_edges;
@@ -285,20 +281,16 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
         side_geom(G, x), P.gam, *dtp, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u,
         [&](int k, double v) { LJ[k * xs + x] = v; });
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      up[k][t] = u[k];
-      uplus[k * xs + x] = u[k];
-    }
+    for (int k = 0; k < kDim; ++k) uplus[k * xs + x] = u[k];
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
   double L[kDim], R[kDim], F[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    L[k] = up[k][i];
-    R[k] = up[k][kEdgeBlock + i];
-  }
-  riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+  EdgeSide<double> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) fe[(size_t)k * G.epad + e] = F[k];
 }
@@ -348,41 +340,48 @@ __global__ void __launch_bounds__(kThreads) adj_edge_kernel(DevGeom G, PhysParam
                                                             const double* __restrict__ lam,
                                                             const uint8_t* __restrict__ mask, int bit,
                                                             double* __restrict__ PU, double* __restrict__ own) {
-  __shared__ double ub[kDim][kThreads];
+  __shared__ SideExchange<double, kThreads> sides;
+  __shared__ double bars[rev::kSideBarValues][kThreads];
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
   const int e = blockIdx.x * kEdgeBlock + i;
   const bool live = e < G.n_edges;
   const size_t fp = G.fpad, xs = G.xs;
+  const Gas gas = gas_of(P);
+  const int x = (t < kEdgeBlock) ? e : G.epad + e;
+  EdgeGeom eg;
+  EdgeSide<double> S;
+  double u[kDim];
+  if (live) {
+    eg = edge_geom(G, e);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) u[k] = uplus[k * xs + x];
+    S = edge_side(u, eg, gas);
+    sides.put(t, u, S);
+  }
+  __syncthreads();
   if (live && t < kEdgeBlock) {
     const double* coef = G.e_side + kSideCoef * xs + e;
     const double c0 = dt_here * coef[0], c1 = dt_here * coef[G.epad];
     const int f0 = G.e_face[e], f1 = G.e_face[G.epad + e];
-    double L[kDim], R[kDim], Fb[kDim], Lb[kDim], Rb[kDim];
+    double R[kDim], Fb[kDim];
+    EdgeSide<double> SR;
+    sides.get(kEdgeBlock + i, R, SR);
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      L[k] = uplus[k * xs + e];
-      R[k] = uplus[k * xs + G.epad + e];
+    for (int k = 0; k < kDim; ++k)
       Fb[k] = fma(c1, masked(lam, mask, bit, fp, k, f1), -(c0 * masked(lam, mask, bit, fp, k, f0)));
-      Lb[k] = 0.0;
-      Rb[k] = 0.0;
-    }
-    rev::riemann_flux_rev(L, R, edge_geom(G, e), gas_of(P), P.solver, Fb, Lb, Rb);
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      ub[k][i] = Lb[k];
-      ub[k][kEdgeBlock + i] = Rb[k];
-    }
+    rev::SideBar BL, BR;
+    rev::riemann_flux_rev(u, R, S, SR, eg, gas, P.solver, Fb, BL, BR);
+    rev::put_bar(&bars[0][i], kThreads, BL);
+    rev::put_bar(&bars[0][kEdgeBlock + i], kThreads, BR);
   }
   __syncthreads();
   if (!live) return;
-  const int x = (t < kEdgeBlock) ? e : G.epad + e;
   const int f = G.e_face[x];
-  double w[kDim], upb[kDim], pu[kDim], mu[kDim], wb[kDim] = {0, 0, 0, 0, 0};
+  double w[kDim], upb[kDim] = {0, 0, 0, 0, 0}, pu[kDim], mu[kDim], wb[kDim] = {0, 0, 0, 0, 0};
+  rev::SideBar B = rev::get_bar(&bars[0][t], kThreads);
+  rev::edge_side_rev(u, S, eg, gas, B, upb);
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    w[k] = W[k * fp + f];
-    upb[k] = ub[k][t];
-  }
+  for (int k = 0; k < kDim; ++k) w[k] = W[k * fp + f];
   rev::recon_side_rev(side_geom(G, x), P.gam, dt, w, upb, [&](int k) { return LJ[k * xs + x]; }, pu, mu, wb);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {

@@ -15,8 +15,7 @@
 //                     the local limiter Jacobian (adiabatic.hpp:685-828) taped
 //   recon_side_rev    reverse of the reconstruction from that tape
 //   source_rev        reverse of the source term (adiabatic.hpp:396-541)
-//                     from a Dual<10> Jacobian of its 5 state and 5
-//                     parameter inputs
+//                     in its 5 state and 5 parameter inputs
 //   prim_rev          reverse of (Sigma, l, E) -> (Sigma, l, Pi)
 #pragma once
 
@@ -37,6 +36,32 @@ struct SideBar {
 SPLASH_HD void zero(SideBar& b) {
   b.u0 = b.u4 = b.vn = b.v2 = b.p = b.e = b.gi = b.a2 = b.a = b.q = 0.0;
   b.l = b.vel = d3(0, 0, 0);
+}
+// a SideBar as values at p[0], p[stride], ... (q is folded into the others
+// before it is handed on)
+constexpr int kSideBarValues = 15;
+SPLASH_HD void put_bar(double* p, int stride, const SideBar& b) {
+  const double v[kSideBarValues] = {b.u0, b.u4, b.vn, b.v2, b.p, b.e, b.gi, b.a2, b.a, b.l.x, b.l.y, b.l.z,
+                                    b.vel.x, b.vel.y, b.vel.z};
+  for (int i = 0; i < kSideBarValues; ++i) p[(size_t)i * stride] = v[i];
+}
+SPLASH_HD SideBar get_bar(const double* p, int stride) {
+  double v[kSideBarValues];
+  for (int i = 0; i < kSideBarValues; ++i) v[i] = p[(size_t)i * stride];
+  SideBar b;
+  b.u0 = v[0];
+  b.u4 = v[1];
+  b.vn = v[2];
+  b.v2 = v[3];
+  b.p = v[4];
+  b.e = v[5];
+  b.gi = v[6];
+  b.a2 = v[7];
+  b.a = v[8];
+  b.q = 0.0;
+  b.l = d3(v[9], v[10], v[11]);
+  b.vel = d3(v[12], v[13], v[14]);
+  return b;
 }
 SPLASH_HD void add_scaled(D3& a, const D3& b, double s) {
   a.x = fma(b.x, s, a.x);
@@ -98,16 +123,16 @@ SPLASH_HD double wave_speed_rev(const EdgeSide<double>& S, double p_star, const 
   return 0.0;
 }
 
-// Adjoint of F = riemann_flux(uL, uR): uLb += (dF/duL)^T Fb, uRb += (dF/duR)^T Fb.
-SPLASH_HD void riemann_flux_rev(const double* uL, const double* uR, const EdgeGeom& g, const Gas& gas, int solver,
-                                const double* Fb, double* uLb, double* uRb) {
-  EdgeSide<double> L = edge_side(uL, g, gas), R = edge_side(uR, g, gas);
+// Adjoint of F = riemann_flux(uL, uR, L, R): the adjoints of the two sides'
+// quantities (edge_side_rev turns them into those of the states).
+SPLASH_HD void riemann_flux_rev(const double* uL, const double* uR, EdgeSide<double> L, EdgeSide<double> R,
+                                const EdgeGeom& g, const Gas& gas, int solver, const double* Fb, SideBar& BL,
+                                SideBar& BR) {
   const double pvrs = fma(-0.125 * ((R.vn - L.vn) * (uL[0] + uR[0])), L.a + R.a, 0.5 * (L.p + R.p));
   const double p_star = smax(0., pvrs);
   L.q = wave_speed(L, p_star, gas);
   R.q = wave_speed(R, p_star, gas);
   const double S_L = L.vn - L.q, S_R = R.vn + R.q;
-  SideBar BL, BR;
   zero(BL);
   zero(BR);
   double SLb = 0.0, SRb = 0.0;
@@ -310,8 +335,6 @@ SPLASH_HD void riemann_flux_rev(const double* uL, const double* uR, const EdgeGe
     BL.a += asb;
     BR.a += asb;
   }
-  edge_side_rev(uL, L, g, gas, BL, uLb);
-  edge_side_rev(uR, R, g, gas, BR, uRb);
 }
 
 // Adjoint of flux_star (states with the energy in field 4)
@@ -329,7 +352,12 @@ SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom&
     for (int k = 0; k < 4; ++k) st[i][k] = us[i][k];
     st[i][4] = ps[i]->v;
   }
-  riemann_flux_rev(st[0], st[1], g, gas_of(gam), solver, Fb, bar[0], bar[1]);
+  const Gas gas = gas_of(gam);
+  const EdgeSide<double> L = edge_side(st[0], g, gas), R = edge_side(st[1], g, gas);
+  SideBar BL, BR;
+  riemann_flux_rev(st[0], st[1], L, R, g, gas, solver, Fb, BL, BR);
+  edge_side_rev(st[0], L, g, gas, BL, bar[0]);
+  edge_side_rev(st[1], R, g, gas, BR, bar[1]);
   double* out[2] = {uLb, uRb};
   for (int i = 0; i < 2; ++i)
     for (int k = 0; k < kDim; ++k) out[i][k] += (k < 4 ? bar[i][k] : 0.0) + bar[i][4] * ps[i]->d[k];
@@ -341,32 +369,60 @@ SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom&
 // Per side and field the limited edge state is up = w + hg dp phi(r, nu)
 // with dp = U+ - w, dm = w - U-, r = hr dm / dp (hr = H+/H-, hg = BM/H+)
 // and nu the side's Courant factor (MUSCL_base.hpp:361-434,
-// adiabatic.hpp:685-828).  The recomputation evaluates phi once on Dual<2>
-// over (r, nu) -- its value is the primal's, bit for bit -- and stores the
-// three partials
+// adiabatic.hpp:685-828).  The recomputation evaluates phi with its two
+// partial derivatives -- its value is the primal's, bit for bit -- and stores
 //   d up / d dp = hg (phi - r phi_r),  d up / d dm = hg hr phi_r,
 //   d up / d nu = hg dp phi_nu
 // so that the reverse sweep needs no transcendental.  Where phi is flat in r
 // (r = +-inf or NaN) d up / d dp = hg phi.
 constexpr int kTapePlanes = 15;  // 3 per field
 
+// limiter_field with its partial derivatives in r and nu; inu = 1 / nu
+// (22 FP64 instructions beside the value's, against 2 per instruction of the
+// value for a dual number over (r, nu))
+struct Phi {
+  double v, r, nu;
+};
+SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double inu) {
+  if (nan_bits(r)) return Phi{0., 0., 0.};
+  if (odd_bits(r)) return Phi{limiter_field(r, l), 0., 0.};
+  // the superbee: max(0, max(min(1, r sb), min(r, eta_p)))
+  Phi A{1., 0., 0.};
+  const double rs = r * l.sb;
+  if (less(rs, 1.)) A = Phi{rs, l.sb, -rs * inu};
+  const Phi B = less(l.eta_p, r) ? Phi{l.eta_p, 0., 0.} : Phi{r, 1., 0.};
+  Phi sb = less(A.v, B.v) ? B : A;
+  if (!less(0., sb.v)) sb = Phi{0., 0., 0.};
+  // the third-order line t1 + ts r below it, not below 0
+  const double t = fma(l.ts, r, l.t1);
+  Phi to = sb;
+  if (less(t, sb.v)) to = Phi{t, l.ts, (r - 1) * (1.0 / 3)};
+  if (!less(0., to.v)) to = Phi{0., 0., 0.};
+  if (to.v == sb.v) return sb;
+  if (!(r > 0.0)) return to;
+  const Dual<1> h = switch_pos(Dual<1>::seed(r, 0));
+  return Phi{fma(h.v, sb.v - to.v, to.v), fma(h.v, sb.r - to.r, fma(h.d[0], sb.v - to.v, to.r)),
+             fma(h.v, sb.nu - to.nu, to.nu)};
+}
+
 // nb as in recon_side; lj(3 k + i) receives the partials of field k
 template <class NbFn, class LjFn>
 SPLASH_HD void recon_side_tape(const SideGeom& g, double gam, double dt, const double* w, NbFn nb, double* up,
                                LjFn lj) {
-  const Dual<2> nu = Dual<2>::seed(side_courant(g, gam, dt, w), 1);
-  const LimiterLine<Dual<2>> line = limiter_line(g, nu);
+  const double nu = side_courant(g, gam, dt, w);
+  const LimiterLine<double> line = limiter_line(g, nu);
+  const double inu = recip(nu);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
     double dp, dm;
     side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
     const double r = slope_ratio(g, dp, dm);
-    const Dual<2> lim = limiter_field(Dual<2>::seed(r, 0), line);
+    const Phi phi = limiter_partials(r, line, inu);
     const double dg = dp * g.hg;
-    up[k] = fm(dg, lim.v, w[k]);
-    lj(3 * k, g.hg * ((lim.d[0] != 0.0) ? fma(-lim.d[0], r, lim.v) : lim.v));
-    lj(3 * k + 1, g.hg * g.hr * lim.d[0]);
-    lj(3 * k + 2, dg * lim.d[1]);
+    up[k] = fm(dg, phi.v, w[k]);
+    lj(3 * k, g.hg * ((phi.r != 0.0) ? fma(-phi.r, r, phi.v) : phi.v));
+    lj(3 * k + 1, g.hg * g.hr * phi.r);
+    lj(3 * k + 2, dg * phi.nu);
   }
 }
 
@@ -458,34 +514,116 @@ SPLASH_HD void recon_face_rev(const DevGeom& G, const PhysParams& P, double dt, 
 SPLASH_HD void source_rev(const double* w, const D3& fcn, const SrcParams<double>& sp, const PhysParams& P,
                           const double* srcb, double* wb, double* pb) {
   if (!P.accretion_on) return;
-  Dual<10> wd[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) wd[k] = Dual<10>::seed(w[k], k);
-  SrcParams<Dual<10>> sd;
-  sd.acc0 = Dual<10>::seed(sp.acc0, 5);
-  sd.omega_acc = v3(Dual<10>(sp.omega_acc.x), Dual<10>::seed(sp.omega_acc.y, 6), Dual<10>::seed(sp.omega_acc.z, 7));
-  sd.acc_rate = Dual<10>::seed(sp.acc_rate, 8);
-  sd.total_mass = Dual<10>::seed(sp.total_mass, 9);
-  Dual<10> res[kDim];
-  source_term(wd, fcn, sd, P, res);
-#pragma unroll
-  for (int i = 0; i < kDim; ++i) {
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) wb[k] += srcb[i] * res[i].d[k];
-#pragma unroll
-    for (int j = 0; j < 5; ++j) pb[j] += srcb[i] * res[i].d[5 + j];
+  const double b0 = srcb[0], b4 = srcb[4];
+  const D3 bl = d3(srcb[1], srcb[2], srcb[3]);
+  const double ir = recip(w[0]), ip = recip(w[4]);
+  const D3 vel = scal(fcross(fcn, d3(w[1], w[2], w[3])), -ir);
+  const double v2 = fdot(vel, vel);
+  const D3 omxr = fcross(sp.omega_acc, fcn);
+  const D3 rxo = fcross(fcn, omxr);
+  const D3 d = sub(omxr, vel);
+  const double H = fma(P.gam_gm1 * w[4], ir, 0.5 * v2);
+  double w0b = 0.0, w4b = 0.0, v2b = 0.0, gb = 0.0, Hb = 0.0, irb = 0.0;
+  // accretion: acc0 (1, r x (omega x r), e_acc + |omega x r - v|^2 / 2)
+  pb[0] += fma(b4, fma(0.5, fdot(d, d), P.e_acc), b0 + fdot(bl, rxo));
+  const D3 db = scal(d, b4 * sp.acc0);
+  D3 ob = fcross(scal(bl, sp.acc0), fcn);
+  add_scaled(ob, db, 1.0);
+  const D3 omb = fcross(fcn, ob);
+  pb[1] += omb.y;
+  pb[2] += omb.z;
+  D3 velb = scal(db, -1.0);
+  if (!P.friction_on) {
+    const D3 rxv = fcross(fcn, vel);
+    const double im = recip(sp.total_mass);
+    const double q = -(sp.acc_rate * (4 * M_PI)) * im, m = q * w[0];
+    const double mb = fma(b4, H, b0 + fdot(bl, rxv));
+    Hb = b4 * m;
+    const D3 x = fcross(scal(bl, m), fcn);
+    add_scaled(velb, x, 1.0);
+    w0b = mb * q;
+    const double qb = mb * w[0];
+    pb[3] += qb * (-4 * M_PI) * im;
+    pb[4] -= qb * q * im;
   }
+  // cooling: - g_eff / kappa (1 - beta(C))
+  const double GM = 0.217909;
+  const double g_eff = GM - v2;
+  const double kappa = 3.4e6;
+  const double C = (12. / 5 * 1.6e-13) * (w[0] * ip) * root(root((3. / 4 * 4.85e36) * (g_eff * w[0])));
+  const double C_switch = -1 - 1 / (0.736194670678821 - 1);
+  double beta, dbeta;
+  if (C <= C_switch) {
+    const double y = recip(1.0 + C);
+    beta = 1.0 - y;
+    dbeta = y * y;
+  } else {
+    const double y = recip(C), x2 = 4.0 * (y * y);
+    beta = 1.0 - x2 * x2;
+    dbeta = 4.0 * (x2 * x2) * y;
+  }
+  const bool floor = beta < 1e-8 || is_nan(beta), ceil = beta > 1 - 1e-8;
+  if (floor) beta = 1e-8;
+  if (ceil) beta = 1 - 1e-8;
+  gb = -b4 * (1 / kappa) * (1.0 - beta);
+  if (!floor && !ceil && C > 0.0) {
+    const double Cb = b4 * g_eff * (1 / kappa) * dbeta * C;  // adjoint of log C
+    w0b = fma(1.25 * Cb, ir, w0b);
+    w4b = -Cb * ip;
+    gb = fma(0.25 * Cb, recip(g_eff), gb);
+  }
+  if (P.friction_on) {
+    const D3 l = d3(w[1], w[2], w[3]);
+    const double rho = P.fric_k * g_eff * w[0] * w[0] * ip;
+    const D3 vel0 = d3(-P.omega_ns * fcn.y, P.omega_ns * fcn.x, 0.0);
+    const D3 rel = sub(vel, vel0);
+    double in;
+    const double n = root_pair(fdot(rel, rel), in);
+    const double k = P.alpha * rho * n;
+    D3 wrb = fcross(bl, fcn);
+    add_scaled(wrb, vel0, b4);
+    const double krb = -fdot(bl, l);
+    const double kb = fma(krb, ir, -fma(b4, H, b0 + fdot(wrb, rel)));
+    irb = krb * k;
+    const double kr = k * ir;
+    wb[1] = fma(-kr, bl.x, wb[1]);
+    wb[2] = fma(-kr, bl.y, wb[2]);
+    wb[3] = fma(-kr, bl.z, wb[3]);
+    Hb -= b4 * k;
+    add_scaled(velb, wrb, -k);
+    if (n > 0.0) add_scaled(velb, rel, kb * P.alpha * rho * in);
+    const double rhob = kb * P.alpha * n;
+    gb = fma(rhob, P.fric_k * w[0] * w[0] * ip, gb);
+    w0b = fma(2.0 * rhob * rho, ir, w0b);
+    w4b = fma(-rhob * rho, ip, w4b);
+  }
+  // H = gam / (gam - 1) Pi / Sigma + v2 / 2, g_eff = GM - v2
+  w4b = fma(Hb * P.gam_gm1, ir, w4b);
+  irb = fma(Hb * P.gam_gm1, w[4], irb);
+  v2b = fma(0.5, Hb, -gb);
+  add_scaled(velb, vel, 2.0 * v2b);
+  // vel = -(r x l) / Sigma
+  w0b -= ir * fma(irb, ir, fdot(velb, vel));
+  const D3 lb = fcross(scal(velb, -ir), fcn);
+  wb[0] += w0b;
+  wb[1] += lb.x;
+  wb[2] += lb.y;
+  wb[3] += lb.z;
+  wb[4] += w4b;
 }
 
 // Reverse of prim_of: ub += J^T wb for w = (u0..u3, pressure_fc(u)).
 SPLASH_HD void prim_rev(const double* u, const D3& r, double gam, const double* wb, double* ub) {
-  Dual<5> ud[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) ud[k] = Dual<5>::seed(u[k], k);
-  const Dual<5> p = pressure_fc(ud, r, gam);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) ub[k] += wb[k] + wb[4] * p.d[k];
-  ub[4] += wb[4] * p.d[4];
+  const D3 c = fcross(r, d3(u[1], u[2], u[3]));
+  const double ir = recip(u[0]), h = 0.5 * fdot(c, c);
+  // the floored pressure is a constant
+  const double b = less(1e-16, fma(-h, ir, u[4]) * (gam - 1)) ? wb[4] * (gam - 1) : 0.0;
+  const D3 lb = fcross(scal(c, -b * ir), r);
+  ub[0] += fma(b * h, ir * ir, wb[0]);
+  ub[1] += wb[1] + lb.x;
+  ub[2] += wb[2] + lb.y;
+  ub[3] += wb[3] + lb.z;
+  ub[4] += b;
 }
 
 }  // namespace rev

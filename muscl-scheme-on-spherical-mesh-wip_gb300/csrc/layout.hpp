@@ -21,7 +21,7 @@ namespace splash {
 
 constexpr int kDim = 5;          // conserved fields: Sigma, l_x, l_y, l_z, E
 constexpr int kMaxSlots = 6;     // hexagons (pentagons and quads use fewer)
-constexpr int kEdgeBlock = 64;   // edges per block of the FP64 edge launches
+constexpr int kEdgeBlock = 32;   // edges per block of the FP64 edge launches
 
 // Physics constants of the adiabatic model (physics/adiabatic.hpp).
 struct PhysParams {

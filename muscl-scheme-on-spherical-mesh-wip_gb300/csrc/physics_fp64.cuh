@@ -154,10 +154,12 @@ SPLASH_HD T hllcp_fstar(const T& mm, T& M) {
 // (S_K - S*) = s (p_K - P) - P it is alpha Sigma, alpha l + beta (n x R) and
 // alpha E + s (S_K P - p_K V_K), 2 instructions per momentum component, of
 // the one side that S* selects.
+//
+// L and R are the edge_side of the states (their q is not read).
 template <class T>
-SPLASH_HD unsigned riemann_flux(const T* uL, const T* uR, const EdgeGeom& g, const Gas& gas, int solver, T* F) {
+SPLASH_HD unsigned riemann_flux(const T* uL, const T* uR, EdgeSide<T> L, EdgeSide<T> R, const EdgeGeom& g,
+                                const Gas& gas, int solver, T* F) {
   unsigned bits = 0;
-  EdgeSide<T> L = edge_side(uL, g, gas), R = edge_side(uR, g, gas);
   const T p_star = star_pressure(uL, uR, L, R);
   L.q = wave_speed(L, p_star, gas);
   R.q = wave_speed(R, p_star, gas);
@@ -251,6 +253,11 @@ SPLASH_HD unsigned riemann_flux(const T* uL, const T* uR, const EdgeGeom& g, con
     F[4] = fm(w, f1 * dV * S_star, F[4]);
   }
   return bits;
+}
+
+template <class T>
+SPLASH_HD unsigned riemann_flux(const T* uL, const T* uR, const EdgeGeom& g, const Gas& gas, int solver, T* F) {
+  return riemann_flux(uL, uR, edge_side(uL, g, gas), edge_side(uR, g, gas), g, gas, solver, F);
 }
 
 // Geometry of one slot with the edge centre as evaluated (not exactly unit).

@@ -195,6 +195,50 @@ SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt, cons
   }
 }
 
+#if defined(__CUDACC__)
+// What the two threads of an edge exchange: each puts the state and the
+// EdgeSide of its side, the one that evaluates the flux takes both.  One
+// shared-memory plane per value (and one per tangent), indexed by thread.
+template <class T, int THREADS>
+struct SideExchange {
+  static constexpr int kValues = kDim + 10;
+  static constexpr int kParts = is_dual<T>::value ? 2 : 1;
+  double v[kParts][kValues][THREADS];
+
+  __device__ __forceinline__ void put(int i, int t, const T& x) {
+    v[0][i][t] = val(x);
+    if constexpr (is_dual<T>::value) v[1][i][t] = x.d[0];
+  }
+  __device__ __forceinline__ T get(int i, int t) const {
+    T x(v[0][i][t]);
+    if constexpr (is_dual<T>::value) x.d[0] = v[1][i][t];
+    return x;
+  }
+  __device__ __forceinline__ void put(int t, const T* u, const EdgeSide<T>& S) {
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) put(k, t, u[k]);
+    const T s[10] = {S.vel.x, S.vel.y, S.vel.z, S.vn, S.v2, S.p, S.e, S.gi, S.a2, S.a};
+#pragma unroll
+    for (int k = 0; k < 10; ++k) put(kDim + k, t, s[k]);
+  }
+  __device__ __forceinline__ void get(int t, T* u, EdgeSide<T>& S) const {
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) u[k] = get(k, t);
+    T s[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) s[k] = get(kDim + k, t);
+    S.vel = v3(s[0], s[1], s[2]);
+    S.vn = s[3];
+    S.v2 = s[4];
+    S.p = s[5];
+    S.e = s[6];
+    S.gi = s[7];
+    S.a2 = s[8];
+    S.a = s[9];
+  }
+};
+#endif
+
 // res2d + the RK combine with the density floor (MUSCL_base.hpp:238-276,
 // 124-161) for face f: the updated conserved state
 // U0 + dt_here (source - flux divergence), floored, from the edges' fluxes

@@ -33,11 +33,9 @@ namespace f64 {
 namespace {
 
 // Edge launches: blocks of kEdgeBlock edges and twice as many threads.
-// Thread t reconstructs one side of edge t mod kEdgeBlock, the two states
-// meet in shared memory, and the first half of the threads evaluates the
-// fluxes.  The other half has nothing left to do then, but the pipe is fed by
-// the SM's other blocks: a block of 64 edges measured as fast as larger ones
-// on hex(7) and spreads the smallest meshes over the most SMs.
+// Thread t reconstructs one side of edge t mod kEdgeBlock and evaluates what
+// the flux needs of that side alone (EdgeSide); the two meet in shared memory,
+// and the first half of the threads evaluates the fluxes.
 constexpr int kThreads = 2 * kEdgeBlock;
 constexpr int kFaceBlock = 64;
 
@@ -63,12 +61,13 @@ __global__ void __launch_bounds__(kFaceBlock) prepare_kernel(DevGeom G, DevState
 // find_U_edges (MUSCL_base.hpp:361-434) of both sides of every edge and the
 // Riemann flux (find_flux_var, MUSCL_base.hpp:345-359).
 template <int STAGE>
-__global__ void __launch_bounds__(kThreads, 3) edge_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
+__global__ void __launch_bounds__(kThreads) edge_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
   griddep_launch_dependents();
-  __shared__ double up[kDim][kThreads];
+  __shared__ SideExchange<double, kThreads> sides;
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
   const int e = blockIdx.x * kEdgeBlock + i;
   const bool live = e < G.n_edges;
+  const Gas gas = gas_of(P);
   if (live) {
     const int x = (t < kEdgeBlock) ? e : G.epad + e;
     const SideGeom g = side_geom(G, x);
@@ -82,23 +81,20 @@ __global__ void __launch_bounds__(kThreads, 3) edge_kernel(DevGeom G, DevState S
 #pragma unroll
     for (int k = 0; k < kDim; ++k) w[k] = W[k * fp + f];
     recon_side(g, P.gam, dt, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u);
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) up[k][t] = u[k];
     if (STAGE == 2) {
 #pragma unroll
       for (int k = 0; k < kDim; ++k) S.uplus[(size_t)k * G.xs + x] = u[k];
     }
     if (STAGE == 1 && x == 0) publish_dt(S, dt);
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
   double L[kDim], R[kDim], F[kDim];
-#pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    L[k] = up[k][i];
-    R[k] = up[k][kEdgeBlock + i];
-  }
-  unsigned bits = riemann_flux(L, R, edge_geom(G, e), gas_of(P), P.solver, F);
+  EdgeSide<double> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
     if (nan_bits(F[k])) bits |= 1u;
