@@ -39,7 +39,7 @@ cudaError_t fp64_gather_state(const double* U, const int* iperm, double* aos, in
 // the same layout.
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
                        cudaStream_t st, cudaEvent_t* ev = nullptr, bool per_launch = false);
-const void* mixed_dt0_kernel_ptr();
+const void* mixed_dt0_kernel_ptr(const DevGeomMixed& G);
 // The last step's stage-2 edge states into S.uplus32 (for write_t_curl),
 // recomputed from the stage-2 input face states S.W32b and the step's dt.
 cudaError_t mixed_edge_states(const DevGeomMixed& G, const DevState& S, const PhysParams& P, cudaStream_t st);

@@ -738,6 +738,79 @@ __global__ void __launch_bounds__(kBlock, 8) edge_kernel(DevGeomMixed G, DevStat
   edge_body<STAGE, STAGE == 1, true>(G, S, P, blockIdx.x * blockDim.x + threadIdx.x, dt0, dt0f);
 }
 
+// The same step with a thread per side of an edge, for meshes that do not
+// fill the GPU: there a launch takes the latency of one thread's chain of
+// loads and instructions, and the two sides' reconstructions, one after the
+// other in edge_kernel, run side by side here.  Thread t of a block serves
+// edge t mod kHalf, its owner slot below kHalf and its reverse slot above; the
+// edge states meet in shared memory and the lower half evaluates the fluxes.
+// The step scalars are published by a block of their own (FP64 work, 36 ns
+// per dependent instruction, off every edge's chain).  Each edge's arithmetic
+// is edge_body's.
+constexpr int kHalf = kBlock / 2;
+template <int STAGE>
+__global__ void __launch_bounds__(kBlock) edge_sides_kernel(DevGeomMixed G, DevState S, PhysParams P, double dt0,
+                                                            float dt0f) {
+  griddep_launch_dependents();
+  __shared__ float up[kDim][kBlock];
+  const int t = threadIdx.x;
+  if (STAGE == 1 && blockIdx.x == gridDim.x - 1) {
+    if (t == 0) {
+      griddep_wait();
+      publish_dt(S, clip_dt(S.keys, P, dt0), dt0);
+    }
+    return;
+  }
+  const int e = blockIdx.x * kHalf + (t & (kHalf - 1));
+  const bool live = e < G.n_edges, owner = t < kHalf;
+  SlotGeomF g{};
+  if (live) {
+    const int4 ids = ld_rec_i4(G.e_ids, e);
+    const float4 ce = ld_rec_f4(G.e_ec, e), ne = ld_rec_f4(G.e_en, e);
+    const size_t x = owner ? (size_t)e : (size_t)G.epad + e;
+    SlotConsts sc;
+    sc.st = ld_rec_i4(G.e_sten, x);
+    sc.bt = ld_rec_f4(G.e_beta, x);
+    sc.hh = ld_rec_f4(G.e_h, x);
+    sc.eta_p = __fdividef(1.0f, sc.hh.x * sc.hh.z);
+    sc.eta_m = __fdividef(1.0f, sc.hh.y * sc.hh.z);
+    g.ec = f3(ce.x, ce.y, ce.z);
+    g.en = f3(ne.x, ne.y, ne.z);
+    g.nxr = f3(ce.w, ne.w, __int_as_float(ids.z));
+    const int id = owner ? ids.x : ids.y;
+    griddep_wait();
+    const float dt = (STAGE == 1) ? clip_dt_f32(S.keys, P, dt0f) : reinterpret_cast<const float2*>(S.scal + kScDtF)->x;
+    float u[kDim];
+    // whole warps take one branch or the other; one call with a selected
+    // normal rounds differently
+    if (owner)
+      recon_slot(stage_input<STAGE>(S), G.fpad, id & 0x0fffffff, id >> 28, sc, g.ec, g.en, dt, P, u);
+    else
+      recon_slot(stage_input<STAGE>(S), G.fpad, id & 0x0fffffff, id >> 28, sc, g.ec,
+                 f3(-g.en.x, -g.en.y, -g.en.z), dt, P, u);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) up[k][t] = u[k];
+  }
+  __syncthreads();
+  if (!owner) return;
+  unsigned bits = 0;
+  if (live) {
+    float uL[kDim], uR[kDim], F[kDim] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      uL[k] = up[k][t];
+      uR[k] = up[k][t + kHalf];
+    }
+    bits = (P.solver == kSolverIsoHLLE) ? iso_flux_star(uL, uR, g, F) : flux_star(uL, uR, g, P.gam_f, P.solver, F);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k)
+      if (isnan(F[k])) bits |= 1u;
+    st5(S.fe32, G.epad, e, F);
+  }
+  bits = __reduce_or_sync(0xffffffffu, bits);
+  if ((t & 31) == 0 && bits) atomicOr(S.err, bits);
+}
+
 // res2d + RK combine (MUSCL_base.hpp:238-276, 124-161) of face f: the
 // slot contributions -dt_here coef F (F the edge flux, negated on the
 // reverse side) summed in slot order (Neumaier-compensated FP32), plus
@@ -752,12 +825,30 @@ __global__ void __launch_bounds__(kBlock, 8) edge_kernel(DevGeomMixed G, DevStat
 // edge launch that read them has completed); EARLY_STATE: the face's own
 // FP32 and FP64 states are loaded right after the dependency wait, in
 // flight with the flux gathers (one memory round trip less per thread, at
-// more registers: for the one-wave launches of one solver)
+// more registers: for the one-wave launches of one solver); SPLIT (kBlock
+// threads): a face has two threads, the one of the block's upper half
+// evaluates the source while the other sums the fluxes
 template <int STAGE, int MAXS = kMaxFaceSlots, bool BLOCK_FOLD = false, bool RESTART_KEYS = false,
-          bool EARLY_STATE = false>
+          bool EARLY_STATE = false, bool SPLIT = false>
 __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevState& S, const PhysParams& P,
                                             int f) {
   const int fp = G.fpad;
+  __shared__ float src_of[SPLIT ? kDim : 1][SPLIT ? kHalf : 1];
+  if (SPLIT && threadIdx.x >= kHalf) {
+    if (f < G.n_faces) {
+      const F3 fcn32 = plane3f(G.fcn32, fp, f);
+      const double acc0 = G.acc_src[f];
+      griddep_wait();
+      float w[kDim], src[kDim];
+      ld5(stage_input<STAGE>(S), fp, f, w);
+      source_f32(w, fcn32, fpc::d2f(acc0), P, src);
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) src_of[k][threadIdx.x - kHalf] = src[k];
+    }
+    __syncthreads();
+    if (STAGE == 2) fold_candidates_block(0.f, kNoBound, S.keys);
+    return;
+  }
   const bool live = f < G.n_faces;
   F3 fcn32 = f3(0.f, 0.f, 0.f), fcn_lo = f3(0.f, 0.f, 0.f);
   double acc0 = 0.0;
@@ -779,19 +870,20 @@ __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevStat
   griddep_wait();
   if (RESTART_KEYS && f == 0) restart_keys(S.keys);
   float vmax = 0.f, dmin = kNoBound;
+  float w[kDim];
+  double u0[kDim];
+  float dtf = 0.f;
+  // fields 0-1 and 2-3 accumulate in packed pairs, field 4 alone
+  Acc2 a01{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, a23 = a01;
+  Acc a4{0.f, 0.f};
   if (live) {
-    float w[kDim];
-    double u0[kDim];
     if (EARLY_STATE) {
-      ld5(stage_input<STAGE>(S), fp, f, w);
+      if (!SPLIT) ld5(stage_input<STAGE>(S), fp, f, w);
 #pragma unroll
       for (int k = 0; k < kDim; ++k) u0[k] = S.U[k * fp + f];
     }
     const float2 dtf2 = *reinterpret_cast<const float2*>(S.scal + kScDtF);
-    const float dtf = (STAGE == 1) ? dtf2.y : dtf2.x;
-    // fields 0-1 and 2-3 accumulate in packed pairs, field 4 alone
-    Acc2 a01{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, a23 = a01;
-    Acc a4{0.f, 0.f};
+    dtf = (STAGE == 1) ? dtf2.y : dtf2.x;
     // unrolled over the slot bound so that every slot's gather is in flight
     // before the first is summed; the sum stays in slot order
 #pragma unroll
@@ -809,11 +901,19 @@ __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevStat
         a4.add(c * fe4);
       }
     }
+  }
+  if (SPLIT) __syncthreads();  // every thread of the block comes here or to the upper half's
+  if (live) {
     const Acc acc[kDim] = {{a01.hi.x, a01.lo.x}, {a01.hi.y, a01.lo.y}, {a23.hi.x, a23.lo.x},
                            {a23.hi.y, a23.lo.y}, a4};
     float src[kDim];
-    if (!EARLY_STATE) ld5(stage_input<STAGE>(S), fp, f, w);
-    source_f32(w, fcn32, fpc::d2f(acc0), P, src);
+    if (SPLIT) {
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) src[k] = src_of[k][threadIdx.x];
+    } else {
+      if (!EARLY_STATE) ld5(stage_input<STAGE>(S), fp, f, w);
+      source_f32(w, fcn32, fpc::d2f(acc0), P, src);
+    }
     // the FP32 increment (flux sum + dt source, one rounding) is added to
     // the FP64 state; U0 stays in S.U until stage 2 overwrites it
     double u[kDim];
@@ -868,6 +968,14 @@ template <int STAGE, int MAXS>
 __global__ void __launch_bounds__(kBlock, 9) update_early_kernel(DevGeomMixed G, DevState S, PhysParams P) {
   griddep_launch_dependents();
   update_body<STAGE, MAXS, true, STAGE == 1, true>(G, S, P, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// the same with two threads per face
+template <int STAGE, int MAXS>
+__global__ void __launch_bounds__(kBlock) update_split_kernel(DevGeomMixed G, DevState S, PhysParams P) {
+  griddep_launch_dependents();
+  update_body<STAGE, MAXS, true, STAGE == 1, true, true>(G, S, P,
+                                                         blockIdx.x * kHalf + (threadIdx.x & (kHalf - 1)));
 }
 
 // ---------------------------------------------------------------- ensemble
@@ -1024,7 +1132,20 @@ inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
 }  // namespace
 }  // namespace mx
 
-const void* mixed_dt0_kernel_ptr() { return (const void*)mx::edge_kernel<1>; }
+namespace {
+// Two threads per edge and per face (edge_sides_kernel, update_split_kernel)
+// on meshes that leave the GPU's issue slots idle, where a launch takes the
+// latency of one thread's chain; past that the doubled warps cost more than
+// they hide.  us per step back to back, one thread / two: hex(3) 16.1 / 13.7,
+// hex(4) 17.0 / 14.4, hex(5) 18.5 / 17.2, quad(6) 20.1 / 16.5, hex(6) (40,962
+// faces) 28.2 / 24.1; quad(7) (98,304) 31.0 / 33.4, hex(7) 53.7 / 61.4.
+constexpr int kTwoThreadFaces = 65536;
+bool two_threads(const DevGeomMixed& G) { return G.n_faces <= kTwoThreadFaces; }
+}  // namespace
+
+const void* mixed_dt0_kernel_ptr(const DevGeomMixed& G) {
+  return two_threads(G) ? (const void*)mx::edge_sides_kernel<1> : (const void*)mx::edge_kernel<1>;
+}
 
 cudaError_t mixed_scatter_prepare(const double* aos, const int* iperm, const DevGeomMixed& G, const DevState& S,
                                   const PhysParams& P, int dim, cudaStream_t st) {
@@ -1038,8 +1159,9 @@ cudaError_t mixed_scatter_prepare(const double* aos, const int* iperm, const Dev
 
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
                        cudaStream_t st, cudaEvent_t* ev, bool /*per_launch: four launches, same layout*/) {
-  const dim3 egrid(mx::blocks_for(G.n_edges));
-  const dim3 ugrid(mx::blocks_for(G.n_faces));
+  const bool two = two_threads(G);
+  const int ne = two ? (G.n_edges + mx::kHalf - 1) / mx::kHalf : mx::blocks_for(G.n_edges);
+  dim3 ugrid(mx::blocks_for(G.n_faces));
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t r) {
     if (e == cudaSuccess) e = r;
@@ -1061,18 +1183,28 @@ cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParam
   const bool early = G.max_slots > 4 && G.max_slots <= 6 && (int)ugrid.x > 6 * sms && (int)ugrid.x <= 9 * sms;
   void (*upd1)(DevGeomMixed, DevState, PhysParams) = mx::update_kernel<1, 8>;
   void (*upd2)(DevGeomMixed, DevState, PhysParams) = mx::update_kernel<2, 8>;
-  if (G.max_slots <= 4) {
+  if (two) {
+    ugrid.x = (G.n_faces + mx::kHalf - 1) / mx::kHalf;
+    upd1 = G.max_slots <= 4   ? mx::update_split_kernel<1, 4>
+           : G.max_slots <= 6 ? mx::update_split_kernel<1, 6>
+                              : mx::update_split_kernel<1, 8>;
+    upd2 = G.max_slots <= 4   ? mx::update_split_kernel<2, 4>
+           : G.max_slots <= 6 ? mx::update_split_kernel<2, 6>
+                              : mx::update_split_kernel<2, 8>;
+  } else if (G.max_slots <= 4) {
     upd1 = mx::update_kernel<1, 4>;
     upd2 = mx::update_kernel<2, 4>;
   } else if (G.max_slots <= 6) {
     upd1 = early ? mx::update_early_kernel<1, 6> : mx::update_kernel<1, 6>;
     upd2 = early ? mx::update_early_kernel<2, 6> : mx::update_kernel<2, 6>;
   }
-  chk(launch_pdl(mx::edge_kernel<1>, egrid, dim3(mx::kBlock), st, G, S, P, dt0, dt0f));
+  chk(launch_pdl(two ? mx::edge_sides_kernel<1> : mx::edge_kernel<1>, dim3(two ? ne + 1 : ne), dim3(mx::kBlock), st,
+                 G, S, P, dt0, dt0f));
   if (ev) cudaEventRecord(ev[2], st);
   chk(launch_pdl(upd1, ugrid, dim3(mx::kBlock), st, G, S, P));
   if (ev) cudaEventRecord(ev[3], st);
-  chk(launch_pdl(mx::edge_kernel<2>, egrid, dim3(mx::kBlock), st, G, S, P, dt0, dt0f));
+  chk(launch_pdl(two ? mx::edge_sides_kernel<2> : mx::edge_kernel<2>, dim3(ne), dim3(mx::kBlock), st, G, S, P, dt0,
+                 dt0f));
   if (ev) cudaEventRecord(ev[4], st);
   chk(launch_pdl(upd2, ugrid, dim3(mx::kBlock), st, G, S, P));
   if (ev) cudaEventRecord(ev[5], st);

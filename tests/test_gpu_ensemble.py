@@ -239,3 +239,29 @@ def test_full_batched_workload_matches_oracle_record():
             assert abs(en - r["energy"]) <= 1e-6 * abs(r["energy"]), (i, en, r["energy"])
     assert sum(1 for r in rec["members"] if r["bits"]) == 3
     ens.close()
+
+
+@pytest.mark.parametrize("kind,level", [("hex", 2), ("hex", 3), ("hex", 5), ("quad", 3), ("quad", 5)])
+@pytest.mark.parametrize("solver", [1, 2, 3, 4])
+def test_two_thread_launches_equal_batched_launches(kind, level, solver):
+    """Small meshes of one solver run with two threads per edge and face, the batched launches with one: the same bits
+    in a full and a partial last block, for every solver, with and without friction and accretion."""
+    import splash_gb300 as sg
+
+    from helpers import mesh_of
+
+    gam = sg.initial_conditions.gam2d(4 / 3)
+    mesh = mesh_of(kind, level)
+    r = sg.Geometry(mesh).unit_face_centers()
+    U = sg.initial_conditions.rotating_blob(r, gam, seed=solver)
+    U = np.ascontiguousarray(U[:, :4]) if solver == 4 else U
+    params = sg.SolverParams(accretion_rate=1e-2, e_acc=0.5, omega_acc_abs=0.5, tilt_angle=0.2, acc_width=0.1,
+                             alpha=1e-6, friction_on=solver != 2)
+    ens = sg.Ensemble([dict(mesh=mesh, U_in=U, gam=gam, accretion_on=solver != 1, params=params, solver=solver)],
+                      autotune=False)
+    s = sg.Solver(mesh, U, U.shape[1], gam, 0.0, solver != 1, params=params, solver=solver, precision=sg.PREC_MIXED)
+    ens.do_steps(11, 1e-2)
+    s.do_steps(11, 1e-2)
+    assert np.array_equal(ens.get_state(0), s.get_state())
+    info = ens.member_info(0)
+    assert info["t"] == s.time() and info["dt"] == s.last_dt() and info["err"] == s.error_word()
