@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -45,6 +46,7 @@ struct Level {
   RefGeometry geom;
   SlotPlanes sp;
   DevGeomMixed G{};  // acc_src filled per member
+  int* d_iperm = nullptr;  // reference face -> internal face
 };
 
 }  // namespace
@@ -76,19 +78,29 @@ struct Ensemble {
   unsigned* d_bar = nullptr;  // [0..1] grid barrier, [2] status (kEnsBarrierTimeout)
   cudaGraphNode_t p_node = nullptr;
   int graph_steps = 1;
+  bool used_persistent = false;  // do_steps has run the persistent launch
   std::vector<void*> allocs;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t dt0_node = nullptr;
+  // one step, and several in one graph (programmatic dependent launch works
+  // within a graph, not across graph launches)
+  static constexpr int kGraphSteps = 4;
+  struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    std::vector<cudaGraphNode_t> dt0_nodes;
+    void free() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (graph) cudaGraphDestroy(graph);
+      *this = StepGraph{};
+    }
+  } one, several;
   double graph_dt0 = 0.0;
   size_t total_faces = 0;
-  double* h_stage = nullptr;
-  size_t stage_len = 0;
+  double* h_stage = nullptr;  // page-locked: one member's state in reference order
+  bool host_direct = false;   // the device writes pageable host memory (coherent link)
 
   ~Ensemble() {
     cudaSetDevice(device);
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    for (StepGraph* g : {&one, &several}) g->free();
     for (void* p : allocs) cudaFree(p);
     if (h_stage) cudaFreeHost(h_stage);
     if (stream) cudaStreamDestroy(stream);
@@ -167,8 +179,10 @@ struct Ensemble {
     return ensemble_persistent(d_inst, n, d_ftiles, n_ftiles, d_etiles, n_etiles, dt0, steps, d_bar, d_bar + 2,
                                pgrid, stream);
   }
-  // the persistent launch's status word (after the stream has drained)
+  // the persistent launch's status word (after the stream has drained; the
+  // trials read it at their end)
   int check_status() {
+    if (!used_persistent) return SPLASH_OK;
     unsigned st = 0;
     ENS_CUDA(cudaMemcpy(&st, d_bar + 2, sizeof st, cudaMemcpyDeviceToHost));
     if (st & kEnsBarrierTimeout)
@@ -231,8 +245,10 @@ struct Ensemble {
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
+    used_persistent = true;  // by the trials
     int rc = check_status();
     if (rc) return rc;
+    used_persistent = false;
     rc = set_schedule(best_o, best_w);
     if (rc) return rc;
     persistent = best_p;
@@ -245,14 +261,19 @@ struct Ensemble {
   }
 
   int capture() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    exec = nullptr;
-    graph = nullptr;
-    dt0_node = p_node = nullptr;
+    for (StepGraph* g : {&one, &several}) g->free();
+    p_node = nullptr;
     graph_steps = 1;
+    if (persistent) return capture_into(one, 0);
+    const int rc = capture_into(one, 1);
+    return rc ? rc : capture_into(several, kGraphSteps);
+  }
+
+  // n_steps steps of five launches, or the persistent launch (n_steps 0)
+  int capture_into(StepGraph& sg, int n_steps) {
     ENS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t le = persistent ? launch_persistent(graph_dt0, 1) : launch_step(graph_dt0);
+    cudaError_t le = n_steps ? cudaSuccess : launch_persistent(graph_dt0, 1);
+    for (int k = 0; k < n_steps && le == cudaSuccess; ++k) le = launch_step(graph_dt0);
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(stream, &g);
     if (le != cudaSuccess) {
@@ -260,36 +281,38 @@ struct Ensemble {
       return set_error(SPLASH_E_CUDA, "ensemble capture: %s", cudaGetErrorString(le));
     }
     ENS_CUDA(ce);
-    graph = g;
-    ENS_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    sg.graph = g;
+    ENS_CUDA(cudaGraphInstantiate(&sg.exec, g, 0));
     size_t nn = 0;
-    ENS_CUDA(cudaGraphGetNodes(graph, nullptr, &nn));
+    ENS_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
     std::vector<cudaGraphNode_t> nodes(nn);
-    ENS_CUDA(cudaGraphGetNodes(graph, nodes.data(), &nn));
+    ENS_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
     for (cudaGraphNode_t nd : nodes) {
       cudaGraphNodeType t;
       ENS_CUDA(cudaGraphNodeGetType(nd, &t));
       if (t != cudaGraphNodeTypeKernel) continue;
       cudaKernelNodeParams kp{};
       ENS_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
-      if (kp.func == ensemble_finalize_kernel_ptr()) dt0_node = nd;
+      if (kp.func == ensemble_finalize_kernel_ptr()) sg.dt0_nodes.push_back(nd);
       if (kp.func == ensemble_persistent_kernel_ptr()) p_node = nd;
     }
-    if (!(persistent ? p_node : dt0_node)) return set_error(SPLASH_E_CUDA, "ensemble dt node not found");
+    if (n_steps ? (int)sg.dt0_nodes.size() != n_steps : !p_node)
+      return set_error(SPLASH_E_CUDA, "ensemble dt node not found");
     return SPLASH_OK;
   }
 
-  // do_steps: the five-launch graph replayed once per step, or the
-  // persistent graph (one launch) replayed once for all n steps
+  // do_steps: the five-launch graphs (kGraphSteps steps, then single ones),
+  // or the persistent graph (one launch) replayed once for all n steps
   int steps(int nst, double dt0) {
     if (nst <= 0) return SPLASH_OK;
     if (!persistent) {
-      for (int i = 0; i < nst; ++i) {
-        const int rc = step(dt0);
-        if (rc) return rc;
-      }
+      const int rc = set_dt0(dt0);
+      if (rc) return rc;
+      for (; nst >= kGraphSteps; nst -= kGraphSteps) ENS_CUDA(cudaGraphLaunch(several.exec, stream));
+      for (; nst > 0; --nst) ENS_CUDA(cudaGraphLaunch(one.exec, stream));
       return SPLASH_OK;
     }
+    used_persistent = true;
     if (dt0 != graph_dt0 || nst != graph_steps) {
       cudaKernelNodeParams kp{};
       ENS_CUDA(cudaGraphKernelNodeGetParams(p_node, &kp));
@@ -301,27 +324,27 @@ struct Ensemble {
       void* args[] = {&di, &nn, &ft, &nft, &et, &net, &d0, &ns, &bar, &status};
       kp.kernelParams = args;
       kp.extra = nullptr;
-      ENS_CUDA(cudaGraphExecKernelNodeSetParams(exec, p_node, &kp));
+      ENS_CUDA(cudaGraphExecKernelNodeSetParams(one.exec, p_node, &kp));
       graph_dt0 = dt0;
       graph_steps = nst;
     }
-    ENS_CUDA(cudaGraphLaunch(exec, stream));
+    ENS_CUDA(cudaGraphLaunch(one.exec, stream));
     return SPLASH_OK;
   }
 
-  int step(double dt0) {
-    if (dt0 != graph_dt0) {
-      cudaKernelNodeParams kp{};
-      ENS_CUDA(cudaGraphKernelNodeGetParams(dt0_node, &kp));
-      const EnsInstance* di = d_inst;
-      int nn = n;
-      void* args[] = {&di, &nn, &dt0};
-      kp.kernelParams = args;
-      kp.extra = nullptr;
-      ENS_CUDA(cudaGraphExecKernelNodeSetParams(exec, dt0_node, &kp));
-      graph_dt0 = dt0;
-    }
-    ENS_CUDA(cudaGraphLaunch(exec, stream));
+  // dt0 of the five-launch graphs: an argument of their finalize nodes
+  int set_dt0(double dt0) {
+    if (dt0 == graph_dt0) return SPLASH_OK;
+    cudaKernelNodeParams kp{};
+    ENS_CUDA(cudaGraphKernelNodeGetParams(one.dt0_nodes[0], &kp));
+    const EnsInstance* di = d_inst;
+    int nn = n;
+    void* args[] = {&di, &nn, &dt0};
+    kp.kernelParams = args;
+    kp.extra = nullptr;
+    for (StepGraph* g : {&one, &several})
+      for (cudaGraphNode_t nd : g->dt0_nodes) ENS_CUDA(cudaGraphExecKernelNodeSetParams(g->exec, nd, &kp));
+    graph_dt0 = dt0;
     return SPLASH_OK;
   }
 };
@@ -374,6 +397,7 @@ int splash_ensemble_create(const splash_member* members, int n, int device, int 
         L.G.fpad = L.sp.fpad;
         L.G.max_slots = L.sp.max_slots;
         L.G.nslots = e->upload(L.sp.nslots);
+        L.d_iperm = e->upload(L.sp.iperm);
         L.G.fcn = e->upload(L.sp.fcn);
         L.G.fcn32 = e->upload(mp.fcn32);
         L.G.fcn_lo = e->upload(mp.fcn_lo);
@@ -424,8 +448,10 @@ int splash_ensemble_create(const splash_member* members, int n, int device, int 
     ENS_CUDA(cudaMemset(e->err, 0, (size_t)n * 4 * sizeof(unsigned)));
     size_t max_fpad = 0;
     for (const auto& L : e->levels) max_fpad = std::max(max_fpad, (size_t)L.sp.fpad);
-    e->stage_len = max_fpad * kDim;
-    ENS_CUDA(cudaMallocHost(&e->h_stage, e->stage_len * sizeof(double)));
+    ENS_CUDA(cudaMallocHost(&e->h_stage, max_fpad * kDim * sizeof(double)));
+    int pma = 0;
+    if (cudaDeviceGetAttribute(&pma, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess)
+      e->host_direct = pma != 0 && std::getenv("SPLASH_STAGED_TRANSFERS") == nullptr;
     for (int i = 0; i < n; ++i) {
       const splash_member& m = members[i];
       const splash::Level& L = e->levels[e->member_level[i]];
@@ -559,13 +585,14 @@ int splash_ensemble_get_state(splash_ensemble* h, int member, double* U) {
   const splash::Level& L = e->levels[e->member_level[member]];
   const int nf = L.sp.n_faces, fp = L.sp.fpad;
   const int mdim = (e->inst[member].P.solver == splash::kSolverIsoHLLE) ? 4 : splash::kDim;
-  ENS_CUDA(cudaMemcpyAsync(e->h_stage, e->inst[member].S.U, (size_t)fp * splash::kDim * sizeof(double),
-                           cudaMemcpyDeviceToHost, e->stream));
+  // one gather kernel into the caller's array, or into the page-locked stage
+  // (a strided copy loop on the host took 48 members on hex(3..7) 2.2 ms)
+  double* dst = e->host_direct ? U : e->h_stage;
+  ENS_CUDA(splash::fp64_gather_state(e->inst[member].S.U, L.d_iperm, dst, nf, fp, e->stream, mdim));
   ENS_CUDA(cudaStreamSynchronize(e->stream));
   const int rc = e->check_status();
   if (rc) return rc;
-  for (int q = 0; q < nf; ++q)
-    for (int k = 0; k < mdim; ++k) U[(size_t)L.sp.perm[q] * mdim + k] = e->h_stage[(size_t)k * fp + q];
+  if (!e->host_direct) std::memcpy(U, dst, (size_t)nf * mdim * sizeof(double));
   return SPLASH_OK;
 }
 

@@ -265,3 +265,23 @@ def test_two_thread_launches_equal_batched_launches(kind, level, solver):
     assert np.array_equal(ens.get_state(0), s.get_state())
     info = ens.member_info(0)
     assert info["t"] == s.time() and info["dt"] == s.last_dt() and info["err"] == s.error_word()
+
+
+@pytest.mark.parametrize("direct", [True, False])
+@pytest.mark.parametrize("steps", [1, 3, 4, 6, 9])
+def test_multi_step_graphs_and_downloads(monkeypatch, steps, direct):
+    """do_steps(n) is n single steps, whether n fills the graphs of several steps or not, across a change of dt0; a
+    member's state comes back the same straight into the caller's array and through the page-locked stage."""
+    import splash_gb300 as sg
+
+    if not direct:
+        monkeypatch.setenv("SPLASH_STAGED_TRANSFERS", "1")
+    ms = members()[:3]
+    a, b = sg.Ensemble(ms, autotune=False), sg.Ensemble(ms, autotune=False)
+    for dt0 in (1e-3, 5e-4):
+        a.do_steps(steps, dt0)
+        for _ in range(steps):
+            b.do_steps(1, dt0)
+    for i in range(len(ms)):
+        assert np.array_equal(a.get_state(i), b.get_state(i)), i
+        assert a.member_info(i) == b.member_info(i)
