@@ -377,52 +377,23 @@ SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom&
 // (r = +-inf or NaN) d up / d dp = hg phi.
 constexpr int kTapePlanes = 15;  // 3 per field
 
-// limiter_field with its partial derivatives in r and nu; inu = 1 / nu
-// (22 FP64 instructions beside the value's, against 2 per instruction of the
-// value for a dual number over (r, nu))
-struct Phi {
-  double v, r, nu;
-};
-SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double inu) {
-  if (nan_bits(r)) return Phi{0., 0., 0.};
-  if (odd_bits(r)) return Phi{limiter_field(r, l), 0., 0.};
-  // the superbee: max(0, max(min(1, r sb), min(r, eta_p)))
-  Phi A{1., 0., 0.};
-  const double rs = r * l.sb;
-  if (less(rs, 1.)) A = Phi{rs, l.sb, -rs * inu};
-  const Phi B = less(l.eta_p, r) ? Phi{l.eta_p, 0., 0.} : Phi{r, 1., 0.};
-  Phi sb = less(A.v, B.v) ? B : A;
-  if (!less(0., sb.v)) sb = Phi{0., 0., 0.};
-  // the third-order line t1 + ts r below it, not below 0
-  const double t = fma(l.ts, r, l.t1);
-  Phi to = sb;
-  if (less(t, sb.v)) to = Phi{t, l.ts, (r - 1) * (1.0 / 3)};
-  if (!less(0., to.v)) to = Phi{0., 0., 0.};
-  if (to.v == sb.v) return sb;
-  if (!(r > 0.0)) return to;
-  const Dual<1> h = switch_pos(Dual<1>::seed(r, 0));
-  return Phi{fma(h.v, sb.v - to.v, to.v), fma(h.v, sb.r - to.r, fma(h.d[0], sb.v - to.v, to.r)),
-             fma(h.v, sb.nu - to.nu, to.nu)};
-}
-
 // nb as in recon_side; lj(3 k + i) receives the partials of field k
 template <class NbFn, class LjFn>
 SPLASH_HD void recon_side_tape(const SideGeom& g, double gam, double dt, const double* w, NbFn nb, double* up,
                                LjFn lj) {
-  const double nu = side_courant(g, gam, dt, w);
-  const LimiterLine<double> line = limiter_line(g, nu);
-  const double inu = recip(nu);
+  double c;
+  const double nu = side_courant(g, gam, dt, w, c);
+  const SideLimiterPartials limiter(g, nu, w[0], w[4], c);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    double dp, dm;
+    double dp, dm, r;
     side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
-    const double r = slope_ratio(g, dp, dm);
-    const Phi phi = limiter_partials(r, line, inu);
-    const double dg = dp * g.hg;
-    up[k] = fm(dg, phi.v, w[k]);
+    const double num = dm * g.hr, dpg = dp * g.hg;
+    const Phi phi = limiter(k, dp, num, dpg, r);
+    up[k] = fm(dpg, phi.v, w[k]);
     lj(3 * k, g.hg * ((phi.r != 0.0) ? fma(-phi.r, r, phi.v) : phi.v));
     lj(3 * k + 1, g.hg * g.hr * phi.r);
-    lj(3 * k + 2, dg * phi.nu);
+    lj(3 * k + 2, dpg * phi.nu);
   }
 }
 

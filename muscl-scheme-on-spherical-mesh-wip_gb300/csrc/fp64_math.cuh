@@ -263,60 +263,63 @@ SPLASH_HD double switch_formula(double r, double& slope) {
   return 0.0;
 }
 
-#if defined(__CUDACC__) && defined(SPLASH_SWITCH_TABLE)
+#if defined(SPLASH_SWITCH_TABLE)
+#if defined(__CUDACC__)
+#define SPLASH_TABLE __device__ __align__(64)
+#else
+#define SPLASH_TABLE static
+#endif
 #include "limiter_switch_table.inc"  // written by limiter_table.py at build time
+#endif
 
+#if defined(__CUDACC__) && defined(SPLASH_SWITCH_TABLE)
 __device__ __forceinline__ double horner8(const double* __restrict__ row, double d) {
   const double2* c = reinterpret_cast<const double2*>(row);
   const double2 a = __ldg(c), b = __ldg(c + 1), e = __ldg(c + 2), f = __ldg(c + 3);
   return ::fma(::fma(::fma(::fma(::fma(::fma(::fma(f.y, d, f.x), d, e.y), d, e.x), d, b.y), d, b.x), d, a.y), d, a.x);
 }
-// The row of r > 0 and the offset from its centre; row -1: r - 1 below
-// -2^-16 or past the table (limiter_table.py describes the intervals).
+// The row of r > 0 and the offset from its centre; row -1: 1 - r below
+// 2^-40 or past the table (limiter_table.py describes the intervals).
 __device__ __forceinline__ int switch_row(double r, double& d) {
   const uint32_t hr = high_word(r);
   const bool above = hr >= 0x3ff00000u;
   const double u = above ? r : 1 - r;
   const uint32_t hu = high_word(u);
   const int sh = above ? 12 : 15;
-  int row = (int)(hu >> sh) - (above ? (1023 << 8) - 512 : 1007 << 5);
+  int row = (int)(hu >> sh) - (above ? (1023 << 8) - 1280 : 983 << 5);
   uint32_t mid = ((hu >> sh) << sh) | (1u << (sh - 1));
   if (!above && hu == 0x3ff00000u) {  // u = 1: the end of the last interval
-    row = 511;
+    row = 1279;
     mid = 0x3fefc000u;
   }
   d = u - __hiloint2double((int)mid, 0);
-  return (above ? row < 800 : row >= 0) ? row : -1;
+  return (above ? row < 1568 : row >= 0) ? row : -1;
 }
 #endif
 
-// h(r) for r > 0 (not NaN)
-template <class T>
-SPLASH_HD T switch_pos(const T& r) {
-  const double x = val(r);
-  double h, slope = 0.0;
+// h(r) for r > 0 (not NaN), and dh/dr
+SPLASH_HD double switch_pos(double r, double& slope) {
 #if defined(__CUDA_ARCH__) && defined(SPLASH_SWITCH_TABLE)
-  if (high_word(x) >= 0x40020000u) {  // r >= 2.25
-    h = 1.0;
-  } else {
-    double d;
-    const int row = switch_row(x, d);
-    if (row >= 0) {
-      h = horner8(kSwitchTable[row], d);
-      if constexpr (is_dual<T>::value) slope = horner8(kSwitchSlope[row], d);
-    } else {
-      h = switch_formula(x, slope);
-    }
+  slope = 0.0;
+  if (high_word(r) >= 0x40020000u) return 1.0;  // r >= 2.25
+  double d;
+  const int row = switch_row(r, d);
+  if (row >= 0) {
+    slope = horner8(kSwitchSlope[row], d);
+    return horner8(kSwitchTable[row], d);
   }
-#else
-  h = switch_formula(x, slope);
 #endif
-  T o(h);
-  if constexpr (is_dual<T>::value) {
-#pragma unroll
-    for (int i = 0; i < T::kN; ++i) o.d[i] = slope * r.d[i];
-  }
-  return o;
+  return switch_formula(r, slope);
+}
+SPLASH_HD double switch_pos(double r) {
+#if defined(__CUDA_ARCH__) && defined(SPLASH_SWITCH_TABLE)
+  if (high_word(r) >= 0x40020000u) return 1.0;
+  double d;
+  const int row = switch_row(r, d);
+  if (row >= 0) return horner8(kSwitchTable[row], d);
+#endif
+  double slope;
+  return switch_formula(r, slope);
 }
 
 // 1 - h^M with h = min(a / b, b / a) for a, b > 0 (the pressure switch of

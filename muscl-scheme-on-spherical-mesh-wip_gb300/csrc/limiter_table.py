@@ -11,13 +11,16 @@ and seven fused multiply-adds) instead of a logarithm, two exponentials and a
 division.  The intervals follow the bits of the argument, so that a shift of
 its high word is the row and its centre:
 
-    0 < r < 1    u = 1 - r, 32 intervals per power of two, 2^-16 <= u <= 1
-                 (rows 0 .. 511; h is smooth in log u, its slope unbounded at 0)
-    1 <= r < 2   u = r, 256 intervals (rows 512 .. 767)
-    2 <= r < 2.25  32 intervals (rows 768 .. 799); from 2.25 on h is 1 to the
+    0 < r < 1    u = 1 - r, 32 intervals per power of two, 2^-40 <= u <= 1
+                 (rows 0 .. 1279; h is smooth in log u, its slope unbounded at 0)
+    1 <= r < 2   u = r, 256 intervals (rows 1280 .. 1535)
+    2 <= r < 2.25  32 intervals (rows 1536 .. 1567); from 2.25 on h is 1 to the
                  last bit
 
-A second table holds dh/dr in the same form, for the derivative kernels.
+A second table holds dh/dr in the same form, for the derivative kernels, and
+a third the coefficients of h for pairs of floats (limiter_pair.cuh): the
+first four as a float and its remainder, the others, whose terms are below
+2^-24 of h, rounded to a float; below 1 they are those of u scaled to [1, 2).
 Each polynomial interpolates at the 8 Chebyshev nodes of its interval and is
 evaluated here in 45-digit decimal arithmetic; only the coefficients are
 rounded.  Against the formulas h is within 1.1e-16 (absolute)
@@ -26,12 +29,13 @@ and dh/dr within 5e-16 of the larger of 1 and its interval's largest value.
 from __future__ import annotations
 
 import math
+import struct
 import sys
 from decimal import Decimal as D, getcontext
 from pathlib import Path
 
 DEGREE = 7
-OCTAVES, PER_OCTAVE = 16, 32
+OCTAVES, PER_OCTAVE = 40, 32
 ROWS_BELOW = OCTAVES * PER_OCTAVE
 ROWS_1_2, ROWS_2_UP = 256, 32
 ROWS = ROWS_BELOW + ROWS_1_2 + ROWS_2_UP
@@ -95,13 +99,30 @@ def tables() -> tuple[list[list[float]], list[list[float]]]:
     return value, slope
 
 
+def to_float(x: float) -> float:
+    return struct.unpack("f", struct.pack("f", x))[0]
+
+
+def pair_row(row: list[float]) -> list[float]:
+    """c0 .. c3 as a float and its remainder, then c4 .. c7 (48 bytes)."""
+    out = []
+    for c in row[:4]:
+        out += [to_float(c), to_float(c - to_float(c))]
+    return out + [to_float(c) for c in row[4:]]
+
+
 def write(path: Path) -> None:
     value, slope = tables()
     lines = ["// written by limiter_table.py: rows of " + str(DEGREE + 1) + " coefficients, constant term first"]
     for name, table in (("kSwitchTable", value), ("kSwitchSlope", slope)):
-        lines.append(f"__device__ const double __align__(64) {name}[{ROWS}][{DEGREE + 1}] = {{")
+        lines.append(f"SPLASH_TABLE const double {name}[{ROWS}][{DEGREE + 1}] = {{")
         lines += ["  {" + ", ".join(c.hex() for c in row) + "}," for row in table]
         lines.append("};")
+    lines.append(f"SPLASH_TABLE const float kSwitchPairs[{ROWS}][12] = {{")
+    for i, row in enumerate(value):
+        scale = 2.0 ** (i // PER_OCTAVE - OCTAVES) if i < ROWS_BELOW else 1.0
+        lines.append("  {" + ", ".join(c.hex() + "f" for c in pair_row([c * scale**k for k, c in enumerate(row)])) + "},")
+    lines.append("};")
     path.write_text("\n".join(lines) + "\n")
 
 

@@ -302,17 +302,11 @@ struct LimiterLine {
 template <class T>
 SPLASH_HD T limiter_field(const T& r, const LimiterLine<T>& l) {
   if (is_nan(r)) return T(0.);
-  if constexpr (is_dual<T>::value) {
-    // r = +-inf (a zero forward difference): the limiter is flat there in r
-    // and in the Courant factor; the dual chain would form 0 * inf
-    if (is_inf(r))
-      return T(limiter_field(val(r), LimiterLine<double>{l.eta_p, val(l.sb), val(l.ts), val(l.t1)}));
-  }
   const T sb = smax(T(0.), smax(smin(T(1.), r * l.sb), smin(r, T(l.eta_p))));
   const T to = smax(T(0.), smin(sb, fm(l.ts, r, l.t1)));
   if (val(to) == val(sb)) return sb;
   if (!(val(r) > 0.0)) return to;
-  return fm(switch_pos(r), sb - to, to);
+  return fm(switch_pos(val(r)), sb - to, to);
 }
 // The same for a positive, finite superbee scale (nu > 0: no supersonic
 // inflow) on integer comparisons alone: then every operand of the min and max

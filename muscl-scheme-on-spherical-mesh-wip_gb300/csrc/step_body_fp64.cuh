@@ -11,6 +11,7 @@
 
 #include "dual.cuh"
 #include "layout.hpp"
+#include "limiter_pair.cuh"
 #include "physics_fp64.cuh"
 
 namespace splash {
@@ -118,16 +119,15 @@ SPLASH_HD EdgeGeom edge_geom(const DevGeom& G, int e) {
 // face state w on one side of an edge, (c + v.n) dt arc / area with
 // v.n = -(l . (n x R)) / Sigma, and what the limiter makes of it.
 template <class T>
-SPLASH_HD T side_courant(const SideGeom& g, double gam, double dt, const T* w) {
+SPLASH_HD T side_courant(const SideGeom& g, double gam, double dt, const T* w, T& c) {
   const T ir = recip(w[0]);
-  const T c = root(gam * (w[4] * ir));
+  c = root(gam * (w[4] * ir));
   const T vn = -(fdot(g.nxr, v3(w[1], w[2], w[3])) * ir);
   return (c + vn) * (dt * g.arc_a);
 }
-template <class T>
-SPLASH_HD LimiterLine<T> limiter_line(const SideGeom& g, const T& nu) {
-  const T ts = fm(nu, 1.0 / 3, T(1.0 / 3));
-  return LimiterLine<T>{g.eta_p, divide(g.sbs, nu), ts, 1.0 - ts};
+SPLASH_HD LimiterLine<double> limiter_line(double eta_p, double sbs, double nu) {
+  const double ts = fma(nu, 1.0 / 3, 1.0 / 3);
+  return LimiterLine<double>{eta_p, divide(sbs, nu), ts, 1.0 - ts};
 }
 
 // The differences of one field across the side: dp = U+ - w, dm = w - U-
@@ -138,39 +138,170 @@ SPLASH_HD void side_differences(const SideGeom& g, const T& w, const T& a, const
   dp = fm(g.b1, b, fm(g.b0, a, -w));
   dm = fm(-g.b3, d, fm(-g.b2, c, w));
 }
-// r = (dm / H-) / (dp / H+)
-template <class T>
-SPLASH_HD T slope_ratio(const SideGeom& g, const T& dp, const T& dm) {
-  const T num = dm * g.hr;
-  const double y = recip(val(dp));
-  double v = val(num) * y;
-  if (odd_bits(v)) v = exact_quotient(val(num), val(dp));
-  T r(v);
-  if constexpr (is_dual<T>::value) {
-#pragma unroll
-    for (int i = 0; i < T::kN; ++i) r.d[i] = fma(-v, dp.d[i], num.d[i]) * y;
-  }
-  return r;
+// r = num / dp with num = hr dm: (dm / H-) / (dp / H+)
+SPLASH_HD double slope_ratio(double dp, double num) {
+  const double v = num * recip(dp);
+  return odd_bits(v) ? exact_quotient(num, dp) : v;
 }
+
+// The limiter of one field in FP64; out of line, as the rarer path.
+SPLASH_COLD double limiter_full(double dp, double num, double eta_p, double sb, double ts, double t1) {
+  const LimiterLine<double> line{eta_p, sb, ts, t1};
+  const bool pos = (int64_t)bits_of(sb) > 0 && !odd_bits(sb);
+  const double r = slope_ratio(dp, num);
+  return pos ? limiter_field_pos(r, line) : limiter_field(r, line);
+}
+
+// One side's limiter: what its fields share, and the value for one field.
+struct SideLimiter {
+  double eta_p, sbs, nu;
+#if defined(SPLASH_SWITCH_TABLE)
+  PairLine pairs;
+#endif
+  int scale[kDim];  // exponent fields that the differences are measured against
+
+  // The differences of Sigma and Pi are measured against the face's own
+  // values, those of l against Sigma c: the momentum equation carries Pi =
+  // Sigma c^2 / gam beside them.
+  SPLASH_HD SideLimiter(const SideGeom& g, double nu_, double w0, double w4, double c)
+      : eta_p(g.eta_p), sbs(g.sbs), nu(nu_) {
+    scale[0] = exponent_field(w0);
+    scale[1] = scale[2] = scale[3] = scale[0] + exponent_field(c) - 1023;
+    scale[4] = exponent_field(w4);
+#if defined(SPLASH_SWITCH_TABLE)
+    pairs = pair_line(eta_p, sbs, nu);
+#endif
+  }
+  // the limiter in pairs of floats, where they serve; dpg = dp BM / H+
+  SPLASH_HD bool in_pairs(int k, double dp, double num, double dpg, double& lim) const {
+#if defined(SPLASH_SWITCH_TABLE)
+    return shallow(dpg, scale[k]) && limiter_pair(dp, num, dp - num, pairs, lim);
+#else
+    return false;
+#endif
+  }
+  // line: limiter_line of the side, used where pairs do not serve
+  SPLASH_HD double operator()(int k, double dp, double num, double dpg, const LimiterLine<double>& line) const {
+    double lim;
+    if (in_pairs(k, dp, num, dpg, lim)) return lim;
+    return limiter_full(dp, num, line.eta_p, line.sb, line.ts, line.t1);
+  }
+  // whether any field may need the line
+  SPLASH_HD bool needs_line(const double* dp, const double* num, const double* dpg) const {
+#if defined(SPLASH_SWITCH_TABLE)
+    bool need = !pairs.ok;
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) need = need || !shallow(dpg[k], scale[k]) || !pair_range(dp[k], num[k]);
+    return need;
+#else
+    return true;
+#endif
+  }
+};
+
+// The limiter of one field with its partial derivatives in r and nu.  The
+// value is SideLimiter's, bit for bit.
+struct Phi {
+  double v, r, nu;
+};
+SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double inu) {
+  if (nan_bits(r)) return Phi{0., 0., 0.};
+  if (odd_bits(r)) return Phi{limiter_field(r, l), 0., 0.};  // flat in r and in the Courant factor
+  // the superbee: max(0, max(min(1, r sb), min(r, eta_p)))
+  Phi A{1., 0., 0.};
+  const double rs = r * l.sb;
+  if (less(rs, 1.)) A = Phi{rs, l.sb, -rs * inu};
+  const Phi B = less(l.eta_p, r) ? Phi{l.eta_p, 0., 0.} : Phi{r, 1., 0.};
+  Phi sb = less(A.v, B.v) ? B : A;
+  if (!less(0., sb.v)) sb = Phi{0., 0., 0.};
+  // the third-order line t1 + ts r below it, not below 0
+  const double t = fma(l.ts, r, l.t1);
+  Phi to = sb;
+  if (less(t, sb.v)) to = Phi{t, l.ts, (r - 1) * (1.0 / 3)};
+  if (!less(0., to.v)) to = Phi{0., 0., 0.};
+  if (to.v == sb.v) return sb;
+  if (!(r > 0.0)) return to;
+  double slope;
+  const double h = switch_pos(r, slope);
+  return Phi{fma(h, sb.v - to.v, to.v), fma(h, sb.r - to.r, fma(slope, sb.v - to.v, to.r)),
+             fma(h, sb.nu - to.nu, to.nu)};
+}
+struct SideLimiterPartials : SideLimiter {
+  LimiterLine<double> line;
+  double inu;
+  SPLASH_HD SideLimiterPartials(const SideGeom& g, double nu_, double w0, double w4, double c)
+      : SideLimiter(g, nu_, w0, w4, c), line(limiter_line(g.eta_p, g.sbs, nu_)), inu(recip(nu_)) {}
+  // r receives the ratio
+  SPLASH_HD Phi operator()(int k, double dp, double num, double dpg, double& r) const {
+    r = slope_ratio(dp, num);
+    Phi phi = limiter_partials(r, line, inu);
+    double v;
+    if (in_pairs(k, dp, num, dpg, v)) phi.v = v;
+    return phi;
+  }
+};
 
 // The limited state (Sigma, l, Pi) of one side: up = w + dp phi(r) BM / H+.
 // nb(k, q) returns field k of stencil face q (0, 1: plus pair, 2, 3: minus).
 template <class T, class NbFn>
 SPLASH_HD void recon_side(const SideGeom& g, double gam, double dt, const T* w, NbFn nb, T* up) {
-  const T nu = side_courant(g, gam, dt, w);
-  const LimiterLine<T> line = limiter_line(g, nu);
-  const bool pos = (int64_t)bits_of(val(line.sb)) > 0 && !odd_bits(val(line.sb));
+  T c;
+  const T nu = side_courant(g, gam, dt, w, c);
+  using Limiter = std::conditional_t<is_dual<T>::value, SideLimiterPartials, SideLimiter>;
+  const Limiter limiter(g, val(nu), val(w[0]), val(w[4]), val(c));
+  T num[kDim], dpg[kDim], dp[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    T dp, dm;
-    side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
-    const T r = slope_ratio(g, dp, dm);
-    T lim;
-    if constexpr (std::is_same<T, double>::value)
-      lim = pos ? limiter_field_pos(r, line) : limiter_field(r, line);
-    else
-      lim = limiter_field(r, line);
-    up[k] = fm(dp * g.hg, lim, w[k]);
+    T dm;
+    side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp[k], dm);
+    num[k] = dm * g.hr;
+    dpg[k] = dp[k] * g.hg;
+  }
+  if constexpr (is_dual<T>::value) {
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      double r;
+      const Phi phi = limiter(k, dp[k].v, num[k].v, dpg[k].v, r);
+      const bool flat = odd_bits(r);  // the limiter is flat where the ratio is no number
+      const double idp = flat ? 0.0 : recip(dp[k].v);
+      T lim(phi.v);
+#pragma unroll
+      for (int i = 0; i < T::kN; ++i) {
+        const double rd = flat ? 0.0 : fma(-r, dp[k].d[i], num[k].d[i]) * idp;
+        lim.d[i] = fma(phi.r, rd, phi.nu * nu.d[i]);
+      }
+      up[k] = fm(dpg[k], lim, w[k]);
+    }
+  } else {
+    double dpv[kDim], numv[kDim], dpgv[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      dpv[k] = val(dp[k]);
+      numv[k] = val(num[k]);
+      dpgv[k] = val(dpg[k]);
+    }
+    LimiterLine<double> line{};
+    if (limiter.needs_line(dpv, numv, dpgv)) {
+#if defined(__CUDA_ARCH__)
+      asm volatile("");  // a branch: evaluated beside it, the line costs 8 FP64 instructions on every path
+#endif
+      line = limiter_line(g.eta_p, g.sbs, val(nu));
+    }
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      T lim;
+      if constexpr (std::is_same<T, double>::value) {
+        lim = limiter(k, dpv[k], numv[k], dpgv[k], line);
+      } else {
+        // the recorded branches decide; where they are the values' own, so is the value
+        const LimiterLine<double> all = limiter_line(g.eta_p, g.sbs, val(nu));
+        const double r = slope_ratio(dpv[k], numv[k]);
+        lim = limiter_field(T(r), LimiterLine<T>{all.eta_p, T(all.sb), T(all.ts), T(all.t1)});
+        if (bits_of(val(lim)) == bits_of(limiter_field(r, all)))
+          lim = T(limiter(k, dpv[k], numv[k], dpgv[k], line));
+      }
+      up[k] = fm(dpg[k], lim, w[k]);
+    }
   }
 }
 

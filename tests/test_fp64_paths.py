@@ -29,9 +29,14 @@ def _p(a):
 def lib(tmp_path_factory):
     if shutil.which("g++") is None:
         pytest.skip("g++ not available")
-    out = tmp_path_factory.mktemp("fp64paths") / "libfp64paths.so"
+    sys.path.insert(0, str(CSRC))
+    import limiter_table
+
+    tmp = tmp_path_factory.mktemp("fp64paths")
+    limiter_table.write(tmp / "limiter_switch_table.inc")
+    out = tmp / "libfp64paths.so"
     subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-ffp-contract=off", "-Wno-unknown-pragmas",
-                    f"-I{CSRC}", f"-I{REPO / 'include'}", str(REPO / "tests" / "cpp" / "fp64_paths.cpp"), "-o", str(out)],
+                    "-DSPLASH_SWITCH_TABLE", f"-I{tmp}", f"-I{CSRC}", f"-I{REPO / 'include'}", str(REPO / "tests" / "cpp" / "fp64_paths.cpp"), "-o", str(out)],
                    check=True, capture_output=True)
     return ctypes.CDLL(str(out))
 
@@ -53,6 +58,43 @@ def test_limiter_positive_path_is_the_general_path(lib, eta_p):
     assert (a > 0).any() and np.isfinite(a).all()
 
 
+@pytest.mark.parametrize("eta_p", [1.0, 1.7, 2.24])
+def test_limiter_in_pairs_of_floats(lib, eta_p):
+    """Against the FP64 limiter, with ratios over the whole range, near 1, near the switch's table edges and near eta_p,
+    differences of every size and sign, Courant factors from 1e-5 to 4: within 2^-44 (the ratio and its distance from 1
+    carry 2^-46 each; they reach the value with weights up to 2.3 and with the switch's slope, up to 5.6 there where the
+    distance is below 1)."""
+    rng = np.random.default_rng(2)
+    n = 400_000
+    r = np.concatenate([rng.uniform(0, 4, n), 1 + rng.choice([-1, 1], n) * np.exp2(rng.uniform(-52, -1, n)),
+                        np.exp(rng.uniform(-30, 30, n)), eta_p * (1 + np.exp2(rng.uniform(-52, -4, n))),
+                        1 - np.exp2(-rng.integers(1, 39, n).astype(float)) * (1 + rng.choice([-1e-9, 0, 1e-9], n)),
+                        1 + rng.integers(0, 320, n) / 256.0, -rng.uniform(0, 3, n)])
+    dp = rng.choice([-1, 1], r.size) * np.exp2(rng.uniform(-200, 200, r.size))
+    num = r * dp
+    nu = np.exp(rng.uniform(np.log(1e-5), np.log(4), r.size))
+    pairs, full, served = np.empty_like(r), np.empty_like(r), np.empty(r.size, dtype=np.int32)
+    lib.limiter_pairs(len(r), _p(dp), _p(num), _p(nu), ctypes.c_double(eta_p), ctypes.c_double(0.16), _p(pairs), _p(full),
+                      served.ctypes.data_as(ctypes.POINTER(ctypes.c_int)))
+    ok = served == 1
+    assert ok.mean() > 0.9
+    assert np.abs(pairs - full)[ok].max() <= 2.0**-44
+
+
+def test_limiter_pairs_leave_the_odd_cases(lib):
+    """Zero, subnormal, infinite and NaN differences, ratios past 2^60 or within 2^-40 below 1, and Courant factors that
+    are not positive and finite are left to FP64; a vanishing numerator gives 0."""
+    tiny, inf, nan = 5e-324, np.inf, np.nan
+    dp = np.array([0.0, tiny, inf, nan, 1.0, 1.0, 1.0, 1e-300, 1.0, 1.0, 1.0, 1.0, 1.0, 3.0, 1.0])
+    num = np.array([1.0, 1.0, 1.0, 1.0, inf, nan, 1 - 2.0**-45, 1.0, 0.5, 0.5, 0.5, 0.5, 0.5, 0.0, -0.5])
+    nu = np.array([0.1, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1, 0.0, -0.1, inf, nan, 1e-30, 0.1, 0.1])
+    pairs, full, served = np.empty_like(dp), np.empty_like(dp), np.empty(dp.size, dtype=np.int32)
+    lib.limiter_pairs(len(dp), _p(dp), _p(num), _p(nu), ctypes.c_double(2.0), ctypes.c_double(0.16), _p(pairs), _p(full),
+                      served.ctypes.data_as(ctypes.POINTER(ctypes.c_int)))
+    assert list(served) == [0] * 13 + [1, 1]
+    assert pairs[-2] == pairs[-1] == 0.0
+
+
 def test_switch_table_is_the_switch():
     """Each row at its two ends and inside, its polynomial evaluated in double as the kernels do (without their fused
     rounding): h within 2 ulp of 1 (the row's constant and the sum round once each), dh/dr within 1e-14 of the larger
@@ -61,7 +103,7 @@ def test_switch_table_is_the_switch():
     import limiter_table as lt
 
     value, slope = lt.tables()
-    assert len(value) == len(slope) == lt.ROWS == 800
+    assert len(value) == len(slope) == lt.ROWS == 1568
     for i, (centre, half, formula) in enumerate(lt.rows()):
         for x in (-1.0, -0.37, 0.0, 0.61, 1.0):
             d = float(half) * x
