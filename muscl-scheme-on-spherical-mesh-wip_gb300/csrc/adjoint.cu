@@ -56,6 +56,7 @@ constexpr int kBlock = 64;                // faces per block
 constexpr int kThreads = 2 * kEdgeBlock;  // edge launches: a thread per side, as in step_fp64.cu
 
 inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
+inline int face_blocks(int n) { return (n + kFaces - 1) / kFaces; }
 inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
 
 __device__ __forceinline__ D1 dual1(double v, double d) {
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState
     }
     dt_fold(wv, r, P, vel2, rate2, negative);
   }
-  fold_block<kBlock>(vel2, rate2, negative, S, P);
+  fold_warp(vel2, rate2, negative, S, P, gridDim.x * (kBlock / 32));
 }
 
 template <int STAGE>
@@ -128,27 +129,42 @@ __global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState 
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) tlm_update_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vel2 = 0.0, rate2 = 0.0;
-  bool negative = false;
-  if (f < G.n_faces) {
-    const size_t fp = G.fpad;
-    const double dt = S.scal[kScDt];
+__global__ void __launch_bounds__(kFaceThreads) tlm_update_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
+  __shared__ FaceParts<D1, 2 * kDim> parts;
+  const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
+  const bool live = f < G.n_faces;
+  const size_t fp = G.fpad;
+  if (live && part < kDim) {
+    const Planes<D1> fe{S.fe, T.dfe, 0};
+    parts.put(part, i, flux_sum<D1>(G, f, [&](int e) { return fe.ld((size_t)part * G.epad + e); }));
+  } else if (live) {
     const SrcParams<D1> sp{dual1(G.acc_src[f], T.dacc[f]),
                            v3(D1(P.omega_acc_x), dual1(P.omega_acc_y, T.d_omega_y), dual1(P.omega_acc_z, T.d_omega_z)),
                            dual1(P.acc_rate, T.d_rate), dual1(P.total_mass, T.d_total_mass)};
     const Planes<D1> Win = (STAGE == 1) ? Planes<D1>{S.W0, T.dW0, 0} : Planes<D1>{S.W1, T.dW1, 0};
-    const Planes<D1> U{S.U, T.dU, 0}, fe{S.fe, T.dfe, 0};
-    D1 w[kDim], u0[kDim], u[kDim];
+    D1 w[kDim], src[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) w[k] = Win.ld(k * fp + f);
+    source_term(w, plane3(G.fcn, G.fpad, f), sp, P, src);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) parts.put(kDim + k, i, src[k]);
+  }
+  __syncthreads();
+  if (part != 0) return;
+  double vel2 = 0.0, rate2 = 0.0;
+  bool negative = false;
+  if (live) {
+    const double dt = S.scal[kScDt];
+    const Planes<D1> U{S.U, T.dU, 0};
+    D1 sum[kDim], src[kDim], u0[kDim], u[kDim], w[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) {
-      w[k] = Win.ld(k * fp + f);
+      sum[k] = parts.get(k, i);
+      src[k] = parts.get(kDim + k, i);
       u0[k] = U.ld(k * fp + f);
     }
     bool floored;
-    update_face<D1, D1>(G, P, sp, (STAGE == 1) ? 0.5 * dt : dt, w, u0,
-                        [&](int k, int e) { return fe.ld((size_t)k * G.epad + e); }, f, u, floored);
+    combine_face((STAGE == 1) ? 0.5 * dt : dt, src, sum, u0, u, floored);
     const D3 fcn = plane3(G.fcn, G.fpad, f);
     prim_of(u, fcn, P.gam, w);
     const Planes<D1> Wout = (STAGE == 1) ? Planes<D1>{S.W1, T.dW1, 0} : Planes<D1>{S.W0, T.dW0, 0};
@@ -161,7 +177,7 @@ __global__ void __launch_bounds__(kBlock) tlm_update_kernel(DevGeom G, DevState 
     }
     if (STAGE == 2) dt_fold(wv, fcn, P, vel2, rate2, negative);
   }
-  if (STAGE == 2) fold_block<kBlock>(vel2, rate2, negative, S, P);
+  if (STAGE == 2) fold_warp(vel2, rate2, negative, S, P, gridDim.x);
 }
 
 // ---------------------------------------------------------------------
@@ -219,23 +235,27 @@ __global__ void __launch_bounds__(kBlock) tp_flux_kernel(DevGeom G, PhysParams P
     u0[k] = Taped(U0[k * fp + f]);
   }
   const Gas gas = gas_of(P);
-  int have = -1;  // the edge whose flux F holds: the sum asks for its fields in turn
+  Taped src[kDim], sum[kDim];
+  source_term(w, plane3(G.fcn, G.fpad, f), face_src_params<double>(G, P, f), P, src);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) sum[k] = Taped(0.);
+  const int n = G.nslots[f];
+  for (int j = 0; j < n; ++j) {
+    const int se = G.slot_edge[(size_t)j * fp + f];
+    const int e = se & 0x7fffffff;
+    Taped L[kDim], R[kDim];
+#pragma unroll
+    for (int q = 0; q < kDim; ++q) {
+      L[q] = Taped(uplus[q * xs + e]);
+      R[q] = Taped(uplus[q * xs + (G.e_twin ? G.e_twin[e] : G.epad + e)]);
+    }
+    riemann_flux(L, R, edge_geom(G, e), gas, P.solver, F);
+    const double c = G.e_side[kSideCoef * xs + side_index(G, se)];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) sum[k] = fm((se < 0) ? c : -c, F[k], sum[k]);  // flux_sum
+  }
   bool floored;
-  update_face<Taped, double>(
-      G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
-      [&](int k, int e) {
-        if (have != e) {
-          Taped L[kDim], R[kDim];
-          for (int q = 0; q < kDim; ++q) {
-            L[q] = Taped(uplus[q * xs + e]);
-            R[q] = Taped(uplus[q * xs + (G.e_twin ? G.e_twin[e] : G.epad + e)]);
-          }
-          riemann_flux(L, R, edge_geom(G, e), gas, P.solver, F);
-          have = e;
-        }
-        return F[k];
-      },
-      f, u, floored);
+  combine_face((STAGE == 1) ? 0.5 * dt : dt, src, sum, u0, u, floored);
   prim_of(u, plane3(G.fcn, G.fpad, f), P.gam, w);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
@@ -296,24 +316,37 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) rc_update_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                           const double* __restrict__ Win,
-                                                           const double* __restrict__ U0, const double* __restrict__ fe,
-                                                           double* __restrict__ Uout, double* __restrict__ Wout,
-                                                           uint8_t* __restrict__ mask) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= G.n_faces) return;
+__global__ void __launch_bounds__(kFaceThreads) rc_update_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
+                                                                 const double* __restrict__ Win,
+                                                                 const double* __restrict__ U0,
+                                                                 const double* __restrict__ fe, double* __restrict__ Uout,
+                                                                 double* __restrict__ Wout, uint8_t* __restrict__ mask) {
+  __shared__ FaceParts<double, 2 * kDim> parts;
+  const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
+  const bool live = f < G.n_faces;
   const size_t fp = G.fpad;
+  if (live && part < kDim) {
+    parts.put(part, i, flux_sum<double>(G, f, [&](int e) { return fe[(size_t)part * G.epad + e]; }));
+  } else if (live) {
+    double w[kDim], src[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) w[k] = Win[k * fp + f];
+    source_term(w, plane3(G.fcn, G.fpad, f), face_src_params<double>(G, P, f), P, src);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) parts.put(kDim + k, i, src[k]);
+  }
+  __syncthreads();
+  if (part != 0 || !live) return;
   const double dt = *dtp;
-  double w[kDim], u0[kDim], u[kDim];
+  double sum[kDim], src[kDim], u0[kDim], u[kDim], w[kDim];
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    w[k] = Win[k * fp + f];
+    sum[k] = parts.get(k, i);
+    src[k] = parts.get(kDim + k, i);
     u0[k] = U0[k * fp + f];
   }
   bool floored;
-  update_face<double, double>(G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
-                              [&](int k, int e) { return fe[(size_t)k * G.epad + e]; }, f, u, floored);
+  combine_face((STAGE == 1) ? 0.5 * dt : dt, src, sum, u0, u, floored);
   prim_of(u, plane3(G.fcn, G.fpad, f), P.gam, w);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
@@ -392,54 +425,64 @@ __global__ void __launch_bounds__(kThreads) adj_edge_kernel(DevGeom G, PhysParam
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kBlock) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
-                                                          const double* __restrict__ Win,
-                                                          const double* __restrict__ Uin,
-                                                          const uint8_t* __restrict__ mask, const double* lam,
-                                                          double* lam_out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= G.n_faces) return;
+__global__ void __launch_bounds__(kFaceThreads) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
+                                                                const double* __restrict__ Win,
+                                                                const double* __restrict__ Uin,
+                                                                const uint8_t* __restrict__ mask, const double* lam,
+                                                                double* lam_out) {
+  __shared__ FaceParts<double, 2 * kDim> parts;
+  const int part = face_part(), i = threadIdx.x % kFaces, g = blockIdx.x * kFaces + i;
+  const bool live = g < G.n_faces;
   const size_t fp = G.fpad, xs = G.xs;
-  double wb[kDim] = {0, 0, 0, 0, 0};
-  // the interpolants whose stencils hold face g, and the sides that are its own
-  for (int e = X.inv_off[g]; e < X.inv_off[g + 1]; ++e) {
-    const int code = X.inv_ent[e];
-    const size_t x = (size_t)(code >> 3);
-    const int pos = code & 7;
-    if (pos == 4) {
-#pragma unroll
-      for (int k = 0; k < kDim; ++k) wb[k] += X.own[k * xs + x];
-      continue;
-    }
-    const double bt = G.e_side[(size_t)(kSideBeta + pos) * xs + x];
-    const double* src = X.PU + (pos >= 2 ? kDim : 0) * xs;
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) wb[k] = fma(bt, src[k * xs + x], wb[k]);
-  }
-  const D3 fcn = plane3(G.fcn, G.fpad, g);
   // the adjoint of this stage's output state: stage 2's is lam, stage 1's lam1
   const double* out = (STAGE == 2) ? lam : X.lam1;
-  double w[kDim], u[kDim], la[kDim], srcb[kDim], ub[kDim] = {0, 0, 0, 0, 0}, pb[5] = {0, 0, 0, 0, 0};
+  if (live && part < kDim) {
+    // one field over the interpolants whose stencils hold face g, and the
+    // sides that are its own
+    const double *own = X.own + part * xs, *pu = X.PU + part * xs, *mu = X.PU + (kDim + part) * xs;
+    double s = 0.0;
+    const int end = X.inv_off[g + 1];
+#pragma unroll 4
+    for (int e = X.inv_off[g]; e < end; ++e) {
+      const int code = X.inv_ent[e];
+      const size_t x = (size_t)(code >> 3);
+      const int pos = code & 7;
+      const double bt = (pos == 4) ? 1.0 : G.e_side[(size_t)(kSideBeta + (pos & 3)) * xs + x];
+      s = fma(bt, (pos == 4 ? own : pos >= 2 ? mu : pu)[x], s);
+    }
+    parts.put(part, i, s);
+  } else if (live) {
+    double w[kDim], srcb[kDim], wb[kDim] = {0, 0, 0, 0, 0}, pb[5] = {0, 0, 0, 0, 0};
+    if (P.accretion_on) {
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) {
+        w[k] = Win[k * fp + g];
+        srcb[k] = dt_here * masked(out, mask, STAGE, fp, k, g);
+      }
+      rev::source_rev(w, plane3(G.fcn, G.fpad, g), face_src_params<double>(G, P, g), P, srcb, wb, pb);
+#pragma unroll
+      for (int j = 0; j < 5; ++j) X.th[j * fp + g] += pb[j];
+    }
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) parts.put(kDim + k, i, wb[k]);
+  }
+  __syncthreads();
+  if (part != 0 || !live) return;
+  double wb[kDim], u[kDim], ub[kDim] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    w[k] = Win[k * fp + g];
+    wb[k] = parts.get(k, i) + parts.get(kDim + k, i);
     u[k] = Uin[k * fp + g];
-    la[k] = masked(out, mask, STAGE, fp, k, g);
-    srcb[k] = dt_here * la[k];
   }
-  if (P.accretion_on) {
-    rev::source_rev(w, fcn, face_src_params<double>(G, P, g), P, srcb, wb, pb);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) X.th[j * fp + g] += pb[j];
-  }
-  rev::prim_rev(u, fcn, P.gam, wb, ub);
+  rev::prim_rev(u, plane3(G.fcn, G.fpad, g), P.gam, wb, ub);
   if (STAGE == 2) {
 #pragma unroll
     for (int k = 0; k < kDim; ++k) lam_out[k * fp + g] = ub[k];
   } else {
     // U1 = floor(U + acc1) and U2 = floor(U + acc2) both hold U directly
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) lam_out[k * fp + g] = ub[k] + la[k] + masked(lam, mask, 2, fp, k, g);
+    for (int k = 0; k < kDim; ++k)
+      lam_out[k * fp + g] = ub[k] + masked(out, mask, 1, fp, k, g) + masked(lam, mask, 2, fp, k, g);
   }
 }
 
@@ -457,11 +500,11 @@ cudaError_t tlm_prepare(const DevGeom& G, const DevState& S, const TlmTangents& 
 
 cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P, double dt0,
                      cudaStream_t st) {
-  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
   adj::tlm_edge_kernel<1><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
-  adj::tlm_update_kernel<1><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
+  adj::tlm_update_kernel<1><<<nb, f64::kFaceThreads, 0, st>>>(G, S, T, P);
   adj::tlm_edge_kernel<2><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
-  adj::tlm_update_kernel<2><<<nb, adj::kBlock, 0, st>>>(G, S, T, P);
+  adj::tlm_update_kernel<2><<<nb, f64::kFaceThreads, 0, st>>>(G, S, T, P);
   return cudaGetLastError();
 }
 
@@ -514,8 +557,8 @@ cudaError_t rc_prim(const DevGeom& G, const PhysParams& P, const double* U, doub
 
 cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t, double* fe,
                     double* U_next, double* W_next, cudaStream_t st) {
-  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
-  constexpr int B = adj::kBlock, E = adj::kThreads;
+  const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  constexpr int B = f64::kFaceThreads, E = adj::kThreads;
   adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W0, t.P0, t.J0, fe);
   adj::rc_update_kernel<1><<<nb, B, 0, st>>>(G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask);
   adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W1, t.P1, t.J1, fe);
@@ -525,8 +568,8 @@ cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, co
 
 cudaError_t adj_step(const DevGeom& G, const PhysParams& P, double dt, const StepTape& t, const AdjScratch& X,
                      double* lam, cudaStream_t st) {
-  const int nb = adj::blocks_for(G.n_faces), ne = adj::edge_blocks(G.n_edges);
-  constexpr int B = adj::kBlock, E = adj::kThreads;
+  const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
+  constexpr int B = f64::kFaceThreads, E = adj::kThreads;
   // stage 2: U2 = floor(U + dt Phi(W1, P1))
   adj::adj_edge_kernel<<<ne, E, 0, st>>>(G, P, dt, dt, t.W1, t.P1, t.J1, lam, t.mask, 2, X.PU, X.own);
   adj::adj_face_kernel<2><<<nb, B, 0, st>>>(G, P, dt, X, t.W1, t.U1, t.mask, lam, X.lam1);

@@ -370,30 +370,58 @@ struct SideExchange {
 };
 #endif
 
-// res2d + the RK combine with the density floor (MUSCL_base.hpp:238-276,
-// 124-161) for face f: the updated conserved state
-// U0 + dt_here (source - flux divergence), floored, from the edges' fluxes
-// (flux(k, e) gives field k of edge e).
-template <class T, class Q, class FluxFn>
-SPLASH_HD void update_face(const DevGeom& G, const PhysParams& P, const SrcParams<Q>& sp, double dt_here,
-                           const T* w, const T* u0, FluxFn flux, int f, T* u, bool& floored) {
-  const int fp = G.fpad;
-  T acc[kDim];
-  source_term(w, plane3(G.fcn, fp, f), sp, P, acc);
+// res2d and the RK combine with the density floor (MUSCL_base.hpp:238-276,
+// 124-161) of face f, in three parts that the kernels spread over threads:
+// the sum over the face's slots of -+ coef flux of one field (flux(e): that
+// field of edge e's flux), the source (source_term), and the combination.
+template <class T, class FluxFn>
+SPLASH_HD T flux_sum(const DevGeom& G, int f, FluxFn flux) {
+  T acc(0.);
   const int n = G.nslots[f];
   for (int j = 0; j < n; ++j) {
-    const int se = G.slot_edge[j * fp + f];
+    const int se = G.slot_edge[j * G.fpad + f];
     const int e = se & 0x7fffffff;
     const double c = G.e_side[(size_t)kSideCoef * G.xs + (se < 0 ? G.epad + e : e)];
-    const double coef = (se < 0) ? c : -c;
-#pragma unroll
-    for (int k = 0; k < kDim; ++k) acc[k] = fm(coef, flux(k, e), acc[k]);
+    acc = fm((se < 0) ? c : -c, flux(e), acc);
   }
+  return acc;
+}
+// U0 + dt_here (source + sum), floored; `floored` reports the density floor
+template <class T>
+SPLASH_HD void combine_face(double dt_here, const T* src, const T* sum, const T* u0, T* u, bool& floored) {
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) u[k] = fm(dt_here, acc[k], u0[k]);
+  for (int k = 0; k < kDim; ++k) u[k] = fm(dt_here, src[k] + sum[k], u0[k]);
   floored = less(u[0], T(1e-8));
   if (floored) u[0] = T(1e-8);
 }
+
+#if defined(__CUDACC__)
+// A block of the face launches: kFaces faces, and for each of them kDim
+// threads that sum one field's fluxes and one for the source, a warp per
+// part, so that the parts run side by side on the SM's four schedulers; the
+// warp of part 0 then combines them.  One thread per face runs all of it in
+// sequence, 194 dependent FP64 instructions of 36 ns on a mesh that leaves
+// the SMs a warp or two.  The parts rotate from block to block, since a
+// warp's place in the block decides its scheduler and the source is the
+// longest part.
+constexpr int kFaces = 32;
+constexpr int kFaceThreads = kFaces * (kDim + 1);
+__device__ __forceinline__ int face_part() { return (int)((threadIdx.x / kFaces + blockIdx.x) % (kDim + 1)); }
+template <class T, int N>
+struct FaceParts {
+  static constexpr int kParts = is_dual<T>::value ? 2 : 1;
+  double v[kParts][N][kFaces];
+  __device__ __forceinline__ void put(int i, int t, const T& x) {
+    v[0][i][t] = val(x);
+    if constexpr (is_dual<T>::value) v[1][i][t] = x.d[0];
+  }
+  __device__ __forceinline__ T get(int i, int t) const {
+    T x(v[0][i][t]);
+    if constexpr (is_dual<T>::value) x.d[0] = v[1][i][t];
+    return x;
+  }
+};
+#endif
 
 }  // namespace f64
 }  // namespace splash

@@ -10,43 +10,31 @@
 namespace splash {
 namespace f64 {
 
-// max over the block of non-negative doubles' bit patterns, in thread 0
-template <int BLOCK>
-__device__ __forceinline__ unsigned long long block_max(unsigned long long v, unsigned long long* sm) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long a = __shfl_down_sync(0xffffffffu, v, o);
-    v = a > v ? a : v;
-  }
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < BLOCK / 32; ++w) v = sm[w] > v ? sm[w] : v;
-  }
-  return v;
-}
-
-// Folds the block's candidates (integer maxima: exact in any order) and, in
-// the last block to do so, makes the bounds of the next step's dt of them:
+// Folds a warp's candidates (integer maxima: exact in any order) and, in the
+// last of n_warps warps to do so, makes the bounds of the next step's dt of
+// them:
 //   CFL bound h0 0.1 / max_vel, max_vel = max(1e-8, sqrt(vel2)),
 //   extra dt 0.01 / (alpha fric_k sqrt(rate2)), at most 1e20; 1e20 and a flag
 //   when some face's is negative (physics/adiabatic.hpp:543-580),
-// and gives the folds a fresh start.  Every thread of the block calls it.
-template <int BLOCK>
-__device__ __forceinline__ void fold_block(double vel2, double rate2, bool negative, const DevState& S,
-                                           const PhysParams& P) {
-  __shared__ unsigned long long sm[2][BLOCK / 32];
-  const int neg = __syncthreads_or(negative);
-  const unsigned long long v = block_max<BLOCK>(bits_of(vel2), sm[0]);
-  const unsigned long long r = block_max<BLOCK>(bits_of(rate2), sm[1]);
-  if (threadIdx.x != 0) return;
+// and gives the folds a fresh start.  Every lane of the warp calls it.
+__device__ __forceinline__ void fold_warp(double vel2, double rate2, bool negative, const DevState& S,
+                                          const PhysParams& P, unsigned long long n_warps) {
+  unsigned long long v = bits_of(vel2), r = bits_of(rate2);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long a = __shfl_down_sync(0xffffffffu, v, o);
+    const unsigned long long b = __shfl_down_sync(0xffffffffu, r, o);
+    v = a > v ? a : v;
+    r = b > r ? b : r;
+  }
+  const bool neg = __any_sync(0xffffffffu, negative);
+  if ((threadIdx.x & 31) != 0) return;
   unsigned long long* F = S.fold;
   if (v) atomicMax(F + kFoldVel2, v);
   if (r) atomicMax(F + kFoldRate2, r);
   if (neg) atomicMax(F + kFoldNeg, 1ull);
   __threadfence();
-  if (atomicAdd(F + kFoldDone, 1ull) != gridDim.x - 1) return;
+  if (atomicAdd(F + kFoldDone, 1ull) != n_warps - 1) return;
   __threadfence();
   const double vmax = fmax(1e-8, sqrt(from_bits(atomicExch(F + kFoldVel2, 0ull))));
   const double rate = sqrt(from_bits(atomicExch(F + kFoldRate2, 0ull)));

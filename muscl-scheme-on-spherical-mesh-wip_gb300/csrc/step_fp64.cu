@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kFaceBlock) prepare_kernel(DevGeom G, DevState
     for (int k = 0; k < kDim; ++k) S.W0[k * G.fpad + f] = w[k];
     dt_fold(w, r, P, vel2, rate2, negative);
   }
-  fold_block<kFaceBlock>(vel2, rate2, negative, S, P);
+  fold_warp(vel2, rate2, negative, S, P, gridDim.x * (kFaceBlock / 32));
 }
 
 // find_U_edges (MUSCL_base.hpp:361-434) of both sides of every edge and the
@@ -104,27 +104,21 @@ __global__ void __launch_bounds__(kThreads) edge_kernel(DevGeom G, DevState S, P
 }
 
 // res2d + the RK combine; stage 1: dt/2, writes W1; stage 2: dt, writes U, W0
-// and folds the candidates of the next dt.
+// and folds the candidates of the next dt.  This is the part after the sums
+// and the source, of one face per lane; every lane of the warp calls it.
 template <int STAGE>
-__global__ void __launch_bounds__(kFaceBlock) update_kernel(DevGeom G, DevState S, PhysParams P) {
-  griddep_launch_dependents();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void finish_face(const DevGeom& G, const DevState& S, const PhysParams& P, int f, bool live,
+                                            const double* src, const double* sum, unsigned long long n_warps) {
   double vel2 = 0.0, rate2 = 0.0;
   bool negative = false;
-  griddep_wait();
-  if (f < G.n_faces) {
+  if (live) {
     const int fp = G.fpad;
     const double dt = S.scal[kScDt];
-    const double* Win = (STAGE == 1) ? S.W0 : S.W1;
-    double w[kDim], u0[kDim], u[kDim];
+    double u0[kDim], u[kDim], w[kDim];
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      w[k] = Win[k * fp + f];
-      u0[k] = S.U[k * fp + f];
-    }
+    for (int k = 0; k < kDim; ++k) u0[k] = S.U[k * fp + f];
     bool floored;
-    update_face<double, double>(G, P, face_src_params<double>(G, P, f), (STAGE == 1) ? 0.5 * dt : dt, w, u0,
-                                [&](int k, int e) { return S.fe[(size_t)k * G.epad + e]; }, f, u, floored);
+    combine_face((STAGE == 1) ? 0.5 * dt : dt, src, sum, u0, u, floored);
     const D3 fcn = plane3(G.fcn, fp, f);
     prim_of(u, fcn, P.gam, w);
     double* Wout = (STAGE == 1) ? S.W1 : S.W0;
@@ -136,7 +130,66 @@ __global__ void __launch_bounds__(kFaceBlock) update_kernel(DevGeom G, DevState 
       dt_fold(w, fcn, P, vel2, rate2, negative);
     }
   }
-  if (STAGE == 2) fold_block<kFaceBlock>(vel2, rate2, negative, S, P);
+  if (STAGE == 2) fold_warp(vel2, rate2, negative, S, P, n_warps);
+}
+template <int STAGE>
+__device__ __forceinline__ void face_source(const DevGeom& G, const DevState& S, const PhysParams& P, int f,
+                                            double* src) {
+  const double* Win = (STAGE == 1) ? S.W0 : S.W1;
+  double w[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) w[k] = Win[k * G.fpad + f];
+  source_term(w, plane3(G.fcn, G.fpad, f), face_src_params<double>(G, P, f), P, src);
+}
+
+// one thread per face
+template <int STAGE>
+__global__ void __launch_bounds__(kFaceBlock) update_kernel(DevGeom G, DevState S, PhysParams P) {
+  griddep_launch_dependents();
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = f < G.n_faces;
+  double src[kDim] = {0, 0, 0, 0, 0}, sum[kDim] = {0, 0, 0, 0, 0};
+  griddep_wait();
+  if (live) {
+    face_source<STAGE>(G, S, P, f, src);
+    // flux_sum of the five fields in one walk over the slots
+    const int n = G.nslots[f];
+    for (int j = 0; j < n; ++j) {
+      const int se = G.slot_edge[j * G.fpad + f];
+      const int e = se & 0x7fffffff;
+      const double c = G.e_side[(size_t)kSideCoef * G.xs + (se < 0 ? G.epad + e : e)];
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) sum[k] = fma((se < 0) ? c : -c, S.fe[(size_t)k * G.epad + e], sum[k]);
+    }
+  }
+  finish_face<STAGE>(G, S, P, f, live, src, sum, gridDim.x * (kFaceBlock / 32));
+}
+// kDim + 1 threads per face (face_part)
+template <int STAGE>
+__global__ void __launch_bounds__(kFaceThreads) update_parts_kernel(DevGeom G, DevState S, PhysParams P) {
+  griddep_launch_dependents();
+  __shared__ FaceParts<double, 2 * kDim> parts;
+  const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
+  const bool live = f < G.n_faces;
+  griddep_wait();
+  if (live && part < kDim) {
+    const double* fe = S.fe + (size_t)part * G.epad;
+    parts.put(part, i, flux_sum<double>(G, f, [&](int e) { return fe[e]; }));
+  } else if (live) {
+    double src[kDim];
+    face_source<STAGE>(G, S, P, f, src);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) parts.put(kDim + k, i, src[k]);
+  }
+  __syncthreads();
+  if (part != 0) return;
+  double src[kDim], sum[kDim];
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    sum[k] = live ? parts.get(k, i) : 0.0;
+    src[k] = live ? parts.get(kDim + k, i) : 0.0;
+  }
+  finish_face<STAGE>(G, S, P, f, live, src, sum, gridDim.x);
 }
 
 // ---- isothermal solver (MUSCL_HLLE, 4 fields; planes 0..3 of U/W/U+) ----
@@ -154,7 +207,7 @@ __global__ void __launch_bounds__(kFaceBlock) iso_prepare_kernel(DevGeom G, DevS
     }
     vel2 = iso::dt_fold(u, plane3(G.fcn, G.fpad, f));
   }
-  fold_block<kFaceBlock>(vel2, 0.0, false, S, P);
+  fold_warp(vel2, 0.0, false, S, P, gridDim.x * (kFaceBlock / 32));
 }
 
 // the two sides' states with the isothermal limiter (MUSCL_base.hpp:361-434,
@@ -251,7 +304,7 @@ __global__ void __launch_bounds__(kFaceBlock) iso_update_kernel(DevGeom G, DevSt
     }
     if (STAGE == 2) vel2 = iso::dt_fold(u, plane3(G.fcn, fp, f));
   }
-  if (STAGE == 2) fold_block<kFaceBlock>(vel2, 0.0, false, S, P);
+  if (STAGE == 2) fold_warp(vel2, 0.0, false, S, P, gridDim.x * (kFaceBlock / 32));
 }
 
 // reference order [F][dim] <-> internal planes
@@ -300,7 +353,7 @@ __global__ void gather_state2_kernel(const double* __restrict__ U, const int* __
 }
 constexpr int kMoveBlock = 256;
 
-inline int face_blocks(int n) { return (n + kFaceBlock - 1) / kFaceBlock; }
+inline int face_blocks(int n, int per = kFaceBlock) { return (n + per - 1) / per; }
 inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
 
 }  // namespace
@@ -323,8 +376,22 @@ const void* fp64_dt0_kernel_ptr(int solver) {
 
 cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, double dt0, cudaStream_t st,
                       cudaEvent_t* ev) {
-  const bool iso = P.solver == kSolverIsoHLLE;
-  const dim3 eg(f64::edge_blocks(G.n_edges)), fg(f64::face_blocks(G.n_faces)), eb(f64::kThreads), fb(f64::kFaceBlock);
+  using Edge = void (*)(DevGeom, DevState, PhysParams, double);
+  using Update = void (*)(DevGeom, DevState, PhysParams);
+  // six threads per face where one per face leaves the pipe to a warp or two
+  // per SM; where it does not, the combining warp's share of a block's
+  // registers costs more.  us per step, one / six: hex(4) 53.9 / 52.4, hex(5)
+  // 97 / 76 (shear 131 / 97), hex(6) (40,962 faces) 250 / 224, quad(7) (98,304)
+  // 366 / 367, hex(7) 760 / 798, quad(8) 1262 / 1352.
+  constexpr int kPartsFaces = 65536;
+  const bool iso = P.solver == kSolverIsoHLLE, parts = !iso && G.n_faces <= kPartsFaces;
+  const Edge edge1 = iso ? f64::iso_edge_kernel<1> : f64::edge_kernel<1>;
+  const Edge edge2 = iso ? f64::iso_edge_kernel<2> : f64::edge_kernel<2>;
+  const Update upd1 = iso ? f64::iso_update_kernel<1> : parts ? f64::update_parts_kernel<1> : f64::update_kernel<1>;
+  const Update upd2 = iso ? f64::iso_update_kernel<2> : parts ? f64::update_parts_kernel<2> : f64::update_kernel<2>;
+  const dim3 eg(f64::edge_blocks(G.n_edges)), eb(f64::kThreads);
+  const dim3 fg(f64::face_blocks(G.n_faces, parts ? f64::kFaces : f64::kFaceBlock));
+  const dim3 fb(parts ? f64::kFaceThreads : f64::kFaceBlock);
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t r) {
     if (e == cudaSuccess) e = r;
@@ -333,13 +400,13 @@ cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, 
   // launch evaluates itself
   if (ev) cudaEventRecord(ev[0], st);
   if (ev) cudaEventRecord(ev[1], st);
-  chk(launch_pdl(iso ? f64::iso_edge_kernel<1> : f64::edge_kernel<1>, eg, eb, st, G, S, P, dt0));
+  chk(launch_pdl(edge1, eg, eb, st, G, S, P, dt0));
   if (ev) cudaEventRecord(ev[2], st);
-  chk(launch_pdl(iso ? f64::iso_update_kernel<1> : f64::update_kernel<1>, fg, fb, st, G, S, P));
+  chk(launch_pdl(upd1, fg, fb, st, G, S, P));
   if (ev) cudaEventRecord(ev[3], st);
-  chk(launch_pdl(iso ? f64::iso_edge_kernel<2> : f64::edge_kernel<2>, eg, eb, st, G, S, P, dt0));
+  chk(launch_pdl(edge2, eg, eb, st, G, S, P, dt0));
   if (ev) cudaEventRecord(ev[4], st);
-  chk(launch_pdl(iso ? f64::iso_update_kernel<2> : f64::update_kernel<2>, fg, fb, st, G, S, P));
+  chk(launch_pdl(upd2, fg, fb, st, G, S, P));
   if (ev) cudaEventRecord(ev[5], st);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
