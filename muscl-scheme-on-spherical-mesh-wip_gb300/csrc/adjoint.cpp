@@ -231,8 +231,9 @@ int Adjoint::forward(const double* U0, const double* theta, int n, double dt0_, 
   for (int i = 0; i < n; ++i) {
     if (i % K == 0)
       ADJ_CUDA(cudaMemcpyAsync(d_ck + (size_t)(i / K) * FS, S.U, FS * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    ADJ_CUDA(fp64_step(G, S, P, dt0_, st));
-    ADJ_CUDA(cudaMemcpyAsync(d_dts + i, S.scal + kScDt, sizeof(double), cudaMemcpyDeviceToDevice, st));
+    DevState step = S;
+    step.dt_log = d_dts + i;
+    ADJ_CUDA(fp64_step(G, step, P, dt0_, st));
   }
   ADJ_CUDA(cudaEventRecord(e1, st));
   ADJ_CUDA(cudaEventSynchronize(e1));

@@ -17,6 +17,10 @@
 //   adj_face    per face: lamW = sum over the inverse stencil of beta * PU and
 //               the own parts, + source reverse (dt_here la), -> prim reverse
 // Every sum has a fixed order (no atomics): the adjoint is deterministic.
+//
+// The launches overlap by programmatic dependent launch (pdl.cuh), so what a
+// predecessor writes is read with ordinary loads: no __restrict__ on those
+// pointers, which would let the compiler take the non-coherent path.
 // Like the step itself (step_fp64.cu) all of it is bound by the FP64 pipe:
 // the flux reverse runs once per edge, the reconstruction on a thread per
 // side.
@@ -28,6 +32,7 @@
 #include "adjoint_rev.cuh"
 #include "dual.cuh"
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "physics_fp64.cuh"
 #include "step_body_fp64.cuh"
 #include "step_fold_fp64.cuh"
@@ -68,6 +73,8 @@ __device__ __forceinline__ D1 dual1(double v, double d) {
 // ---------------------------------------------------------------------
 // tangent-linear model
 __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   double vel2 = 0.0, rate2 = 0.0;
   bool negative = false;
@@ -91,8 +98,10 @@ __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
+__global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
                                                             double dt0) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ SideExchange<D1, kThreads> sides;
   const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
@@ -130,6 +139,8 @@ __global__ void __launch_bounds__(kThreads) tlm_edge_kernel(DevGeom G, DevState 
 
 template <int STAGE>
 __global__ void __launch_bounds__(kFaceThreads) tlm_update_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ FaceParts<D1, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
   const bool live = f < G.n_faces;
@@ -266,8 +277,10 @@ __global__ void __launch_bounds__(kBlock) tp_flux_kernel(DevGeom G, PhysParams P
 
 // ---------------------------------------------------------------------
 // recomputation (double, extra outputs)
-__global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P, const double* __restrict__ U,
-                                                         double* __restrict__ W) {
+__global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P, const double* U,
+                                                         double* W) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= G.n_faces) return;
   const int fp = G.fpad;
@@ -281,9 +294,11 @@ __global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P
 
 // the edge launch of the step with the limiter's Jacobian (LJ) and the edge
 // states (uplus) kept
-__global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                           const double* __restrict__ W, double* __restrict__ uplus,
-                                                           double* __restrict__ LJ, double* __restrict__ fe) {
+__global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams P, const double* dtp,
+                                                           const double* W, double* uplus,
+                                                           double* LJ, double* fe) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ SideExchange<double, kThreads> sides;
   const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
@@ -316,11 +331,13 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(kFaceThreads) rc_update_kernel(DevGeom G, PhysParams P, const double* __restrict__ dtp,
-                                                                 const double* __restrict__ Win,
-                                                                 const double* __restrict__ U0,
-                                                                 const double* __restrict__ fe, double* __restrict__ Uout,
-                                                                 double* __restrict__ Wout, uint8_t* __restrict__ mask) {
+__global__ void __launch_bounds__(kFaceThreads) rc_update_kernel(DevGeom G, PhysParams P, const double* dtp,
+                                                                 const double* Win,
+                                                                 const double* U0,
+                                                                 const double* fe, double* Uout,
+                                                                 double* Wout, uint8_t* mask) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ FaceParts<double, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
   const bool live = f < G.n_faces;
@@ -366,13 +383,15 @@ __device__ __forceinline__ double masked(const double* lam, const uint8_t* mask,
   return (k == 0 && (mask[f] & bit)) ? 0.0 : lam[k * fp + f];
 }
 
-__global__ void __launch_bounds__(kThreads) adj_edge_kernel(DevGeom G, PhysParams P, double dt, double dt_here,
-                                                            const double* __restrict__ W,
-                                                            const double* __restrict__ uplus,
-                                                            const double* __restrict__ LJ,
-                                                            const double* __restrict__ lam,
-                                                            const uint8_t* __restrict__ mask, int bit,
-                                                            double* __restrict__ PU, double* __restrict__ own) {
+__global__ void __launch_bounds__(kThreads, 7) adj_edge_kernel(DevGeom G, PhysParams P, double dt, double dt_here,
+                                                            const double* W,
+                                                            const double* uplus,
+                                                            const double* LJ,
+                                                            const double* lam,
+                                                            const uint8_t* mask, int bit,
+                                                            double* PU, double* own) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ SideExchange<double, kThreads> sides;
   __shared__ double bars[rev::kSideBarValues][kThreads];
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
@@ -426,10 +445,12 @@ __global__ void __launch_bounds__(kThreads) adj_edge_kernel(DevGeom G, PhysParam
 
 template <int STAGE>
 __global__ void __launch_bounds__(kFaceThreads) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
-                                                                const double* __restrict__ Win,
-                                                                const double* __restrict__ Uin,
-                                                                const uint8_t* __restrict__ mask, const double* lam,
+                                                                const double* Win,
+                                                                const double* Uin,
+                                                                const uint8_t* mask, const double* lam,
                                                                 double* lam_out) {
+  griddep_launch_dependents();
+  griddep_wait();
   __shared__ FaceParts<double, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, g = blockIdx.x * kFaces + i;
   const bool live = g < G.n_faces;
@@ -500,12 +521,13 @@ cudaError_t tlm_prepare(const DevGeom& G, const DevState& S, const TlmTangents& 
 
 cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P, double dt0,
                      cudaStream_t st) {
+  FirstError chk;
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
-  adj::tlm_edge_kernel<1><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
-  adj::tlm_update_kernel<1><<<nb, f64::kFaceThreads, 0, st>>>(G, S, T, P);
-  adj::tlm_edge_kernel<2><<<ne, adj::kThreads, 0, st>>>(G, S, T, P, dt0);
-  adj::tlm_update_kernel<2><<<nb, f64::kFaceThreads, 0, st>>>(G, S, T, P);
-  return cudaGetLastError();
+  chk(launch_pdl(adj::tlm_edge_kernel<1>, dim3(ne), dim3(adj::kThreads), st, G, S, T, P, dt0));
+  chk(launch_pdl(adj::tlm_update_kernel<1>, dim3(nb), dim3(f64::kFaceThreads), st, G, S, T, P));
+  chk(launch_pdl(adj::tlm_edge_kernel<2>, dim3(ne), dim3(adj::kThreads), st, G, S, T, P, dt0));
+  chk(launch_pdl(adj::tlm_update_kernel<2>, dim3(nb), dim3(f64::kFaceThreads), st, G, S, T, P));
+  return chk.status();
 }
 
 namespace {
@@ -557,27 +579,29 @@ cudaError_t rc_prim(const DevGeom& G, const PhysParams& P, const double* U, doub
 
 cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, const StepTape& t, double* fe,
                     double* U_next, double* W_next, cudaStream_t st) {
+  FirstError chk;
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
   constexpr int B = f64::kFaceThreads, E = adj::kThreads;
-  adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W0, t.P0, t.J0, fe);
-  adj::rc_update_kernel<1><<<nb, B, 0, st>>>(G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask);
-  adj::rc_edge_kernel<<<ne, E, 0, st>>>(G, P, dtp, t.W1, t.P1, t.J1, fe);
-  adj::rc_update_kernel<2><<<nb, B, 0, st>>>(G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask);
-  return cudaGetLastError();
+  chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W0, t.P0, t.J0, fe));
+  chk(launch_pdl(adj::rc_update_kernel<1>, dim3(nb), dim3(B), st, G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask));
+  chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W1, t.P1, t.J1, fe));
+  chk(launch_pdl(adj::rc_update_kernel<2>, dim3(nb), dim3(B), st, G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask));
+  return chk.status();
 }
 
 cudaError_t adj_step(const DevGeom& G, const PhysParams& P, double dt, const StepTape& t, const AdjScratch& X,
                      double* lam, cudaStream_t st) {
+  FirstError chk;
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
   constexpr int B = f64::kFaceThreads, E = adj::kThreads;
   // stage 2: U2 = floor(U + dt Phi(W1, P1))
-  adj::adj_edge_kernel<<<ne, E, 0, st>>>(G, P, dt, dt, t.W1, t.P1, t.J1, lam, t.mask, 2, X.PU, X.own);
-  adj::adj_face_kernel<2><<<nb, B, 0, st>>>(G, P, dt, X, t.W1, t.U1, t.mask, lam, X.lam1);
+  chk(launch_pdl(adj::adj_edge_kernel, dim3(ne), dim3(E), st, G, P, dt, dt, t.W1, t.P1, t.J1, lam, t.mask, 2, X.PU, X.own));
+  chk(launch_pdl(adj::adj_face_kernel<2>, dim3(nb), dim3(B), st, G, P, dt, X, t.W1, t.U1, t.mask, lam, X.lam1));
   // stage 1: U1 = floor(U + dt/2 Phi(W0, P0))
   const double dt_half = dt / 2;
-  adj::adj_edge_kernel<<<ne, E, 0, st>>>(G, P, dt, dt_half, t.W0, t.P0, t.J0, X.lam1, t.mask, 1, X.PU, X.own);
-  adj::adj_face_kernel<1><<<nb, B, 0, st>>>(G, P, dt_half, X, t.W0, t.U, t.mask, lam, lam);
-  return cudaGetLastError();
+  chk(launch_pdl(adj::adj_edge_kernel, dim3(ne), dim3(E), st, G, P, dt, dt_half, t.W0, t.P0, t.J0, X.lam1, t.mask, 1, X.PU, X.own));
+  chk(launch_pdl(adj::adj_face_kernel<1>, dim3(nb), dim3(B), st, G, P, dt_half, X, t.W0, t.U, t.mask, lam, lam));
+  return chk.status();
 }
 
 }  // namespace splash

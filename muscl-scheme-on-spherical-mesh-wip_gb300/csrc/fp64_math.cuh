@@ -297,8 +297,9 @@ __device__ __forceinline__ int switch_row(double r, double& d) {
 }
 #endif
 
-// h(r) for r > 0 (not NaN), and dh/dr
-SPLASH_HD double switch_pos(double r, double& slope) {
+// h(r) for r > 0 (not NaN) and dh/dr; with `known`, h comes in and only the
+// slope is evaluated
+SPLASH_HD double switch_slope(double r, bool known, double h, double& slope) {
 #if defined(__CUDA_ARCH__) && defined(SPLASH_SWITCH_TABLE)
   slope = 0.0;
   if (high_word(r) >= 0x40020000u) return 1.0;  // r >= 2.25
@@ -306,7 +307,7 @@ SPLASH_HD double switch_pos(double r, double& slope) {
   const int row = switch_row(r, d);
   if (row >= 0) {
     slope = horner8(kSwitchSlope[row], d);
-    return horner8(kSwitchTable[row], d);
+    return known ? h : horner8(kSwitchTable[row], d);
   }
 #endif
   return switch_formula(r, slope);

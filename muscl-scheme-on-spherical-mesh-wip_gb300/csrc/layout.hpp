@@ -174,6 +174,7 @@ struct DevState {
   double* W1;     // (Sigma, l, Pi) after stage 1, kDim planes
   double* uplus;  // the last stage-2 edge states (Sigma, l, Pi), kDim planes of xs
   double* fe;     // Riemann flux of every edge, kDim planes of epad
+  double* dt_log = nullptr;  // FP64 path: where the step also leaves its dt (may be null)
   unsigned long long* fold;  // FP64 path: the candidates of the next dt, see FoldSlot
   float* W32;     // mixed path: stage-1 input (Sigma, l, Pi) in FP32: [fpad] float4 (Sigma, l), then a Pi plane
   float* W32b;    // mixed path: stage-2 input, the same layout (written by the stage-1 update)

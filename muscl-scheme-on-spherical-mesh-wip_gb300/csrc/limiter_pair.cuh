@@ -196,8 +196,9 @@ SPLASH_HD bool pair_range(double dp, double num) {
 }
 
 // The limiter of one field from dp, num = hr dm (r = num / dp) and
-// e = dp - num (1 - r = e / dp); false where pairs do not serve.
-SPLASH_HD bool limiter_pair(double dp, double num, double e, const PairLine& l, double& lim) {
+// e = dp - num (1 - r = e / dp); false where pairs do not serve.  hp receives
+// the switch where it is needed.
+SPLASH_HD bool limiter_pair(double dp, double num, double e, const PairLine& l, double& lim, Pair& hp) {
   if (!l.ok || !pair_range(dp, num)) return false;
   const int e0 = exponent_field(dp);
   Pair D, N, E;
@@ -220,10 +221,15 @@ SPLASH_HD bool limiter_pair(double dp, double num, double e, const PairLine& l, 
   Pair v = S;
   if (pair_less(T, S)) {
     if (T.h < 0.0f) T = Pair{0.0f, 0.0f};
-    v = pair_add(T, pair_mul(switch_pair(r, t), pair_add(S, pair_neg(T))));
+    hp = switch_pair(r, t);
+    v = pair_add(T, pair_mul(hp, pair_add(S, pair_neg(T))));
   }
   lim = widen(v.h) + widen(v.l);
   return true;
+}
+SPLASH_HD bool limiter_pair(double dp, double num, double e, const PairLine& l, double& lim) {
+  Pair hp;
+  return limiter_pair(dp, num, e, l, lim, hp);
 }
 #endif
 

@@ -33,4 +33,13 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// The first error of a sequence of launches.
+struct FirstError {
+  cudaError_t e = cudaSuccess;
+  void operator()(cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+  }
+  cudaError_t status() const { return e != cudaSuccess ? e : cudaGetLastError(); }
+};
+
 }  // namespace splash

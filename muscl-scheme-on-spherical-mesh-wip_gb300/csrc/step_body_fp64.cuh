@@ -204,7 +204,8 @@ struct SideLimiter {
 struct Phi {
   double v, r, nu;
 };
-SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double inu) {
+// known: the switch is h (8 FP64 instructions less).
+SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double inu, bool known, double hk) {
   if (nan_bits(r)) return Phi{0., 0., 0.};
   if (odd_bits(r)) return Phi{limiter_field(r, l), 0., 0.};  // flat in r and in the Courant factor
   // the superbee: max(0, max(min(1, r sb), min(r, eta_p)))
@@ -222,7 +223,7 @@ SPLASH_HD Phi limiter_partials(double r, const LimiterLine<double>& l, double in
   if (to.v == sb.v) return sb;
   if (!(r > 0.0)) return to;
   double slope;
-  const double h = switch_pos(r, slope);
+  const double h = switch_slope(r, known, hk, slope);
   return Phi{fma(h, sb.v - to.v, to.v), fma(h, sb.r - to.r, fma(slope, sb.v - to.v, to.r)),
              fma(h, sb.nu - to.nu, to.nu)};
 }
@@ -234,9 +235,18 @@ struct SideLimiterPartials : SideLimiter {
   // r receives the ratio
   SPLASH_HD Phi operator()(int k, double dp, double num, double dpg, double& r) const {
     r = slope_ratio(dp, num);
-    Phi phi = limiter_partials(r, line, inu);
-    double v;
-    if (in_pairs(k, dp, num, dpg, v)) phi.v = v;
+    // in pairs the switch comes with the value and serves the derivatives
+    // too, where it was needed (h > 0)
+    bool in_pairs = false, known = false;
+    double v = 0.0, hk = 0.0;
+#if defined(SPLASH_SWITCH_TABLE)
+    Pair h{0.0f, 0.0f};
+    in_pairs = shallow(dpg, scale[k]) && limiter_pair(dp, num, dp - num, pairs, v, h);
+    known = in_pairs && h.h > 0.0f;
+    if (known) hk = widen(h.h) + widen(h.l);
+#endif
+    Phi phi = limiter_partials(r, line, inu, known, hk);
+    if (in_pairs) phi.v = v;
     return phi;
   }
 };

@@ -58,6 +58,7 @@ __device__ __forceinline__ double step_dt(const double* scal, double dt0) {
 // extra dt, which the reference latches when the step begins.
 __device__ __forceinline__ void publish_dt(const DevState& S, double dt) {
   S.scal[kScDt] = dt;
+  if (S.dt_log) *S.dt_log = dt;
   S.scal[kScTime] = S.scal[kScTime] + dt;
   if (S.scal[kScNegExtra] != 0.0) atomicOr(S.err, 8u);  // SPLASH_STOP_NEG_EXTRA_DT
 }

@@ -392,10 +392,7 @@ cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, 
   const dim3 eg(f64::edge_blocks(G.n_edges)), eb(f64::kThreads);
   const dim3 fg(f64::face_blocks(G.n_faces, parts ? f64::kFaces : f64::kFaceBlock));
   const dim3 fb(parts ? f64::kFaceThreads : f64::kFaceBlock);
-  cudaError_t e = cudaSuccess;
-  auto chk = [&](cudaError_t r) {
-    if (e == cudaSuccess) e = r;
-  };
+  FirstError chk;
   // ev[0]..ev[1] is the (empty) slot of the dt clip, which the stage-1 edge
   // launch evaluates itself
   if (ev) cudaEventRecord(ev[0], st);
@@ -408,7 +405,7 @@ cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, 
   if (ev) cudaEventRecord(ev[4], st);
   chk(launch_pdl(upd2, fg, fb, st, G, S, P));
   if (ev) cudaEventRecord(ev[5], st);
-  return e != cudaSuccess ? e : cudaGetLastError();
+  return chk.status();
 }
 
 cudaError_t fp64_scatter_state(const double* aos, const int* iperm, double* U, int n_faces,
