@@ -531,17 +531,18 @@ __device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n,
   const F3 vel = scal(cross3(ec, f3(w[1], w[2], w[3])), inv_rho);
   const float nu_plus = (c + dot3(vel, en)) * dt * arc_a;
   const float sb_scale = __fdividef(sc.eta_m, (float)(2 * n) * nu_plus);
+  const float third = (1.f + nu_plus) * (1.f / 3.f);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const float pp = (bp0 * wa[k] + bp1 * wb[k] - w[k]) * ihp;
     const float pm = (w[k] - (bm0 * wc[k] + bm1 * wd[k])) * ihm;
-    const float lim = limiter_field(__fdividef(pm, pp), nu_plus, sc.eta_p, sb_scale);
+    const float lim = limiter_field(__fdividef(pm, pp), third, sc.eta_p, sb_scale);
     up[k] = w[k] + pp * lim * bmd;
   }
   {
     const float pp = (bp0 * Wp[ia] + bp1 * Wp[ib] - wp) * ihp;
     const float pm = (wp - (bm0 * Wp[ic] + bm1 * Wp[id])) * ihm;
-    const float lim = limiter_field(__fdividef(pm, pp), nu_plus, sc.eta_p, sb_scale);
+    const float lim = limiter_field(__fdividef(pm, pp), third, sc.eta_p, sb_scale);
     up[4] = wp + pp * lim * bmd;
   }
 }
