@@ -341,8 +341,9 @@ int Solver::capture_steps(int n_steps, cudaGraph_t* g, cudaGraphExec_t* exec, st
 }
 
 int Solver::capture_graph() {
+  in_cluster = precision == SPLASH_PREC_MIXED && mixed_in_cluster(GM);
   const int rc = capture_steps(1, &graph, &graph_exec, &dt0_nodes);
-  return rc ? rc : capture_steps(kGraphSteps, &graph_k, &graph_k_exec, &dt0_nodes_k);
+  return rc || in_cluster ? rc : capture_steps(kGraphSteps, &graph_k, &graph_k_exec, &dt0_nodes_k);
 }
 
 int Solver::set_graph_dt0(double dt0) {
@@ -371,6 +372,15 @@ int Solver::step(double dt0) {
 }
 
 int Solver::steps_n(int n, double dt0) {
+  if (in_cluster && n != 1) {
+    for (int left = n; left > 0;) {
+      const int k = left < kClusterSteps ? left : kClusterSteps;
+      SPLASH_CUDA(mixed_cluster_steps(GM, S, P, dt0, k, stream));
+      steps += k;
+      left -= k;
+    }
+    return SPLASH_OK;
+  }
   const int rc = set_graph_dt0(dt0);
   if (rc) return rc;
   int left = n;

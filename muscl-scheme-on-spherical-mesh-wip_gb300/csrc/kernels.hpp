@@ -40,6 +40,11 @@ cudaError_t fp64_gather_state(const double* U, const int* iperm, double* aos, in
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
                        cudaStream_t st, cudaEvent_t* ev = nullptr, bool per_launch = false);
 const void* mixed_dt0_kernel_ptr(const DevGeomMixed& G);
+// The same for meshes that fit one thread-block cluster (mixed_in_cluster):
+// n steps in one launch.
+bool mixed_in_cluster(const DevGeomMixed& G);
+cudaError_t mixed_cluster_steps(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0, int n,
+                                cudaStream_t st);
 // The last step's stage-2 edge states into S.uplus32 (for write_t_curl),
 // recomputed from the stage-2 input face states S.W32b and the step's dt.
 cudaError_t mixed_edge_states(const DevGeomMixed& G, const DevState& S, const PhysParams& P, cudaStream_t st);

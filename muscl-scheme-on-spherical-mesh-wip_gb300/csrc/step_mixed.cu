@@ -185,8 +185,8 @@ __device__ __forceinline__ void fold_candidates_block(float vmax2, float dmin, u
   }
 }
 
-// The FP32 face state (Sigma, l, Pi) of the FP64 state u of face f, stored
-// to W32 and returned in w: (Sigma, l) rounded to the nearest float and the
+// The FP32 face state w = (Sigma, l, Pi) of the FP64 state u of a face:
+// (Sigma, l) rounded to the nearest float and the
 // pressure recovery Pi = (E - |r x l|^2 / (2 Sigma)) (gam - 1), floored at
 // 1e-16 (MUSCL_base.hpp:538).  Where the kinetic term cancels part of E
 // (above E / 8: low density, fast flow) the recovery runs in double-word
@@ -200,8 +200,7 @@ __device__ __forceinline__ void fold_candidates_block(float vmax2, float dmin, u
 // just below E / 8, 1.0 when the kinetic term is negligible): on hex(7) the
 // same density L1 error against FP64 after 200 steps (6.0e-8) with both
 // update launches at 12.3 us instead of 12.4 / 14.3 us.
-__device__ __forceinline__ void store_face_state(float* W32, int fp, int f, const double* u, F3 r32, F3 lo,
-                                                 const PhysParams& P, float* w) {
+__device__ __forceinline__ void face_state(const double* u, F3 r32, F3 lo, const PhysParams& P, float* w) {
   w[0] = fpc::d2f(u[0]);
   w[1] = fpc::d2f(u[1]);
   w[2] = fpc::d2f(u[2]);
@@ -215,6 +214,10 @@ __device__ __forceinline__ void store_face_state(float* W32, int fp, int f, cons
     const dw::DW r[3] = {{r32.x, lo.x}, {r32.y, lo.y}, {r32.z, lo.z}};
     dw::face_state_dw(u, r, dw::DW{P.gam_m1_h, P.gam_m1_l}, w);
   }
+}
+__device__ __forceinline__ void store_face_state(float* W32, int fp, int f, const double* u, F3 r32, F3 lo,
+                                                 const PhysParams& P, float* w) {
+  face_state(u, r32, lo, P, w);
   st5(W32, fp, f, w);
 }
 
@@ -323,14 +326,20 @@ __device__ __forceinline__ void source_f32(const float* w, F3 fcn, float acc0, c
 // Isothermal state (4 fields): W32 is the state itself (field 4 unused) and
 // the CFL candidate is max(|v|^2, a^2) with a = 1 (find_v_max with the
 // isothermal sound speed); no extra constraint (isothermal.hpp:262-267).
-__device__ __forceinline__ void iso_w32_candidates(const double* u, F3 r, float* W32, int fp, int f,
-                                                   float& vmax2, float& dmin) {
-  const float v[kDim] = {fpc::d2f(u[0]), fpc::d2f(u[1]), fpc::d2f(u[2]), fpc::d2f(u[3]), 0.f};
-  st5(W32, fp, f, v);
+__device__ __forceinline__ void iso_state_candidates(const double* u, F3 r, float* v, float& vmax2, float& dmin) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = fpc::d2f(u[k]);
+  v[4] = 0.f;
   const float ir = 1.0f / v[0];
   const F3 c = cross3(r, f3(v[1], v[2], v[3]));
   vmax2 = fmaxf(dot3(c, c) * (ir * ir), 1.f);
   dmin = kNoBound;
+}
+__device__ __forceinline__ void iso_w32_candidates(const double* u, F3 r, float* W32, int fp, int f,
+                                                   float& vmax2, float& dmin) {
+  float v[kDim];
+  iso_state_candidates(u, r, v, vmax2, dmin);
+  st5(W32, fp, f, v);
 }
 
 // W32 and the dt candidates of the state u of internal face f
@@ -495,14 +504,23 @@ struct SlotConsts {
   float eta_p, eta_m;
 };
 
-__device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n, const SlotConsts& sc, F3 ec,
-                                           F3 en, float dt, const PhysParams& P, float* up) {
-  const int ia = sc.st.x, ib = sc.st.y, ic = sc.st.z, id = sc.st.w;
+// States of the slot's face (q = 0) and its stencil faces (q = 1..4) from a
+// packed array.
+struct ArrayStates {
+  const float* W;
+  int fp, i[5];
+  __device__ __forceinline__ float4 sigma_l(int q) const { return ld4(W, i[q]); }
+  __device__ __forceinline__ float pi(int q) const { return W[4 * (size_t)fp + i[q]]; }
+};
+
+template <class States>
+__device__ __forceinline__ void recon_slot_of(const States& W, int n, const SlotConsts& sc, F3 ec, F3 en, float dt,
+                                              const PhysParams& P, float* up) {
   const float bp0 = sc.bt.x, bp1 = sc.bt.y, bm0 = sc.bt.z, bm1 = sc.bt.w;
   const float ihp = sc.hh.x, ihm = sc.hh.y, bmd = sc.hh.z, arc_a = sc.hh.w;
   // the face and its four stencil faces: one 16-byte gather each for
   // (Sigma, l), one more each for Pi (adiabatic only)
-  const float4 w4 = ld4(W, f), a4 = ld4(W, ia), b4 = ld4(W, ib), c4 = ld4(W, ic), d4 = ld4(W, id);
+  const float4 w4 = W.sigma_l(0), a4 = W.sigma_l(1), b4 = W.sigma_l(2), c4 = W.sigma_l(3), d4 = W.sigma_l(4);
   const float w[4] = {w4.x, w4.y, w4.z, w4.w};
   const float wa[4] = {a4.x, a4.y, a4.z, a4.w}, wb[4] = {b4.x, b4.y, b4.z, b4.w};
   const float wc[4] = {c4.x, c4.y, c4.z, c4.w}, wd[4] = {d4.x, d4.y, d4.z, d4.w};
@@ -523,8 +541,7 @@ __device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n,
     up[4] = 0.f;
     return;
   }
-  const float* Wp = W + 4 * (size_t)fp;
-  const float wp = Wp[f];
+  const float wp = W.pi(0);
   const float gam = P.gam_f;
   const float inv_rho = __fdividef(-1.0f, w[0]);
   const float c = sqrtf(__fdividef(gam * wp, w[0]));
@@ -540,11 +557,15 @@ __device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n,
     up[k] = w[k] + pp * lim * bmd;
   }
   {
-    const float pp = (bp0 * Wp[ia] + bp1 * Wp[ib] - wp) * ihp;
-    const float pm = (wp - (bm0 * Wp[ic] + bm1 * Wp[id])) * ihm;
+    const float pp = (bp0 * W.pi(1) + bp1 * W.pi(2) - wp) * ihp;
+    const float pm = (wp - (bm0 * W.pi(3) + bm1 * W.pi(4))) * ihm;
     const float lim = limiter_field(__fdividef(pm, pp), third, sc.eta_p, sb_scale);
     up[4] = wp + pp * lim * bmd;
   }
+}
+__device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n, const SlotConsts& sc, F3 ec,
+                                           F3 en, float dt, const PhysParams& P, float* up) {
+  recon_slot_of(ArrayStates{W, fp, {f, sc.st.x, sc.st.y, sc.st.z, sc.st.w}}, n, sc, ec, en, dt, P, up);
 }
 
 // One stage's reconstruction and Riemann fluxes, one thread per interior
@@ -979,6 +1000,263 @@ __global__ void __launch_bounds__(kBlock) update_split_kernel(DevGeomMixed G, De
                                                          blockIdx.x * kHalf + (threadIdx.x & (kHalf - 1)));
 }
 
+// ---- whole steps of a mesh that fits one thread-block cluster ----
+// On such a mesh a step takes the latency of four chains of loads and
+// instructions and of the four launch boundaries between them, each of which
+// also loads the threads' geometry again.  Here one cluster runs n_steps
+// steps in one launch: the phases of a step meet at cluster barriers, and
+// each thread keeps the geometry and the FP64 state of its edge side and its
+// face in registers.  The states and fluxes that phases exchange stay in
+// global memory (the L2).  us per step of do_steps, four launches / cluster:
+// hex(1) 12.9 / 8.8, hex(3) 13.4 / 10.0, quad(3) 12.5 / 8.5, quad(4)
+// 13.0 / 9.4.  In distributed shared memory instead, a stencil's gathers
+// take about a cycle per lane: hex(3) 15.6, and 11.8 with every block pulling
+// all face states first.
+//
+// A block has `half` edges and a 16th of the faces: thread t < half serves
+// the owner side of edge t and sums face t's fluxes, thread half + t its
+// reverse side and face t's source (as edge_sides_kernel and
+// update_split_kernel), and one more warp clips the dt in FP64.  The
+// arithmetic is theirs.
+constexpr int kClusterBlocks = 16;
+constexpr int kClusterHalf = 192;  // the most edges of a block (416 threads leave them 128 registers)
+// Every thread arrives and waits once per phase: the arrival releases its
+// writes to the cluster, the wait acquires the others'.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+struct ClusterShared {
+  float w[kDim][kClusterHalf];  // the input states of the block's faces
+  float up[kDim][2 * kClusterHalf];
+  float src[kDim][kClusterHalf];
+  double dt, dt_half;
+};
+
+// one side of an edge, and the flux in the lower half
+template <int STAGE>
+__device__ __forceinline__ void cluster_edge(const DevGeomMixed& G, const DevState& S, const PhysParams& P,
+                                             ClusterShared& sh, int x, int half, int id,
+                                             const SlotConsts& sc, const SlotGeomF& g, float dt) {
+  const int t = threadIdx.x;
+  const bool owner = t < half, live = x < G.n_edges;
+  if (live) {
+    const ArrayStates W{stage_input<STAGE>(S), G.fpad, {id & 0x0fffffff, sc.st.x, sc.st.y, sc.st.z, sc.st.w}};
+    const int n = id >> 28;
+    float u[kDim];
+    // two calls for the same reason as in edge_sides_kernel
+    if (owner)
+      recon_slot_of(W, n, sc, g.ec, g.en, dt, P, u);
+    else
+      recon_slot_of(W, n, sc, g.ec, f3(-g.en.x, -g.en.y, -g.en.z), dt, P, u);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) sh.up[k][t] = u[k];
+  }
+  __syncthreads();
+  if (!owner) return;
+  unsigned bits = 0;
+  if (live) {
+    float uL[kDim], uR[kDim], F[kDim] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) {
+      uL[k] = sh.up[k][t];
+      uR[k] = sh.up[k][t + half];
+    }
+    bits = (P.solver == kSolverIsoHLLE) ? iso_flux_star(uL, uR, g, F) : flux_star(uL, uR, g, P.gam_f, P.solver, F);
+#pragma unroll
+    for (int k = 0; k < kDim; ++k)
+      if (isnan(F[k])) bits |= 1u;
+    st5(S.fe32, G.epad, x, F);
+  }
+  bits = __reduce_or_sync(0xffffffffu, bits);
+  if ((t & 31) == 0 && bits) atomicOr(S.err, bits);
+}
+
+// The constants of a face: its slots' edges and flux coefficients
+// (negated on the owner side), centre and mass source.
+template <int MAXS>
+struct ClusterFace {
+  int e[MAXS];
+  float co[MAXS];
+  int n;
+  F3 r, lo;
+  double acc0;
+};
+
+// update_body for face x (-1: none): u0 is its FP64 state U0, replaced by the
+// new one in stage 2 and stored by the launch's last step
+template <int STAGE, int MAXS>
+__device__ __forceinline__ void cluster_face(const DevGeomMixed& G, const DevState& S, const PhysParams& P,
+                                             ClusterShared& sh, int x, int half, const ClusterFace<MAXS>& c,
+                                             float dtf, double* u0, bool last) {
+  const int t = threadIdx.x;
+  const bool live = x >= 0;
+  if (t >= half) {
+    if (live) {
+      float w[kDim], src[kDim];
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) w[k] = sh.w[k][t - half];
+      source_f32(w, c.r, fpc::d2f(c.acc0), P, src);
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) sh.src[k][t - half] = src[k];
+    }
+    __syncthreads();
+    return;
+  }
+  Acc2 a01{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, a23 = a01;
+  Acc a4{0.f, 0.f};
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < MAXS; ++j) {
+      if (j < c.n) {
+        const float k = dtf * c.co[j];
+        const float4 fe = ld4(S.fe32, c.e[j]);
+        const float fe4 = S.fe32[4 * (size_t)G.epad + c.e[j]];
+        const float2 k2 = make_float2(k, k);
+        a01.add(mul2(k2, make_float2(fe.x, fe.y)));
+        a23.add(mul2(k2, make_float2(fe.z, fe.w)));
+        a4.add(k * fe4);
+      }
+    }
+  }
+  __syncthreads();
+  float vmax = 0.f, dmin = kNoBound;
+  if (live) {
+    const Acc acc[kDim] = {{a01.hi.x, a01.lo.x}, {a01.hi.y, a01.lo.y}, {a23.hi.x, a23.lo.x},
+                           {a23.hi.y, a23.lo.y}, a4};
+    double u[kDim];
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) u[k] = u0[k] + fpc::f2d((acc[k].hi + acc[k].lo) + dtf * sh.src[k][t]);
+    if (P.accretion_on) u[0] += ((STAGE == 1) ? sh.dt_half : sh.dt) * c.acc0;
+    if (u[0] < 1e-8) u[0] = 1e-8;
+    float w[kDim];
+    if (P.solver == kSolverIsoHLLE) {
+      u[4] = 0.0;
+      iso_state_candidates(u, c.r, w, vmax, dmin);
+    } else {
+      face_state(u, c.r, c.lo, P, w);
+      if (STAGE == 2) dt_candidates_f32(w, c.r, P, vmax, dmin);
+    }
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) sh.w[k][t] = w[k];
+    st5(stage_output<STAGE>(S), G.fpad, x, w);
+    if (STAGE == 2) {
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) u0[k] = u[k];
+    }
+    if (STAGE == 2 && last) {
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) S.U[k * G.fpad + x] = u[k];
+    }
+  }
+  if (STAGE == 2) fold_candidates(vmax, dmin, S.keys);
+}
+
+template <int MAXS>
+__global__ void __launch_bounds__(2 * kClusterHalf + 32) cluster_steps_kernel(DevGeomMixed G, DevState S, PhysParams P,
+                                                                              double dt0, float dt0f, int n_steps) {
+  __shared__ ClusterShared sh;
+  const int half = (blockDim.x - 32) / 2, t = threadIdx.x;
+  const bool spare = t >= 2 * half, lower = t < half;
+  const int i = lower ? t : t - half;  // edge and face of the block
+  const int x = blockIdx.x * half + i;
+  // the block's faces, and this thread's: -1 for none
+  const int faces = (G.n_faces + kClusterBlocks - 1) / kClusterBlocks;
+  const int f0 = (int)blockIdx.x * faces + i, f = (!spare && i < faces && f0 < G.n_faces) ? f0 : -1;
+  SlotConsts sc{};
+  SlotGeomF g{};
+  int id = 0;
+  if (!spare && x < G.n_edges) {
+    const int4 ids = ld_rec_i4(G.e_ids, x);
+    const float4 ce = ld_rec_f4(G.e_ec, x), ne = ld_rec_f4(G.e_en, x);
+    const size_t side = lower ? (size_t)x : (size_t)G.epad + x;
+    sc.st = ld_rec_i4(G.e_sten, side);
+    sc.bt = ld_rec_f4(G.e_beta, side);
+    sc.hh = ld_rec_f4(G.e_h, side);
+    sc.eta_p = __fdividef(1.0f, sc.hh.x * sc.hh.z);
+    sc.eta_m = __fdividef(1.0f, sc.hh.y * sc.hh.z);
+    g.ec = f3(ce.x, ce.y, ce.z);
+    g.en = f3(ne.x, ne.y, ne.z);
+    g.nxr = f3(ce.w, ne.w, __int_as_float(ids.z));
+    id = lower ? ids.x : ids.y;
+  }
+  ClusterFace<MAXS> c{};
+  double u0[kDim] = {0, 0, 0, 0, 0};
+  if (f >= 0) {
+    c.r = plane3f(G.fcn32, G.fpad, f);
+    c.acc0 = G.acc_src[f];
+    if (lower) {
+      if (P.solver != kSolverIsoHLLE) c.lo = plane3f(G.fcn_lo, G.fpad, f);
+      c.n = G.nslots[f];
+#pragma unroll
+      for (int j = 0; j < MAXS; ++j) {
+        if (j < c.n) {
+          const int se = G.slot_edge[j * G.fpad + f], e = se & 0x7fffffff;
+          const float co = G.coef[j * G.fpad + f];
+          c.co[j] = (se < 0) ? co : -co;
+          c.e[j] = e;
+        }
+      }
+      float w[kDim];
+      ld5(S.W32, G.fpad, f, w);
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) sh.w[k][t] = w[k];
+#pragma unroll
+      for (int k = 0; k < kDim; ++k) u0[k] = S.U[k * G.fpad + f];
+    }
+  }
+  const bool clock = t == 2 * half && blockIdx.x == gridDim.x - 1;
+  double time = clock ? S.scal[kScTime] : 0.0;
+  cluster_arrive();
+  for (int s = 0; s < n_steps; ++s) {
+    const bool last = s == n_steps - 1;
+    cluster_wait();
+    const float dtf = clip_dt_f32(S.keys, P, dt0f);
+    if (!spare) {
+      cluster_edge<1>(G, S, P, sh, x, half, id, sc, g, dtf);
+    } else {
+      if (t == 2 * half) {
+        const StepDt d = clip_dt(S.keys, P, dt0);
+        sh.dt = d.dt;
+        sh.dt_half = d.dt / 2;
+        if (clock) {
+          time = time + d.dt;
+          if (d.neg_extra) atomicOr(S.err, 8u);  // SPLASH_STOP_NEG_EXTRA_DT
+          if (last) {
+            S.scal[kScDt] = d.dt;
+            S.scal[kScDtHalf] = d.dt / 2;
+            *reinterpret_cast<float2*>(S.scal + kScDtF) = make_float2((float)d.dt, (float)(d.dt / 2));
+            S.scal[kScDt0] = dt0;
+            S.scal[kScMaxVel] = d.max_vel;
+            S.scal[kScExtraDt] = d.extra;
+            S.scal[kScTime] = time;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (t == 0 && blockIdx.x == 0) restart_keys(S.keys);
+    if (!spare)
+      cluster_face<1>(G, S, P, sh, f, half, c, 0.5f * dtf, u0, last);
+    else
+      __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+    if (!spare)
+      cluster_edge<2>(G, S, P, sh, x, half, id, sc, g, dtf);
+    else
+      __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+    if (!spare)
+      cluster_face<2>(G, S, P, sh, f, half, c, dtf, u0, last);
+    else
+      __syncthreads();
+    cluster_arrive();
+  }
+  cluster_wait();
+}
+
 // ---------------------------------------------------------------- ensemble
 // Batched launches over many independent instances: every block looks up
 // its (instance, first face) tile and runs the same bodies as a single
@@ -1146,6 +1424,50 @@ bool two_threads(const DevGeomMixed& G) { return G.n_faces <= kTwoThreadFaces; }
 
 const void* mixed_dt0_kernel_ptr(const DevGeomMixed& G) {
   return two_threads(G) ? (const void*)mx::edge_sides_kernel<1> : (const void*)mx::edge_kernel<1>;
+}
+
+namespace {
+using ClusterKernel = void (*)(DevGeomMixed, DevState, PhysParams, double, float, int);
+ClusterKernel cluster_kernel(const DevGeomMixed& G) {
+  return G.max_slots <= 4   ? mx::cluster_steps_kernel<4>
+         : G.max_slots <= 6 ? mx::cluster_steps_kernel<6>
+                            : mx::cluster_steps_kernel<8>;
+}
+// one cluster over the mesh: the edges of a block are a multiple of a warp
+cudaLaunchConfig_t cluster_config(const DevGeomMixed& G, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  const int n = G.n_edges > G.n_faces ? G.n_edges : G.n_faces;
+  const int half = ((n + mx::kClusterBlocks - 1) / mx::kClusterBlocks + 31) / 32 * 32;
+  cfg.gridDim = dim3(mx::kClusterBlocks);
+  cfg.blockDim = dim3(2 * half + 32);
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = mx::kClusterBlocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+}  // namespace
+
+bool mixed_in_cluster(const DevGeomMixed& G) {
+  const int n = G.n_edges > G.n_faces ? G.n_edges : G.n_faces;
+  if (n > mx::kClusterBlocks * mx::kClusterHalf) return false;
+  ClusterKernel k = cluster_kernel(G);
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cluster_config(G, nullptr, attr);
+  int clusters = 0;
+  const bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok && clusters > 0;
+}
+
+cudaError_t mixed_cluster_steps(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0, int n,
+                                cudaStream_t st) {
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cluster_config(G, st, attr);
+  return cudaLaunchKernelEx(&cfg, cluster_kernel(G), G, S, P, dt0, fpc::d2f(dt0), n);
 }
 
 cudaError_t mixed_scatter_prepare(const double* aos, const int* iperm, const DevGeomMixed& G, const DevState& S,
