@@ -507,6 +507,15 @@ struct SlotConsts {
 // States of the slot's face (q = 0) and its stencil faces (q = 1..4) from a
 // packed array.
 struct ArrayStates {
+  const float *W, *Wp;
+  int i[5];
+  __device__ __forceinline__ float4 sigma_l(int q) const { return ld4(W, i[q]); }
+  __device__ __forceinline__ float pi(int q) const { return Wp[i[q]]; }
+};
+// The same with one base address for the launches that are bound by their
+// chains (two registers fewer: hex(6) 24.2 -> 23.5 us per step, hex(5) 17.0
+// -> 16.8; the full launches are slower with it, hex(9) 756 -> 776).
+struct OneBaseStates {
   const float* W;
   int fp, i[5];
   __device__ __forceinline__ float4 sigma_l(int q) const { return ld4(W, i[q]); }
@@ -565,7 +574,7 @@ __device__ __forceinline__ void recon_slot_of(const States& W, int n, const Slot
 }
 __device__ __forceinline__ void recon_slot(const float* W, int fp, int f, int n, const SlotConsts& sc, F3 ec,
                                            F3 en, float dt, const PhysParams& P, float* up) {
-  recon_slot_of(ArrayStates{W, fp, {f, sc.st.x, sc.st.y, sc.st.z, sc.st.w}}, n, sc, ec, en, dt, P, up);
+  recon_slot_of(ArrayStates{W, W + 4 * (size_t)fp, {f, sc.st.x, sc.st.y, sc.st.z, sc.st.w}}, n, sc, ec, en, dt, P, up);
 }
 
 // One stage's reconstruction and Riemann fluxes, one thread per interior
@@ -805,11 +814,11 @@ __global__ void __launch_bounds__(kBlock) edge_sides_kernel(DevGeomMixed G, DevS
     float u[kDim];
     // whole warps take one branch or the other; one call with a selected
     // normal rounds differently
+    const OneBaseStates W{stage_input<STAGE>(S), G.fpad, {id & 0x0fffffff, sc.st.x, sc.st.y, sc.st.z, sc.st.w}};
     if (owner)
-      recon_slot(stage_input<STAGE>(S), G.fpad, id & 0x0fffffff, id >> 28, sc, g.ec, g.en, dt, P, u);
+      recon_slot_of(W, id >> 28, sc, g.ec, g.en, dt, P, u);
     else
-      recon_slot(stage_input<STAGE>(S), G.fpad, id & 0x0fffffff, id >> 28, sc, g.ec,
-                 f3(-g.en.x, -g.en.y, -g.en.z), dt, P, u);
+      recon_slot_of(W, id >> 28, sc, g.ec, f3(-g.en.x, -g.en.y, -g.en.z), dt, P, u);
 #pragma unroll
     for (int k = 0; k < kDim; ++k) up[k][t] = u[k];
   }
@@ -875,7 +884,11 @@ __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevStat
   F3 fcn32 = f3(0.f, 0.f, 0.f), fcn_lo = f3(0.f, 0.f, 0.f);
   double acc0 = 0.0;
   int n = 0;
-  // the slots' edges and flux coefficients: geometry, loaded before the wait
+  // The slots' edges and flux coefficients: geometry, loaded before the wait,
+  // and not after the load of n that says which of them the face has (the
+  // planes hold max_slots of every face): hex(9) 755 -> 744 us per step,
+  // hex(5) 17.0 -> 16.5.  The early variant, at its register limit, spills
+  // with it (hex(7) 51.7 -> 52.0).
   int se[MAXS];
   float co[MAXS];
   if (live) {
@@ -886,8 +899,9 @@ __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevStat
   }
 #pragma unroll
   for (int j = 0; j < MAXS; ++j) {
-    se[j] = (j < n) ? G.slot_edge[j * fp + f] : 0;
-    co[j] = (j < n) ? G.coef[j * fp + f] : 0.f;
+    const bool plane = (EARLY_STATE && !SPLIT) ? j < n : live && j < G.max_slots;
+    se[j] = plane ? G.slot_edge[j * fp + f] : 0;
+    co[j] = plane ? G.coef[j * fp + f] : 0.f;
   }
   griddep_wait();
   if (RESTART_KEYS && f == 0) restart_keys(S.keys);
@@ -1039,7 +1053,7 @@ __device__ __forceinline__ void cluster_edge(const DevGeomMixed& G, const DevSta
   const int t = threadIdx.x;
   const bool owner = t < half, live = x < G.n_edges;
   if (live) {
-    const ArrayStates W{stage_input<STAGE>(S), G.fpad, {id & 0x0fffffff, sc.st.x, sc.st.y, sc.st.z, sc.st.w}};
+    const OneBaseStates W{stage_input<STAGE>(S), G.fpad, {id & 0x0fffffff, sc.st.x, sc.st.y, sc.st.z, sc.st.w}};
     const int n = id >> 28;
     float u[kDim];
     // two calls for the same reason as in edge_sides_kernel
