@@ -101,7 +101,6 @@ template <int STAGE>
 __global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
                                                             double dt0) {
   griddep_launch_dependents();
-  griddep_wait();
   __shared__ SideExchange<D1, kThreads> sides;
   const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
@@ -109,15 +108,17 @@ __global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevSta
   const bool live = e < G.n_edges;
   if (live) {
     const int x = (t < kEdgeBlock) ? e : G.epad + e;
+    const SideGeom g = side_geom(G, x);
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[G.xs + x], G.e_sten[2 * G.xs + x], G.e_sten[3 * G.xs + x]};
+    griddep_wait();
     const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
     const Planes<D1> W = (STAGE == 1) ? Planes<D1>{S.W0, T.dW0, 0} : Planes<D1>{S.W1, T.dW1, 0};
     const size_t fp = G.fpad;
-    const int f = G.e_face[x];
-    const int st[4] = {G.e_sten[x], G.e_sten[G.xs + x], G.e_sten[2 * G.xs + x], G.e_sten[3 * G.xs + x]};
     D1 w[kDim], u[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) w[k] = W.ld(k * fp + f);
-    recon_side(side_geom(G, x), P.gam, dt, w, [&](int k, int q) { return W.ld(k * fp + st[q]); }, u);
+    recon_side(g, P.gam, dt, w, [&](int k, int q) { return W.ld(k * fp + st[q]); }, u);
     if (STAGE == 1 && x == 0) publish_dt(S, dt);
     sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
   }
@@ -140,14 +141,16 @@ __global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevSta
 template <int STAGE>
 __global__ void __launch_bounds__(kFaceThreads) tlm_update_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P) {
   griddep_launch_dependents();
-  griddep_wait();
   __shared__ FaceParts<D1, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
   const bool live = f < G.n_faces;
+  FluxTerms terms;
+  if (live && part < kDim) terms = flux_terms(G, f);
+  griddep_wait();
   const size_t fp = G.fpad;
   if (live && part < kDim) {
     const Planes<D1> fe{S.fe, T.dfe, 0};
-    parts.put(part, i, flux_sum<D1>(G, f, [&](int e) { return fe.ld((size_t)part * G.epad + e); }));
+    parts.put(part, i, flux_sum<D1>(G, f, terms, [&](int e) { return fe.ld((size_t)part * G.epad + e); }));
   } else if (live) {
     const SrcParams<D1> sp{dual1(G.acc_src[f], T.dacc[f]),
                            v3(D1(P.omega_acc_x), dual1(P.omega_acc_y, T.d_omega_y), dual1(P.omega_acc_z, T.d_omega_z)),
@@ -298,7 +301,6 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
                                                            const double* W, double* uplus,
                                                            double* LJ, double* fe) {
   griddep_launch_dependents();
-  griddep_wait();
   __shared__ SideExchange<double, kThreads> sides;
   const Gas gas = gas_of(P);
   const int t = threadIdx.x, i = t & (kEdgeBlock - 1);
@@ -307,13 +309,15 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
   if (live) {
     const int x = (t < kEdgeBlock) ? e : G.epad + e;
     const size_t fp = G.fpad, xs = G.xs;
+    const SideGeom g = side_geom(G, x);
     const int f = G.e_face[x];
     const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    griddep_wait();
     double w[kDim], u[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) w[k] = W[k * fp + f];
     rev::recon_side_tape(
-        side_geom(G, x), P.gam, *dtp, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u,
+        g, P.gam, *dtp, w, [&](int k, int q) { return W[k * fp + st[q]]; }, u,
         [&](int k, double v) { LJ[k * xs + x] = v; });
 #pragma unroll
     for (int k = 0; k < kDim; ++k) uplus[k * xs + x] = u[k];
@@ -337,13 +341,15 @@ __global__ void __launch_bounds__(kFaceThreads) rc_update_kernel(DevGeom G, Phys
                                                                  const double* fe, double* Uout,
                                                                  double* Wout, uint8_t* mask) {
   griddep_launch_dependents();
-  griddep_wait();
   __shared__ FaceParts<double, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
   const bool live = f < G.n_faces;
+  FluxTerms terms;
+  if (live && part < kDim) terms = flux_terms(G, f);
+  griddep_wait();
   const size_t fp = G.fpad;
   if (live && part < kDim) {
-    parts.put(part, i, flux_sum<double>(G, f, [&](int e) { return fe[(size_t)part * G.epad + e]; }));
+    parts.put(part, i, flux_sum<double>(G, f, terms, [&](int e) { return fe[(size_t)part * G.epad + e]; }));
   } else if (live) {
     double w[kDim], src[kDim];
 #pragma unroll

@@ -384,17 +384,42 @@ struct SideExchange {
 // 124-161) of face f, in three parts that the kernels spread over threads:
 // the sum over the face's slots of -+ coef flux of one field (flux(e): that
 // field of edge e's flux), the source (source_term), and the combination.
+// The edges of slots j0 .. j0 + kTerms - 1 of face f and their coefficients
+// (negated on the owner side), loaded without waiting for the slot count: the
+// planes hold max_slots entries of every face.
+constexpr int kTerms = 6;
+struct FluxTerms {
+  int e[kTerms];
+  double c[kTerms];
+};
+SPLASH_HD FluxTerms flux_terms(const DevGeom& G, int f, int j0 = 0) {
+  FluxTerms t;
+#pragma unroll
+  for (int j = 0; j < kTerms; ++j) {
+    const int se = (j0 + j < G.max_slots) ? G.slot_edge[(size_t)(j0 + j) * G.fpad + f] : 0;
+    t.e[j] = se & 0x7fffffff;
+    const double c = G.e_side[(size_t)kSideCoef * G.xs + (se < 0 ? G.epad + t.e[j] : t.e[j])];
+    t.c[j] = (se < 0) ? c : -c;
+  }
+  return t;
+}
+// `first` is flux_terms of slot 0; a chunk's fluxes are in flight together
 template <class T, class FluxFn>
-SPLASH_HD T flux_sum(const DevGeom& G, int f, FluxFn flux) {
+SPLASH_HD T flux_sum(const DevGeom& G, int f, const FluxTerms& first, FluxFn flux) {
   T acc(0.);
   const int n = G.nslots[f];
-  for (int j = 0; j < n; ++j) {
-    const int se = G.slot_edge[j * G.fpad + f];
-    const int e = se & 0x7fffffff;
-    const double c = G.e_side[(size_t)kSideCoef * G.xs + (se < 0 ? G.epad + e : e)];
-    acc = fm((se < 0) ? c : -c, flux(e), acc);
+  FluxTerms t = first;
+  for (int j0 = 0;;) {
+    T F[kTerms];
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j) F[j] = flux(t.e[j]);
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j)
+      if (j0 + j < n) acc = fm(t.c[j], F[j], acc);
+    j0 += kTerms;
+    if (j0 >= n) return acc;
+    t = flux_terms(G, f, j0);
   }
-  return acc;
 }
 // U0 + dt_here (source + sum), floored; `floored` reports the density floor
 template <class T>

@@ -171,10 +171,12 @@ __global__ void __launch_bounds__(kFaceThreads) update_parts_kernel(DevGeom G, D
   __shared__ FaceParts<double, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
   const bool live = f < G.n_faces;
+  FluxTerms terms;
+  if (live && part < kDim) terms = flux_terms(G, f);
   griddep_wait();
   if (live && part < kDim) {
     const double* fe = S.fe + (size_t)part * G.epad;
-    parts.put(part, i, flux_sum<double>(G, f, [&](int e) { return fe[e]; }));
+    parts.put(part, i, flux_sum<double>(G, f, terms, [&](int e) { return fe[e]; }));
   } else if (live) {
     double src[kDim];
     face_source<STAGE>(G, S, P, f, src);
