@@ -322,7 +322,7 @@ int Solver::capture_steps(int n_steps, cudaGraph_t* g, cudaGraphExec_t* exec, st
   SPLASH_CUDA(ce);
   *g = got;
   SPLASH_CUDA(cudaGraphInstantiate(exec, got, 0));
-  const void* first = precision == SPLASH_PREC_MIXED ? mixed_dt0_kernel_ptr(GM) : fp64_dt0_kernel_ptr(solver_kind);
+  const void* first = precision == SPLASH_PREC_MIXED ? mixed_dt0_kernel_ptr(GM) : fp64_dt0_kernel_ptr(G, solver_kind);
   size_t n = 0;
   SPLASH_CUDA(cudaGraphGetNodes(got, nullptr, &n));
   std::vector<cudaGraphNode_t> nodes(n);

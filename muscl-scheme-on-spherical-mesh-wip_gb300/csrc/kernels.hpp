@@ -19,7 +19,7 @@ cudaError_t fp64_prepare(const DevGeom& G, const DevState& S, const PhysParams& 
 // dt slot, after every launch).
 cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, double dt0, cudaStream_t st,
                       cudaEvent_t* ev = nullptr);
-const void* fp64_dt0_kernel_ptr(int solver);
+const void* fp64_dt0_kernel_ptr(const DevGeom& G, int solver);
 // reference-order [n_faces][dim] <-> internal planes (dim 5, or 4 for the
 // isothermal solver, whose fifth plane is zero); iperm[reference face] =
 // internal face.  aos may be host memory the device can access.

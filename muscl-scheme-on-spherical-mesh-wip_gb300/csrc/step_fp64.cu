@@ -58,6 +58,22 @@ __global__ void __launch_bounds__(kFaceBlock) prepare_kernel(DevGeom G, DevState
   fold_warp(vel2, rate2, negative, S, P, gridDim.x * (kFaceBlock / 32));
 }
 
+// the flux of edge e, whose sides are columns i and kEdgeBlock + i
+__device__ __forceinline__ void store_flux(const DevGeom& G, const DevState& S, const PhysParams& P, const Gas& gas,
+                                           const SideExchange<double, kThreads>& sides, int e, int i) {
+  double L[kDim], R[kDim], F[kDim];
+  EdgeSide<double> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    if (nan_bits(F[k])) bits |= 1u;
+    S.fe[(size_t)k * G.epad + e] = F[k];
+  }
+  if (bits) atomicOr(S.err, bits);
+}
+
 // find_U_edges (MUSCL_base.hpp:361-434) of both sides of every edge and the
 // Riemann flux (find_flux_var, MUSCL_base.hpp:345-359).
 template <int STAGE>
@@ -90,17 +106,79 @@ __global__ void __launch_bounds__(kThreads) edge_kernel(DevGeom G, DevState S, P
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
-  double L[kDim], R[kDim], F[kDim];
-  EdgeSide<double> SL, SR;
-  sides.get(i, L, SL);
-  sides.get(kEdgeBlock + i, R, SR);
-  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
+  store_flux(G, S, P, gas, sides, e, i);
+}
+
+// The same with kDim threads per side, one per field, for meshes whose sides
+// leave the SMs a warp or two: there a launch takes the latency of one
+// thread's chain, 255 dependent FP64 instructions of 36 ns and 3,100 in all.
+// Warp 2 k + s of a block serves field k of side s of its 32 edges; the field
+// 0 warps evaluate the side's Courant factor while the others form their
+// differences, then every warp limits its field, and the field 0 warps go on
+// as in edge_kernel.  Two blocks per SM: at one (112 registers) hex(4) takes
+// two waves, 51.6 us per step instead of 40.7.
+constexpr int kEdgePartThreads = kThreads * kDim;
+template <int STAGE>
+__global__ void __launch_bounds__(kEdgePartThreads, 2) edge_parts_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
+  griddep_launch_dependents();
+  __shared__ SideExchange<double, kThreads> sides;
+  __shared__ double up[kDim][kThreads];
+  __shared__ __align__(8) unsigned char limiters[kThreads * sizeof(SideLimiter)];
+  const int warp = threadIdx.x / 32, k = warp >> 1, i = threadIdx.x & 31;
+  const int t = (warp & 1) * kEdgeBlock + i;  // the side, as in edge_kernel
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  const int x = (t < kEdgeBlock) ? e : G.epad + e;
+  const size_t fp = G.fpad, xs = G.xs;
+  SideLimiter& limiter = reinterpret_cast<SideLimiter*>(limiters)[t];
+  SideGeom g{};
+  double wk = 0.0, dp = 0.0, num = 0.0, dpg = 0.0;
+  if (live) {
+    g = side_geom(G, x);
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    griddep_wait();
+    const double* W = (STAGE == 1) ? S.W0 : S.W1;
+    const double* Wk = W + k * fp;
+    wk = Wk[f];
+    double dm;
+    side_differences(g, wk, Wk[st[0]], Wk[st[1]], Wk[st[2]], Wk[st[3]], dp, dm);
+    num = dm * g.hr;
+    dpg = dp * g.hg;
+    if (k == 0) {
+      const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
+      double w[kDim], c;
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    if (nan_bits(F[k])) bits |= 1u;
-    S.fe[(size_t)k * G.epad + e] = F[k];
+      for (int q = 0; q < kDim; ++q) w[q] = W[q * fp + f];
+      const double nu = side_courant(g, P.gam, dt, w, c);
+      limiter = SideLimiter(g, nu, w[0], w[4], c);
+    } else if (STAGE == 1 && k == kDim - 1 && x == 0) {
+      publish_dt(S, step_dt(S.scal, dt0));
+    }
   }
-  if (bits) atomicOr(S.err, bits);
+  __syncthreads();
+  if (live) {
+    double lim;
+    if (!limiter.in_pairs(k, dp, num, dpg, lim)) {
+      const LimiterLine<double> line = limiter_line(g.eta_p, g.sbs, limiter.nu);
+      lim = limiter_full(dp, num, line.eta_p, line.sb, line.ts, line.t1);
+    }
+    const double u = fm(dpg, lim, wk);
+    up[k][t] = u;
+    if (STAGE == 2) S.uplus[k * xs + x] = u;
+  }
+  __syncthreads();
+  if (k != 0) return;
+  const Gas gas = gas_of(P);
+  double u[kDim];
+  if (live) {
+#pragma unroll
+    for (int q = 0; q < kDim; ++q) u[q] = up[q][t];
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
+  }
+  asm volatile("bar.sync 1, 64;" ::: "memory");  // the two field 0 warps
+  if (!live || t >= kEdgeBlock) return;
+  store_flux(G, S, P, gas, sides, e, i);
 }
 
 // res2d + the RK combine; stage 1: dt/2, writes W1; stage 2: dt, writes U, W0
@@ -372,8 +450,20 @@ cudaError_t fp64_prepare(const DevGeom& G, const DevState& S, const PhysParams& 
   return cudaGetLastError();
 }
 
-const void* fp64_dt0_kernel_ptr(int solver) {
-  return solver == kSolverIsoHLLE ? (const void*)f64::iso_edge_kernel<1> : (const void*)f64::edge_kernel<1>;
+namespace {
+// kDim threads per side on meshes of at most a wave and a quarter of its
+// blocks (two per SM).  us per step of MUSCL_HLLE_p / HLLC+, one thread per
+// side / kDim: hex(3) 48.8 / 37.5 and 54.5 / 43.3, hex(4) 53.9 / 40.7 and 59.7
+// / 45.8, quad(5) (12,288 edges) 58.8 / 55.0 and 67.2 / 66.1; hex(5) (30,720)
+// 72.3 / 122 and 81.6 / 160.
+constexpr int kEdgePartsEdges = 12288;
+bool edge_parts(const DevGeom& G) { return G.n_edges <= kEdgePartsEdges; }
+}  // namespace
+
+const void* fp64_dt0_kernel_ptr(const DevGeom& G, int solver) {
+  return solver == kSolverIsoHLLE ? (const void*)f64::iso_edge_kernel<1>
+         : edge_parts(G)          ? (const void*)f64::edge_parts_kernel<1>
+                                  : (const void*)f64::edge_kernel<1>;
 }
 
 cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, double dt0, cudaStream_t st,
@@ -387,11 +477,12 @@ cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, 
   // 366 / 367, hex(7) 760 / 798, quad(8) 1262 / 1352.
   constexpr int kPartsFaces = 65536;
   const bool iso = P.solver == kSolverIsoHLLE, parts = !iso && G.n_faces <= kPartsFaces;
-  const Edge edge1 = iso ? f64::iso_edge_kernel<1> : f64::edge_kernel<1>;
-  const Edge edge2 = iso ? f64::iso_edge_kernel<2> : f64::edge_kernel<2>;
+  const bool fields = !iso && edge_parts(G);
+  const Edge edge1 = iso ? f64::iso_edge_kernel<1> : fields ? f64::edge_parts_kernel<1> : f64::edge_kernel<1>;
+  const Edge edge2 = iso ? f64::iso_edge_kernel<2> : fields ? f64::edge_parts_kernel<2> : f64::edge_kernel<2>;
   const Update upd1 = iso ? f64::iso_update_kernel<1> : parts ? f64::update_parts_kernel<1> : f64::update_kernel<1>;
   const Update upd2 = iso ? f64::iso_update_kernel<2> : parts ? f64::update_parts_kernel<2> : f64::update_kernel<2>;
-  const dim3 eg(f64::edge_blocks(G.n_edges)), eb(f64::kThreads);
+  const dim3 eg(f64::edge_blocks(G.n_edges)), eb(fields ? f64::kEdgePartThreads : f64::kThreads);
   const dim3 fg(f64::face_blocks(G.n_faces, parts ? f64::kFaces : f64::kFaceBlock));
   const dim3 fb(parts ? f64::kFaceThreads : f64::kFaceBlock);
   FirstError chk;

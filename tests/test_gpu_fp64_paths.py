@@ -31,3 +31,23 @@ def test_step_equals_the_tangent_models_values(kind, level, solver, friction):
     base.do_steps(3, 1e-2)
     assert np.array_equal(base.get_state(), Ut)
     assert base.last_dt() < 1e-2 or level < 4
+
+
+@pytest.mark.parametrize("kind,level", [("hex", 0), ("hex", 1), ("quad", 1), ("ico", 2), ("hex", 4), ("quad", 5)])
+@pytest.mark.parametrize("solver,noise", [(1, 0.2), (2, 1e-3), (3, 1e-2)])
+def test_fields_on_threads_of_their_own(kind, level, solver, noise):
+    """The smallest meshes give every field of a side a thread: the tangent model's values, which one thread per side makes,
+    with partial blocks (30, 120, 24, 480 edges), up to the largest such mesh, smooth and steep."""
+    import splash_gb300 as sg
+
+    mesh = mesh_of(kind, level)
+    r = sg.Geometry(mesh).unit_face_centers()
+    U = sg.initial_conditions.rotating_blob(r, GAM, seed=solver)
+    U[:, 0] *= 1 + noise * np.random.default_rng(level).uniform(-1, 1, len(U))
+    params = sg.SolverParams(accretion_rate=1e-2, e_acc=0.5, omega_acc_abs=0.5, tilt_angle=0.2, acc_width=0.1,
+                             alpha=1e-6, friction_on=True)
+    base = sg.Solver(mesh, U, 5, GAM, 0.0, True, params=params, solver=solver, precision=sg.PREC_FP64)
+    Ut, _ = sg.Adjoint(base, checkpoint_every=1).tlm(U, np.array([1e-2, 0.2, 0.5]), np.ones_like(U), np.zeros(3), 5, 1e-3)
+    base.do_steps(5, 1e-3)
+    # equal_nan: the coarsest quad mesh leaves the range of the method, on both paths alike
+    assert np.array_equal(base.get_state(), Ut, equal_nan=True)
