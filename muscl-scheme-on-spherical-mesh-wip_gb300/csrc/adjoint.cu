@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
   for (int k = 0; k < kDim; ++k) fe[(size_t)k * G.epad + e] = F[k];
 }
 
-template <int STAGE>
-__global__ void __launch_bounds__(kFaceThreads) rc_update_kernel(DevGeom G, PhysParams P, const double* dtp,
+template <int STAGE, int BLOCKS>
+__global__ void __launch_bounds__(kFaceThreads, BLOCKS) rc_update_kernel(DevGeom G, PhysParams P, const double* dtp,
                                                                  const double* Win,
                                                                  const double* U0,
                                                                  const double* fe, double* Uout,
@@ -449,8 +449,11 @@ __global__ void __launch_bounds__(kThreads, 7) adj_edge_kernel(DevGeom G, PhysPa
   }
 }
 
+// Four blocks per SM (80 registers instead of 108): the gathers of the five
+// field warps wait on memory, and three blocks cover less of it.  20 steps'
+// gradient on hex(4) 4.65 -> 4.34 ms, hex(5) 6.99 -> 6.77, hex(6) 21.1 -> 20.4.
 template <int STAGE>
-__global__ void __launch_bounds__(kFaceThreads) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
+__global__ void __launch_bounds__(kFaceThreads, 4) adj_face_kernel(DevGeom G, PhysParams P, double dt_here, AdjScratch X,
                                                                 const double* Win,
                                                                 const double* Uin,
                                                                 const uint8_t* mask, const double* lam,
@@ -589,9 +592,10 @@ cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, co
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
   constexpr int B = f64::kFaceThreads, E = adj::kThreads;
   chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W0, t.P0, t.J0, fe));
-  chk(launch_pdl(adj::rc_update_kernel<1>, dim3(nb), dim3(B), st, G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask));
+  const bool five = f64::five_face_blocks(G.n_faces);
+  chk(launch_pdl(five ? adj::rc_update_kernel<1, 5> : adj::rc_update_kernel<1, 4>, dim3(nb), dim3(B), st, G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask));
   chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W1, t.P1, t.J1, fe));
-  chk(launch_pdl(adj::rc_update_kernel<2>, dim3(nb), dim3(B), st, G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask));
+  chk(launch_pdl(five ? adj::rc_update_kernel<2, 5> : adj::rc_update_kernel<2, 4>, dim3(nb), dim3(B), st, G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask));
   return chk.status();
 }
 

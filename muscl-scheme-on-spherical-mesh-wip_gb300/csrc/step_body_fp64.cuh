@@ -441,6 +441,11 @@ SPLASH_HD void combine_face(double dt_here, const T* src, const T* sum, const T*
 // longest part.
 constexpr int kFaces = 32;
 constexpr int kFaceThreads = kFaces * (kDim + 1);
+// Blocks per SM that a face launch of n_faces is compiled for: 5 (64
+// registers) where more than the 4 that fit at 66-70 registers are there for
+// each of the GB300's 152 SMs.  us per step, 4 / 5: hex(5) 76 / 79, hex(6)
+// 230 / 217.
+inline bool five_face_blocks(int n_faces) { return (n_faces + kFaces - 1) / kFaces > 4 * 152; }
 __device__ __forceinline__ int face_part() { return (int)((threadIdx.x / kFaces + blockIdx.x) % (kDim + 1)); }
 template <class T, int N>
 struct FaceParts {

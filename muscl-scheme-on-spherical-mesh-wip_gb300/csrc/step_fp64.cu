@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(kFaceBlock) update_kernel(DevGeom G, DevState 
   finish_face<STAGE>(G, S, P, f, live, src, sum, gridDim.x * (kFaceBlock / 32));
 }
 // kDim + 1 threads per face (face_part)
-template <int STAGE>
-__global__ void __launch_bounds__(kFaceThreads) update_parts_kernel(DevGeom G, DevState S, PhysParams P) {
+template <int STAGE, int BLOCKS>
+__global__ void __launch_bounds__(kFaceThreads, BLOCKS) update_parts_kernel(DevGeom G, DevState S, PhysParams P) {
   griddep_launch_dependents();
   __shared__ FaceParts<double, 2 * kDim> parts;
   const int part = face_part(), i = threadIdx.x % kFaces, f = blockIdx.x * kFaces + i;
@@ -480,8 +480,15 @@ cudaError_t fp64_step(const DevGeom& G, const DevState& S, const PhysParams& P, 
   const bool fields = !iso && edge_parts(G);
   const Edge edge1 = iso ? f64::iso_edge_kernel<1> : fields ? f64::edge_parts_kernel<1> : f64::edge_kernel<1>;
   const Edge edge2 = iso ? f64::iso_edge_kernel<2> : fields ? f64::edge_parts_kernel<2> : f64::edge_kernel<2>;
-  const Update upd1 = iso ? f64::iso_update_kernel<1> : parts ? f64::update_parts_kernel<1> : f64::update_kernel<1>;
-  const Update upd2 = iso ? f64::iso_update_kernel<2> : parts ? f64::update_parts_kernel<2> : f64::update_kernel<2>;
+  const bool five = parts && f64::five_face_blocks(G.n_faces);
+  const Update upd1 = iso     ? f64::iso_update_kernel<1>
+                      : five  ? f64::update_parts_kernel<1, 5>
+                      : parts ? f64::update_parts_kernel<1, 4>
+                              : f64::update_kernel<1>;
+  const Update upd2 = iso     ? f64::iso_update_kernel<2>
+                      : five  ? f64::update_parts_kernel<2, 5>
+                      : parts ? f64::update_parts_kernel<2, 4>
+                              : f64::update_kernel<2>;
   const dim3 eg(f64::edge_blocks(G.n_edges)), eb(fields ? f64::kEdgePartThreads : f64::kThreads);
   const dim3 fg(f64::face_blocks(G.n_faces, parts ? f64::kFaces : f64::kFaceBlock));
   const dim3 fb(parts ? f64::kFaceThreads : f64::kFaceBlock);

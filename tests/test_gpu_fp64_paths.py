@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 GAM = 2 - 1 / (4 / 3)
 
 
-@pytest.mark.parametrize("kind,level", [("hex", 2), ("hex", 3), ("hex", 5), ("quad", 5), ("quad", 7), ("hex", 7)])
+@pytest.mark.parametrize("kind,level", [("hex", 2), ("hex", 3), ("hex", 5), ("quad", 5), ("quad", 6), ("quad", 7), ("hex", 7)])
 @pytest.mark.parametrize("solver,friction", [(1, True), (2, False), (3, True)])
 def test_step_equals_the_tangent_models_values(kind, level, solver, friction):
     """Small meshes update with six threads per face, large ones with one, the tangent-linear model always with six and on
