@@ -1003,7 +1003,7 @@ __device__ __forceinline__ void update_body(const DevGeomMixed& G, const DevStat
 // stage 2, hex(9) 741 us per step instead of 732; the copy for 4 slots spills
 // with it (quad(8) 86.5 us uncapped, 88.3 capped).
 template <int STAGE, int MAXS>
-__global__ void __launch_bounds__(kBlock, MAXS <= 4 ? 1 : 9) update_kernel(DevGeomMixed G, DevState S, PhysParams P) {
+__global__ void __launch_bounds__(kBlock, MAXS <= 4 ? 0 : 9) update_kernel(DevGeomMixed G, DevState S, PhysParams P) {
   griddep_launch_dependents();
   update_body<STAGE, MAXS, true, STAGE == 1>(G, S, P, blockIdx.x * blockDim.x + threadIdx.x);
 }
