@@ -316,24 +316,6 @@ def algorithmic_bytes_mixed(geom, kernel: str) -> float:
     return F * (20 + 40 + 24 + 12 + 8 + 1) + S * 8 + E * 20 + F * (20 + 40 / 2)
 
 
-def algorithmic_bytes(geom, kernel: str) -> float:
-    """Compulsory bytes per launch of one kernel of the FP64 path.
-
-    reconstruct: read W (5 x 8 B per face), per slot 4 int32 stencil ids +
-      4 betas + H+, H-, BM + edge centre (3) + |ec| + normal (3) + Courant
-      factor + 2 eta (8 B each except ids) ; write U+ (5 x 8 B per slot).
-    flux_update: read U+ (5 x 8 B per slot, each read once algorithmically),
-      per slot edge centre, |ec|, normal, n x R, chord (11 x 8 B) + reverse
-      index (4 B); per face W, U0, unit centre, area, accretion source
-      (5+5+3+1+1 doubles) ; write U (or W1) and W (10 x 8 B).
-    """
-    F = geom.n_faces
-    S = geom.n_slots
-    if kernel == "reconstruct":
-        return F * 40 + S * (16 + 8 * (4 + 3 + 3 + 1 + 3 + 1 + 2)) + S * 40
-    return S * 40 + S * (11 * 8 + 4) + F * 8 * (5 + 5 + 3 + 1 + 1) + F * 80
-
-
 # ------------------------------------------------------------------ arms
 STOP_BITS = {1: "nan_flux", 2: "nan_wave_speed", 4: "wave_order", 8: "negative_extra_dt"}
 
@@ -729,8 +711,7 @@ def run_ours(args):
     kern = {"dt_clip_slot": lt[0], "edge": (lt[1] + lt[3]) / 2, "update": (lt[2] + lt[4]) / 2,
             "edge_stage1": lt[1], "edge_stage2": lt[3], "update_stage1": lt[2], "update_stage2": lt[4]}
     per_step = {"edge": lt[1] + lt[3], "update": lt[2] + lt[4]}
-    kern64 = {"dt_reduce": ms64[0], "reconstruct": (ms64[1] + ms64[3]) / 2,
-              "flux_update": (ms64[2] + ms64[4]) / 2}
+    kern64 = {"dt_clip_slot": ms64[0], "edge": (ms64[1] + ms64[3]) / 2, "update": (ms64[2] + ms64[4]) / 2}
     dom = max(per_step, key=per_step.get)
     hbm, src = peaks()
     ach = algorithmic_bytes_mixed(geom, dom) / (kern[dom] * 1e-3) / 1e9

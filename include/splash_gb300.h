@@ -150,23 +150,16 @@ SPLASH_API int splash_synchronize(splash_solver* s);
 SPLASH_API int splash_stream(splash_solver* s, void** stream);
 /* Runs `reps` un-captured steps with CUDA events between the step's phases
  * and returns the mean device time per phase in milliseconds:
- * ms[0] dt reduction (FP64 path; on the mixed path the stage-1 edge
- * launch clips dt itself and ms[0] is an empty slot); FP64 path: ms[1]
- * reconstruct (stage 1),
- * ms[2] flux+update (stage 1), ms[3] reconstruct (stage 2), ms[4]
- * flux+update (stage 2); mixed path: ms[1] edge (reconstruction + Riemann
- * flux, stage 1), ms[2] update (stage 1), ms[3] edge (stage 2), ms[4] update
- * (stage 2).  The steps advance the state like do_step(dt0). */
+ * ms[0] an empty slot (the stage-1 edge launch clips the step's dt itself),
+ * ms[1] edge (reconstruction + Riemann flux, stage 1), ms[2] update (stage 1),
+ * ms[3] edge (stage 2), ms[4] update (stage 2).  The steps advance the state
+ * like do_step(dt0). */
 SPLASH_API int splash_kernel_times(splash_solver* s, int reps, double dt0, double ms[5]);
 /* Mean device ms of every launch of one step over `reps` un-captured steps,
  * with a CUDA event between consecutive launches (which serialises the
  * step's programmatic overlap, so the sum exceeds the captured step's time).
- * Five slots on either path: mixed, the dt clip (an empty slot: the
- * stage-1 edge launch clips dt itself, so a mixed step is four launches),
- * edge (reconstruction + Riemann flux, stage 1), update (stage 1), edge
- * (stage 2), update (stage 2); FP64, dt reduction, reconstruct,
- * flux+update, reconstruct, flux+update.  Writes min(cap, *count) values;
- * *count = 5.
+ * Five slots, as splash_kernel_times (a step is four launches).  Writes
+ * min(cap, *count) values; *count = 5.
  * The steps advance the state like do_step(dt0). */
 SPLASH_API int splash_launch_times(splash_solver* s, int reps, double dt0, double* ms, int cap, int* count);
 /* Device bytes held by the solver: out[0] geometry, out[1] state + scratch. */
@@ -274,7 +267,8 @@ SPLASH_API int splash_ensemble_create(const splash_member* members, int n, int d
                            splash_ensemble** out);
 SPLASH_API int splash_ensemble_destroy(splash_ensemble* e);
 /* n steps of every member: member i advances by min(dt0, its CFL clip).
- * One graph replay per step, or one (the persistent schedule) for all n. */
+ * Graph replays of four steps and of one, or one (the persistent schedule)
+ * for all n. */
 SPLASH_API int splash_ensemble_do_steps(splash_ensemble* e, int n, double dt0);
 /* Waits for the ensemble's stream; SPLASH_E_CUDA if a grid barrier of the
  * persistent launch timed out (its bounded wait, about 0.25 s). */
@@ -340,7 +334,7 @@ SPLASH_API int splash_cfl_dt_noalloc(const double* U, const double* unit_centres
  * must outlive it) and owns its own state.  The forward run keeps the state
  * every `checkpoint_every` steps; the backward run recomputes each interval
  * from its checkpoint (the tape of one interval: checkpoint_every *
- * (20 + 42 * max_slots) * 8 bytes per face, 4.5 GB for icosphere_hex(6) at
+ * (20 + 40 n) * 8 bytes per face of n edges, 4.3 GB for icosphere_hex(6) at
  * 50 steps) and sweeps it in reverse.  States and adjoints are [n_faces][5] in reference face
  * order; every call is synchronous. */
 typedef struct splash_adjoint splash_adjoint;

@@ -378,16 +378,14 @@ class Solver:
         return int(p.value or 0)
 
     def kernel_times(self, reps: int, dt0: float) -> np.ndarray:
-        """Mean device ms per launch: dt, recon1, flux1, recon2, flux2."""
+        """Mean device ms per launch: an empty slot (the stage-1 edge launch clips dt), edge 1, update 1, edge 2, update 2."""
         out = np.zeros(5)
         _check(self._lib.splash_kernel_times(self.handle, reps, dt0, _dptr(out)))
         return out
 
     def launch_times(self, reps: int, dt0: float) -> np.ndarray:
-        """Mean device ms of every timing slot of one step (mixed: the dt clip
-        (an empty slot: the stage-1 edge launch clips dt), edge 1, update 1,
-        edge 2, update 2; FP64: dt, recon1, flux1, recon2, flux2), with events
-        between launches."""
+        """Mean device ms of every timing slot of one step (those of
+        kernel_times), with events between launches."""
         out = np.zeros(8)
         n = C.c_int(0)
         _check(self._lib.splash_launch_times(self.handle, reps, dt0, _dptr(out), 8, C.byref(n)))
