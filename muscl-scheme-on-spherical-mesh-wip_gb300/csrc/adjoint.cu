@@ -59,10 +59,21 @@ using D1 = Dual<1>;
 static_assert(kTapeJ == rev::kTapePlanes, "tape plane count");
 constexpr int kBlock = 64;                // faces per block
 constexpr int kThreads = 2 * kEdgeBlock;  // edge launches: a thread per side, as in step_fp64.cu
+inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
+// Edge launches with a thread per field of a side up to kPartsEdges edges, at
+// two blocks per SM where one for each of the 152 SMs is not enough.  20 steps,
+// one thread per side / kDim: tangent on hex(3) 2.20 / 1.70 ms, hex(4) 3.29 /
+// 1.97 (one block per SM 2.43), quad(5) 4.45 / 3.32; gradient on hex(3) 3.52 /
+// 3.20, quad(4) 4.10 / 3.98 (two blocks per SM, 96 registers: 4.66), hex(4)
+// 4.39 / 4.20, quad(5) 7.0 / 6.4.
+constexpr int kPartsEdges = 12288;
+enum class Split { kSides, kFields, kFieldsTwo };
+inline Split edge_split(int n_edges) {
+  return n_edges > kPartsEdges ? Split::kSides : edge_blocks(n_edges) > 152 ? Split::kFieldsTwo : Split::kFields;
+}
 
 inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
 inline int face_blocks(int n) { return (n + kFaces - 1) / kFaces; }
-inline int edge_blocks(int n) { return (n + kEdgeBlock - 1) / kEdgeBlock; }
 
 __device__ __forceinline__ D1 dual1(double v, double d) {
   D1 r(v);
@@ -97,6 +108,24 @@ __global__ void __launch_bounds__(kBlock) tlm_prepare_kernel(DevGeom G, DevState
   fold_warp(vel2, rate2, negative, S, P, gridDim.x * (kBlock / 32));
 }
 
+// the flux of edge e, whose sides are columns i and kEdgeBlock + i
+__device__ __forceinline__ void tlm_flux(const DevGeom& G, const DevState& S, const TlmTangents& T,
+                                         const PhysParams& P, const Gas& gas, const SideExchange<D1, kThreads>& sides,
+                                         int e, int i) {
+  D1 L[kDim], R[kDim], F[kDim];
+  EdgeSide<D1> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
+  const Planes<D1> fe{S.fe, T.dfe, 0};
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) {
+    if (nan_bits(F[k].v)) bits |= 1u;
+    fe.st((size_t)k * G.epad + e, F[k]);
+  }
+  if (bits) atomicOr(S.err, bits);
+}
+
 template <int STAGE>
 __global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevState S, TlmTangents T, PhysParams P,
                                                             double dt0) {
@@ -124,18 +153,69 @@ __global__ void __launch_bounds__(kThreads, 7) tlm_edge_kernel(DevGeom G, DevSta
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
-  D1 L[kDim], R[kDim], F[kDim];
-  EdgeSide<D1> SL, SR;
-  sides.get(i, L, SL);
-  sides.get(kEdgeBlock + i, R, SR);
-  unsigned bits = riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
-  const Planes<D1> fe{S.fe, T.dfe, 0};
+  tlm_flux(G, S, T, P, gas, sides, e, i);
+}
+
+// with a thread per field of a side, as edge_parts_kernel of step_fp64.cu
+template <int STAGE, int BLOCKS>
+__global__ void __launch_bounds__(kEdgePartThreads, BLOCKS) tlm_edge_parts_kernel(DevGeom G, DevState S, TlmTangents T,
+                                                                          PhysParams P, double dt0) {
+  griddep_launch_dependents();
+  __shared__ SideExchange<D1, kThreads> sides;
+  __shared__ double up[2][kDim][kThreads], nus[2][kThreads];
+  __shared__ __align__(8) unsigned char limiters[kThreads * sizeof(SideLimiterPartials)];
+  const int warp = threadIdx.x / 32, k = warp >> 1, i = threadIdx.x & 31;
+  const int t = (warp & 1) * kEdgeBlock + i;
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  const int x = (t < kEdgeBlock) ? e : G.epad + e;
+  const size_t fp = G.fpad, xs = G.xs;
+  SideLimiterPartials& limiter = reinterpret_cast<SideLimiterPartials*>(limiters)[t];
+  SideGeom g{};
+  D1 wk, dp, num, dpg;
+  if (live) {
+    g = side_geom(G, x);
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    griddep_wait();
+    const Planes<D1> W = (STAGE == 1) ? Planes<D1>{S.W0, T.dW0, 0} : Planes<D1>{S.W1, T.dW1, 0};
+    wk = W.ld(k * fp + f);
+    D1 dm;
+    side_differences(g, wk, W.ld(k * fp + st[0]), W.ld(k * fp + st[1]), W.ld(k * fp + st[2]), W.ld(k * fp + st[3]), dp,
+                     dm);
+    num = dm * g.hr;
+    dpg = dp * g.hg;
+    if (k == 0) {
+      const double dt = (STAGE == 1) ? step_dt(S.scal, dt0) : S.scal[kScDt];
+      D1 w[kDim], c;
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) {
-    if (nan_bits(F[k].v)) bits |= 1u;
-    fe.st((size_t)k * G.epad + e, F[k]);
+      for (int q = 0; q < kDim; ++q) w[q] = W.ld(q * fp + f);
+      const D1 nu = side_courant(g, P.gam, dt, w, c);
+      limiter = SideLimiterPartials(g, nu.v, w[0].v, w[4].v, c.v);
+      nus[0][t] = nu.v;
+      nus[1][t] = nu.d[0];
+    } else if (STAGE == 1 && k == kDim - 1 && x == 0) {
+      publish_dt(S, step_dt(S.scal, dt0));
+    }
   }
-  if (bits) atomicOr(S.err, bits);
+  __syncthreads();
+  if (live) {
+    const D1 u = limited_dual(limiter, k, wk, dp, num, dpg, dual1(nus[0][t], nus[1][t]));
+    up[0][k][t] = u.v;
+    up[1][k][t] = u.d[0];
+  }
+  __syncthreads();
+  if (k != 0) return;
+  const Gas gas = gas_of(P);
+  D1 u[kDim];
+  if (live) {
+#pragma unroll
+    for (int q = 0; q < kDim; ++q) u[q] = dual1(up[0][q][t], up[1][q][t]);
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
+  }
+  field0_sync();
+  if (!live || t >= kEdgeBlock) return;
+  tlm_flux(G, S, T, P, gas, sides, e, i);
 }
 
 template <int STAGE>
@@ -295,6 +375,16 @@ __global__ void __launch_bounds__(kBlock) rc_prim_kernel(DevGeom G, PhysParams P
   for (int k = 0; k < kDim; ++k) W[(size_t)k * fp + f] = w[k];
 }
 
+__device__ __forceinline__ void rc_flux(const DevGeom& G, const PhysParams& P, const Gas& gas,
+                                        const SideExchange<double, kThreads>& sides, double* fe, int e, int i) {
+  double L[kDim], R[kDim], F[kDim];
+  EdgeSide<double> SL, SR;
+  sides.get(i, L, SL);
+  sides.get(kEdgeBlock + i, R, SR);
+  riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
+#pragma unroll
+  for (int k = 0; k < kDim; ++k) fe[(size_t)k * G.epad + e] = F[k];
+}
 // the edge launch of the step with the limiter's Jacobian (LJ) and the edge
 // states (uplus) kept
 __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams P, const double* dtp,
@@ -325,13 +415,61 @@ __global__ void __launch_bounds__(kThreads) rc_edge_kernel(DevGeom G, PhysParams
   }
   __syncthreads();
   if (!live || t >= kEdgeBlock) return;
-  double L[kDim], R[kDim], F[kDim];
-  EdgeSide<double> SL, SR;
-  sides.get(i, L, SL);
-  sides.get(kEdgeBlock + i, R, SR);
-  riemann_flux(L, R, SL, SR, edge_geom(G, e), gas, P.solver, F);
+  rc_flux(G, P, gas, sides, fe, e, i);
+}
+
+// with a thread per field of a side
+template <int BLOCKS>
+__global__ void __launch_bounds__(kEdgePartThreads, BLOCKS) rc_edge_parts_kernel(DevGeom G, PhysParams P, const double* dtp,
+                                                                         const double* W, double* uplus, double* LJ,
+                                                                         double* fe) {
+  griddep_launch_dependents();
+  __shared__ SideExchange<double, kThreads> sides;
+  __shared__ double up[kDim][kThreads];
+  __shared__ __align__(8) unsigned char limiters[kThreads * sizeof(SideLimiterPartials)];
+  const int warp = threadIdx.x / 32, k = warp >> 1, i = threadIdx.x & 31;
+  const int t = (warp & 1) * kEdgeBlock + i;
+  const int e = blockIdx.x * kEdgeBlock + i;
+  const bool live = e < G.n_edges;
+  const int x = (t < kEdgeBlock) ? e : G.epad + e;
+  const size_t fp = G.fpad, xs = G.xs;
+  SideLimiterPartials& limiter = reinterpret_cast<SideLimiterPartials*>(limiters)[t];
+  SideGeom g{};
+  double wk = 0.0, dp = 0.0, dm = 0.0;
+  if (live) {
+    g = side_geom(G, x);
+    const int f = G.e_face[x];
+    const int st[4] = {G.e_sten[x], G.e_sten[xs + x], G.e_sten[2 * xs + x], G.e_sten[3 * xs + x]};
+    griddep_wait();
+    const double* Wk = W + k * fp;
+    wk = Wk[f];
+    side_differences(g, wk, Wk[st[0]], Wk[st[1]], Wk[st[2]], Wk[st[3]], dp, dm);
+    if (k == 0) {
+      double w[kDim], c;
 #pragma unroll
-  for (int k = 0; k < kDim; ++k) fe[(size_t)k * G.epad + e] = F[k];
+      for (int q = 0; q < kDim; ++q) w[q] = W[q * fp + f];
+      const double nu = side_courant(g, P.gam, *dtp, w, c);
+      limiter = SideLimiterPartials(g, nu, w[0], w[4], c);
+    }
+  }
+  __syncthreads();
+  if (live) {
+    const double u = rev::limited_tape(g, limiter, k, wk, dp, dm, [&](int q, double v) { LJ[q * xs + x] = v; });
+    up[k][t] = u;
+    uplus[k * xs + x] = u;
+  }
+  __syncthreads();
+  if (k != 0) return;
+  const Gas gas = gas_of(P);
+  double u[kDim];
+  if (live) {
+#pragma unroll
+    for (int q = 0; q < kDim; ++q) u[q] = up[q][t];
+    sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
+  }
+  field0_sync();
+  if (!live || t >= kEdgeBlock) return;
+  rc_flux(G, P, gas, sides, fe, e, i);
 }
 
 template <int STAGE, int BLOCKS>
@@ -532,9 +670,18 @@ cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, 
                      cudaStream_t st) {
   FirstError chk;
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
-  chk(launch_pdl(adj::tlm_edge_kernel<1>, dim3(ne), dim3(adj::kThreads), st, G, S, T, P, dt0));
+  const adj::Split split = adj::edge_split(G.n_edges);
+  const dim3 eb(split == adj::Split::kSides ? adj::kThreads : f64::kEdgePartThreads);
+  using Edge = void (*)(DevGeom, DevState, TlmTangents, PhysParams, double);
+  const Edge edge1 = split == adj::Split::kSides    ? adj::tlm_edge_kernel<1>
+                     : split == adj::Split::kFields ? adj::tlm_edge_parts_kernel<1, 1>
+                                                    : adj::tlm_edge_parts_kernel<1, 2>;
+  const Edge edge2 = split == adj::Split::kSides    ? adj::tlm_edge_kernel<2>
+                     : split == adj::Split::kFields ? adj::tlm_edge_parts_kernel<2, 1>
+                                                    : adj::tlm_edge_parts_kernel<2, 2>;
+  chk(launch_pdl(edge1, dim3(ne), eb, st, G, S, T, P, dt0));
   chk(launch_pdl(adj::tlm_update_kernel<1>, dim3(nb), dim3(f64::kFaceThreads), st, G, S, T, P));
-  chk(launch_pdl(adj::tlm_edge_kernel<2>, dim3(ne), dim3(adj::kThreads), st, G, S, T, P, dt0));
+  chk(launch_pdl(edge2, dim3(ne), eb, st, G, S, T, P, dt0));
   chk(launch_pdl(adj::tlm_update_kernel<2>, dim3(nb), dim3(f64::kFaceThreads), st, G, S, T, P));
   return chk.status();
 }
@@ -590,11 +737,17 @@ cudaError_t rc_step(const DevGeom& G, const PhysParams& P, const double* dtp, co
                     double* U_next, double* W_next, cudaStream_t st) {
   FirstError chk;
   const int nb = adj::face_blocks(G.n_faces), ne = adj::edge_blocks(G.n_edges);
-  constexpr int B = f64::kFaceThreads, E = adj::kThreads;
-  chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W0, t.P0, t.J0, fe));
+  constexpr int B = f64::kFaceThreads;
   const bool five = f64::five_face_blocks(G.n_faces);
+  const adj::Split split = adj::edge_split(G.n_edges);
+  const dim3 eb(split == adj::Split::kSides ? adj::kThreads : f64::kEdgePartThreads);
+  using Edge = void (*)(DevGeom, PhysParams, const double*, const double*, double*, double*, double*);
+  const Edge edge = split == adj::Split::kSides    ? adj::rc_edge_kernel
+                    : split == adj::Split::kFields ? adj::rc_edge_parts_kernel<1>
+                                                   : adj::rc_edge_parts_kernel<2>;
+  chk(launch_pdl(edge, dim3(ne), eb, st, G, P, dtp, t.W0, t.P0, t.J0, fe));
   chk(launch_pdl(five ? adj::rc_update_kernel<1, 5> : adj::rc_update_kernel<1, 4>, dim3(nb), dim3(B), st, G, P, dtp, t.W0, t.U, fe, t.U1, t.W1, t.mask));
-  chk(launch_pdl(adj::rc_edge_kernel, dim3(ne), dim3(E), st, G, P, dtp, t.W1, t.P1, t.J1, fe));
+  chk(launch_pdl(edge, dim3(ne), eb, st, G, P, dtp, t.W1, t.P1, t.J1, fe));
   chk(launch_pdl(five ? adj::rc_update_kernel<2, 5> : adj::rc_update_kernel<2, 4>, dim3(nb), dim3(B), st, G, P, dtp, t.W1, t.U, fe, U_next, W_next, t.mask));
   return chk.status();
 }

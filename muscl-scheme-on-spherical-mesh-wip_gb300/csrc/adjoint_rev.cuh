@@ -377,7 +377,19 @@ SPLASH_HD void flux_star_rev(const double* uL, const double* uR, const SlotGeom&
 // (r = +-inf or NaN) d up / d dp = hg phi.
 constexpr int kTapePlanes = 15;  // 3 per field
 
-// nb as in recon_side; lj(3 k + i) receives the partials of field k
+// field k; lj(3 k + i) receives its partials
+template <class LjFn>
+SPLASH_HD double limited_tape(const SideGeom& g, const SideLimiterPartials& limiter, int k, double w, double dp,
+                              double dm, LjFn lj) {
+  const double num = dm * g.hr, dpg = dp * g.hg;
+  double r;
+  const Phi phi = limiter(k, dp, num, dpg, r);
+  lj(3 * k, g.hg * ((phi.r != 0.0) ? fma(-phi.r, r, phi.v) : phi.v));
+  lj(3 * k + 1, g.hg * g.hr * phi.r);
+  lj(3 * k + 2, dpg * phi.nu);
+  return fm(dpg, phi.v, w);
+}
+// nb as in recon_side
 template <class NbFn, class LjFn>
 SPLASH_HD void recon_side_tape(const SideGeom& g, double gam, double dt, const double* w, NbFn nb, double* up,
                                LjFn lj) {
@@ -386,14 +398,9 @@ SPLASH_HD void recon_side_tape(const SideGeom& g, double gam, double dt, const d
   const SideLimiterPartials limiter(g, nu, w[0], w[4], c);
 #pragma unroll
   for (int k = 0; k < kDim; ++k) {
-    double dp, dm, r;
+    double dp, dm;
     side_differences(g, w[k], nb(k, 0), nb(k, 1), nb(k, 2), nb(k, 3), dp, dm);
-    const double num = dm * g.hr, dpg = dp * g.hg;
-    const Phi phi = limiter(k, dp, num, dpg, r);
-    up[k] = fm(dpg, phi.v, w[k]);
-    lj(3 * k, g.hg * ((phi.r != 0.0) ? fma(-phi.r, r, phi.v) : phi.v));
-    lj(3 * k + 1, g.hg * g.hr * phi.r);
-    lj(3 * k + 2, dpg * phi.nu);
+    up[k] = limited_tape(g, limiter, k, w[k], dp, dm, lj);
   }
 }
 

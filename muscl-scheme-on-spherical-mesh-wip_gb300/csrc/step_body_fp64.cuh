@@ -251,6 +251,23 @@ struct SideLimiterPartials : SideLimiter {
   }
 };
 
+// up = w + dpg phi(r, nu) of field k with its tangents
+template <int N>
+SPLASH_HD Dual<N> limited_dual(const SideLimiterPartials& limiter, int k, const Dual<N>& w, const Dual<N>& dp,
+                               const Dual<N>& num, const Dual<N>& dpg, const Dual<N>& nu) {
+  double r;
+  const Phi phi = limiter(k, dp.v, num.v, dpg.v, r);
+  const bool flat = odd_bits(r);  // the limiter is flat where the ratio is no number
+  const double idp = flat ? 0.0 : recip(dp.v);
+  Dual<N> lim(phi.v);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double rd = flat ? 0.0 : fma(-r, dp.d[i], num.d[i]) * idp;
+    lim.d[i] = fma(phi.r, rd, phi.nu * nu.d[i]);
+  }
+  return fm(dpg, lim, w);
+}
+
 // The limited state (Sigma, l, Pi) of one side: up = w + dp phi(r) BM / H+.
 // nb(k, q) returns field k of stencil face q (0, 1: plus pair, 2, 3: minus).
 template <class T, class NbFn>
@@ -269,19 +286,7 @@ SPLASH_HD void recon_side(const SideGeom& g, double gam, double dt, const T* w, 
   }
   if constexpr (is_dual<T>::value) {
 #pragma unroll
-    for (int k = 0; k < kDim; ++k) {
-      double r;
-      const Phi phi = limiter(k, dp[k].v, num[k].v, dpg[k].v, r);
-      const bool flat = odd_bits(r);  // the limiter is flat where the ratio is no number
-      const double idp = flat ? 0.0 : recip(dp[k].v);
-      T lim(phi.v);
-#pragma unroll
-      for (int i = 0; i < T::kN; ++i) {
-        const double rd = flat ? 0.0 : fma(-r, dp[k].d[i], num[k].d[i]) * idp;
-        lim.d[i] = fma(phi.r, rd, phi.nu * nu.d[i]);
-      }
-      up[k] = fm(dpg[k], lim, w[k]);
-    }
+    for (int k = 0; k < kDim; ++k) up[k] = limited_dual(limiter, k, w[k], dp[k], num[k], dpg[k], nu);
   } else {
     double dpv[kDim], numv[kDim], dpgv[kDim];
 #pragma unroll
@@ -337,6 +342,12 @@ SPLASH_HD void recon_face(const DevGeom& G, const PhysParams& P, double dt, cons
 }
 
 #if defined(__CUDACC__)
+// The edge launches with a thread per field of a side (small meshes): warp
+// 2 k + s of a block serves field k of side s of its kEdgeBlock edges.
+constexpr int kEdgePartThreads = 2 * kEdgeBlock * kDim;
+// the barrier of the two field 0 warps, which go on alone
+__device__ __forceinline__ void field0_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
 // What the two threads of an edge exchange: each puts the state and the
 // EdgeSide of its side, the one that evaluates the flux takes both.  One
 // shared-memory plane per value (and one per tangent), indexed by thread.

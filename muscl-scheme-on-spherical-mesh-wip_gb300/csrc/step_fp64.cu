@@ -117,7 +117,6 @@ __global__ void __launch_bounds__(kThreads) edge_kernel(DevGeom G, DevState S, P
 // differences, then every warp limits its field, and the field 0 warps go on
 // as in edge_kernel.  Two blocks per SM: at one (112 registers) hex(4) takes
 // two waves, 51.6 us per step instead of 40.7.
-constexpr int kEdgePartThreads = kThreads * kDim;
 template <int STAGE>
 __global__ void __launch_bounds__(kEdgePartThreads, 2) edge_parts_kernel(DevGeom G, DevState S, PhysParams P, double dt0) {
   griddep_launch_dependents();
@@ -176,7 +175,7 @@ __global__ void __launch_bounds__(kEdgePartThreads, 2) edge_parts_kernel(DevGeom
     for (int q = 0; q < kDim; ++q) u[q] = up[q][t];
     sides.put(t, u, edge_side(u, edge_geom(G, e), gas));
   }
-  asm volatile("bar.sync 1, 64;" ::: "memory");  // the two field 0 warps
+  field0_sync();
   if (!live || t >= kEdgeBlock) return;
   store_flux(G, S, P, gas, sides, e, i);
 }

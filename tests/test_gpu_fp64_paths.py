@@ -36,8 +36,9 @@ def test_step_equals_the_tangent_models_values(kind, level, solver, friction):
 @pytest.mark.parametrize("kind,level", [("hex", 0), ("hex", 1), ("quad", 1), ("ico", 2), ("hex", 4), ("quad", 5)])
 @pytest.mark.parametrize("solver,noise", [(1, 0.2), (2, 1e-3), (3, 1e-2)])
 def test_fields_on_threads_of_their_own(kind, level, solver, noise):
-    """The smallest meshes give every field of a side a thread: the tangent model's values, which one thread per side makes,
-    with partial blocks (30, 120, 24, 480 edges), up to the largest such mesh, smooth and steep."""
+    """The smallest meshes give every field of a side a thread, in the step and on dual numbers in the tangent model: the
+    same values, with partial blocks (30, 120, 24, 480 edges), up to the largest such mesh, smooth and steep, and the
+    recorded forward's, which one thread per face makes."""
     import splash_gb300 as sg
 
     mesh = mesh_of(kind, level)
@@ -47,7 +48,10 @@ def test_fields_on_threads_of_their_own(kind, level, solver, noise):
     params = sg.SolverParams(accretion_rate=1e-2, e_acc=0.5, omega_acc_abs=0.5, tilt_angle=0.2, acc_width=0.1,
                              alpha=1e-6, friction_on=True)
     base = sg.Solver(mesh, U, 5, GAM, 0.0, True, params=params, solver=solver, precision=sg.PREC_FP64)
-    Ut, _ = sg.Adjoint(base, checkpoint_every=1).tlm(U, np.array([1e-2, 0.2, 0.5]), np.ones_like(U), np.zeros(3), 5, 1e-3)
+    adj, theta = sg.Adjoint(base, checkpoint_every=1), np.array([1e-2, 0.2, 0.5])
+    Ut, _ = adj.tlm(U, theta, np.ones_like(U), np.zeros(3), 5, 1e-3)
     base.do_steps(5, 1e-3)
     # equal_nan: the coarsest quad mesh leaves the range of the method, on both paths alike
     assert np.array_equal(base.get_state(), Ut, equal_nan=True)
+    assert np.array_equal(adj.forward(U, theta, 5, 1e-3), Ut, equal_nan=True)
+    assert np.array_equal(adj.branch_tape(U, theta, 5, "record")[0], Ut, equal_nan=True)
