@@ -23,7 +23,7 @@
 // pointers, which would let the compiler take the non-coherent path.
 // Like the step itself (step_fp64.cu) all of it is bound by the FP64 pipe:
 // the flux reverse runs once per edge, the reconstruction on a thread per
-// side.
+// side (forward and tangent: per field of a side on small meshes).
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -3,7 +3,9 @@
 // One step is four launches: per stage an edge launch (reconstruction of
 // both slots of every interior edge and one Riemann flux per edge; the
 // stage-1 launch also clips the step's dt) and a per-face update launch.
-// The batched (ensemble) launches add a dt finalize per step.  Work split:
+// The batched (ensemble) launches add a dt finalize per step; the smallest
+// meshes run several steps in one launch of a thread-block cluster
+// (cluster_steps_kernel).  Work split:
 //   FP32: slopes and limiter, edge states, Riemann fluxes, source terms,
 //         the per-slot flux contributions, the dt candidates;
 //   FP64: the conserved state U, the RK combine U0 + dt*Phi, the dt and
