@@ -349,8 +349,9 @@ SPLASH_HD void dt_candidates(const double* u, D3 r, double area, const PhysParam
 // rate2 = (g_eff Sigma |v - v0| / Pi)^2, the squared reciprocal of the extra
 // dt 0.01 Pi / (alpha fric_k g_eff Sigma |v - v0|) but for the constant factor
 // (no root and no quotient but 1 / Sigma and 1 / Pi per face).  `negative`
-// reports a negative extra dt; NaN candidates are 0, like the reference's
-// comparisons skip them.  w holds (Sigma, l, Pi).
+// reports a negative extra dt, by the signs of g_eff Sigma / Pi and of alpha
+// (a zero counts by its sign: it makes the extra dt infinite); NaN candidates
+// are 0, like the reference's comparisons skip them.  w holds (Sigma, l, Pi).
 SPLASH_HD void dt_fold(const double* w, const D3& r, const PhysParams& P, double& vel2, double& rate2,
                        bool& negative) {
   const double ir = recip(w[0]);
@@ -365,7 +366,7 @@ SPLASH_HD void dt_fold(const double* w, const D3& r, const PhysParams& P, double
   if (!nan_bits(v2)) vel2 = v2;
   if (not_below_zero(a2) && less_pos(vel2, a2)) vel2 = a2;
   rate2 = t * t * n2;
-  negative = below_zero(t) && !nan_bits(n2);
+  negative = (high_word(t) ^ high_word(P.alpha)) >> 31 && !odd_bits(t) && !odd_bits(n2);
   if (nan_bits(rate2)) rate2 = 0.0;
 }
 

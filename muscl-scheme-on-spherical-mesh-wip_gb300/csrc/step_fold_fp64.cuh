@@ -10,13 +10,31 @@
 namespace splash {
 namespace f64 {
 
+// What the folds say of the next step's dt (MUSCL_base.hpp:100-115):
+//   CFL bound h0 0.1 / max_vel, max_vel = max(1e-8, sqrt(vel2)),
+//   extra dt 0.01 / (|alpha| fric_k sqrt(rate2)), at most 1e20; 1e20 and a flag
+//   when some face's is negative (physics/adiabatic.hpp:543-580).
+// Where none is, alpha has the sign of every face's rate, so its size serves.
+struct DtBounds {
+  double max_vel, extra, dt;  // dt: the smaller of the CFL bound and the extra dt
+  bool negative;
+};
+SPLASH_HD DtBounds dt_bounds(double vel2, double rate2, bool negative, const PhysParams& P) {
+  DtBounds b;
+  b.max_vel = fmax(1e-8, sqrt(vel2));
+  const double rate = sqrt(rate2);
+  b.negative = negative && !odd_bits(P.alpha);  // an extra dt of -0, or none
+  b.extra = 1e20;
+  if (!b.negative && rate > 0) b.extra = fmin(1e20, 0.01 / (fabs(P.alpha) * P.fric_k * rate));
+  const double cfl = P.h0 * 0.1 / b.max_vel;
+  b.dt = (cfl > b.extra) ? b.extra : cfl;
+  return b;
+}
+
+#if defined(__CUDACC__)
 // Folds a warp's candidates (integer maxima: exact in any order) and, in the
 // last of n_warps warps to do so, makes the bounds of the next step's dt of
-// them:
-//   CFL bound h0 0.1 / max_vel, max_vel = max(1e-8, sqrt(vel2)),
-//   extra dt 0.01 / (alpha fric_k sqrt(rate2)), at most 1e20; 1e20 and a flag
-//   when some face's is negative (physics/adiabatic.hpp:543-580),
-// and gives the folds a fresh start.  Every lane of the warp calls it.
+// them and gives the folds a fresh start.  Every lane of the warp calls it.
 __device__ __forceinline__ void fold_warp(double vel2, double rate2, bool negative, const DevState& S,
                                           const PhysParams& P, unsigned long long n_warps) {
   unsigned long long v = bits_of(vel2), r = bits_of(rate2);
@@ -36,17 +54,13 @@ __device__ __forceinline__ void fold_warp(double vel2, double rate2, bool negati
   __threadfence();
   if (atomicAdd(F + kFoldDone, 1ull) != n_warps - 1) return;
   __threadfence();
-  const double vmax = fmax(1e-8, sqrt(from_bits(atomicExch(F + kFoldVel2, 0ull))));
-  const double rate = sqrt(from_bits(atomicExch(F + kFoldRate2, 0ull)));
-  const bool below = atomicExch(F + kFoldNeg, 0ull) != 0;
+  const double v2 = from_bits(atomicExch(F + kFoldVel2, 0ull)), r2 = from_bits(atomicExch(F + kFoldRate2, 0ull));
+  const DtBounds b = dt_bounds(v2, r2, atomicExch(F + kFoldNeg, 0ull) != 0, P);
   atomicExch(F + kFoldDone, 0ull);
-  double extra = 1e20;
-  if (!below && rate > 0) extra = fmin(1e20, 0.01 / (P.alpha * P.fric_k * rate));
-  const double cfl = P.h0 * 0.1 / vmax;
-  S.scal[kScMaxVel] = vmax;
-  S.scal[kScExtraDt] = extra;
-  S.scal[kScBound] = (cfl > extra) ? extra : cfl;
-  S.scal[kScNegExtra] = below ? 1.0 : 0.0;
+  S.scal[kScMaxVel] = b.max_vel;
+  S.scal[kScExtraDt] = b.extra;
+  S.scal[kScBound] = b.dt;
+  S.scal[kScNegExtra] = b.negative ? 1.0 : 0.0;
 }
 
 // dt = min(dt0, 0.1 h0 / max_vel, extra_dt)
@@ -62,6 +76,7 @@ __device__ __forceinline__ void publish_dt(const DevState& S, double dt) {
   S.scal[kScTime] = S.scal[kScTime] + dt;
   if (S.scal[kScNegExtra] != 0.0) atomicOr(S.err, 8u);  // SPLASH_STOP_NEG_EXTRA_DT
 }
+#endif
 
 }  // namespace f64
 }  // namespace splash
