@@ -168,12 +168,21 @@ SPLASH_HD double recip(double b) {
 #endif
   return exact_quotient(1.0, b);
 }
-// a / b given y = recip(b): Markstein's correction
+// normal, and twice the smallest normal number or more
+SPLASH_HD bool well_normal(double x) { return (high_word(x) & 0x7fffffffu) - 0x00200000u < 0x7fd00000u; }
+// a / b given y = recip(b): Markstein's correction, the operator's bits.  It
+// needs the remainder a - b q exactly, which holds from |a| = 2^-899 on (its
+// last place is 2^-106 of a), and a quotient and a reciprocal with all their
+// bits; the rest is the operator's.  Zeros, which quiet flows are full of, are
+// a y, whose sign the correction would lose (-0 + 0).
 SPLASH_HD double quotient(double a, double b, double y) {
 #if defined(__CUDA_ARCH__)
   const double q = a * y;
   const double c = ::fma(::fma(-b, q, a), y, q);
-  if (!odd_bits(c)) return c;
+  if (well_normal(y)) {
+    if ((high_word(a) & 0x7fffffffu) >= 0x07c00000u && well_normal(c)) return c;
+    if (bits_of(a) << 1 == 0) return q;
+  }
 #endif
   return exact_quotient(a, b);
 }
