@@ -464,6 +464,7 @@ int splash_adjoint_create(splash_solver* base_h, int checkpoint_every, splash_ad
     a->P = base->P;
     a->par = base->par;
     const size_t fp = a->fpad, XS = a->XS, FS = a->FS;
+    if (XS > splash::kMaxAdjointSides) return splash::set_error(SPLASH_E_UNSUPPORTED, "mesh too large for the adjoint");
     // host copies of the geometry the adjoint needs
     a->fcn_h.assign(3 * fp, 0.0);
     std::vector<int> sten(4 * XS), face(XS);

@@ -250,6 +250,12 @@ EdgeList make_edge_list(const SlotPlanes& sp) {
   return el;
 }
 
+int padded_edges(int n_edges) {
+  const size_t pad = ((size_t)n_edges + kEdgeBlock - 1) / kEdgeBlock * kEdgeBlock;
+  if (2 * pad > kMaxSides) throw std::runtime_error("too many edges");
+  return (int)pad;
+}
+
 EdgePlanes make_edge_planes(const SlotPlanes& sp, bool isothermal) {
   EdgePlanes ep;
   const size_t PS = sp.PS();
@@ -279,8 +285,7 @@ EdgePlanes make_edge_planes(const SlotPlanes& sp, bool isothermal) {
     for (int q : el.nbr) ep.twin.push_back(el.slot_edge[q]);
   }
   const int ne = ep.n_edges = el.n_edges;
-  const size_t pad = ep.epad = (ne + kEdgeBlock - 1) / kEdgeBlock * kEdgeBlock, xs = 2 * pad;
-  if (xs >= (size_t)1 << 28) throw std::runtime_error("too many edges");
+  const size_t pad = ep.epad = padded_edges(ne), xs = 2 * pad;
   ep.slot_edge = std::move(el.slot_edge);
   ep.face.resize(xs);
   ep.sten.resize(4 * xs);

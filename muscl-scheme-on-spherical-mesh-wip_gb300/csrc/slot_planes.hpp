@@ -94,6 +94,12 @@ struct EdgePlanes {
   RawVector<double> side, geo;
 };
 EdgePlanes make_edge_planes(const SlotPlanes& sp, bool isothermal);
+// n_edges rounded up to the edges of a block; throws where the planes of two
+// sides per edge would be too long: the kernels address the four of e_sten by
+// int (2^29 sides: quad_sphere(12), icosphere_hex(11)), the adjoint's inverse
+// stencil holds side * 8 + position (2^28).
+constexpr size_t kMaxSides = (size_t)1 << 29, kMaxAdjointSides = (size_t)1 << 28;
+int padded_edges(int n_edges);
 
 // FP32 planes of the mixed path.  The mixed step works per interior edge:
 // one thread reconstructs the edge states of the edge's two slots (owner:
