@@ -372,7 +372,13 @@ int Solver::step(double dt0) {
 }
 
 int Solver::steps_n(int n, double dt0) {
-  if (in_cluster && n != 1) {
+  if (in_cluster && n > 1) {
+    // refused like the graph launches of the other meshes: a captured launch
+    // would count steps that have not run
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    SPLASH_CUDA(cudaStreamIsCapturing(stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone)
+      return fail(SPLASH_E_CUDA, "steps are not permitted while the solver's stream is being captured");
     for (int left = n; left > 0;) {
       const int k = left < kClusterSteps ? left : kClusterSteps;
       SPLASH_CUDA(mixed_cluster_steps(GM, S, P, dt0, k, stream));
