@@ -17,13 +17,13 @@
 // writes each record it later reads, so nothing needs clearing between
 // calls.
 //
-// The kernels are the FP64 path's own per-face candidates and reduction
-// (physics_fp64.cuh, reduce.cuh), and this file is compiled with the same
-// -fmad=false as step_fp64.cu.  dt, max_vel and extra_dt are maxima and
-// minima, exact in any order, so they equal what an FP64 adiabatic (dim 5)
+// The kernels use the FP64 path's own face states, candidates and bounds
+// (prim_of, dt_fold, dt_bounds), and this file is compiled with the same
+// -fmad=false as step_fp64.cu.  The candidates are folded by maxima, exact in
+// any order, so dt, max_vel and extra_dt equal what an FP64 adiabatic (dim 5)
 // solver's splash_do_step computes for the same state; the five sums are
-// reduced over 256-face blocks here and 64-face blocks in the solver, so
-// they agree to rounding, not bit for bit.  A mixed-precision solver clips
+// reduced in another order than the solver's diagnostics, so they agree to
+// rounding, not bit for bit.  A mixed-precision solver clips
 // dt from FP32 candidates of its FP32 face state (within ~1e-7 relative of
 // this value), and the isothermal (dim 4) state layout is not accepted.
 #include <cuda_runtime.h>
@@ -34,6 +34,8 @@
 #include "reduce.cuh"
 #include "solver.hpp"
 #include "splash_gb300.h"
+#include "step_body_fp64.cuh"
+#include "step_fold_fp64.cuh"
 
 namespace splash {
 namespace noalloc {
@@ -56,59 +58,45 @@ __global__ void __launch_bounds__(kBlock) candidates_kernel(const double* __rest
                                                             int n_faces, PhysParams P,
                                                             double* __restrict__ scratch) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double vmax = 0.0, dmin = 1e20, sums[5] = {0, 0, 0, 0, 0};
+  double v[kPartialStride] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (f < n_faces) {
-    double u[kDim];
+    double u[kDim], w[kDim];
 #pragma unroll
     for (int k = 0; k < kDim; ++k) u[k] = U[(size_t)f * kDim + k];
     const f64::D3 rf{r[3 * (size_t)f], r[3 * (size_t)f + 1], r[3 * (size_t)f + 2]};
-    f64::dt_candidates(u, rf, area[f], P, vmax, dmin, sums);
+    f64::prim_of(u, rf, P.gam, w);
+    bool negative;
+    f64::dt_fold(w, rf, P, v[kFoldVel2], v[kFoldRate2], negative);
+    v[kFoldNeg] = negative ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < kDim; ++k) v[kPartialMaxima + k] = u[k] * area[f];
   }
-  red::block_partials<kBlock>(vmax, dmin, sums, scratch + (size_t)blockIdx.x * kPartialStride);
+  red::block_partials<kBlock>(v, scratch + (size_t)blockIdx.x * kPartialStride);
 }
 
 // MUSCL_base.hpp:100-115 and physics/adiabatic.hpp:573-577
 __global__ void __launch_bounds__(256) finalize_kernel(const double* __restrict__ scratch,
                                                        int nblocks, PhysParams P, double dt0,
                                                        double* __restrict__ out) {
-  __shared__ double sm[256][7];
-  double v[7] = {1e-8, 1e20, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    const double* p = scratch + (size_t)b * kPartialStride;
-    v[0] = fmax(v[0], p[0]);
-    v[1] = fmin(v[1], p[1]);
+  __shared__ double sm[256][kPartialStride];
+  double v[kPartialStride] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) red::merge(v, scratch + (size_t)b * kPartialStride);
 #pragma unroll
-    for (int k = 2; k < 7; ++k) v[k] = v[k] + p[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 7; ++k) sm[threadIdx.x][k] = v[k];
+  for (int k = 0; k < kPartialStride; ++k) sm[threadIdx.x][k] = v[k];
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sm[threadIdx.x][0] = fmax(sm[threadIdx.x][0], sm[threadIdx.x + s][0]);
-      sm[threadIdx.x][1] = fmin(sm[threadIdx.x][1], sm[threadIdx.x + s][1]);
-#pragma unroll
-      for (int k = 2; k < 7; ++k) sm[threadIdx.x][k] = sm[threadIdx.x][k] + sm[threadIdx.x + s][k];
-    }
+    if (threadIdx.x < s) red::merge(sm[threadIdx.x], sm[threadIdx.x + s]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    const double max_vel = sm[0][0];
-    double extra = sm[0][1];
-    double stop = 0.0;
-    if (extra < 0) {
-      stop = 1.0;
-      extra = 1e20;
-    }
-    double dt = dt0;
-    if (dt > P.h0 * 0.1 / max_vel) dt = P.h0 * 0.1 / max_vel;
-    if (dt > extra) dt = extra;
-    out[0] = dt;
-    out[1] = max_vel;
-    out[2] = extra;
-    out[3] = stop;
+    const double* t = sm[0];
+    const f64::DtBounds b = f64::dt_bounds(t[kFoldVel2], t[kFoldRate2], t[kFoldNeg] != 0.0, P);
+    out[0] = f64::clipped_dt(dt0, b.dt);
+    out[1] = b.max_vel;
+    out[2] = b.extra;
+    out[3] = b.negative ? 1.0 : 0.0;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) out[4 + k] = sm[0][2 + k];
+    for (int k = 0; k < kDim; ++k) out[4 + k] = t[kPartialMaxima + k];
   }
 }
 

@@ -324,28 +324,9 @@ SPLASH_HD double limiter_field_pos(double r, const LimiterLine<double>& l) {
   return fma(switch_pos(r), sb - t, t);
 }
 
-// Per-face contributions to the dt clip of the NEXT step and to the
-// diagnostics sums, for a conserved state u (u[4] = energy):
-// find_v_max (MUSCL_base.hpp:311-343) and extra_dt_constr
-// (physics/adiabatic.hpp:543-580).
-SPLASH_HD void dt_candidates(const double* u, D3 r, double area, const PhysParams& P,
-                                              double& vmax, double& dmin, double sums[5]) {
-  const double ir = recip(u[0]);
-  const D3 vel = scal(fcross(r, d3(u[1], u[2], u[3])), -ir);
-  const double v2 = fdot(vel, vel);
-  const double p = smax(1e-16, fma(-0.5 * u[0], v2, u[4]) * (P.gam - 1));
-  vmax = fmax(root(v2), root(P.gam * p * ir));
-  // extra_dt_constr: d = 0.01 Sigma / (alpha rho |v - v0|), rho = fric_k g_eff Sigma^2 / p
-  const D3 rel = d3(fma(P.omega_ns, r.y, vel.x), fma(-P.omega_ns, r.x, vel.y), vel.z);
-  const double GM = 0.217909;
-  const double g_eff = GM - v2;
-  dmin = 0.01 * p / (P.alpha * P.fric_k * g_eff * u[0] * root(fdot(rel, rel)));
-#pragma unroll
-  for (int k = 0; k < 5; ++k) sums[k] = u[k] * area;
-}
-
-// The candidates of one face for the next dt in the form in which they are
-// folded (FoldSlot): the larger of |v|^2 and the squared sound speed, and
+// The candidates of one face for the next dt (find_v_max,
+// MUSCL_base.hpp:311-343; extra_dt_constr, physics/adiabatic.hpp:543-580) in
+// the form in which they are folded (FoldSlot): the larger of |v|^2 and the squared sound speed, and
 // rate2 = (g_eff Sigma |v - v0| / Pi)^2, the squared reciprocal of the extra
 // dt 0.01 Pi / (alpha fric_k g_eff Sigma |v - v0|) but for the constant factor
 // (no root and no quotient but 1 / Sigma and 1 / Pi per face).  `negative`

@@ -30,6 +30,8 @@ SPLASH_HD DtBounds dt_bounds(double vel2, double rate2, bool negative, const Phy
   b.dt = (cfl > b.extra) ? b.extra : cfl;
   return b;
 }
+// dt = min(dt0, 0.1 h0 / max_vel, extra_dt)
+SPLASH_HD double clipped_dt(double dt0, double bound) { return less(bound, dt0) ? bound : dt0; }
 
 #if defined(__CUDACC__)
 // Folds a warp's candidates (integer maxima: exact in any order) and, in the
@@ -63,11 +65,7 @@ __device__ __forceinline__ void fold_warp(double vel2, double rate2, bool negati
   S.scal[kScNegExtra] = b.negative ? 1.0 : 0.0;
 }
 
-// dt = min(dt0, 0.1 h0 / max_vel, extra_dt)
-__device__ __forceinline__ double step_dt(const double* scal, double dt0) {
-  const double bound = scal[kScBound];
-  return less(bound, dt0) ? bound : dt0;
-}
+__device__ __forceinline__ double step_dt(const double* scal, double dt0) { return clipped_dt(dt0, scal[kScBound]); }
 // One thread of the step: its dt and time, and the stop bit of a negative
 // extra dt, which the reference latches when the step begins.
 __device__ __forceinline__ void publish_dt(const DevState& S, double dt) {
