@@ -265,8 +265,8 @@ int Solver::run_diagnostics(double* out9) {
 // computes its face states and dt keys in the set_state pass)
 cudaError_t Solver::launch_prepare() { return fp64_prepare(G, S, P, stream); }
 
-cudaError_t Solver::launch_step(cudaEvent_t* ev, double dt0, bool per_launch) {
-  if (precision == SPLASH_PREC_MIXED) return mixed_step(GM, S, P, dt0, stream, ev, per_launch);
+cudaError_t Solver::launch_step(cudaEvent_t* ev, double dt0) {
+  if (precision == SPLASH_PREC_MIXED) return mixed_step(GM, S, P, dt0, stream, ev);
   return fp64_step(G, S, P, dt0, stream, ev);
 }
 
@@ -507,7 +507,6 @@ int splash_create(const splash_mesh_desc* mesh, const double* U_in, int dim, dou
     S.err = s->dalloc<unsigned int>(4);
     S.keys = s->dalloc<unsigned>(2);
     s->d_stage = s->dalloc<double>((size_t)s->n_faces * dim);
-    s->d_perm = s->upload(s->perm);
     s->d_iperm = s->upload(s->iperm);
     s->d_cos_obs = s->upload(observer_planes(*s));
     s->d_diag_partial = s->dalloc<double>((size_t)splash::diag_partial_blocks(s->n_faces) * 9);
@@ -618,7 +617,7 @@ int splash_launch_times(splash_solver* h, int reps, double dt0, double* ms, int 
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
   int rc = SPLASH_OK;
   for (int r = 0; r < reps && rc == SPLASH_OK; ++r) {
-    cudaError_t e = s->launch_step(ev, dt0, true);
+    cudaError_t e = s->launch_step(ev, dt0);
     if (e == cudaSuccess) e = cudaEventSynchronize(ev[nl]);
     if (e != cudaSuccess) {
       rc = fail(SPLASH_E_CUDA, "launch timing: %s", cudaGetErrorString(e));

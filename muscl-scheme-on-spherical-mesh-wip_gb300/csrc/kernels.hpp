@@ -35,10 +35,9 @@ cudaError_t fp64_gather_state(const double* U, const int* iperm, double* aos, in
 // them.  Capturable; the stage-1 edge node's dt0 can be updated in an
 // instantiated graph (mixed_dt0_kernel_ptr identifies the node).
 // ev (optional): six events recorded on st (before the step, an empty dt
-// slot, after each stage's edge launch and update launch); per_launch gives
-// the same layout.
+// slot, after each stage's edge launch and update launch).
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
-                       cudaStream_t st, cudaEvent_t* ev = nullptr, bool per_launch = false);
+                       cudaStream_t st, cudaEvent_t* ev = nullptr);
 const void* mixed_dt0_kernel_ptr(const DevGeomMixed& G);
 // The same for meshes that fit one thread-block cluster (mixed_in_cluster):
 // n steps in one launch.

@@ -52,7 +52,6 @@ struct Solver {
   DevGeomMixed GM{};
   DevState S{};
   double* d_stage = nullptr;  // [n_faces][5] reference-order staging
-  int* d_perm = nullptr;
   int* d_iperm = nullptr;   // reference face -> internal face
   // device diagnostics (diagnostics.cu): observer planes, partials, block counter
   double* d_cos_obs = nullptr;
@@ -99,7 +98,7 @@ struct Solver {
   int step(double dt0);
   // one un-captured step; ev as for mixed_step (six events, five slots on
   // both paths)
-  cudaError_t launch_step(cudaEvent_t* ev, double dt0, bool per_launch = false);
+  cudaError_t launch_step(cudaEvent_t* ev, double dt0);
   int launches_per_step() const { return 5; }  // timing slots (a step launches 4 kernels; the dt slot is empty)
   cudaError_t launch_prepare();
   static int check_cuda(cudaError_t e, const char* what);

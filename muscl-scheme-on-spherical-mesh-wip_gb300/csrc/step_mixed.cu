@@ -26,9 +26,7 @@
 #include "fp_convert.cuh"
 #include "kernels.hpp"
 #include "pdl.cuh"
-#include "physics_fp64.cuh"
 #include "physics_mixed.cuh"
-#include "reduce.cuh"
 #include "solver.hpp"
 
 namespace splash {
@@ -1507,7 +1505,7 @@ cudaError_t mixed_scatter_prepare(const double* aos, const int* iperm, const Dev
 }
 
 cudaError_t mixed_step(const DevGeomMixed& G, const DevState& S, const PhysParams& P, double dt0,
-                       cudaStream_t st, cudaEvent_t* ev, bool /*per_launch: four launches, same layout*/) {
+                       cudaStream_t st, cudaEvent_t* ev) {
   const bool two = two_threads(G);
   const int ne = two ? (G.n_edges + mx::kHalf - 1) / mx::kHalf : mx::blocks_for(G.n_edges);
   dim3 ugrid(mx::blocks_for(G.n_faces));
