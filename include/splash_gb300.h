@@ -146,7 +146,9 @@ SPLASH_API int splash_do_steps(splash_solver* s, int n, double dt0);
 SPLASH_API int splash_synchronize(splash_solver* s);
 
 /* The cudaStream_t the solver launches on (as void*), so a caller can
- * order its own work or record CUDA events against the step. */
+ * order its own work or record CUDA events against the step.  Steps cannot be
+ * captured from it (they are graph launches): they return SPLASH_E_CUDA while
+ * it is being captured. */
 SPLASH_API int splash_stream(splash_solver* s, void** stream);
 /* Runs `reps` un-captured steps with CUDA events between the step's phases
  * and returns the mean device time per phase in milliseconds:

@@ -59,8 +59,8 @@ struct AdjScratch {
 // ---- tangent-linear model (value state S + tangents T) ----
 cudaError_t tlm_prepare(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P,
                         cudaStream_t st);
-// One step: dt clip of the value state, then the four stage launches on
-// Dual<1> (values bit-identical to fp64_step).
+// One step: four launches on Dual<1>, the first of which clips dt from the
+// value state (values bit-identical to fp64_step).
 cudaError_t tlm_step(const DevGeom& G, const DevState& S, const TlmTangents& T, const PhysParams& P, double dt0,
                      cudaStream_t st);
 

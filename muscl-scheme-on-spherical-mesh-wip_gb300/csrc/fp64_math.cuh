@@ -1,9 +1,11 @@
 // Arithmetic of the FP64 path, written for a narrow FP64 pipe.
 //
-// GB300 issues one FP64 warp instruction per SM every 9.8 ns (3.27 thread
-// operations per SM and ns measured, FMA, add, multiply and compare alike,
-// 1/80 of FP32), so the FP64 kernels' time is the number of FP64
-// instructions; everything else issues beside them for free.  Hence
+// GB300 issues one FP64 warp instruction per SM every 16 cycles (8.16 ns
+// measured from 4 warps per SM on, 2 thread operations per SM and cycle, FMA,
+// add, multiply and compare alike, 1/64 of FP32), one per scheduler every 33
+// ns, whether it depends on the last or not.  So the FP64 kernels' time is the
+// number of FP64 instructions; what else issues beside them is nearly free.
+// Hence
 //   * multiply-adds are written as fma explicitly (these files are compiled
 //     with -fmad=false, so nothing else is fused and the scalar types below
 //     agree to the last bit),
@@ -11,9 +13,9 @@
 //     2^-19.9, on the special-function unit), one third-order Newton step
 //     (Householder's method) and, where the quotient itself is kept, the
 //     residual correction of Markstein (1990): 4 or 6 instructions; a root
-//     is the same from rsqrt.approx.ftz.f64 (2^-20.0).  Zero, subnormal,
-//     infinite and NaN operands leave through an integer test to the exact
-//     operator, so those give what it gives,
+//     is the same from rsqrt.approx.ftz.f64 (2^-20.0).  Operands or quotients
+//     that are subnormal, infinite, NaN or next to the ends of the range leave
+//     through integer tests to the exact operator, so those give what it gives,
 //   * comparisons are integer comparisons of the bit patterns.
 // Every function is a template over the scalar: double, Dual<N> (values by
 // the same operations, derivatives by the chain rule) and Taped (taped.cuh).
@@ -218,7 +220,7 @@ SPLASH_HD T recip(const T& b) {
   }
   return r;
 }
-// a / b, rounded like the operator wherever the operands are in range
+// a / b, rounded like the operator
 template <class A, class B>
 SPLASH_HD wider_t<A, B> divide(const A& a, const B& b) {
   using R = wider_t<A, B>;

@@ -209,8 +209,8 @@ enum FoldSlot : int {
 enum ScalarSlot : int {
   kScDt = 0,       // dt of the current step (clipped)
   kScTime = 1,     // simulation time after the current step
-  kScMaxVel = 2,   // max_vel of the step's input state
-  kScExtraDt = 3,  // extra_dt_constr of the step's input state
+  kScMaxVel = 2,   // max_vel; mixed path: of the step's input state, FP64 path: of the current state
+  kScExtraDt = 3,  // extra_dt_constr, likewise
   kScBound = 4,    // FP64 path: min(CFL bound, extra dt) of the current state
   kScNegExtra = 5, // FP64 path: 1 if the current state's extra dt is negative
   kScDt0 = 9,      // mixed path: dt0 requested by the caller

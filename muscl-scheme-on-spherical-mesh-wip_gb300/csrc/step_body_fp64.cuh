@@ -446,7 +446,7 @@ SPLASH_HD void combine_face(double dt_here, const T* src, const T* sum, const T*
 // threads that sum one field's fluxes and one for the source, a warp per
 // part, so that the parts run side by side on the SM's four schedulers; the
 // warp of part 0 then combines them.  One thread per face runs all of it in
-// sequence, 194 dependent FP64 instructions of 36 ns on a mesh that leaves
+// sequence, 194 dependent FP64 instructions of 33 ns on a mesh that leaves
 // the SMs a warp or two.  The parts rotate from block to block, since a
 // warp's place in the block decides its scheduler and the source is the
 // longest part.

@@ -11,7 +11,7 @@
 //                          the bounds of them
 //
 // What bounds them is the FP64 pipe (fp64_math.cuh: one warp instruction per
-// SM every 9.8 ns), so the layout serves the instruction count: every edge's
+// SM every 8.2 ns), so the layout serves the instruction count: every edge's
 // flux is evaluated once (every Riemann solver here satisfies
 // F(uR, uL, -n) = -F(uL, uR, n) term by term; the reference evaluates it from
 // both faces), and the work is spread over sides and edges instead of faces,
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads) edge_kernel(DevGeom G, DevState S, P
 
 // The same with kDim threads per side, one per field, for meshes whose sides
 // leave the SMs a warp or two: there a launch takes the latency of one
-// thread's chain, 255 dependent FP64 instructions of 36 ns and 3,100 in all.
+// thread's chain, 255 dependent FP64 instructions of 33 ns and 3,100 in all.
 // Warp 2 k + s of a block serves field k of side s of its 32 edges; the field
 // 0 warps evaluate the side's Courant factor while the others form their
 // differences, then every warp limits its field, and the field 0 warps go on

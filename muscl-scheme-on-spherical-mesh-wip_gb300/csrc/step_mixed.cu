@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kBlock, 8) edge_kernel(DevGeomMixed G, DevStat
 // other in edge_kernel, run side by side here.  Thread t of a block serves
 // edge t mod kHalf, its owner slot below kHalf and its reverse slot above; the
 // edge states meet in shared memory and the lower half evaluates the fluxes.
-// The step scalars are published by a block of their own (FP64 work, 36 ns
+// The step scalars are published by a block of their own (FP64 work, 33 ns
 // per dependent instruction, off every edge's chain).  Each edge's arithmetic
 // is edge_body's.
 constexpr int kHalf = kBlock / 2;
